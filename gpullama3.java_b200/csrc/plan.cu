@@ -7,6 +7,7 @@
 #include "prefill.cuh"
 #include "stream_matvec.cuh"
 #include "stream_matvec_f16.cuh"
+#include "exact_prefill.cuh"
 #include "kquant.cuh"
 #include "decode_persistent.cuh"
 #include "sampler.cuh"
@@ -123,6 +124,14 @@ struct b200_plan {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
     PrefillCtx prefill;
+    // batched exact prefill (exact_prefill.cuh); rows = prefill_batch padded to whole token tiles, 0 = not built for this plan
+    struct {
+        int rows = 0;
+        float *X = nullptr, *QKV = nullptr, *AS = nullptr, *HS = nullptr;
+        int8_t *AQ = nullptr, *HQ = nullptr;
+        float *scratch = nullptr; // score rows of contexts whose rows do not fit shared memory
+        size_t scratch_bytes = 0;
+    } xp;
     // persistent decode kernel
     bool pd_ok = false;           // the plan fits the kernel's restrictions
     std::string pd_why;           // ... or why not
@@ -850,6 +859,7 @@ int set_smem_attrs(b200_plan *p) {
 }
 
 int prefill_init(b200_plan *p);
+int exact_prefill_init(b200_plan *p);
 
 int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
     const b200_config &c = p->cfg;
@@ -1106,9 +1116,122 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
     if ((rc = set_smem_attrs(p))) return rc;
     if (c.tp_size > 1) { CK(cudaStreamSynchronize(p->stream)); return B200_OK; } // graphs are captured by b200_tp_attach
     if ((rc = capture_all(p))) return rc;
-    if (p->prefill_batch > 1)
+    if (p->prefill_batch > 1) {
         if ((rc = prefill_init(p))) return rc;
+        if ((rc = exact_prefill_init(p))) return rc;
+    }
     CK(cudaStreamSynchronize(p->stream));
+    return B200_OK;
+}
+
+// ---- batched exact prefill of Q8_0 plans (exact_prefill.cuh) ------------------------------------------------------------------------
+template <typename F> int xp_by_head_size(int hs, F &&f) { // f(integral_constant<head size>)
+    if (hs == 128) return f(std::integral_constant<int, 128>());
+    if (hs == 64) return f(std::integral_constant<int, 64>());
+    if (hs == 256) return f(std::integral_constant<int, 256>());
+    if (hs == 96) return f(std::integral_constant<int, 96>());
+    return f(std::integral_constant<int, 32>());
+}
+const size_t XP_SMEM_MAX = 220 * 1024;
+const size_t XP_SCRATCH_MAX = (size_t)256 << 20;
+
+// Buffers of one chunk.  Plans off the streaming path (row-major weights) and tensor-parallel ones keep the token-by-token graph.
+int exact_prefill_init(b200_plan *p) {
+    const b200_config &g = p->cfg;
+    if (!p->use_stream || g.tp_size > 1 || p->wtype != B200_GGML_Q8_0) return B200_OK;
+    const int rows = (p->prefill_batch + 63) / 64 * 64, nqkv = p->qd + 2 * p->kvd, wide = p->qd > g.dim ? p->qd : g.dim;
+    int rc;
+    if ((rc = dalloc(p, &p->xp.X, (size_t)rows * g.dim * 4))) return rc;
+    if ((rc = dalloc(p, &p->xp.QKV, (size_t)rows * nqkv * 4))) return rc;
+    if ((rc = dalloc(p, &p->xp.AQ, (size_t)rows * wide))) return rc;
+    if ((rc = dalloc(p, &p->xp.AS, (size_t)rows * (wide / 32) * 4))) return rc;
+    if ((rc = dalloc(p, &p->xp.HQ, (size_t)rows * g.hidden_dim))) return rc;
+    if ((rc = dalloc(p, &p->xp.HS, (size_t)rows * (g.hidden_dim / 32) * 4))) return rc;
+    CK(cudaMemset(p->xp.AQ, 0, (size_t)rows * wide)); // rows behind the chunk's last token are multiplied too (and dropped)
+    CK(cudaMemset(p->xp.AS, 0, (size_t)rows * (wide / 32) * 4));
+    CK(cudaMemset(p->xp.HQ, 0, (size_t)rows * g.hidden_dim));
+    CK(cudaMemset(p->xp.HS, 0, (size_t)rows * (g.hidden_dim / 32) * 4));
+    if (!p->prefill.tok && (rc = dalloc(p, &p->prefill.tok, (size_t)rows * 4))) return rc;
+    if (xp_att_smem_bytes(g.head_size, 32, g.context_length, false) > XP_SMEM_MAX) { // one slot of 32 score rows per SM, as far as that goes
+        const size_t slot = (size_t)32 * xp_score_stride(g.context_length) * 4;
+        size_t want = slot * p->n_sms;
+        if (want > XP_SCRATCH_MAX) want = slot > XP_SCRATCH_MAX ? slot : XP_SCRATCH_MAX;
+        if ((rc = dalloc(p, &p->xp.scratch, want))) return rc;
+        p->xp.scratch_bytes = want;
+    }
+    p->xp.rows = rows;
+    return B200_OK;
+}
+
+template <int MODE>
+int xp_gemm(b200_plan *p, const TileMat &W, const int8_t *aq, const float *as, int n, float *out, int ldo, int8_t *hq, float *hs, float *hb1) {
+    const int mt = (W.rows + XP_ROWS - 1) / XP_ROWS;
+    auto go = [&](auto nj) -> int {
+        constexpr int NJ = decltype(nj)::value;
+        auto kern = k_xp_gemm<MODE, NJ>;
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<NJ>::BYTES));
+        kern<<<dim3(mt, (n + 8 * NJ - 1) / (8 * NJ)), XP_THREADS, XpTile<NJ>::BYTES, p->stream>>>(W, aq, as, p->xp.rows, n, out, ldo, hq, hs, hb1);
+        CK(cudaGetLastError());
+        return B200_OK;
+    };
+    // the largest token tile that leaves no SM without a CTA (and is not mostly padding): a wider tile reads a weight fewer times, a narrower one
+    // shortens the chain of a column block
+    auto fits = [&](int tok) { return (tok == 8 || n > tok / 2) && (tok == 8 || mt * ((n + tok - 1) / tok) >= p->n_sms); };
+    if (fits(64)) return go(std::integral_constant<int, 8>());
+    if (fits(32)) return go(std::integral_constant<int, 4>());
+    if (fits(16)) return go(std::integral_constant<int, 2>());
+    return go(std::integral_constant<int, 1>());
+}
+
+// n tokens already in prefill.tok (device), positions start_pos .. start_pos + n - 1
+int exact_prefill(b200_plan *p, int n, int start_pos) {
+    const b200_config &g = p->cfg;
+    auto &c = p->xp;
+    const int nqkv = p->qd + 2 * p->kvd;
+    const size_t ctx_kv = (size_t)g.context_length * p->kvd;
+    const size_t norm_smem = (size_t)g.dim * 4, rope_smem = (size_t)(g.n_heads + g.n_kv_heads) * (g.head_size + 1) * 4;
+    CK(cudaFuncSetAttribute(k_xp_rope_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
+    auto attention = [&](float *kc, float *vc) {
+        return xp_by_head_size(g.head_size, [&](auto hs_c) -> int {
+            constexpr int HS = decltype(hs_c)::value;
+            const int nt = start_pos + n;
+            auto go = [&](auto kern, int qt) -> int {
+                const bool scratch = xp_att_smem_bytes(HS, qt, nt, false) > XP_SMEM_MAX;
+                const size_t smem = xp_att_smem_bytes(HS, qt, nt, scratch);
+                int ctas = (n + qt - 1) / qt * g.n_heads;
+                if (scratch) {
+                    const size_t slots = c.scratch_bytes / ((size_t)qt * xp_score_stride(nt) * 4);
+                    if ((size_t)ctas > slots) ctas = (int)slots;
+                }
+                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
+                kern<<<ctas, XP_ATT_THREADS, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, c.AS, c.rows, scratch ? c.scratch : nullptr);
+                CK(cudaGetLastError());
+                return B200_OK;
+            };
+            // 32 tokens per CTA share the staged keys and values; a chunk too small to fill the SMs that way takes 8
+            return (n + 31) / 32 * g.n_heads >= p->n_sms ? go(k_xp_attention<HS, 4>, 32) : go(k_xp_attention<HS, 1>, 8);
+        });
+    };
+    for (int l = 0; l < g.n_layers; l++) {
+        const LayerW &L = p->layers[l];
+        float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
+        int rc;
+        if (l == 0) k_xp_norm<true><<<n, XP_NORM_THREADS, norm_smem, p->stream>>>(c.X, p->prefill.tok, p->emb, L.attn_norm, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
+        else k_xp_norm<false><<<n, XP_NORM_THREADS, norm_smem, p->stream>>>(c.X, nullptr, p->emb, L.attn_norm, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
+        CK(cudaGetLastError());
+        if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, c.AQ, c.AS, n, c.QKV, nqkv, nullptr, nullptr, nullptr))) return rc;
+        k_xp_rope_kv<<<n, 256, rope_smem, p->stream>>>(c.QKV, kc, vc, g.head_size, g.n_heads, g.n_kv_heads, p->kflags, L.q_norm, L.k_norm, g.rms_norm_eps, p->rope_cr, p->rope_ci, start_pos);
+        CK(cudaGetLastError());
+        if ((rc = attention(kc, vc))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, L.two, c.AQ, c.AS, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
+        k_xp_norm<false><<<n, XP_NORM_THREADS, norm_smem, p->stream>>>(c.X, nullptr, p->emb, L.ffn_norm, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
+        CK(cudaGetLastError());
+        if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, c.AQ, c.AS, n, nullptr, 0, c.HQ, c.HS, p->hb))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, L.tw2, c.HQ, c.HS, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
+    }
+    // the single-token buffers hold what the last token's own step would have left there
+    CK(cudaMemcpyAsync(p->x, c.X + (size_t)(n - 1) * g.dim, (size_t)g.dim * 4, cudaMemcpyDeviceToDevice, p->stream));
+    CK(cudaMemcpyAsync(p->qkv, c.QKV + (size_t)(n - 1) * nqkv, (size_t)nqkv * 4, cudaMemcpyDeviceToDevice, p->stream));
     return B200_OK;
 }
 
@@ -1488,10 +1611,17 @@ int b200_forward_batch_prefill(b200_plan *p, const int32_t *tokens, int32_t n, i
         CK(cudaEventElapsedTime(&p->prefill_ms, p->ev0, p->ev1));
         return B200_OK;
     }
-    // Exact path: the prefill graph token by token (bit-identical KV cache to the CPU
-    // batchForwardJavaPrefill, InferenceCoreBatchPrefillDecode.java:62-168).
+    // Exact path (bit-identical KV cache to the CPU batchForwardJavaPrefill, InferenceCoreBatchPrefillDecode.java:62-168): the whole chunk
+    // at once where the plan has the buffers for it, else the prefill graph token by token.
     if (n > p->seq_cap) return fail(p, B200_ERR_BAD_ARG, "chunk too long");
     memcpy(p->h_ids, tokens, (size_t)n * 4);
+    if (p->xp.rows && n > 1) {
+        CK(cudaMemcpyAsync(p->prefill.tok, p->h_ids, (size_t)n * 4, cudaMemcpyHostToDevice, p->stream));
+        int rc2 = exact_prefill(p, n, start_pos);
+        if (rc2) return rc2;
+        CK(cudaStreamSynchronize(p->stream));
+        return B200_OK;
+    }
     CK(cudaMemcpyAsync(p->seq_tokens, p->h_ids, (size_t)n * 4, cudaMemcpyHostToDevice, p->stream));
     int rc;
     if ((rc = set_state(p, tokens[0], start_pos, n, 0))) return rc;

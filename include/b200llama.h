@@ -346,7 +346,9 @@ int b200_forward_batch_prefill(b200_plan *plan, const int32_t *tokens, int32_t n
 
 /* How b200_forward_batch_prefill computes (the reference has the same two families:
  * LlamaFP16LayersBatchPrefill vs ...BatchPrefillMMA, selected by TensorCoreSupport.java):
- *   B200_PREFILL_EXACT       the single-token prefill graph per token: KV cache bit-identical to the CPU path;
+ *   B200_PREFILL_EXACT       KV cache bit-identical to the CPU path: single-GPU Q8_0 plans on the streaming path created with
+ *                            prefill_batch_size > 1 multiply the whole chunk at once in the CPU path's float order, other plans
+ *                            run the single-token prefill graph per token;
  *   B200_PREFILL_TENSOR_CORE TMA + tcgen05 GEMMs over the whole chunk, FP16 operands / FP32 accumulation:
  *                            KV cache within FP16 tolerance of the CPU path.  Default for FP16 plans created
  *                            with prefill_batch_size > 1.  Opt-in for single-GPU Q8_0 plans: the first call
