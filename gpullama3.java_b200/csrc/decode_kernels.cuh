@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "seqsum.cuh"
 #include "seqsum2.cuh"
+#include "seqsum3.cuh"
 
 enum { MODE_STORE = 0, MODE_RESID = 1 };
 
@@ -407,6 +408,216 @@ __global__ void k_swiglu(float *__restrict__ hb, const float *__restrict__ hb2, 
 // ------------------------------------------------------------------------------------------
 #define ATT_THREADS 512 // four threads per key (scores) and per output element (weighted sum): head size <= ATT_THREADS / 4
 
+// Long contexts.  One CTA per head leaves most SMs idle, and its score loads touch 32 cache lines per instruction: 9 us per 128 keys.  So a head
+// gets a cluster of C = head size / 32 CTAs, and beyond ATT_SPLIT keys they share its work (up to ATT_SPLIT the first CTA works alone and the
+// others leave at once):
+//   scores    blocks of 32 keys go round robin over the 8 C scoring warps; a lane owns a key's whole chain.  The rows arrive through a per-warp ring of
+//             cp.async stages (32 keys x 16 elements, coalesced, conflict-free to read), so nothing waits for another warp.
+//   softmax   the maximum over the cluster, the exponentials of the CTA's own keys, and the sequential sum (seqsum3.cuh), which every CTA takes for
+//             itself; the row lives in global memory (L2) and is handed over at two cluster barriers.
+//   output    a CTA owns 32 elements of the head: one warp walks the positions (one dependent add each: 4 cycles per position, the bound of this part),
+//             the others stage V rows and the quotients ahead of it.
+// 8B geometry, 3000 keys: 165 us -> see the table in the measurement notes of the plan; the dependent adds alone are 6.3 us.
+#define ATT_SPLIT 128
+#define ATT_KW 8           // scoring warps of a CTA
+#define ATT_KSTAGES 4      // stages of a scoring warp's ring
+#define ATT_KROW 80        // bytes between the 64-byte row pieces of a stage: lanes read 16 bytes without bank conflicts
+#define ATT_VT 128         // positions per V stage
+#define ATT_VSTAGES 4
+__host__ __device__ inline int att_cluster(int hs, int ctx) { return ctx > ATT_SPLIT && hs >= 64 ? hs / 32 : 1; }
+struct AttSplitSmem { // behind q | k | out
+    alignas(16) unsigned char ring[ATT_KW * ATT_KSTAGES * 32 * ATT_KROW]; // K rings; afterwards the V ring (ATT_VSTAGES x ATT_VT x 128 bytes)
+    alignas(16) float e[4096];                                            // exponentials of the piece being summed
+    SeqSum3Scratch sum;
+    alignas(16) float a[2][ATT_VT];                                       // weights of a V stage
+};
+static_assert(ATT_VSTAGES * ATT_VT * 128 <= ATT_KW * ATT_KSTAGES * 32 * ATT_KROW, "the V ring reuses the K rings");
+struct AttSumSync { __device__ __forceinline__ void operator()() const { asm volatile("bar.sync 4, 256;" ::: "memory"); } };
+__device__ __forceinline__ void att_cluster_sync() { // every thread of every CTA of the cluster; global writes before it are visible behind it
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ void att_cp16(unsigned dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// The cluster's share of one head (k_attention, above).  q (rotated) at sm, the current position's key at sm + HS; kc / vc point at the head's first element
+// of position 0; row: the head's score row, maxima: its 8 words behind all rows (both global).
+template <int HS>
+__device__ __forceinline__ void attention_split(float *sm, float *qkv, const float *kc, const float *vc, int kvd, int h, int rank, int cluster, int pos, float sqrt_hs, const float *vcur, int8_t *xq,
+                                                float *xs, float *xb, const TpCtx &tp, int head_base, float *row, float *maxima) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = pos + 1;
+    const float *sq = sm, *sk = sm + HS;
+    AttSplitSmem &S = *reinterpret_cast<AttSplitSmem *>(sm + 3 * HS);
+    __shared__ float red[ATT_THREADS / 32];
+    const unsigned ring = (unsigned)__cvta_generic_to_shared(S.ring);
+    float lmax = -INFINITY;
+    // ---- scores (scalarDot, FloatTensor.java:86-92)
+    const int n_blocks = (pos + 31) / 32, stride_b = ATT_KW * cluster;
+    if (warp < ATT_KW) {
+        constexpr int CH = HS / 16; // 16-element pieces of a row
+        const int b0 = rank * ATT_KW + warp;
+        const int items = b0 < n_blocks ? ((n_blocks - 1 - b0) / stride_b + 1) * CH : 0;
+        const unsigned wr = ring + warp * ATT_KSTAGES * 32 * ATT_KROW;
+        auto fetch = [&](int i) {
+            const int b = b0 + (i / CH) * stride_b, c = i % CH;
+            const unsigned dst = wr + (i % ATT_KSTAGES) * 32 * ATT_KROW;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int r = (lane >> 2) + 8 * u, t = b * 32 + r;
+                if (t < pos) att_cp16(dst + r * ATT_KROW + (lane & 3) * 16, kc + (size_t)t * kvd + c * 16 + (lane & 3) * 4);
+            }
+        };
+#pragma unroll
+        for (int i = 0; i < ATT_KSTAGES - 1; i++) {
+            if (i < items) fetch(i);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        float acc = 0.0f;
+        for (int i = 0; i < items; i++) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(ATT_KSTAGES - 2) : "memory");
+            __syncwarp(); // the stage is complete for every lane, and every lane is done with the stage that is fetched into next
+            if (i + ATT_KSTAGES - 1 < items) fetch(i + ATT_KSTAGES - 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            const int c = i % CH;
+            const float4 *k = reinterpret_cast<const float4 *>(S.ring + (warp * ATT_KSTAGES + i % ATT_KSTAGES) * 32 * ATT_KROW + lane * ATT_KROW);
+            const float4 *q = reinterpret_cast<const float4 *>(sq + c * 16);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const float4 kk = k[u], qq = q[u];
+                acc = __fadd_rn(acc, __fmul_rn(qq.x, kk.x));
+                acc = __fadd_rn(acc, __fmul_rn(qq.y, kk.y));
+                acc = __fadd_rn(acc, __fmul_rn(qq.z, kk.z));
+                acc = __fadd_rn(acc, __fmul_rn(qq.w, kk.w));
+            }
+            if (c == CH - 1) {
+                const int t = (b0 + (i / CH) * stride_b) * 32 + lane;
+                if (t < pos) {
+                    const float s = __fdiv_rn(acc, sqrt_hs);
+                    row[t] = s;
+                    lmax = fmaxf(lmax, s);
+                }
+                acc = 0.0f;
+            }
+        }
+    } else if (warp == ATT_KW && rank == 0) { // the current position's key is in shared memory
+        float acc = 0.0f;
+#pragma unroll 4
+        for (int d = 0; d < HS; d++) acc = __fadd_rn(acc, __fmul_rn(sq[d], sk[d]));
+        const float s = __fdiv_rn(acc, sqrt_hs);
+        if (lane == 0) row[pos] = s;
+        lmax = s;
+    }
+    lmax = warp_max_f(lmax);
+    if (lane == 0) red[warp] = lmax;
+    __syncthreads(); // also: the K rings are free
+    auto fetch_v = [&](int c, int t0, int n_thr) { // V stage c: positions [c * ATT_VT, + ATT_VT) of this CTA's 32 elements
+        const unsigned dst = ring + (c % ATT_VSTAGES) * ATT_VT * 128;
+        for (int i = t0; i < ATT_VT * 8; i += n_thr) {
+            const int t = c * ATT_VT + (i >> 3);
+            if (t < pos) att_cp16(dst + i * 16, vc + (size_t)t * kvd + rank * 32 + (i & 7) * 4);
+        }
+    };
+    const int n_vc = (pos + ATT_VT - 1) / ATT_VT;
+#pragma unroll
+    for (int c = 0; c < ATT_VSTAGES - 1; c++) { // in flight through the softmax
+        if (c < n_vc) fetch_v(c, tid, ATT_THREADS);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (tid == 0) {
+        float m = red[0];
+#pragma unroll
+        for (int w = 1; w < ATT_THREADS / 32; w++) m = fmaxf(m, red[w]);
+        maxima[rank] = m;
+    }
+    att_cluster_sync();
+    // ---- softmax (FloatTensor.java:211-219)
+    float mx = ldcg_f32c(maxima);
+    for (int k = 1; k < cluster; k++) mx = fmaxf(mx, ldcg_f32c(maxima + k));
+    if (rank == 0 && tid < HS) qkv[h * HS + tid] = sq[tid]; // the rotated q, for read-back: every CTA of the cluster has its copy by now
+    for (int o = warp;; o += ATT_THREADS / 32) { // the blocks this CTA scored
+        const int b = (o / ATT_KW) * stride_b + rank * ATT_KW + o % ATT_KW;
+        if ((o / ATT_KW) * stride_b + rank * ATT_KW >= n_blocks) break;
+        const int t = b * 32 + lane;
+        if (b < n_blocks && t < pos) row[t] = (float)exp((double)__fsub_rn(ldcg_f32c(row + t), mx));
+    }
+    if (rank == 0 && tid == ATT_THREADS - 1) row[pos] = (float)exp((double)__fsub_rn(ldcg_f32c(row + pos), mx));
+    att_cluster_sync();
+    if (tid < SEQSUM3_THREADS) {
+        float s = 0.0f;
+        auto piece = [&](auto e_c, int p0) {
+            constexpr int E = decltype(e_c)::value;
+            float t[E];
+#pragma unroll
+            for (int k = 0; k < E; k += 4) {
+                const int at = p0 + tid * E + k;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (at < nt) v = __ldcg(reinterpret_cast<const float4 *>(row + at)); // (rows are padded to whole pieces of four)
+                t[k] = v.x; t[k + 1] = at + 1 < nt ? v.y : 0.f; t[k + 2] = at + 2 < nt ? v.z : 0.f; t[k + 3] = at + 3 < nt ? v.w : 0.f;
+                *reinterpret_cast<float4 *>(S.e + tid * E + k) = make_float4(t[k], t[k + 1], t[k + 2], t[k + 3]);
+            }
+            s = block_seqsum3<E>(t, S.e, S.sum, tid, AttSumSync(), s);
+            AttSumSync()(); // the next piece overwrites the terms
+        };
+        if (nt <= 1024) piece(SeqSumTerms<4>(), 0);
+        else
+            for (int p0 = 0; p0 < nt; p0 += 4096) piece(SeqSumTerms<16>(), p0);
+    }
+    __syncthreads();
+    const float sum = S.sum.result;
+    // ---- output (saxpyInPlace, FloatTensor.java:221-227): warp 0 walks, the others stay a stage ahead
+    auto weights = [&](int c) {
+        const int i = tid - 32, t = c * ATT_VT + i;
+        if (i >= 0 && i < ATT_VT && t < nt) S.a[c & 1][i] = __fdiv_rn(ldcg_f32c(row + t), sum);
+    };
+    weights(0);
+    float acc = 0.0f;
+    for (int c = 0; c < n_vc; c++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ATT_VSTAGES - 2) : "memory");
+        __syncthreads(); // stage c and its weights are there for every thread, and stage c - 1 is consumed
+        if (warp == 0) {
+            const float *v = reinterpret_cast<const float *>(S.ring) + (c % ATT_VSTAGES) * ATT_VT * 32 + lane, *a = S.a[c & 1];
+            const int n = min(ATT_VT, pos - c * ATT_VT);
+            int t = 0;
+            for (; t + 16 <= n; t += 16) {
+                float p[16];
+#pragma unroll
+                for (int u = 0; u < 16; u += 4) {
+                    const float4 w = *reinterpret_cast<const float4 *>(a + t + u);
+                    p[u] = __fmul_rn(w.x, v[(t + u) * 32]); p[u + 1] = __fmul_rn(w.y, v[(t + u + 1) * 32]);
+                    p[u + 2] = __fmul_rn(w.z, v[(t + u + 2) * 32]); p[u + 3] = __fmul_rn(w.w, v[(t + u + 3) * 32]);
+                }
+#pragma unroll
+                for (int u = 0; u < 16; u++) acc = __fadd_rn(p[u], acc);
+            }
+            for (; t < n; t++) acc = __fadd_rn(__fmul_rn(a[t], v[t * 32]), acc);
+        } else {
+            if (c + ATT_VSTAGES - 1 < n_vc) fetch_v(c + ATT_VSTAGES - 1, tid - 32, ATT_THREADS - 32);
+            weights(c + 1);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (warp == 0) {
+        const float wl = __fdiv_rn(ldcg_f32c(row + pos), sum);
+        const int d = rank * 32 + lane;
+        acc = __fadd_rn(__fmul_rn(wl, vcur[d]), acc);
+        if (xb) xb[h * HS + d] = acc;
+        if (xq) {
+            float as;
+            const int q = quant_block_lane(acc, as);
+            if (tp.n > 1) {
+                const int gh = head_base + h;
+                for (int k = 0; k < tp.n; k++) {
+                    tp_ptr<int8_t>(tp, k, tp.off_attq)[gh * HS + d] = (int8_t)q;
+                    if (lane == 0) tp_ptr<float>(tp, k, tp.off_atts)[(gh * HS) / 32 + rank] = as;
+                }
+            } else {
+                xq[h * HS + d] = (int8_t)q;
+                if (lane == 0) xs[(h * HS) / 32 + rank] = as;
+            }
+        }
+    }
+}
+
 template <int HS>
 __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ qkv, float *__restrict__ kc, float *__restrict__ vc,
                                                           const StepState *__restrict__ st, const float *__restrict__ cr,
@@ -414,13 +625,14 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
                                                           const float *__restrict__ qnorm_w, const float *__restrict__ knorm_w,
                                                           float eps, float sqrt_hs, int8_t *__restrict__ xq,
                                                           float *__restrict__ xs, float *__restrict__ xb, TraceBuf tr, TpCtx tp,
-                                                          unsigned tp_out_op, int head_base, float *att_scratch, int ctx) {
-    extern __shared__ __align__(16) float sm[]; // q[HS] | k[HS] | out[HS] | att[ctx] (att in global scratch for long contexts)
+                                                          unsigned tp_out_op, int head_base, float *att_scratch, int ctx, int cluster) {
+    // q[HS] | k[HS] | out[HS] | att[ctx] (cluster > 1: att[ATT_SPLIT] or AttSplitSmem; else, for long contexts, att in global scratch)
+    extern __shared__ __align__(16) float sm[];
     __shared__ float red[ATT_THREADS / 32];
     __shared__ float s_val[2];
     float *sq = sm, *sk = sm + HS, *so = sm + 2 * HS;
-    float *att = att_scratch ? att_scratch + (size_t)blockIdx.x * ctx : sm + 3 * HS;
-    const int h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int h = blockIdx.x / cluster, rank = blockIdx.x % cluster, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float *att = att_scratch && cluster == 1 ? att_scratch + (size_t)h * ctx : sm + 3 * HS;
     constexpr int HALF = HS / 2;
     trace_entry(tr);
     pdl_launch_dependents();
@@ -429,7 +641,9 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     pdl_wait();
     trace_mark(tr, 2);
     const int pos = st->pos, nt = pos + 1;
-    { // K/V rows of the earlier positions -> L2, one 128-byte line per request, so the score loads below hit L2 (the weight stream carries an
+    const bool split = cluster > 1 && nt > ATT_SPLIT; // uniform over the grid
+    if (rank && !split) return;
+    if (!split) { // K/V rows of the earlier positions -> L2, one 128-byte line per request, so the score loads below hit L2 (the weight stream carries an
       // evict_first policy; without the prefetch these rows come from HBM every layer)
         constexpr int LINES = HS / 32;
         for (int i = tid; i < pos * LINES; i += ATT_THREADS) {
@@ -475,7 +689,7 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
         float *dst = is_q ? sq : sk;
         dst[i0] = r0;
         dst[i1] = r1;
-        if (h % kv_mul == 0) { // first query head of the KV group owns the cache / debug write-back
+        if (h % kv_mul == 0 && rank == 0) { // first query head of the KV group owns the cache / debug write-back
             if (!is_q) {
                 const size_t o = (size_t)pos * kvd + kvh * HS;
                 kc[o + i0] = r0;
@@ -486,9 +700,21 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
                 //  unrotated k from there concurrently)
             }
         }
-        if (is_q) { qkv[h * HS + i0] = r0; qkv[h * HS + i1] = r1; }
+        if (is_q && !split) { qkv[h * HS + i0] = r0; qkv[h * HS + i1] = r1; } // (split: the other CTAs of the cluster may not have read q yet)
     }
     __syncthreads();
+    if constexpr (HS >= 64) {
+        if (split) {
+            attention_split<HS>(sm, qkv, kc + kvh * HS, vc + kvh * HS, kvd, h, rank, cluster, pos, sqrt_hs, vsrc, xq, xs, xb, tp, head_base, att_scratch + (size_t)h * ctx,
+                                att_scratch + (size_t)n_heads * ctx + h * 8);
+            if (tp.n > 1) {
+                __syncthreads();
+                if (tid == 0) tp_cta_done(tp, TP_SLOT_ATT, tp_seq(tp, tp_out_op), gridDim.x);
+            }
+            trace_mark(tr, 3);
+            return;
+        }
+    }
     // ---- scores (scalarDot, FloatTensor.java:86-92: one sequential unfused mul/add chain per key).  Four threads share a key: each loads
     // ITS quarter of the K row at once (one round trip per pass of ATT_THREADS/4 keys), then the chain runs through the quad in element
     // order, handed on by shuffle.  The V rows of the first round of the weighted sum are requested here too (they do not depend on the scores).
@@ -609,7 +835,7 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     }
     if (tp.n > 1) {
         __syncthreads();
-        if (tid == 0) tp_cta_done(tp, TP_SLOT_ATT, tp_seq(tp, tp_out_op), gridDim.x);
+        if (tid == 0) tp_cta_done(tp, TP_SLOT_ATT, tp_seq(tp, tp_out_op), gridDim.x / cluster);
     }
     trace_mark(tr, 3);
 }

@@ -108,6 +108,7 @@ struct b200_plan {
     unsigned l2_window = 0, pd_l2_ahead = 0, pd_max_fly = 0, pd_evict_first = 1;
     int pd_max_stages = 0; // 0 = as many as shared memory holds
     float *att_scratch = nullptr; // [heads][ctx] score rows when the context does not fit shared memory
+    float *att_rows = nullptr;    // [heads][ctx] score rows and [heads][8] maxima of heads that a cluster of CTAs shares (k_attention)
     int *smp_indices = nullptr, *smp_out = nullptr; // device-side sampler scratch (sampler.cuh): candidate list, {id, info[4]}
 
     // tensor parallelism (tp.n == 1: single GPU).  *_l = this rank's share.
@@ -486,6 +487,7 @@ template <int MODE> int launch_matvec_f16(b200_plan *p, const DevMat &m, const f
 
 // FP16 plans on the streaming path (stream_matvec_f16.cuh); m2 = ffn_up for SF_GATEUP.
 template <typename... KA, typename... A> int launch_k(b200_plan *p, bool pdl, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args);
+template <typename... KA, typename... A> int launch_cluster(b200_plan *p, bool pdl, int cluster, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args);
 int sf_grid(const b200_plan *p, int rows, int cols, bool gateup) { // CTAs of an FP16 streaming launch
     const int lanes = p->cfg.fp16_lanes;
     const SfLayout L = sf_layout(rows, cols, lanes, gateup);
@@ -512,16 +514,29 @@ template <int MODE> int launch_stream_f16(b200_plan *p, const DevMat &m, const D
 // a programmatic edge): the kernel may become resident while its predecessor is still running.
 template <typename... KA, typename... A>
 int launch_k(b200_plan *p, bool pdl, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args) {
+    return launch_cluster(p, pdl, 1, kern, grid, block, smem, args...);
+}
+template <typename... KA, typename... A>
+int launch_cluster(b200_plan *p, bool pdl, int cluster, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = p->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        n++;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     CK(cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...));
     return B200_OK;
 }
@@ -583,8 +598,13 @@ bool gateup_fits(int hidden, int n_sms) { // epilogue buffer holds this CTA's hi
     return 2 * ((hidden / 2) / n_sms + 1) <= SMV_HVALS;
 }
 
-// k_attention's dynamic shared memory: q | k | out | score row (the row lives in a global scratch buffer for long contexts).
-size_t att_smem_bytes(int head_size, int ctx, bool scratch) { return (size_t)(3 * head_size + (scratch ? 0 : ctx)) * 4; }
+// k_attention's dynamic shared memory: q | k | out | score row (the row lives in a global scratch buffer for long contexts), or what a cluster's CTA needs.
+size_t att_smem_bytes(int head_size, int ctx, bool scratch) {
+    if (att_cluster(head_size, ctx) > 1) return (size_t)3 * head_size * 4 + sizeof(AttSplitSmem);
+    return (size_t)(3 * head_size + (scratch ? 0 : ctx)) * 4;
+}
+
+int att_row_stride(int ctx) { return (ctx + PD_CT - 1) / PD_CT * PD_CT; } // score rows in global memory: whole accumulator chunks
 
 // Enqueue one single-token forward on p->stream (captured into a CUDA graph at creation).
 // with_logits=false is the prefill variant (InferenceCoreBatchPrefillDecode.java:166-167).
@@ -622,11 +642,12 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
         {
             const size_t att_smem = att_smem_bytes(c.head_size, c.context_length, p->att_scratch != nullptr);
+            const int cluster = att_cluster(c.head_size, c.context_length);
             auto att = [&](auto kern) {
-                return launch_k(p, pdl, kern, dim3(p->nh_l), dim3(ATT_THREADS), att_smem, p->qkv, kc, vc, (const StepState *)p->st,
+                return launch_cluster(p, pdl, cluster, kern, dim3(p->nh_l * cluster), dim3(ATT_THREADS), att_smem, p->qkv, kc, vc, (const StepState *)p->st,
                                 (const float *)p->rope_cr, (const float *)p->rope_ci, p->nh_l, p->nkv_l, p->kflags, (const float *)L.q_norm,
                                 (const float *)L.k_norm, c.rms_norm_eps, (float)sqrt((double)c.head_size), q8 ? p->attq : nullptr, q8 ? p->atts : nullptr, xbf, TR(4),
-                                p->tp, (unsigned)(4 * l + 0), rank * p->nh_l, p->att_scratch, c.context_length);
+                                p->tp, (unsigned)(4 * l + 0), rank * p->nh_l, cluster > 1 ? p->att_rows : p->att_scratch, att_row_stride(c.context_length), cluster);
             };
             if (c.head_size == 128) rc = att(k_attention<128>);
             else if (c.head_size == 64) rc = att(k_attention<64>);
@@ -1111,7 +1132,10 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
     p->tp.err = p->pd_sync + PD_S_ERR;
     p->tp.host_err = p->d_err;
     if (3 * c.head_size + c.context_length > ATT_SMEM_FLOATS_MAX) { // long context: score rows in global memory
-        if ((rc = dalloc(p, &p->att_scratch, (size_t)p->nh_l * ((c.context_length + PD_CT - 1) / PD_CT * PD_CT) * 4))) return rc;
+        if ((rc = dalloc(p, &p->att_scratch, (size_t)p->nh_l * att_row_stride(c.context_length) * 4))) return rc;
+    }
+    if (att_cluster(c.head_size, c.context_length) > 1) {
+        if ((rc = dalloc(p, &p->att_rows, (size_t)p->nh_l * (att_row_stride(c.context_length) + 8) * 4))) return rc;
     }
     if ((rc = set_smem_attrs(p))) return rc;
     if (c.tp_size > 1) { CK(cudaStreamSynchronize(p->stream)); return B200_OK; } // graphs are captured by b200_tp_attach

@@ -24,12 +24,13 @@ struct SeqSum3Scratch {
     int pad;
     int2 items[SEQSUM3_WARPS][32]; // x = first thread << 16 | last thread << 8 | biased exponent (0: one literal thread), y = the run's integer
 };
+template <int E> struct SeqSumTerms { static constexpr int value = E; };
 // Shared copy of the terms: thread t's E terms start at t * E; a thread's 16-byte pieces are read by one lane at a time (broadcast), so the layout needs no padding.
 
 // t: this thread's E terms (zero behind the last one); sq: all terms in shared memory, written by the caller BEFORE the call (a barrier inside
-// orders them); sync: a barrier over the 256 threads.  Every thread returns the sum.
+// orders them); s0: where the sum starts (a long sum comes in pieces); sync: a barrier over the 256 threads.  Every thread returns the sum.
 template <int E, class Sync>
-__device__ __forceinline__ float block_seqsum3(const float (&t)[E], const float *sq, SeqSum3Scratch &sc, int tid, Sync sync) {
+__device__ __forceinline__ float block_seqsum3(const float (&t)[E], const float *sq, SeqSum3Scratch &sc, int tid, Sync sync, float s0 = 0.0f) {
     static_assert(E % 4 == 0, "terms move in 16-byte pieces");
     const int lane = tid & 31, warp = tid >> 5;
     // ---- a float prefix over the threads' own sums predicts the binade of every thread
@@ -44,7 +45,7 @@ __device__ __forceinline__ float block_seqsum3(const float (&t)[E], const float 
     }
     if (lane == 31) sc.wsum[warp] = inc;
     sync();
-    float before = 0.0f;
+    float before = s0;
 #pragma unroll
     for (int w = 0; w < SEQSUM3_WARPS - 1; w++)
         if (w < warp) before += sc.wsum[w];
@@ -94,7 +95,7 @@ __device__ __forceinline__ float block_seqsum3(const float (&t)[E], const float 
     sync();
     // ---- the walk: warp 0, every lane the same; lane k holds item k of the warp region in hand
     if (warp == 0) {
-        float s = 0.0f;
+        float s = s0;
         int items = 0, replays = 0;
         int2 mine = sc.items[0][lane];
         int cnt = sc.wcnt[0];
