@@ -409,15 +409,14 @@ __global__ void k_swiglu(float *__restrict__ hb, const float *__restrict__ hb2, 
 #define ATT_THREADS 512 // four threads per key (scores) and per output element (weighted sum): head size <= ATT_THREADS / 4
 
 // Long contexts.  One CTA per head leaves most SMs idle, and its score loads touch 32 cache lines per instruction: 9 us per 128 keys.  So a head
-// gets a cluster of C = head size / 32 CTAs, and beyond ATT_SPLIT keys they share its work (up to ATT_SPLIT the first CTA works alone and the
-// others leave at once):
+// gets a cluster of C = head size / 32 CTAs that share its work from position ATT_SPLIT on (a second decode graph; below it a CTA per head is faster):
 //   scores    blocks of 32 keys go round robin over the 8 C scoring warps; a lane owns a key's whole chain.  The rows arrive through a per-warp ring of
 //             cp.async stages (32 keys x 16 elements, coalesced, conflict-free to read), so nothing waits for another warp.
 //   softmax   the maximum over the cluster, the exponentials of the CTA's own keys, and the sequential sum (seqsum3.cuh), which every CTA takes for
 //             itself; the row lives in global memory (L2) and is handed over at two cluster barriers.
 //   output    a CTA owns 32 elements of the head: one warp walks the positions (one dependent add each: 4 cycles per position, the bound of this part),
 //             the others stage V rows and the quotients ahead of it.
-// 8B geometry, 3000 keys: 165 us -> see the table in the measurement notes of the plan; the dependent adds alone are 6.3 us.
+// Decode step of two layers of the 8B geometry at position 3000: 562 us with a CTA per head, 316 us so; the dependent adds alone are 6.3 us a layer.
 #define ATT_SPLIT 128
 #define ATT_KW 8           // scoring warps of a CTA
 #define ATT_KSTAGES 4      // stages of a scoring warp's ring
@@ -626,7 +625,7 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
                                                           float eps, float sqrt_hs, int8_t *__restrict__ xq,
                                                           float *__restrict__ xs, float *__restrict__ xb, TraceBuf tr, TpCtx tp,
                                                           unsigned tp_out_op, int head_base, float *att_scratch, int ctx, int cluster) {
-    // q[HS] | k[HS] | out[HS] | att[ctx] (cluster > 1: att[ATT_SPLIT] or AttSplitSmem; else, for long contexts, att in global scratch)
+    // q[HS] | k[HS] | out[HS] | att[ctx] (cluster > 1: AttSplitSmem; else, for long contexts, att in global scratch)
     extern __shared__ __align__(16) float sm[];
     __shared__ float red[ATT_THREADS / 32];
     __shared__ float s_val[2];
@@ -641,8 +640,7 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     pdl_wait();
     trace_mark(tr, 2);
     const int pos = st->pos, nt = pos + 1;
-    const bool split = cluster > 1 && nt > ATT_SPLIT; // uniform over the grid
-    if (rank && !split) return;
+    const bool split = cluster > 1; // (the host launches clusters from ATT_SPLIT positions on)
     if (!split) { // K/V rows of the earlier positions -> L2, one 128-byte line per request, so the score loads below hit L2 (the weight stream carries an
       // evict_first policy; without the prefetch these rows come from HBM every layer)
         constexpr int LINES = HS / 32;
@@ -835,7 +833,7 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     }
     if (tp.n > 1) {
         __syncthreads();
-        if (tid == 0) tp_cta_done(tp, TP_SLOT_ATT, tp_seq(tp, tp_out_op), gridDim.x / cluster);
+        if (tid == 0) tp_cta_done(tp, TP_SLOT_ATT, tp_seq(tp, tp_out_op), gridDim.x);
     }
     trace_mark(tr, 3);
 }

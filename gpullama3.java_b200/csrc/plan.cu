@@ -98,6 +98,7 @@ struct b200_plan {
     int *h_ids = nullptr;      // pinned, seq_cap
 
     cudaGraphExec_t g_decode = nullptr, g_prefill = nullptr, g_trace = nullptr; // the multi-kernel decode graph (round 1)
+    cudaGraphExec_t g_decode_deep = nullptr, g_prefill_deep = nullptr; // the same with clusters in the attention: positions from ATT_SPLIT on (null: not for this plan)
     cudaGraphExec_t g_pdecode = nullptr, g_pprefill = nullptr, g_ptrace = nullptr; // one persistent kernel per token (decode_persistent.cuh)
     unsigned long long *trace_rec = nullptr;
     int decode_mode = B200_DECODE_GRAPH; // which of the two the forward entry points launch
@@ -487,27 +488,42 @@ template <int MODE> int launch_matvec_f16(b200_plan *p, const DevMat &m, const f
 
 // FP16 plans on the streaming path (stream_matvec_f16.cuh); m2 = ffn_up for SF_GATEUP.
 template <typename... KA, typename... A> int launch_k(b200_plan *p, bool pdl, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args);
+template <typename F> int by_norm_terms(int dim, F &&f) { // f(integral_constant<entries per thread>) (fused_norm.cuh)
+    switch (norm_terms(dim)) {
+    case 4: return f(std::integral_constant<int, 4>());
+    case 8: return f(std::integral_constant<int, 8>());
+    case 16: return f(std::integral_constant<int, 16>());
+    default: return f(std::integral_constant<int, 32>());
+    }
+}
 template <typename... KA, typename... A> int launch_cluster(b200_plan *p, bool pdl, int cluster, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args);
-int sf_grid(const b200_plan *p, int rows, int cols, bool gateup) { // CTAs of an FP16 streaming launch
+int sf_grid(const b200_plan *p, int rows, int cols, bool gateup, bool norm) { // CTAs of an FP16 streaming launch
     const int lanes = p->cfg.fp16_lanes;
-    const SfLayout L = sf_layout(rows, cols, lanes, gateup);
+    const SfLayout L = sf_layout(rows, cols, lanes, gateup, norm);
     const int rw = 64 / lanes, mr = gateup ? rw / 2 : rw;
     const int grid = L.ctas_per_sm * p->n_sms;
     return grid > rows / mr ? rows / mr : grid;
 }
 template <int MODE> int launch_stream_f16(b200_plan *p, const DevMat &m, const DevMat *m2, const float *x, float *out, TraceBuf tr = TraceBuf{nullptr, 0, 0},
-                                          bool argmax = false) {
+                                          bool argmax = false, const NormIn *norm = nullptr) {
     const int lanes = p->cfg.fp16_lanes;
-    const SfLayout L = sf_layout(m.rows, m.cols, lanes, MODE == SF_GATEUP);
+    const SfLayout L = sf_layout(m.rows, m.cols, lanes, MODE == SF_GATEUP, norm != nullptr);
     if (!L.ok) return fail(p, B200_ERR_STATE, "f16 streaming layout does not fit %d x %d", m.rows, m.cols);
-    SfArgs a;
+    SfArgs a{};
     a.w0 = (const __half *)m.qs; a.w1 = m2 ? (const __half *)m2->qs : nullptr; a.x = x; a.out = out; a.rows = m.rows; a.cols = m.cols;
     a.seg = L.seg; a.nseg = L.nseg; a.stages = L.stages; a.tr = tr;
     a.part_val = argmax ? p->part_val : nullptr;
     a.part_idx = argmax ? p->part_idx : nullptr;
-    const int grid = sf_grid(p, m.rows, m.cols, MODE == SF_GATEUP);
-    if (lanes == 16) return launch_k(p, p->use_pdl, k_stream_matvec_f16<16, MODE>, dim3(grid), dim3(SF_THREADS), L.total, a);
-    return launch_k(p, p->use_pdl, k_stream_matvec_f16<8, MODE>, dim3(grid), dim3(SF_THREADS), L.total, a);
+    if (norm) a.norm = *norm;
+    const int grid = sf_grid(p, m.rows, m.cols, MODE == SF_GATEUP, norm != nullptr);
+    auto go = [&](auto e_c) -> int {
+        constexpr int E = decltype(e_c)::value;
+        if (lanes == 16) return launch_k(p, p->use_pdl, k_stream_matvec_f16<16, MODE, E>, dim3(grid), dim3(SF_THREADS), L.total, a);
+        return launch_k(p, p->use_pdl, k_stream_matvec_f16<8, MODE, E>, dim3(grid), dim3(SF_THREADS), L.total, a);
+    };
+    if constexpr (MODE != SF_RESID)
+        if (norm) return by_norm_terms(m.cols, go);
+    return go(std::integral_constant<int, 0>());
 }
 
 // Kernel launch with the programmatic-dependent-launch attribute (captured into the CUDA graph as
@@ -574,9 +590,9 @@ size_t smv_budget(const b200_plan *p, int cols) {
 template <int MODE>
 int launch_stream(b200_plan *p, const TileMat &W, const int8_t *xq, const float *xs, float *out, int8_t *hq, float *hs, bool argmax = false,
                   TraceBuf tr = TraceBuf{nullptr, 0, 0}, int wait_slot = -1, unsigned wait_op = 0, int out_slot = -1, unsigned out_op = 0,
-                  int row_base = 0) {
-    SmvSmem L = smv_layout(W.cols, W.seg, smv_budget(p, W.cols));
-    SmvArgs a;
+                  int row_base = 0, const NormIn *norm = nullptr) {
+    SmvSmem L = smv_layout(W.cols, W.seg, smv_budget(p, W.cols), norm != nullptr);
+    SmvArgs a{};
     a.W = W; a.xq = xq; a.xs = xs; a.out = out; a.hq = hq; a.hs = hs; a.blk_cnt = p->blk_cnt;
     a.part_val = argmax ? p->part_val : nullptr;
     a.part_idx = argmax ? p->part_idx : nullptr;
@@ -584,14 +600,26 @@ int launch_stream(b200_plan *p, const TileMat &W, const int8_t *xq, const float 
     a.tp = p->tp;
     a.wait_slot = wait_slot; a.wait_op = wait_op; a.out_slot = out_slot; a.out_op = out_op; a.row_base = row_base;
     a.l2_window = p->l2_window;
-    return launch_k(p, p->use_pdl, k_stream_matvec_q8<MODE>, dim3(p->n_sms), dim3(SMV_THREADS), L.total, a, L);
+    if (norm) a.norm = *norm;
+    auto go = [&](auto e_c) -> int { return launch_k(p, p->use_pdl, k_stream_matvec_q8<MODE, decltype(e_c)::value>, dim3(p->n_sms), dim3(SMV_THREADS), L.total, a, L); };
+    if constexpr (MODE != SMV_RESID)
+        if (norm) return by_norm_terms(W.cols, go);
+    return go(std::integral_constant<int, 0>());
+}
+
+// The norm in front of a streaming matvec, for the matvec's own CTAs (fused_norm.cuh).
+NormIn norm_in(const b200_plan *p, bool embed, const float *w) {
+    NormIn n{};
+    n.x = p->x; n.w = w; n.eps = p->cfg.rms_norm_eps; n.embed = embed; n.x_out = p->x; n.emb = p->emb; n.st = p->st;
+    n.xq = p->xq; n.xs = p->xs; n.xb = p->xb;
+    return n;
 }
 
 bool stream_shape_ok(int rows, int cols) {
     if (rows % 4 || cols % 32) return false;
     int nseg = smv_pick_nseg(cols);
     if (!nseg) return false;
-    return smv_layout(cols, cols / nseg, SMV_SMEM_BUDGET_MAX).stages >= 3;
+    return smv_layout(cols, cols / nseg, SMV_SMEM_BUDGET_MAX, cols <= 8192).stages >= 3;
 }
 
 bool gateup_fits(int hidden, int n_sms) { // epilogue buffer holds this CTA's hidden units
@@ -599,8 +627,8 @@ bool gateup_fits(int hidden, int n_sms) { // epilogue buffer holds this CTA's hi
 }
 
 // k_attention's dynamic shared memory: q | k | out | score row (the row lives in a global scratch buffer for long contexts), or what a cluster's CTA needs.
-size_t att_smem_bytes(int head_size, int ctx, bool scratch) {
-    if (att_cluster(head_size, ctx) > 1) return (size_t)3 * head_size * 4 + sizeof(AttSplitSmem);
+size_t att_smem_bytes(int head_size, int ctx, bool scratch, int cluster = 1) {
+    if (cluster > 1) return (size_t)3 * head_size * 4 + sizeof(AttSplitSmem);
     return (size_t)(3 * head_size + (scratch ? 0 : ctx)) * 4;
 }
 
@@ -608,7 +636,7 @@ int att_row_stride(int ctx) { return (ctx + PD_CT - 1) / PD_CT * PD_CT; } // sco
 
 // Enqueue one single-token forward on p->stream (captured into a CUDA graph at creation).
 // with_logits=false is the prefill variant (InferenceCoreBatchPrefillDecode.java:166-167).
-int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = false) {
+int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = false, bool deep = false) {
     const b200_config &c = p->cfg;
     const bool q8 = p->wtype == B200_GGML_Q8_0;
     const bool st = p->use_stream, pdl = p->use_pdl, sf = p->use_f16_stream;
@@ -632,17 +660,21 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         LayerW &L = p->layers[l];
         int rc;
         // TP flag epochs inside one forward: op = 4*l + {0: attention out, 1: x after Wo, 2: hb, 3: x after W2}
-        if ((rc = norm(l == 0, L.attn_norm, l == 0 ? -1 : 4 * (l - 1) + 3))) return rc;
-        n++;
-        if (st) rc = launch_stream<SMV_STORE>(p, L.tqkv, p->xq, p->xs, p->qkv, nullptr, nullptr, false, TR(2));
+        const NormIn nin = norm_in(p, l == 0, L.attn_norm), nff = norm_in(p, false, L.ffn_norm);
+        if (!st && !sf) { // (the streaming matvecs compute the norm themselves)
+            if ((rc = norm(l == 0, L.attn_norm, -1))) return rc;
+            n++;
+        }
+        const int x_slot = tpar && l ? TP_SLOT_X : -1;
+        if (st) rc = launch_stream<SMV_STORE>(p, L.tqkv, nullptr, nullptr, p->qkv, nullptr, nullptr, false, TR(2), x_slot, l ? 4 * (l - 1) + 3 : 0, -1, 0, 0, &nin);
         else if (q8) rc = launch_matvec_q8<MODE_STORE>(p, L.qkv, p->xq, p->xs, p->qkv);
-        else if (sf) rc = launch_stream_f16<SF_STORE>(p, L.qkv, nullptr, p->xb, p->qkv, TR(2));
+        else if (sf) rc = launch_stream_f16<SF_STORE>(p, L.qkv, nullptr, nullptr, p->qkv, TR(2), false, &nin);
         else rc = launch_matvec_f16<MODE_STORE>(p, L.qkv, p->xb, p->qkv);
         if (rc) return rc; n++;
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
         {
-            const size_t att_smem = att_smem_bytes(c.head_size, c.context_length, p->att_scratch != nullptr);
-            const int cluster = att_cluster(c.head_size, c.context_length);
+            const int cluster = deep ? att_cluster(c.head_size, c.context_length) : 1;
+            const size_t att_smem = att_smem_bytes(c.head_size, c.context_length, p->att_scratch != nullptr, cluster);
             auto att = [&](auto kern) {
                 return launch_cluster(p, pdl, cluster, kern, dim3(p->nh_l * cluster), dim3(ATT_THREADS), att_smem, p->qkv, kc, vc, (const StepState *)p->st,
                                 (const float *)p->rope_cr, (const float *)p->rope_ci, p->nh_l, p->nkv_l, p->kflags, (const float *)L.q_norm,
@@ -662,10 +694,12 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         else if (sf) rc = launch_stream_f16<SF_RESID>(p, L.wo, nullptr, p->xb, p->x, TR(5));
         else rc = launch_matvec_f16<MODE_RESID>(p, L.wo, p->xb, p->x);
         if (rc) return rc; n++;
-        if ((rc = norm(false, L.ffn_norm, 4 * l + 1))) return rc;
-        n++;
+        if (!st && !sf) {
+            if ((rc = norm(false, L.ffn_norm, -1))) return rc;
+            n++;
+        }
         if (st) {
-            if ((rc = launch_stream<SMV_GATEUP>(p, L.tgu, p->xq, p->xs, p->hb, p->hq, p->hs, false, TR(6), -1, 0, tpar ? TP_SLOT_HQ : -1, 4 * l + 2, rank * p->hid_l))) return rc; n++;
+            if ((rc = launch_stream<SMV_GATEUP>(p, L.tgu, nullptr, nullptr, p->hb, p->hq, p->hs, false, TR(6), tpar ? TP_SLOT_X : -1, 4 * l + 1, tpar ? TP_SLOT_HQ : -1, 4 * l + 2, rank * p->hid_l, &nff))) return rc; n++;
             if ((rc = launch_stream<SMV_RESID>(p, L.tw2, p->hq, p->hs, p->x, nullptr, nullptr, false, TR(7), tpar ? TP_SLOT_HQ : -1, 4 * l + 2, tpar ? TP_SLOT_X : -1, 4 * l + 3, rank * p->dim_l))) return rc; n++;
         } else if (q8) {
             k_gateup_q8<<<c.hidden_dim / 32, 256, q8_smem_bytes(c.dim, 4, 8), p->stream>>>(
@@ -673,7 +707,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
             CK(cudaGetLastError()); n++;
             if ((rc = launch_matvec_q8<MODE_RESID>(p, L.w2, p->hq, p->hs, p->x))) return rc; n++;
         } else if (sf) { // gate, up and SwiGLU in one launch; then the down projection
-            if ((rc = launch_stream_f16<SF_GATEUP>(p, L.w1, &L.w3, p->xb, p->hb, TR(6)))) return rc; n++;
+            if ((rc = launch_stream_f16<SF_GATEUP>(p, L.w1, &L.w3, nullptr, p->hb, TR(6), false, &nff))) return rc; n++;
             if ((rc = launch_stream_f16<SF_RESID>(p, L.w2, nullptr, p->hb, p->x, TR(7)))) return rc; n++;
         } else {
             if ((rc = launch_matvec_f16<MODE_STORE>(p, L.w1, p->xb, p->hb))) return rc; n++;
@@ -687,11 +721,14 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
     if (with_logits) {
         // rmsnorm(x, x, rms_final_weight) then wcls.matmul (InferenceCore.java:167-169)
         int rc;
-        if ((rc = norm(false, p->out_norm, last_x_op))) return rc;
-        n++;
-        if (st) rc = launch_stream<SMV_STORE>(p, p->tout, p->xq, p->xs, p->logits, nullptr, nullptr, true, TR(8), -1, 0, -1, 0, rank * p->voc_l);
+        const NormIn nout = norm_in(p, false, p->out_norm);
+        if (!st && !sf) {
+            if ((rc = norm(false, p->out_norm, -1))) return rc;
+            n++;
+        }
+        if (st) rc = launch_stream<SMV_STORE>(p, p->tout, nullptr, nullptr, p->logits, nullptr, nullptr, true, TR(8), tpar ? TP_SLOT_X : -1, last_x_op, -1, 0, rank * p->voc_l, &nout);
         else if (q8) rc = launch_matvec_q8<MODE_STORE>(p, p->out, p->xq, p->xs, p->logits);
-        else if (sf) rc = launch_stream_f16<SF_STORE>(p, p->out, nullptr, p->xb, p->logits, TR(8), true);
+        else if (sf) rc = launch_stream_f16<SF_STORE>(p, p->out, nullptr, nullptr, p->logits, TR(8), true, &nout);
         else rc = launch_matvec_f16<MODE_STORE>(p, p->out, p->xb, p->logits);
         if (rc) return rc; n++;
     }
@@ -699,7 +736,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         int rc;
         if ((rc = launch_k(p, pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, c.vocab_size, p->st, (const int *)p->seq_tokens, p->out_ids, with_logits ? 1 : 0,
                            (const float *)(st || sf ? p->part_val : nullptr), (const int *)(st || sf ? p->part_idx : nullptr),
-                           sf ? sf_grid(p, c.vocab_size, c.dim, false) : p->n_sms, TR(9), p->tp, with_logits ? -1 : last_x_op))) return rc;
+                           sf ? sf_grid(p, c.vocab_size, c.dim, false, true) : p->n_sms, TR(9), p->tp, with_logits ? -1 : last_x_op))) return rc;
         n++;
     }
     if (launches) *launches = n;
@@ -786,10 +823,10 @@ int enqueue_persistent(b200_plan *p, bool with_logits, int *launches, bool trace
     return B200_OK;
 }
 
-int capture(b200_plan *p, bool with_logits, cudaGraphExec_t *exec, int *launches, bool trace = false, bool persistent = false) {
+int capture(b200_plan *p, bool with_logits, cudaGraphExec_t *exec, int *launches, bool trace = false, bool persistent = false, bool deep = false) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = persistent ? enqueue_persistent(p, with_logits, launches, trace) : enqueue_forward(p, with_logits, launches, trace);
+    int rc = persistent ? enqueue_persistent(p, with_logits, launches, trace) : enqueue_forward(p, with_logits, launches, trace, deep);
     cudaError_t e = cudaStreamEndCapture(p->stream, &g);
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }
     if (e != cudaSuccess) return fail(p, B200_ERR_CUDA, "cudaStreamEndCapture: %s", cudaGetErrorString(e));
@@ -804,6 +841,10 @@ int capture_all(b200_plan *p) {
     int rc;
     if ((rc = capture(p, true, &p->g_decode, &p->launches_decode))) return rc;
     if ((rc = capture(p, false, &p->g_prefill, nullptr))) return rc;
+    if (p->att_rows) { // two graphs, chosen by the position on the host: up to ATT_SPLIT positions the cluster's launch only costs (measured: 1 - 2 %)
+        if ((rc = capture(p, true, &p->g_decode_deep, nullptr, false, false, true))) return rc;
+        if ((rc = capture(p, false, &p->g_prefill_deep, nullptr, false, false, true))) return rc;
+    }
     if (p->use_stream || p->use_f16_stream) {
         if ((rc = dalloc(p, &p->trace_rec, (size_t)(p->launches_decode + 8) * 32))) return rc;
         if ((rc = capture(p, true, &p->g_trace, nullptr, true))) return rc;
@@ -867,6 +908,19 @@ int set_smem_attrs(b200_plan *p) {
     CK(cudaFuncSetAttribute(k_stream_matvec_q8<SMV_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMV_SMEM_BUDGET_MAX));
     CK(cudaFuncSetAttribute(k_stream_matvec_q8<SMV_RESID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMV_SMEM_BUDGET_MAX));
     CK(cudaFuncSetAttribute(k_stream_matvec_q8<SMV_GATEUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMV_SMEM_BUDGET_MAX));
+    for (int d = 1024; d <= 8192; d *= 2) { // every norm width
+        int rc = by_norm_terms(d, [&](auto e_c) -> int {
+            constexpr int E = decltype(e_c)::value;
+            CK(cudaFuncSetAttribute(k_stream_matvec_q8<SMV_STORE, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMV_SMEM_BUDGET_MAX));
+            CK(cudaFuncSetAttribute(k_stream_matvec_q8<SMV_GATEUP, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMV_SMEM_BUDGET_MAX));
+            CK(set_max_dyn(k_stream_matvec_f16<16, SF_STORE, E>, maxdyn));
+            CK(set_max_dyn(k_stream_matvec_f16<16, SF_GATEUP, E>, maxdyn));
+            CK(set_max_dyn(k_stream_matvec_f16<8, SF_STORE, E>, maxdyn));
+            CK(set_max_dyn(k_stream_matvec_f16<8, SF_GATEUP, E>, maxdyn));
+            return B200_OK;
+        });
+        if (rc) return rc;
+    }
     CK(set_max_dyn(k_matvec_f16<MODE_STORE>, maxdyn));
     CK(set_max_dyn(k_matvec_f16<MODE_RESID>, maxdyn));
     CK(set_max_dyn(k_stream_matvec_f16<16, SF_STORE>, maxdyn));
@@ -930,9 +984,9 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
                         stream_shape_ok(2 * p->hid_l, c.dim) && stream_shape_ok(p->dim_l, c.hidden_dim) && stream_shape_ok(p->voc_l, c.dim) &&
                         gateup_fits(p->hid_l, p->n_sms);
         const char *e3 = getenv("B200_F16_STREAM"); // FP16 plans: 0 = the round-1 k_matvec_f16 launches
-        p->use_f16_stream = !(e3 && e3[0] == '0') && p->wtype == B200_GGML_F16 && c.tp_size == 1 && sf_layout(p->qd + 2 * p->kvd, c.dim, c.fp16_lanes, false).ok &&
-                            sf_layout(c.dim, p->qd, c.fp16_lanes, false).ok && sf_layout(c.hidden_dim, c.dim, c.fp16_lanes, true).ok &&
-                            sf_layout(c.dim, c.hidden_dim, c.fp16_lanes, false).ok && sf_layout(c.vocab_size, c.dim, c.fp16_lanes, false).ok;
+        p->use_f16_stream = !(e3 && e3[0] == '0') && p->wtype == B200_GGML_F16 && c.tp_size == 1 && sf_layout(p->qd + 2 * p->kvd, c.dim, c.fp16_lanes, false, true).ok &&
+                            sf_layout(c.dim, p->qd, c.fp16_lanes, false, false).ok && sf_layout(c.hidden_dim, c.dim, c.fp16_lanes, true, true).ok &&
+                            sf_layout(c.dim, c.hidden_dim, c.fp16_lanes, false, false).ok && sf_layout(c.vocab_size, c.dim, c.fp16_lanes, false, true).ok;
         const char *e2 = getenv("B200_PDL");
         p->use_pdl = (p->use_stream || p->use_f16_stream) && !(e2 && e2[0] == '0');
         if (c.tp_size > 1 && !p->use_stream) return fail(p, B200_ERR_UNSUPPORTED, "tensor parallelism needs the Q8_0 streaming path");
@@ -1466,8 +1520,14 @@ int prefill_forward(b200_plan *p, int n, int start_pos, int *launches) {
     return B200_OK;
 }
 
-cudaGraphExec_t decode_graph(b200_plan *p) { return p->decode_mode == B200_DECODE_PERSISTENT && p->g_pdecode ? p->g_pdecode : p->g_decode; }
-cudaGraphExec_t prefill_graph(b200_plan *p) { return p->decode_mode == B200_DECODE_PERSISTENT && p->g_pprefill ? p->g_pprefill : p->g_prefill; }
+cudaGraphExec_t decode_graph(b200_plan *p, int pos) {
+    if (p->decode_mode == B200_DECODE_PERSISTENT && p->g_pdecode) return p->g_pdecode;
+    return pos >= ATT_SPLIT && p->g_decode_deep ? p->g_decode_deep : p->g_decode;
+}
+cudaGraphExec_t prefill_graph(b200_plan *p, int pos) {
+    if (p->decode_mode == B200_DECODE_PERSISTENT && p->g_pprefill) return p->g_pprefill;
+    return pos >= ATT_SPLIT && p->g_prefill_deep ? p->g_prefill_deep : p->g_prefill;
+}
 
 // After a synchronize: did a device-side wait of the persistent kernel (or a tensor-parallel flag wait) give up?
 int check_device_error(b200_plan *p) {
@@ -1565,7 +1625,7 @@ int b200_forward_decode(b200_plan *p, int32_t token, int32_t position, float *lo
     if ((rc = check_pos(p, token, position))) return rc;
     CK(cudaSetDevice(p->device));
     if ((rc = set_state(p, token, position, 0, 0))) return rc;
-    CK(cudaGraphLaunch(decode_graph(p), p->stream));
+    CK(cudaGraphLaunch(decode_graph(p, position), p->stream));
     if (argmax) CK(cudaMemcpyAsync(p->h_ids, p->out_ids, 4, cudaMemcpyDeviceToHost, p->stream));
     if (logits) CK(cudaMemcpyAsync(logits, p->logits, (size_t)p->cfg.vocab_size * 4, cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
@@ -1583,7 +1643,7 @@ int b200_forward_decode_sample(b200_plan *p, int32_t token, int32_t position, fl
     if ((rc = check_pos(p, token, position))) return rc;
     CK(cudaSetDevice(p->device));
     if ((rc = set_state(p, token, position, 0, 0))) return rc;
-    CK(cudaGraphLaunch(decode_graph(p), p->stream));
+    CK(cudaGraphLaunch(decode_graph(p, position), p->stream));
     const bool greedy = temperature == 0.0f; // Sampler.selectSampler: temperature 0 -> FloatTensor.argmax, already computed by the forward
     if (!greedy) {
         static bool attr = false;
@@ -1609,7 +1669,7 @@ int b200_forward_prefill(b200_plan *p, int32_t token, int32_t position) {
     if ((rc = check_pos(p, token, position))) return rc;
     CK(cudaSetDevice(p->device));
     if ((rc = set_state(p, token, position, 0, 0))) return rc;
-    CK(cudaGraphLaunch(prefill_graph(p), p->stream));
+    CK(cudaGraphLaunch(prefill_graph(p, position), p->stream));
     CK(cudaStreamSynchronize(p->stream));
     return check_device_error(p);
 }
@@ -1649,7 +1709,7 @@ int b200_forward_batch_prefill(b200_plan *p, const int32_t *tokens, int32_t n, i
     CK(cudaMemcpyAsync(p->seq_tokens, p->h_ids, (size_t)n * 4, cudaMemcpyHostToDevice, p->stream));
     int rc;
     if ((rc = set_state(p, tokens[0], start_pos, n, 0))) return rc;
-    for (int i = 0; i < n; i++) CK(cudaGraphLaunch(prefill_graph(p), p->stream));
+    for (int i = 0; i < n; i++) CK(cudaGraphLaunch(prefill_graph(p, start_pos + i), p->stream));
     CK(cudaStreamSynchronize(p->stream));
     return check_device_error(p);
 }
@@ -1670,7 +1730,7 @@ int b200_decode_sequence(b200_plan *p, const int32_t *tokens, int32_t n, int32_t
     int rc;
     if ((rc = set_state(p, tokens[0], start_pos, nt, feedback))) return rc;
     CK(cudaEventRecord(p->ev0, p->stream));
-    for (int i = 0; i < n; i++) CK(cudaGraphLaunch(decode_graph(p), p->stream));
+    for (int i = 0; i < n; i++) CK(cudaGraphLaunch(decode_graph(p, start_pos + i), p->stream));
     CK(cudaEventRecord(p->ev1, p->stream));
     if (out_ids) CK(cudaMemcpyAsync(p->h_ids, p->out_ids, (size_t)n * 4, cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
@@ -1795,15 +1855,16 @@ int b200_time_kernel(b200_plan *p, int32_t which, int32_t reps, float *avg_ms, i
         int launches = 0, rc;
         auto one = [&](int l) -> int {
             LayerW &L = p->layers[l];
+            const NormIn nin = norm_in(p, false, L.attn_norm), nff = norm_in(p, false, L.ffn_norm), nout = norm_in(p, false, p->out_norm);
             bool keep = p->use_pdl;
             p->use_pdl = false;
             int r;
             switch (which) {
-            case 0: bytes = tb(L.tgu); r = launch_stream<SMV_GATEUP>(p, L.tgu, p->xq, p->xs, p->hb, p->hq, p->hs); break;
+            case 0: bytes = tb(L.tgu); r = launch_stream<SMV_GATEUP>(p, L.tgu, nullptr, nullptr, p->hb, p->hq, p->hs, false, TraceBuf{nullptr, 0, 0}, -1, 0, -1, 0, 0, &nff); break;
             case 1: bytes = tb(L.tw2); r = launch_stream<SMV_RESID>(p, L.tw2, p->hq, p->hs, p->x, nullptr, nullptr); break;
-            case 2: bytes = tb(L.tqkv); r = launch_stream<SMV_STORE>(p, L.tqkv, p->xq, p->xs, p->qkv, nullptr, nullptr); break;
+            case 2: bytes = tb(L.tqkv); r = launch_stream<SMV_STORE>(p, L.tqkv, nullptr, nullptr, p->qkv, nullptr, nullptr, false, TraceBuf{nullptr, 0, 0}, -1, 0, -1, 0, 0, &nin); break;
             case 3: bytes = tb(L.two); r = launch_stream<SMV_RESID>(p, L.two, p->xq, p->xs, p->x, nullptr, nullptr); break;
-            default: bytes = tb(p->tout); r = launch_stream<SMV_STORE>(p, p->tout, p->xq, p->xs, p->logits, nullptr, nullptr); break;
+            default: bytes = tb(p->tout); r = launch_stream<SMV_STORE>(p, p->tout, nullptr, nullptr, p->logits, nullptr, nullptr, false, TraceBuf{nullptr, 0, 0}, -1, 0, -1, 0, 0, &nout); break;
             }
             p->use_pdl = keep;
             return r;
@@ -1832,15 +1893,16 @@ int b200_time_kernel(b200_plan *p, int32_t which, int32_t reps, float *avg_ms, i
     auto one = [&](int l) -> int {
         LayerW &L = p->layers[l];
         if (sf) { // FP16 streaming kernels, stand-alone (no PDL overlap)
+            const NormIn nin = norm_in(p, false, L.attn_norm), nff = norm_in(p, false, L.ffn_norm), nout = norm_in(p, false, p->out_norm);
             const bool keep = p->use_pdl;
             p->use_pdl = false;
             int r;
             switch (which) {
-            case 0: bytes = mat_bytes(L.w1) + mat_bytes(L.w3); r = launch_stream_f16<SF_GATEUP>(p, L.w1, &L.w3, p->xb, p->hb); break;
+            case 0: bytes = mat_bytes(L.w1) + mat_bytes(L.w3); r = launch_stream_f16<SF_GATEUP>(p, L.w1, &L.w3, nullptr, p->hb, TraceBuf{nullptr, 0, 0}, false, &nff); break;
             case 1: bytes = mat_bytes(L.w2); r = launch_stream_f16<SF_RESID>(p, L.w2, nullptr, p->hb, p->x); break;
-            case 2: bytes = mat_bytes(L.qkv); r = launch_stream_f16<SF_STORE>(p, L.qkv, nullptr, p->xb, p->qkv); break;
+            case 2: bytes = mat_bytes(L.qkv); r = launch_stream_f16<SF_STORE>(p, L.qkv, nullptr, nullptr, p->qkv, TraceBuf{nullptr, 0, 0}, false, &nin); break;
             case 3: bytes = mat_bytes(L.wo); r = launch_stream_f16<SF_RESID>(p, L.wo, nullptr, p->xb, p->x); break;
-            default: bytes = mat_bytes(p->out); r = launch_stream_f16<SF_STORE>(p, p->out, nullptr, p->xb, p->logits); break;
+            default: bytes = mat_bytes(p->out); r = launch_stream_f16<SF_STORE>(p, p->out, nullptr, nullptr, p->logits, TraceBuf{nullptr, 0, 0}, false, &nout); break;
             }
             p->use_pdl = keep;
             return r;
@@ -1958,7 +2020,7 @@ int b200_profile_norm(b200_plan *p, int64_t *cycles4) {
 
 static int run_seqsum_hook(const float *terms, int32_t n, int threads, float *out, int32_t *info) {
     if (!terms || !out || n <= 0 || n > 8192) return B200_ERR_BAD_ARG;
-    if (threads != 0 && threads != 256 && threads != 512 && threads != 1024) return B200_ERR_BAD_ARG;
+    if (threads != 0 && threads != 3 && threads != 256 && threads != 512 && threads != 1024) return B200_ERR_BAD_ARG;
     float *d = nullptr, *o = nullptr;
     if (cudaMalloc(&d, (size_t)n * 4) != cudaSuccess) return B200_ERR_OOM;
     if (cudaMalloc(&o, 16) != cudaSuccess) { cudaFree(d); return B200_ERR_OOM; }
@@ -1968,6 +2030,12 @@ static int run_seqsum_hook(const float *terms, int32_t n, int threads, float *ou
             const size_t smem = (size_t)((n + 31) & ~31) * 4 + seqsum_scratch_bytes((n + 31) & ~31);
             e = cudaFuncSetAttribute(k_test_seqsum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e == cudaSuccess) k_test_seqsum<<<1, NORM_THREADS, smem>>>(d, n, o, reinterpret_cast<int *>(o) + 1);
+        } else if (threads == 3) { // seqsum3.cuh: what the streaming matvecs' norms run
+            by_norm_terms(n, [&](auto e_c) -> int {
+                constexpr int E = decltype(e_c)::value;
+                k_test_seqsum3<E><<<1, SEQSUM3_THREADS>>>(d, n, o, reinterpret_cast<int *>(o) + 1);
+                return B200_OK;
+            });
         } else if (threads == 1024) {
             const size_t smem = (size_t)1024 * ((n + 1023) / 1024) * 4 + seqsum2_scratch_bytes(1024);
             e = cudaFuncSetAttribute(k_test_seqsum2<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -2067,6 +2135,8 @@ void b200_plan_free(b200_plan *p) {
     prefill_free(p->prefill);
     if (p->g_decode) cudaGraphExecDestroy(p->g_decode);
     if (p->g_prefill) cudaGraphExecDestroy(p->g_prefill);
+    if (p->g_decode_deep) cudaGraphExecDestroy(p->g_decode_deep);
+    if (p->g_prefill_deep) cudaGraphExecDestroy(p->g_prefill_deep);
     if (p->g_trace) cudaGraphExecDestroy(p->g_trace);
     if (p->g_pdecode) cudaGraphExecDestroy(p->g_pdecode);
     if (p->g_pprefill) cudaGraphExecDestroy(p->g_pprefill);

@@ -4,13 +4,14 @@
 // 256 threads with E consecutive terms each, the terms in registers (and, for the replays, in shared memory).  What is different from
 // seqsum2.cuh, whose 1024 threads spend most of their time in barriers and in the scan of composed pairs:
 //   * inside one binade a term that is not an exact tie adds the same integer whatever the parity of the sum, so a thread without ties needs ONE
-//     integer (the sum of its rounded terms) and the scan over a run is an integer prefix sum; a thread with a tie is replayed literally (a handful
+//     integer (the sum of its rounded terms) and the scan over a run is an integer prefix sum; a thread with a tie is replayed literally (a few
 //     of 256: a tie needs the dropped bits to be exactly 100..0);
-//   * every warp emits its own items, so there is no compaction over the block: two barriers in front of the walk, one behind;
-//   * the walk works on the float's bits: within a binade they ARE the integer, and one shift-compare checks that the binade was not left.
+//   * the walk works on the float's bits: within a binade they ARE the integer, and one shift-compare checks that the binade was not left; the items and the terms
+//     of literal threads are fetched one and two items ahead, so that an item costs its own few dependent operations and no shared-memory round trip
+//     (without that a walk of 32 items took 9,360 of 13,900 cycles).
 // The predictions (a float prefix, margin 2^-9 against n * 2^-24 <= 2^-11 for n <= 8192) decide speed and never the result: a run that does not
 // start or end in its binade is replayed literally.
-// A literal chain of 4096 terms is 16,400 cycles and seqsum2.cuh takes about 13,000.
+// Measured at 4096 terms (SM cycles): a literal chain 16,400, seqsum2.cuh about 13,000, here 5,900 of which the walk of 32 items is 4,100.
 #pragma once
 #include "seqsum.cuh"
 
@@ -22,7 +23,7 @@ struct SeqSum3Scratch {
     float result;
     int info[2];               // {items walked, runs replayed}
     int pad;
-    int2 items[SEQSUM3_WARPS][32]; // x = first thread << 16 | last thread << 8 | biased exponent (0: one literal thread), y = the run's integer
+    int2 items[SEQSUM3_THREADS + 2]; // in order; x = first thread << 16 | last thread << 8 | biased exponent (0: one literal thread), y = the run's integer
 };
 template <int E> struct SeqSumTerms { static constexpr int value = E; };
 // Shared copy of the terms: thread t's E terms start at t * E; a thread's 16-byte pieces are read by one lane at a time (broadcast), so the layout needs no padding.
@@ -85,51 +86,59 @@ __device__ __forceinline__ float block_seqsum3(const float (&t)[E], const float 
     const unsigned ends = __ballot_sync(0xffffffffu, is_item);
     const int first = 31 - __clz(starts & (0xffffffffu >> (31 - lane)));
     const int start_excl = __shfl_sync(0xffffffffu, scan - sum, first);
+    if (lane == 0) sc.wcnt[warp] = __popc(ends);
+    sync();
+    int off = 0, n_items = 0;
+#pragma unroll
+    for (int w = 0; w < SEQSUM3_WARPS; w++) {
+        const int c = sc.wcnt[w];
+        if (w < warp) off += c;
+        n_items += c;
+    }
     if (is_item) {
         int2 it;
         it.x = ((warp * 32 + first) << 16) | (tid << 8) | be;
         it.y = scan - start_excl;
-        sc.items[warp][__popc(ends & ((1u << lane) - 1u))] = it;
+        sc.items[off + __popc(ends & ((1u << lane) - 1u))] = it;
     }
-    if (lane == 0) sc.wcnt[warp] = __popc(ends);
     sync();
-    // ---- the walk: warp 0, every lane the same; lane k holds item k of the warp region in hand
+    // ---- the walk: warp 0, every lane the same (shared-memory broadcasts)
     if (warp == 0) {
         float s = s0;
-        int items = 0, replays = 0;
-        int2 mine = sc.items[0][lane];
-        int cnt = sc.wcnt[0];
+        int replays = 0;
+        int2 it = sc.items[0], nx = sc.items[min(1, n_items - 1)];
+        float4 v[E / 4];
+        auto terms = [&](const int2 &i, float4 (&q)[E / 4]) {
+#pragma unroll
+            for (int k = 0; k < E / 4; k++) q[k] = *reinterpret_cast<const float4 *>(sq + (i.x >> 16) * E + 4 * k);
+        };
+        terms(it, v);
+#pragma unroll 2
+        for (int i = 0; i < n_items; i++) {
+            float4 vn[E / 4];
+            terms(nx, vn);
+            const int2 nn = sc.items[min(i + 2, n_items - 1)];
+            const unsigned sb = __float_as_uint(s), mb = sb + (unsigned)it.y, xe = (unsigned)it.x & 0xffu;
+            if (xe != 0u && (sb >> 23) == xe && (mb >> 23) == xe) s = __uint_as_float(mb);
+            else if (xe == 0u) { // a literal thread
+#pragma unroll
+                for (int k = 0; k < E / 4; k++) { s = __fadd_rn(s, v[k].x); s = __fadd_rn(s, v[k].y); s = __fadd_rn(s, v[k].z); s = __fadd_rn(s, v[k].w); }
+            } else { // a run that did not stay in its binade: literally
+                const float4 *q = reinterpret_cast<const float4 *>(sq + (it.x >> 16) * E);
+                const int n4 = (((it.x >> 8) & 0xff) - (it.x >> 16) + 1) * (E / 4);
+                replays++;
 #pragma unroll 1
-        for (int w = 0; w < SEQSUM3_WARPS; w++) {
-            int2 ahead = make_int2(0, 0);
-            int ahead_cnt = 0;
-            if (w + 1 < SEQSUM3_WARPS) { ahead = sc.items[w + 1][lane]; ahead_cnt = sc.wcnt[w + 1]; }
-            int x = __shfl_sync(0xffffffffu, mine.x, 0), y = __shfl_sync(0xffffffffu, mine.y, 0);
-#pragma unroll 1
-            for (int k = 0; k < cnt; k++) {
-                const int nx = __shfl_sync(0xffffffffu, mine.x, (k + 1) & 31), ny = __shfl_sync(0xffffffffu, mine.y, (k + 1) & 31);
-                const unsigned sb = __float_as_uint(s), mb = sb + (unsigned)y;
-                const unsigned xe = (unsigned)x & 0xffu;
-                if (xe != 0u && (sb >> 23) == xe && (mb >> 23) == xe) s = __uint_as_float(mb);
-                else {
-                    const float4 *q = reinterpret_cast<const float4 *>(sq + (x >> 16) * E);
-                    const int n4 = (((x >> 8) & 0xff) - (x >> 16) + 1) * (E / 4);
-                    if (xe) replays++;
-                    float4 v = q[0];
-#pragma unroll 1
-                    for (int i = 0; i < n4; i++) {
-                        const float4 c = v;
-                        if (i + 1 < n4) v = q[i + 1];
-                        s = __fadd_rn(s, c.x); s = __fadd_rn(s, c.y); s = __fadd_rn(s, c.z); s = __fadd_rn(s, c.w);
-                    }
+                for (int k = 0; k < n4; k++) {
+                    const float4 c = q[k];
+                    s = __fadd_rn(s, c.x); s = __fadd_rn(s, c.y); s = __fadd_rn(s, c.z); s = __fadd_rn(s, c.w);
                 }
-                x = nx; y = ny;
             }
-            items += cnt;
-            mine = ahead;
-            cnt = ahead_cnt;
+            it = nx;
+            nx = nn;
+#pragma unroll
+            for (int k = 0; k < E / 4; k++) v[k] = vn[k];
         }
-        if (lane == 0) { sc.result = s; sc.info[0] = items; sc.info[1] = replays; }
+        if (lane == 0) { sc.result = s; sc.info[0] = n_items; sc.info[1] = replays; }
     }
     sync();
     return sc.result;

@@ -17,7 +17,7 @@
 //   tiles are stored in (G, s) order, so a CTA's slice [G0, G1) is one contiguous byte range.
 //   For the fused gate/up projection group G holds rows {gate 2G, gate 2G+1, up 2G, up 2G+1}.
 #pragma once
-#include "common.cuh"
+#include "fused_norm.cuh"
 
 #define SMV_CONSUMER_WARPS 8
 #define SMV_THREADS ((SMV_CONSUMER_WARPS + 1) * 32)
@@ -45,7 +45,7 @@ struct SmvSmem {
     int stages, stage_bytes, nbs_pad;
 };
 
-__host__ __device__ inline SmvSmem smv_layout(int cols, int seg, size_t budget) {
+__host__ __device__ inline SmvSmem smv_layout(int cols, int seg, size_t budget, bool norm = false) {
     SmvSmem L;
     int unit = smv_unit_bytes(seg);
     L.stage_bytes = (4 * unit + 127) & ~127;
@@ -55,7 +55,8 @@ __host__ __device__ inline SmvSmem smv_layout(int cols, int seg, size_t budget) 
     L.off_xq = o; o += (size_t)cols;
     L.off_xs = o; o += (size_t)(cols / 32) * 4;
     o = (o + 15) & ~(size_t)15;
-    L.off_terms = o; o += (size_t)SMV_CONSUMER_WARPS * 4 * L.nbs_pad * 4;
+    const size_t terms = (size_t)SMV_CONSUMER_WARPS * 4 * L.nbs_pad * 4, sq = norm ? (size_t)256 * norm_terms(cols) * 4 : 0;
+    L.off_terms = o; o += terms > sq ? terms : sq; // the norm's squares come first
     L.off_hvals = o; o += SMV_HVALS * 4; // GATEUP: this CTA's swiglu outputs; STORE+argmax: per-warp candidates
     o = (o + 127) & ~(size_t)127;
     L.off_ring = o;
@@ -173,9 +174,12 @@ struct SmvArgs {
     int out_slot;       // slot to raise after this kernel's peer stores (-1: outputs stay local)
     unsigned out_op;
     int row_base;       // global index of this rank's first output row (RESID/STORE) or hidden unit (GATEUP)
+    NormIn norm;        // E > 0: where the activation comes from
 };
+struct SmvConsumerSync { __device__ __forceinline__ void operator()() const { consumer_bar_sync(); } };
 
-template <int MODE>
+// E > 0: the consumers compute the RMSNorm themselves (norm_terms(cols) entries per thread); E == 0: xq / xs are finished.
+template <int MODE, int E = 0>
 __global__ void __launch_bounds__(SMV_THREADS, 1) k_stream_matvec_q8(SmvArgs a, SmvSmem L) {
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -240,13 +244,24 @@ __global__ void __launch_bounds__(SMV_THREADS, 1) k_stream_matvec_q8(SmvArgs a, 
     }
 
     // ===== consumers =====
+    constexpr bool W_EARLY = E > 0 && E <= 16;
+    float nw[E > 0 ? E : 1];
+    if constexpr (W_EARLY) norm_weights<E>(a.norm, W.cols, nw, tid); // immutable: on their way while the kernel in front still runs
     pdl_wait(); // activations come from the previous kernel
     trace_mark(a.tr, 2);
     if (a.tp.n > 1 && a.wait_slot >= 0) { // ... and, under TP, from every rank
         if (tid == 0) tp_wait(a.tp, a.wait_slot, tp_seq(a.tp, a.wait_op));
         consumer_bar_sync();
     }
-    {
+    if constexpr (E > 0) {
+        __shared__ SeqSum3Scratch scratch;
+        float x[E];
+        const float ss = norm_scale<E>(a.norm, W.cols, x, reinterpret_cast<float *>(smem + L.off_terms), scratch, tid, SmvConsumerSync());
+        if constexpr (!W_EARLY) norm_weights<E>(a.norm, W.cols, nw, tid);
+#pragma unroll
+        for (int k = 0; k < E; k++) x[k] = __fmul_rn(nw[k], __fmul_rn(ss, x[k]));
+        norm_quantise<E>(a.norm, W.cols, x, reinterpret_cast<int8_t *>(smem + L.off_xq), reinterpret_cast<float *>(smem + L.off_xs), tid);
+    } else {
         const int nb = W.cols >> 5;
         int4 *sxq = reinterpret_cast<int4 *>(smem + L.off_xq);
         float *sxs = reinterpret_cast<float *>(smem + L.off_xs);
@@ -255,6 +270,7 @@ __global__ void __launch_bounds__(SMV_THREADS, 1) k_stream_matvec_q8(SmvArgs a, 
         for (int b = tid; b < nb; b += SMV_CONSUMER_WARPS * 32) sxs[b] = __ldcg(a.xs + b);
     }
     consumer_bar_sync();
+    if constexpr (E > 0) trace_mark(a.tr, 2); // (the norm counts as part of the wait in the timeline)
 
     const int nbs = W.seg >> 5; // blocks per segment
     float *terms = reinterpret_cast<float *>(smem + L.off_terms) + (size_t)warp * 4 * L.nbs_pad;

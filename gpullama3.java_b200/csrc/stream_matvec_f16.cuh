@@ -39,7 +39,11 @@ struct SfArgs {
     float *part_val;       // SF_STORE on the classifier: per-CTA (max, first index) of the rows this CTA produced (FloatTensor.argmax, first
     int *part_idx;         // strict maximum), merged by k_argmax_advance instead of a pass over all logits; nullptr otherwise
     TraceBuf tr;
+    NormIn norm;           // E > 0: where the activation comes from
 };
+struct SfSync { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
+// Shared memory of the activation; with the norm inside, its squares live there first (256 threads x norm_terms entries).
+__host__ __device__ inline size_t sf_act_bytes(int cols, bool norm) { return ((norm && 256 * norm_terms(cols) > cols ? (size_t)256 * norm_terms(cols) : (size_t)cols) * 4 + 127) & ~(size_t)127; }
 
 struct SfLayout {
     int seg, nseg, stages, ctas_per_sm;
@@ -48,14 +52,14 @@ struct SfLayout {
 };
 
 // Host: pick the segment, the ring depth and the CTAs per SM that maximise the bytes in flight per SM.
-static inline SfLayout sf_layout(int rows, int cols, int lanes, bool gateup) {
+static inline SfLayout sf_layout(int rows, int cols, int lanes, bool gateup, bool norm) {
     SfLayout o{};
     o.ok = false;
     if (lanes != 8 && lanes != 16) return o;
     const int rw = 64 / lanes; // a lane owns two chains: L/2 lanes per row
     if (cols % 256 || cols < 256) return o;
     if (gateup ? rows % (rw / 2) : rows % rw) return o;
-    const size_t fixed = (size_t)cols * 4 + SF_WARPS * SF_MAX_STAGES * 8 + 256;
+    const size_t fixed = sf_act_bytes(cols, norm) + SF_WARPS * SF_MAX_STAGES * 8 + 256 + (norm ? sizeof(SeqSum3Scratch) : 0);
     const size_t per_sm = 220 * 1024;
     size_t best = 0;
     for (int seg = 256; seg <= 512; seg += 256) { // bytes in flight per SM = occ * warps * (stages - 1) * stage bytes; ties -> more CTAs
@@ -83,7 +87,8 @@ __device__ __forceinline__ unsigned f16x2_flush_subnormals(unsigned w) { // both
     return r;
 }
 
-template <int L, int MODE>
+// E > 0: the RMSNorm of the activation happens here too (fused_norm.cuh); E == 0: x is finished.
+template <int L, int MODE, int E = 0>
 __global__ void __launch_bounds__(SF_THREADS) k_stream_matvec_f16(SfArgs a) {
     constexpr int LPR = L / 2;         // lanes per row (a lane owns chains 2u and 2u+1)
     constexpr int RW = 32 / LPR;       // row slots per warp
@@ -91,7 +96,7 @@ __global__ void __launch_bounds__(SF_THREADS) k_stream_matvec_f16(SfArgs a) {
     extern __shared__ __align__(128) unsigned char sf_smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float *sx = reinterpret_cast<float *>(sf_smem);
-    const size_t off_bar = ((size_t)a.cols * 4 + 127) & ~(size_t)127;
+    const size_t off_bar = sf_act_bytes(a.cols, E > 0);
     const unsigned row_b = (unsigned)(a.seg * 2 + SF_ROW_PAD), stage_b = RW * row_b;
     const unsigned bar0 = smem_u32(sf_smem + off_bar) + (unsigned)warp * SF_MAX_STAGES * 8;
     unsigned char *ring = sf_smem + off_bar + SF_WARPS * SF_MAX_STAGES * 8 + (size_t)warp * a.stages * stage_b;
@@ -129,8 +134,26 @@ __global__ void __launch_bounds__(SF_THREADS) k_stream_matvec_f16(SfArgs a) {
     pdl_launch_dependents();
     if (lane == 0)
         for (int k = 0; k < S && k < n_items; k++) issue(k);
+    constexpr bool W_EARLY = E > 0 && E <= 16;
+    float nw[E > 0 ? E : 1];
+    if constexpr (W_EARLY) norm_weights<E>(a.norm, a.cols, nw, tid); // immutable: on their way while the kernel in front still runs
     pdl_wait(); // the activation (and out, SF_RESID) come from the previous kernel
-    for (int i = tid * 4; i < a.cols; i += SF_THREADS * 4) *reinterpret_cast<float4 *>(sx + i) = *reinterpret_cast<const float4 *>(a.x + i);
+    if constexpr (E > 0) {
+        __shared__ SeqSum3Scratch scratch;
+        float x[E];
+        const float ss = norm_scale<E>(a.norm, a.cols, x, sx, scratch, tid, SfSync());
+        if constexpr (!W_EARLY) norm_weights<E>(a.norm, a.cols, nw, tid);
+        if (tid * E < a.cols) { // (behind the sum nobody reads the squares any more)
+#pragma unroll
+            for (int k = 0; k < E; k += 4) {
+                const float4 v = make_float4(__fmul_rn(nw[k], __fmul_rn(ss, x[k])), __fmul_rn(nw[k + 1], __fmul_rn(ss, x[k + 1])), __fmul_rn(nw[k + 2], __fmul_rn(ss, x[k + 2])),
+                                             __fmul_rn(nw[k + 3], __fmul_rn(ss, x[k + 3])));
+                *reinterpret_cast<float4 *>(sx + tid * E + k) = v;
+                if (blockIdx.x == 0) *reinterpret_cast<float4 *>(a.norm.xb + tid * E + k) = v;
+            }
+        }
+    } else
+        for (int i = tid * 4; i < a.cols; i += SF_THREADS * 4) *reinterpret_cast<float4 *>(sx + i) = *reinterpret_cast<const float4 *>(a.x + i);
     __syncthreads();
     trace_mark(a.tr, 2);
 

@@ -449,7 +449,8 @@ int b200_profile_norm(b200_plan *plan, int64_t *cycles);
  * non-negative host floats on the device exactly as `for (i) s += t[i]` would. */
 int b200_test_seqsum(const float *terms, int32_t n, float *out, int32_t *info /* nullable: {entries, first fallback element or -1} */);
 /* Same contract for the round-2 accumulator (csrc/seqsum2.cuh) run by `threads` = 1024 (the RMSNorm kernel's form), 512
- * (the persistent decode kernel's form) or 256 threads; info = {items walked, fallbacks}. */
+ * (the persistent decode kernel's form) or 256 threads; threads = 3: the accumulator of the norms that the streaming matvecs compute themselves
+ * (csrc/seqsum3.cuh); info = {items walked, fallbacks}. */
 int b200_test_seqsum2(const float *terms, int32_t n, int32_t threads, float *out, int32_t *info /* nullable */);
 
 /* Test hook for the device-side K-quant -> Q8_0 re-quantiser the upload pipeline applies to Q4_K / Q5_K / Q6_K tensors (csrc/kquant.cuh;
