@@ -2063,7 +2063,7 @@ static int run_seqsum_hook(const float *terms, int32_t n, int threads, float *ou
 
 int b200_test_seqsum(const float *terms, int32_t n, float *out, int32_t *info) { return run_seqsum_hook(terms, n, 0, out, info); }
 int b200_test_seqsum2(const float *terms, int32_t n, int32_t threads, float *out, int32_t *info) {
-    if (threads != 256 && threads != 512 && threads != 1024) return B200_ERR_BAD_ARG;
+    if (threads != 3 && threads != 256 && threads != 512 && threads != 1024) return B200_ERR_BAD_ARG;
     return run_seqsum_hook(terms, n, threads, out, info);
 }
 
