@@ -1267,14 +1267,24 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     auto &c = p->xp;
     const int nqkv = p->qd + 2 * p->kvd;
     const size_t ctx_kv = (size_t)g.context_length * p->kvd;
-    const size_t norm_smem = (size_t)g.dim * 4, rope_smem = (size_t)(g.n_heads + g.n_kv_heads) * (g.head_size + 1) * 4;
+    const size_t rope_smem = (size_t)(g.n_heads + g.n_kv_heads) * (g.head_size + 1) * 4;
     CK(cudaFuncSetAttribute(k_xp_rope_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
+    auto norm = [&](bool embed, const float *w) {
+        return by_norm_terms(g.dim, [&](auto e_c) -> int {
+            constexpr int E = decltype(e_c)::value;
+            if (embed) k_xp_norm<true, E><<<n, 256, 0, p->stream>>>(c.X, p->prefill.tok, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
+            else k_xp_norm<false, E><<<n, 256, 0, p->stream>>>(c.X, nullptr, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
+            CK(cudaGetLastError());
+            return B200_OK;
+        });
+    };
     auto attention = [&](float *kc, float *vc) {
         return xp_by_head_size(g.head_size, [&](auto hs_c) -> int {
             constexpr int HS = decltype(hs_c)::value;
             const int nt = start_pos + n;
-            auto go = [&](auto kern, int qt) -> int {
-                const bool scratch = xp_att_smem_bytes(HS, qt, nt, false) > XP_SMEM_MAX;
+            auto fits = [&](int qt) { return xp_att_smem_bytes(HS, qt, nt, false) <= XP_SMEM_MAX; };
+            auto go = [&](auto kern, int threads, int qt) -> int {
+                const bool scratch = !fits(qt);
                 const size_t smem = xp_att_smem_bytes(HS, qt, nt, scratch);
                 int ctas = (n + qt - 1) / qt * g.n_heads;
                 if (scratch) {
@@ -1282,28 +1292,27 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
                     if ((size_t)ctas > slots) ctas = (int)slots;
                 }
                 CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
-                kern<<<ctas, XP_ATT_THREADS, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, c.AS, c.rows, scratch ? c.scratch : nullptr);
+                kern<<<ctas, threads, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, c.AS, c.rows, scratch ? c.scratch : nullptr);
                 CK(cudaGetLastError());
                 return B200_OK;
             };
-            // 32 tokens per CTA share the staged keys and values; a chunk too small to fill the SMs that way takes 8
-            return (n + 31) / 32 * g.n_heads >= p->n_sms ? go(k_xp_attention<HS, 4>, 32) : go(k_xp_attention<HS, 1>, 8);
+            // 64 tokens per CTA (16 warps) share the staged keys and values while their score rows fit shared memory, else 32; a chunk too small to
+            // fill the SMs that way takes 8
+            if ((n + 63) / 64 * g.n_heads >= p->n_sms && fits(64)) return go(k_xp_attention<HS, 4, 512>, 512, 64);
+            return (n + 31) / 32 * g.n_heads >= p->n_sms ? go(k_xp_attention<HS, 4, 256>, 256, 32) : go(k_xp_attention<HS, 1, 256>, 256, 8);
         });
     };
     for (int l = 0; l < g.n_layers; l++) {
         const LayerW &L = p->layers[l];
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
         int rc;
-        if (l == 0) k_xp_norm<true><<<n, XP_NORM_THREADS, norm_smem, p->stream>>>(c.X, p->prefill.tok, p->emb, L.attn_norm, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
-        else k_xp_norm<false><<<n, XP_NORM_THREADS, norm_smem, p->stream>>>(c.X, nullptr, p->emb, L.attn_norm, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
-        CK(cudaGetLastError());
+        if ((rc = norm(l == 0, L.attn_norm))) return rc;
         if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, c.AQ, c.AS, n, c.QKV, nqkv, nullptr, nullptr, nullptr))) return rc;
         k_xp_rope_kv<<<n, 256, rope_smem, p->stream>>>(c.QKV, kc, vc, g.head_size, g.n_heads, g.n_kv_heads, p->kflags, L.q_norm, L.k_norm, g.rms_norm_eps, p->rope_cr, p->rope_ci, start_pos);
         CK(cudaGetLastError());
         if ((rc = attention(kc, vc))) return rc;
         if ((rc = xp_gemm<XP_RESID>(p, L.two, c.AQ, c.AS, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
-        k_xp_norm<false><<<n, XP_NORM_THREADS, norm_smem, p->stream>>>(c.X, nullptr, p->emb, L.ffn_norm, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
-        CK(cudaGetLastError());
+        if ((rc = norm(false, L.ffn_norm))) return rc;
         if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, c.AQ, c.AS, n, nullptr, 0, c.HQ, c.HS, p->hb))) return rc;
         if ((rc = xp_gemm<XP_RESID>(p, L.tw2, c.HQ, c.HS, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
     }
