@@ -76,6 +76,7 @@ struct b200_plan {
     bool use_stream = false, use_pdl = false;
     int kflags = 0; // KF_* (common.cuh): what the attention prologues do for this architecture
     size_t kq_off = 0; // K-quant files: offset of the raw (K-quant bytes) area inside each staging buffer; 0 = no K-quant tensor in the file
+    bool sf_norm = false;        // FP16 streaming plans: the matvecs compute the norm in front of them (SF_NORM_MAX_DIM)
     bool use_f16_stream = false; // FP16 plans: per-warp bulk-copy rings (stream_matvec_f16.cuh) instead of k_matvec_f16
     bool f16_copies = false; // Q8_0 plan that also holds f16 weight matrices for the tensor-core prefill
     int n_sms = 148;
@@ -497,6 +498,9 @@ template <typename F> int by_norm_terms(int dim, F &&f) { // f(integral_constant
     }
 }
 template <typename... KA, typename... A> int launch_cluster(b200_plan *p, bool pdl, int cluster, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args);
+// Widest row whose norm the FP16 streaming matvecs compute themselves.  They run two CTAs per SM, which share its issue slots during the norm, and the norm's
+// scratch takes stages from their rings: measured on two layers at position 8 (rows of 1536: three), separate -> inside: dim 1536 188 -> 160 us, 2048 160 -> 152, 3072 208 -> 200, 4096 325 -> 344.
+const int SF_NORM_MAX_DIM = 3072;
 int sf_grid(const b200_plan *p, int rows, int cols, bool gateup, bool norm) { // CTAs of an FP16 streaming launch
     const int lanes = p->cfg.fp16_lanes;
     const SfLayout L = sf_layout(rows, cols, lanes, gateup, norm);
@@ -643,6 +647,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
     const bool tpar = p->tp.n > 1;
     int n = 0;
     auto TR = [&](int id) { return TraceBuf{trace ? p->trace_rec : nullptr, n, id}; };
+    const bool fused = st || (sf && p->sf_norm); // the streaming matvecs compute the norm themselves
     const size_t norm_smem = norm_smem_bytes(c.dim, p->norm_v2);
     int8_t *xq = q8 ? p->xq : nullptr;
     float *xs = q8 ? p->xs : nullptr;
@@ -661,14 +666,14 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         int rc;
         // TP flag epochs inside one forward: op = 4*l + {0: attention out, 1: x after Wo, 2: hb, 3: x after W2}
         const NormIn nin = norm_in(p, l == 0, L.attn_norm), nff = norm_in(p, false, L.ffn_norm);
-        if (!st && !sf) { // (the streaming matvecs compute the norm themselves)
+        if (!fused) {
             if ((rc = norm(l == 0, L.attn_norm, -1))) return rc;
             n++;
         }
         const int x_slot = tpar && l ? TP_SLOT_X : -1;
         if (st) rc = launch_stream<SMV_STORE>(p, L.tqkv, nullptr, nullptr, p->qkv, nullptr, nullptr, false, TR(2), x_slot, l ? 4 * (l - 1) + 3 : 0, -1, 0, 0, &nin);
         else if (q8) rc = launch_matvec_q8<MODE_STORE>(p, L.qkv, p->xq, p->xs, p->qkv);
-        else if (sf) rc = launch_stream_f16<SF_STORE>(p, L.qkv, nullptr, nullptr, p->qkv, TR(2), false, &nin);
+        else if (sf) rc = launch_stream_f16<SF_STORE>(p, L.qkv, nullptr, p->xb, p->qkv, TR(2), false, fused ? &nin : nullptr);
         else rc = launch_matvec_f16<MODE_STORE>(p, L.qkv, p->xb, p->qkv);
         if (rc) return rc; n++;
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
@@ -694,7 +699,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         else if (sf) rc = launch_stream_f16<SF_RESID>(p, L.wo, nullptr, p->xb, p->x, TR(5));
         else rc = launch_matvec_f16<MODE_RESID>(p, L.wo, p->xb, p->x);
         if (rc) return rc; n++;
-        if (!st && !sf) {
+        if (!fused) {
             if ((rc = norm(false, L.ffn_norm, -1))) return rc;
             n++;
         }
@@ -707,7 +712,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
             CK(cudaGetLastError()); n++;
             if ((rc = launch_matvec_q8<MODE_RESID>(p, L.w2, p->hq, p->hs, p->x))) return rc; n++;
         } else if (sf) { // gate, up and SwiGLU in one launch; then the down projection
-            if ((rc = launch_stream_f16<SF_GATEUP>(p, L.w1, &L.w3, nullptr, p->hb, TR(6), false, &nff))) return rc; n++;
+            if ((rc = launch_stream_f16<SF_GATEUP>(p, L.w1, &L.w3, p->xb, p->hb, TR(6), false, fused ? &nff : nullptr))) return rc; n++;
             if ((rc = launch_stream_f16<SF_RESID>(p, L.w2, nullptr, p->hb, p->x, TR(7)))) return rc; n++;
         } else {
             if ((rc = launch_matvec_f16<MODE_STORE>(p, L.w1, p->xb, p->hb))) return rc; n++;
@@ -722,13 +727,13 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         // rmsnorm(x, x, rms_final_weight) then wcls.matmul (InferenceCore.java:167-169)
         int rc;
         const NormIn nout = norm_in(p, false, p->out_norm);
-        if (!st && !sf) {
+        if (!fused) {
             if ((rc = norm(false, p->out_norm, -1))) return rc;
             n++;
         }
         if (st) rc = launch_stream<SMV_STORE>(p, p->tout, nullptr, nullptr, p->logits, nullptr, nullptr, true, TR(8), tpar ? TP_SLOT_X : -1, last_x_op, -1, 0, rank * p->voc_l, &nout);
         else if (q8) rc = launch_matvec_q8<MODE_STORE>(p, p->out, p->xq, p->xs, p->logits);
-        else if (sf) rc = launch_stream_f16<SF_STORE>(p, p->out, nullptr, nullptr, p->logits, TR(8), true, &nout);
+        else if (sf) rc = launch_stream_f16<SF_STORE>(p, p->out, nullptr, p->xb, p->logits, TR(8), true, fused ? &nout : nullptr);
         else rc = launch_matvec_f16<MODE_STORE>(p, p->out, p->xb, p->logits);
         if (rc) return rc; n++;
     }
@@ -736,7 +741,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         int rc;
         if ((rc = launch_k(p, pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, c.vocab_size, p->st, (const int *)p->seq_tokens, p->out_ids, with_logits ? 1 : 0,
                            (const float *)(st || sf ? p->part_val : nullptr), (const int *)(st || sf ? p->part_idx : nullptr),
-                           sf ? sf_grid(p, c.vocab_size, c.dim, false, true) : p->n_sms, TR(9), p->tp, with_logits ? -1 : last_x_op))) return rc;
+                           sf ? sf_grid(p, c.vocab_size, c.dim, false, p->sf_norm) : p->n_sms, TR(9), p->tp, with_logits ? -1 : last_x_op))) return rc;
         n++;
     }
     if (launches) *launches = n;
@@ -984,9 +989,10 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
                         stream_shape_ok(2 * p->hid_l, c.dim) && stream_shape_ok(p->dim_l, c.hidden_dim) && stream_shape_ok(p->voc_l, c.dim) &&
                         gateup_fits(p->hid_l, p->n_sms);
         const char *e3 = getenv("B200_F16_STREAM"); // FP16 plans: 0 = the round-1 k_matvec_f16 launches
-        p->use_f16_stream = !(e3 && e3[0] == '0') && p->wtype == B200_GGML_F16 && c.tp_size == 1 && sf_layout(p->qd + 2 * p->kvd, c.dim, c.fp16_lanes, false, true).ok &&
-                            sf_layout(c.dim, p->qd, c.fp16_lanes, false, false).ok && sf_layout(c.hidden_dim, c.dim, c.fp16_lanes, true, true).ok &&
-                            sf_layout(c.dim, c.hidden_dim, c.fp16_lanes, false, false).ok && sf_layout(c.vocab_size, c.dim, c.fp16_lanes, false, true).ok;
+        p->sf_norm = c.dim <= SF_NORM_MAX_DIM;
+        p->use_f16_stream = !(e3 && e3[0] == '0') && p->wtype == B200_GGML_F16 && c.tp_size == 1 && sf_layout(p->qd + 2 * p->kvd, c.dim, c.fp16_lanes, false, p->sf_norm).ok &&
+                            sf_layout(c.dim, p->qd, c.fp16_lanes, false, false).ok && sf_layout(c.hidden_dim, c.dim, c.fp16_lanes, true, p->sf_norm).ok &&
+                            sf_layout(c.dim, c.hidden_dim, c.fp16_lanes, false, false).ok && sf_layout(c.vocab_size, c.dim, c.fp16_lanes, false, p->sf_norm).ok;
         const char *e2 = getenv("B200_PDL");
         p->use_pdl = (p->use_stream || p->use_f16_stream) && !(e2 && e2[0] == '0');
         if (c.tp_size > 1 && !p->use_stream) return fail(p, B200_ERR_UNSUPPORTED, "tensor parallelism needs the Q8_0 streaming path");
@@ -1907,11 +1913,11 @@ int b200_time_kernel(b200_plan *p, int32_t which, int32_t reps, float *avg_ms, i
             p->use_pdl = false;
             int r;
             switch (which) {
-            case 0: bytes = mat_bytes(L.w1) + mat_bytes(L.w3); r = launch_stream_f16<SF_GATEUP>(p, L.w1, &L.w3, nullptr, p->hb, TraceBuf{nullptr, 0, 0}, false, &nff); break;
+            case 0: bytes = mat_bytes(L.w1) + mat_bytes(L.w3); r = launch_stream_f16<SF_GATEUP>(p, L.w1, &L.w3, p->xb, p->hb, TraceBuf{nullptr, 0, 0}, false, p->sf_norm ? &nff : nullptr); break;
             case 1: bytes = mat_bytes(L.w2); r = launch_stream_f16<SF_RESID>(p, L.w2, nullptr, p->hb, p->x); break;
-            case 2: bytes = mat_bytes(L.qkv); r = launch_stream_f16<SF_STORE>(p, L.qkv, nullptr, nullptr, p->qkv, TraceBuf{nullptr, 0, 0}, false, &nin); break;
+            case 2: bytes = mat_bytes(L.qkv); r = launch_stream_f16<SF_STORE>(p, L.qkv, nullptr, p->xb, p->qkv, TraceBuf{nullptr, 0, 0}, false, p->sf_norm ? &nin : nullptr); break;
             case 3: bytes = mat_bytes(L.wo); r = launch_stream_f16<SF_RESID>(p, L.wo, nullptr, p->xb, p->x); break;
-            default: bytes = mat_bytes(p->out); r = launch_stream_f16<SF_STORE>(p, p->out, nullptr, nullptr, p->logits, TraceBuf{nullptr, 0, 0}, false, &nout); break;
+            default: bytes = mat_bytes(p->out); r = launch_stream_f16<SF_STORE>(p, p->out, nullptr, p->xb, p->logits, TraceBuf{nullptr, 0, 0}, false, p->sf_norm ? &nout : nullptr); break;
             }
             p->use_pdl = keep;
             return r;
