@@ -12,6 +12,7 @@
 //                       a ring of earlier inputs, SiLU, unit vectors per q / k head, beta = sigmoid, decay = exp(-exp(A) softplus);
 //   * k_delta_rule_reg  the recurrence S <- g S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q with the state in registers: eight
 //                       lanes share a state column, the rows of a chunk run in sequence, columns in parallel over warps and CTAs;
+//   * k_delta_rule_blocks (+ k_delta_coef)   the same, four tokens per step of the chain: prefill chunks;
 //   * k_delta_rule      the same for key sizes above 128: one thread per state column, the state tile in shared memory;
 //   * k_head_norm_gate  per-head RMS norm of the read-out (optionally divided by a denominator per head first), weight, SiLU or sigmoid gate.
 // Rotation, scores, decays, gates, unit norms and the state are FP32 in both compute modes; fmaf is explicit because the
@@ -327,6 +328,253 @@ __global__ void __launch_bounds__(DR_THREADS) k_delta_rule_reg(const float *__re
     }
 #pragma unroll
     for (int i = 0; i < R; i++) Sg[(size_t)i * DR_THREADS] = Sr[i];
+}
+
+// ---- four tokens at a time -------------------------------------------------------------------------------------------------------------
+// With S the state before four tokens, G_i the product of their first i decays and g(j, i) = G_i / G_j (formed as products, never divided), the recurrence is
+//     u_i = beta_i v_i - beta_i G_i <S, k_i> - sum_{j < i} beta_i g(j, i) <k_j, k_i> u_j          (each per state column)
+//     o_i = G_i <S, q_i> + sum_{j <= i} g(j, i) <k_j, q_i> u_j
+//     S <- G_4 S + sum_j g(j, 4) k_j u_j
+// so the eight products with S do not wait for one another and a column pays for ONE reduction over its lanes and one short triangular solve per four
+// tokens: the chain per token drops from a shuffle tree to a quarter of one.  What the sums over j need (products of keys and queries, decays) is the same for all
+// columns of a head: k_delta_coef computes it for the whole launch beforehand, 40 floats per (four tokens, head).  All of it is FP32.
+// 16 heads of 128 x 128, 512 tokens: 130 us token by token (k_delta_rule_reg: 418 cycles per token), 101 us here and 7.6 us for the coefficients.
+#define DC_FLOATS 40 // [0, 4) beta_i G_i | [4, 8) beta_i | [8, 14) beta_i g(j, i) <k_j, k_i> of (j, i) = 12 13 23 14 24 34 | [16, 32) g(j, i) <k_j, q_i> at 16 + 4 i + j | [32, 36) G_i | [36, 40) g(j, 4)
+__host__ __device__ inline size_t delta_coef_floats(int rows, int heads) { return (size_t)((rows + 3) / 4) * heads * DC_FLOATS; }
+
+// grid (ceil(n / 4), ceil(heads / 4)), 128 threads: a warp per (four tokens, head).  Tokens behind the last one count as beta = 0, decay = 1.
+__global__ void __launch_bounds__(128) k_delta_coef(const float *__restrict__ D, int ldd, DeltaArgs a, int n, float *__restrict__ coef) {
+    const int b = blockIdx.x, lane = threadIdx.x & 31, h = blockIdx.y * 4 + (threadIdx.x >> 5);
+    if (h >= a.heads) return;
+    const int dk = a.dk, g = h / (a.heads / a.kv_heads), C = delta_channels(a), t0 = 4 * b;
+    float kk[6], kq[10]; // (j, i): 12 13 23 14 24 34 | 11 12 22 13 23 33 14 24 34 44
+#pragma unroll
+    for (int e = 0; e < 6; e++) kk[e] = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 10; e++) kq[e] = 0.0f;
+    for (int e = lane; e < dk; e += 32) {
+        float k[4], q[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const bool ok = t0 + i < n;
+            const float *d = D + (size_t)(ok ? t0 + i : t0) * ldd;
+            k[i] = ok ? d[(size_t)(a.kv_heads + g) * dk + e] : 0.0f;
+            q[i] = ok ? d[(size_t)g * dk + e] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0, x = 0, y = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j <= i; j++) {
+                if (j < i) { kk[x] = fmaf(k[j], k[i], kk[x]); x++; }
+                kq[y] = fmaf(k[j], q[i], kq[y]);
+                y++;
+            }
+    }
+#pragma unroll
+    for (int e = 0; e < 6; e++) kk[e] = warp_sum(kk[e]);
+#pragma unroll
+    for (int e = 0; e < 10; e++) kq[e] = warp_sum(kq[e]);
+    if (lane) return;
+    float beta[4], dec[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const bool ok = t0 + i < n;
+        const float *d = D + (size_t)(ok ? t0 + i : t0) * ldd + C;
+        beta[i] = ok ? d[h] : 0.0f;
+        dec[i] = ok ? d[a.heads + h] : 1.0f;
+    }
+    float *o = coef + ((size_t)b * a.heads + h) * DC_FLOATS;
+    float G = 1.0f;
+#pragma unroll
+    for (int i = 0, x = 0, y = 0; i < 4; i++) {
+        G *= dec[i];
+        o[i] = beta[i] * G;
+        o[4 + i] = beta[i];
+        o[32 + i] = G;
+        float gj[4]; // g(j, i)
+        gj[i] = 1.0f;
+#pragma unroll
+        for (int j = i - 1; j >= 0; j--) gj[j] = gj[j + 1] * dec[j + 1];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (j < i) { o[8 + x] = beta[i] * gj[j] * kk[x]; x++; }
+            o[16 + 4 * i + j] = j <= i ? gj[j] * kq[y] : 0.0f;
+            if (j <= i) y++;
+            if (i == 3) o[36 + j] = gj[j];
+        }
+    }
+    o[14] = o[15] = 0.0f;
+}
+
+// The layout of the state is k_delta_rule_reg's (16 lanes a column); a lane serves columns c and c + 8, so that a loaded key or query entry is used for both
+// (one column a lane, eight warps: 110 us instead of 101).  The sixteen products of a lane's slices are reduced over the 16 lanes by halving:
+// fifteen shuffles leave one complete product in every lane, eight more hand <S, k_i> to all of them.  Bound by the latency of that chain: one warp per scheduler, so
+// the keys and queries of the next four tokens are loaded before the solve of these.
+#define DB_THREADS (DR_THREADS / 2)
+template <int R>
+__global__ void __launch_bounds__(DB_THREADS) k_delta_rule_blocks(const float *__restrict__ D, int ldd, DeltaArgs a, const float *__restrict__ coef, float *__restrict__ S, int n,
+                                                                  float *__restrict__ O, int ldo, const StepState *__restrict__ st) {
+    static_assert(DR_SLICES == 16 && DR_COLS == 16, "two columns a lane, sixteen products over sixteen lanes");
+    constexpr int RP = R > 4 ? R + 4 : R, KR = DR_SLICES * RP;
+    __shared__ __align__(16) float ks[3][DR_TB][KR], qs[3][DR_TB][KR], cf[3][DR_TB / 4][DC_FLOATS];
+    __shared__ float vs[3][DR_TB][DR_COLS], os[2][DR_TB][DR_COLS];
+    const int h = blockIdx.x, tile = blockIdx.y, j0 = tile * DR_COLS, tid = threadIdx.x, lane = tid & 31;
+    const int c = tid / DR_SLICES, s = lane % DR_SLICES; // columns c and c + 8
+    const int dk = a.dk, dv = a.dv, g = h / (a.heads / a.kv_heads);
+    float *Sg = S + ((size_t)h * gridDim.y + tile) * R * DR_THREADS + tid;
+    float S0[R], S1[R];
+    const bool fresh = st->pos == 0;
+    const bool wide = R >= 4 && dk % 4 == 0 && ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(D) & 15) == 0; // rows of whole, aligned 16-byte pieces
+    auto stage = [&](int i) { // tokens behind the last one are zero
+        const int buf = i % 3, t0 = i * DR_TB;
+        if (t0 >= n) return;
+        if (wide) {
+            for (int e = tid; e < DR_TB * DR_SLICES * R / 4; e += DB_THREADS) {
+                const int t = e / (DR_SLICES * R / 4), i = e % (DR_SLICES * R / 4) * 4;
+                const bool ok = i < dk && t0 + t < n;
+                const float *d = D + (size_t)(ok ? t0 + t : 0) * ldd;
+                const int at = (i / R) * RP + i % R;
+                cp_async16(&ks[buf][t][at], ok ? d + (size_t)(a.kv_heads + g) * dk + i : D, ok);
+                cp_async16(&qs[buf][t][at], ok ? d + (size_t)g * dk + i : D, ok);
+            }
+        } else
+            for (int e = tid; e < DR_TB * DR_SLICES * R; e += DB_THREADS) {
+                const int t = e / (DR_SLICES * R), i = e % (DR_SLICES * R);
+                const bool ok = i < dk && t0 + t < n;
+                const float *d = D + (size_t)(ok ? t0 + t : 0) * ldd;
+                const int at = (i / R) * RP + i % R;
+                cp_async4(&ks[buf][t][at], ok ? d + (size_t)(a.kv_heads + g) * dk + i : D, ok);
+                cp_async4(&qs[buf][t][at], ok ? d + (size_t)g * dk + i : D, ok);
+            }
+        for (int e = tid; e < DR_TB * DR_COLS; e += DB_THREADS) {
+            const int t = e / DR_COLS, cc = e % DR_COLS;
+            const bool ok = j0 + cc < dv && t0 + t < n;
+            cp_async4(&vs[buf][t][cc], ok ? D + (size_t)(t0 + t) * ldd + 2 * a.kv_heads * dk + (size_t)h * dv + j0 + cc : D, ok);
+        }
+        for (int e = tid; e < DR_TB / 4 * DC_FLOATS; e += DB_THREADS) {
+            const int b = e / DC_FLOATS;
+            const bool ok = t0 + 4 * b < n;
+            cp_async4(&cf[buf][b][e % DC_FLOATS], ok ? coef + ((size_t)(t0 / 4 + b) * a.heads + h) * DC_FLOATS + e % DC_FLOATS : coef, ok);
+        }
+    };
+    auto flush = [&](int i) { // the outputs of staged block i
+        for (int e = tid; e < DR_TB * DR_COLS; e += DB_THREADS) {
+            const int t = i * DR_TB + e / DR_COLS, cc = e % DR_COLS;
+            if (t < n && j0 + cc < dv) O[(size_t)t * ldo + (size_t)h * dv + j0 + cc] = os[i & 1][e / DR_COLS][cc];
+        }
+    };
+    stage(0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    stage(1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        S0[i] = fresh ? 0.0f : Sg[(size_t)i * DR_THREADS];
+        S1[i] = fresh ? 0.0f : Sg[(size_t)i * DR_THREADS + DB_THREADS];
+    }
+    auto load = [&](const float *row, float (&x)[R]) {
+        if (R >= 4) {
+#pragma unroll
+            for (int i = 0; i < R; i += 4) *reinterpret_cast<float4 *>(&x[i]) = *reinterpret_cast<const float4 *>(row + s * RP + i);
+        } else {
+#pragma unroll
+            for (int i = 0; i < R; i++) x[i] = row[s * RP + i];
+        }
+    };
+    const bool b3 = s & 8, b2 = s & 4, b1 = s & 2, b0 = s & 1;
+    const int own = (s >> 1) & 3; // lanes 0 .. 7 end up with <S, k_own>, lanes 8 .. 15 with <S, q_own>; odd lanes of column c + 8
+    const int blocks = (n + DR_TB - 1) / DR_TB;
+    for (int it = 0; it < blocks; it++) { // one barrier per staged block: behind it block it has arrived everywhere and nobody reads block it - 1 any more
+        const int t0 = it * DR_TB, buf = it % 3;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        stage(it + 2);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (it > 0) flush(it - 1);
+        float k[4][R], q[4][R];
+#pragma unroll
+        for (int i = 0; i < 4; i++) { load(ks[buf][i], k[i]); load(qs[buf][i], q[i]); }
+#pragma unroll 1
+        for (int b = 0; b < DR_TB / 4; b++) {
+            if (t0 + 4 * b >= n) break;
+            const float *w = cf[buf][b];
+            float x[16]; // [column][key products 0 .. 3, query products 0 .. 3]
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                float d0 = 0.0f, d1 = 0.0f, e0 = 0.0f, e1 = 0.0f, f0 = 0.0f, f1 = 0.0f, g0 = 0.0f, g1 = 0.0f;
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    if (r & 1) { d1 = fmaf(S0[r], k[i][r], d1); e1 = fmaf(S0[r], q[i][r], e1); f1 = fmaf(S1[r], k[i][r], f1); g1 = fmaf(S1[r], q[i][r], g1); }
+                    else { d0 = fmaf(S0[r], k[i][r], d0); e0 = fmaf(S0[r], q[i][r], e0); f0 = fmaf(S1[r], k[i][r], f0); g0 = fmaf(S1[r], q[i][r], g0); }
+                }
+                x[i] = d0 + d1; x[4 + i] = e0 + e1; x[8 + i] = f0 + f1; x[12 + i] = g0 + g1;
+            }
+            if (b + 1 < DR_TB / 4) // the queries are used up: the next four tokens' (zero behind the last one)
+#pragma unroll
+                for (int i = 0; i < 4; i++) load(qs[buf][4 * b + 4 + i], q[i]);
+            float y[8], z[4], m2[2], m;
+#pragma unroll
+            for (int i = 0; i < 8; i++) { // (i >> 2: column) lanes with bit 3 keep the queries' products, the others the keys'
+                const int at = (i >> 2) * 8 + (i & 3);
+                const float keep = b3 ? x[at + 4] : x[at], send = b3 ? x[at] : x[at + 4];
+                y[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) { // (i >> 1: column) bit 2: tokens 2, 3 or 0, 1
+                const int at = (i >> 1) * 4 + (i & 1);
+                const float keep = b2 ? y[at + 2] : y[at], send = b2 ? y[at] : y[at + 2];
+                z[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++) { // bit 1: the odd or the even one
+                const float keep = b1 ? z[2 * i + 1] : z[2 * i], send = b1 ? z[2 * i] : z[2 * i + 1];
+                m2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+            }
+            m = (b0 ? m2[1] : m2[0]) + __shfl_xor_sync(0xffffffffu, b0 ? m2[0] : m2[1], 1); // bit 0: the column
+            const int base = lane & ~(DR_SLICES - 1);
+            const float4 A = *reinterpret_cast<const float4 *>(w), B = *reinterpret_cast<const float4 *>(w + 4), L = *reinterpret_cast<const float4 *>(w + 8), Lr = *reinterpret_cast<const float4 *>(w + 12);
+            const float4 gl = *reinterpret_cast<const float4 *>(w + 36);
+            const float4 M = *reinterpret_cast<const float4 *>(w + 16 + 4 * own);
+            const float Gown = w[32 + own], G4 = w[35];
+            float u[2][4];
+#pragma unroll
+            for (int cc = 0; cc < 2; cc++) {
+                const float a0 = __shfl_sync(0xffffffffu, m, base + cc), a1 = __shfl_sync(0xffffffffu, m, base + 2 + cc), a2 = __shfl_sync(0xffffffffu, m, base + 4 + cc),
+                            a3 = __shfl_sync(0xffffffffu, m, base + 6 + cc);
+                const float *v = &vs[buf][4 * b][c + 8 * cc];
+                const float u0 = fmaf(-A.x, a0, B.x * v[0]);
+                const float r1 = fmaf(-A.y, a1, B.y * v[DR_COLS]), r2 = fmaf(-A.z, a2, B.z * v[2 * DR_COLS]), r3 = fmaf(-A.w, a3, B.w * v[3 * DR_COLS]);
+                const float u1 = fmaf(-L.x, u0, r1);
+                const float u2 = fmaf(-L.z, u1, fmaf(-L.y, u0, r2));
+                u[cc][0] = u0; u[cc][1] = u1; u[cc][2] = u2;
+                u[cc][3] = fmaf(-Lr.y, u2, fmaf(-Lr.x, u1, fmaf(-L.w, u0, r3)));
+            }
+            if (b3) { // (a later token's update stays out by selection, not by its zero factor: it may be infinite)
+                float o = fmaf(M.x, b0 ? u[1][0] : u[0][0], Gown * m);
+                if (own >= 1) o = fmaf(M.y, b0 ? u[1][1] : u[0][1], o);
+                if (own >= 2) o = fmaf(M.z, b0 ? u[1][2] : u[0][2], o);
+                if (own >= 3) o = fmaf(M.w, b0 ? u[1][3] : u[0][3], o);
+                os[it & 1][4 * b + own][b0 ? c + 8 : c] = o;
+            }
+            auto update = [&](float (&Sr)[R], const float (&uu)[4]) {
+                const float w0 = gl.x * uu[0], w1 = gl.y * uu[1], w2 = gl.z * uu[2];
+#pragma unroll
+                for (int r = 0; r < R; r++) Sr[r] = fmaf(k[3][r], uu[3], fmaf(k[2][r], w2, fmaf(k[1][r], w1, fmaf(k[0][r], w0, G4 * Sr[r]))));
+            };
+            update(S0, u[0]);
+            update(S1, u[1]);
+            if (b + 1 < DR_TB / 4)
+#pragma unroll
+                for (int i = 0; i < 4; i++) load(ks[buf][4 * b + 4 + i], k[i]);
+        }
+    }
+    __syncthreads();
+    flush(blocks - 1);
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+        Sg[(size_t)i * DR_THREADS] = S0[i];
+        Sg[(size_t)i * DR_THREADS + DB_THREADS] = S1[i];
+    }
 }
 
 // One CTA per row, one warp per head: y = o / sqrt(mean(o^2) + eps) * w[h * w_stride + d] * gate(g[h][d]), gate = silu (sigmoid_gate: sigmoid).

@@ -156,6 +156,7 @@ struct Layered {
     float w_off = 1.0f;   // what the norm kernels add to a norm weight (sandwich: weights are deviations from one)
     bool prenorm = false;
     float *emb_norm = nullptr;
+    float *DCO = nullptr; // coefficients of the delta rule per four rows and head (k_delta_coef)
     float *DLT = nullptr, *DO = nullptr; // prepared q | k | v | beta | decay rows and read-out rows of a delta layer, [cap][...]
     int maxD = 0, maxDO = 0, cring = 0, max_taps = 0;
     // OUTNORM block: kept layer results X_j [layers + 1][cap][width], the shared expert's result, its gate logits, BF16 twin of a convolved row
@@ -416,6 +417,8 @@ static int ly_launch_norm(b200_plan *p, int n, const ly::NormArgs &a) {
     return launch_k(p, false, ly::k_norm_rows<LY_NORM_THREADS>, dim3(n), dim3(LY_NORM_THREADS), sm, a);
 }
 
+const int LY_DELTA_BLOCK_ROWS = 3; // the decode step's single row (and two) stay with the token-by-token kernel: it needs no coefficients
+
 // Enqueue the forward of n rows on p->stream.  decode: the single-token step (row 0, position and token from *st).
 // with_head (decode only): final norm + classifier into p->logits.  Prefill leaves the finished residual rows in X.
 static int ly_enqueue(b200_plan *p, bool decode, int n, const StepState *st, const int *tokens, bool with_head, float *trace, int *launches) {
@@ -469,7 +472,14 @@ static int ly_enqueue(b200_plan *p, bool decode, int n, const StepState *st, con
             if ((rc = launch_k(p, false, ly::k_delta_prep, dim3(n, 2 * L.s.kv_heads + L.s.heads + 1), dim3(DELTA_PREP_THREADS), (size_t)dmax * 4, (const float *)Y.PROJ, Y.maxP, da, R.cstate,
                                Y.DLT, Y.maxD, st))) return rc;
             const dim3 rgrid(L.s.heads, (L.s.value_dim + DR_COLS - 1) / DR_COLS), rblock(DR_THREADS);
-            switch (ly::delta_reg_rows(L.s.key_dim)) {
+            const int reg = ly::delta_reg_rows(L.s.key_dim);
+            if (reg && n >= LY_DELTA_BLOCK_ROWS) {
+                if ((rc = launch_k(p, false, ly::k_delta_coef, dim3((n + 3) / 4, (L.s.heads + 3) / 4), dim3(128), (size_t)0, (const float *)Y.DLT, Y.maxD, da, n, Y.DCO))) return rc;
+                nl++;
+                auto go = [&](auto kern) { return launch_k(p, false, kern, rgrid, dim3(DB_THREADS), (size_t)0, (const float *)Y.DLT, Y.maxD, da, (const float *)Y.DCO, R.S, n, Y.DO, Y.maxDO, st); };
+                rc = reg == 1 ? go(ly::k_delta_rule_blocks<1>) : reg == 2 ? go(ly::k_delta_rule_blocks<2>) : reg == 4 ? go(ly::k_delta_rule_blocks<4>) : go(ly::k_delta_rule_blocks<8>);
+            } else
+            switch (reg) {
             case 1: rc = launch_k(p, false, ly::k_delta_rule_reg<1>, rgrid, rblock, (size_t)0, (const float *)Y.DLT, Y.maxD, da, R.S, n, Y.DO, Y.maxDO, st); break;
             case 2: rc = launch_k(p, false, ly::k_delta_rule_reg<2>, rgrid, rblock, (size_t)0, (const float *)Y.DLT, Y.maxD, da, R.S, n, Y.DO, Y.maxDO, st); break;
             case 4: rc = launch_k(p, false, ly::k_delta_rule_reg<4>, rgrid, rblock, (size_t)0, (const float *)Y.DLT, Y.maxD, da, R.S, n, Y.DO, Y.maxDO, st); break;
@@ -1038,6 +1048,10 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
     }
     if (Y.maxDO > 0 && !Y.DO && (rc = dalloc(p, &Y.DO, cap * Y.maxDO * 4))) return rc;
     if (Y.maxD > 0 && (rc = dalloc(p, &Y.DLT, cap * Y.maxD * 4))) return rc;
+    int delta_heads = 0;
+    for (const LyLayer &L : Y.layers)
+        if (L.s.mixer == B200_MIXER_GATED_DELTA && L.s.heads > delta_heads) delta_heads = L.s.heads;
+    if (delta_heads > 0 && (rc = dalloc(p, &Y.DCO, ly::delta_coef_floats((int)cap, delta_heads) * 4))) return rc;
     if (Y.maxLQ > 0 && (rc = dalloc(p, &Y.LQ16, cap * Y.maxLQ * 2))) return rc;
     if (Y.maxX > 0) { // attention + scan
         if ((rc = dalloc(p, &Y.XP, cap * Y.maxX * 4))) return rc;
