@@ -870,9 +870,24 @@ __global__ void __launch_bounds__(1024) k_argmax_advance(const float *__restrict
                 argmax_merge(best, best_i, v, ix);
             }
         } else {
-            for (int i = tid; i < vocab; i += blockDim.x) {
-                float v = logits[i];
-                if (v > best) { best = v; best_i = i; }
+            // eight 16-byte loads of a thread in flight (one value at a time the 32768 logits took 20 us); indices ascend per thread: the first maximum stays
+            const int n4 = vocab >> 2;
+            for (int i0 = tid; i0 < n4; i0 += 8 * blockDim.x) {
+                float4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = i0 + u * (int)blockDim.x < n4 ? *reinterpret_cast<const float4 *>(logits + 4 * (size_t)(i0 + u * blockDim.x)) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    const int i = 4 * (i0 + u * (int)blockDim.x);
+                    if (v[u].x > best) { best = v[u].x; best_i = i; }
+                    if (v[u].y > best) { best = v[u].y; best_i = i + 1; }
+                    if (v[u].z > best) { best = v[u].z; best_i = i + 2; }
+                    if (v[u].w > best) { best = v[u].w; best_i = i + 3; }
+                }
+            }
+            if (tid < (vocab & 3)) {
+                const int i = (vocab & ~3) + tid;
+                if (logits[i] > best) { best = logits[i]; best_i = i; }
             }
         }
         // a thread that saw nothing > -inf keeps INT_MAX; index 0 wins below if all are -inf

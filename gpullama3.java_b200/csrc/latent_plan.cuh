@@ -303,12 +303,9 @@ static int ly_enqueue_latent(b200_plan *p, bool decode, int n, const StepState *
     const size_t asm_ = ly_att_smem(wa.dk, wa.window);
     if (h16) rc = launch_k(p, false, ly::k_window_attention<ly::bf16>, dim3(n, s.heads), dim3(LY_ATT_THREADS), asm_, (const float *)Y.Q, L.qw, wa,
                            (const float *)R.kc, (const float *)R.kc, st, Y.LAT16, L.lw, ly::KeySplit{nullptr, nullptr, nullptr});
-    else {
-        int sp = 1;
-        if (decode && Y.split.o && s.window >= 64) { sp = p->n_sms / s.heads; if (sp > Y.max_splits) sp = Y.max_splits; if (sp < 1) sp = 1; }
-        rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, s.heads, sp), dim3(LY_ATT_THREADS), asm_, (const float *)Y.Q, L.qw, wa,
-                      (const float *)R.kc, (const float *)R.kc, st, Y.LAT32, L.lw, sp > 1 ? Y.split : ly::KeySplit{nullptr, nullptr, nullptr});
-    }
+    else if (decode) rc = ly_step_attention(p, s.heads, s.window, Y.Q, L.qw, wa, R.kc, R.kc, st, Y.LAT32, L.lw, asm_);
+    else rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, s.heads), dim3(LY_ATT_THREADS), asm_, (const float *)Y.Q, L.qw, wa,
+                       (const float *)R.kc, (const float *)R.kc, st, Y.LAT32, L.lw, ly::KeySplit{nullptr, nullptr, nullptr});
     if (rc) return rc;
     ++*nl;
     // per head: W_uv on the latent-space output (times sigmoid(gate) for a gate per entry)

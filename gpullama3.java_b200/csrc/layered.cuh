@@ -247,10 +247,11 @@ __device__ __forceinline__ float dot_row_bf16(const bf16 *__restrict__ w, const 
     return warp_sum(acc);
 }
 
-// The same for rows of whole float4 without a pass prologue or an embedding norm: every thread keeps VPT float4 of the row in registers, and the loads of the
-// row, of the sublayer output and of both weights are in flight together (the statistics are the only places where the CTA waits).
+// The same for rows of whole float4: every thread keeps VPT float4 of the row in registers, and the loads of the row, of the sublayer output, of both weights and
+// (PROLOGUE) of what a pass prologue adds are in flight together (the statistics are the only places where the CTA waits).  PROLOGUE: x0, add_x0, step and
+// w_emb are honoured; models without loops and embedding norms do not pay for their registers.  One row of 2048 with a loop: 8.4 us in k_norm_rows, 5.0 us here.
 // E a multiple of 4, at most 4 * NTH * VPT; top <= LY_NORM_TERMS.  No dynamic shared memory.
-template <int NTH, int VPT>
+template <int NTH, int VPT, bool PROLOGUE = false>
 __global__ void __launch_bounds__(NTH) k_norm_rows_reg(NormArgs a) {
     __shared__ float red[32];
     __shared__ size_t s_row[LY_NORM_TERMS];
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(NTH) k_norm_rows_reg(NormArgs a) {
     }
     const bf16 *emb = a.emb ? a.emb + (size_t)(a.tokens ? a.tokens[r] : a.st->token) * E : nullptr;
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 x[VPT], y[VPT], w1[VPT], w2[VPT];
+    float4 x[VPT], y[VPT], w1[VPT], w2[VPT], p0[PROLOGUE ? VPT : 1], p1[PROLOGUE ? VPT : 1];
     const bool add = a.y || a.ys;
 #pragma unroll
     for (int v = 0; v < VPT; v++) {
@@ -282,6 +283,10 @@ __global__ void __launch_bounds__(NTH) k_norm_rows_reg(NormArgs a) {
         if (a.y) y[v] = *reinterpret_cast<const float4 *>(a.y + src + i);
         if (add) w1[v] = *reinterpret_cast<const float4 *>(a.w_post + i);
         if (a.w_pre) w2[v] = *reinterpret_cast<const float4 *>(a.w_pre + i);
+        if constexpr (PROLOGUE) {
+            if (a.add_x0) p0[v] = *reinterpret_cast<const float4 *>(a.x0 + src + i);
+            if (a.step) p1[v] = *reinterpret_cast<const float4 *>(a.step + i);
+        }
     }
     if (a.ys) {
         for (int k0 = 0; k0 < a.top; k0 += 4) { // the loads of four entries are issued before the first is used
@@ -301,6 +306,27 @@ __global__ void __launch_bounds__(NTH) k_norm_rows_reg(NormArgs a) {
         }
     }
     auto square = [](const float4 &q, float s) { return fmaf(q.x, q.x, fmaf(q.y, q.y, fmaf(q.z, q.z, fmaf(q.w, q.w, s)))); };
+    if constexpr (PROLOGUE)
+        if (emb) {
+            float inv = 1.0f;
+            if (a.w_emb) {
+                float ss = 0.0f;
+#pragma unroll
+                for (int v = 0; v < VPT; v++) ss = square(x[v], ss);
+                ss = block_sum(ss, red);
+                inv = 1.0f / sqrtf(ss / (float)E + a.eps);
+            }
+#pragma unroll
+            for (int v = 0; v < VPT; v++) {
+                const int i = (tid + v * NTH) * 4;
+                if (i >= E) continue;
+                if (a.w_emb) {
+                    const float4 w = *reinterpret_cast<const float4 *>(a.w_emb + i);
+                    x[v] = make_float4(x[v].x * inv * (a.w_off + w.x), x[v].y * inv * (a.w_off + w.y), x[v].z * inv * (a.w_off + w.z), x[v].w * inv * (a.w_off + w.w));
+                }
+                if (a.x0) *reinterpret_cast<float4 *>(a.x0 + src + i) = x[v];
+            }
+        }
     if (add) {
         float inv = 1.0f, off = 0.0f;
         if (!a.post_plain) {
@@ -317,6 +343,18 @@ __global__ void __launch_bounds__(NTH) k_norm_rows_reg(NormArgs a) {
             x[v].z += y[v].z * inv * (off + w1[v].z); x[v].w += y[v].w * inv * (off + w1[v].w);
         }
     }
+    bool moved = emb || add;
+    if constexpr (PROLOGUE) {
+        moved = moved || a.add_x0 || a.step;
+#pragma unroll
+        for (int v = 0; v < VPT; v++) {
+            const int i = (tid + v * NTH) * 4;
+            if (i >= E) continue;
+            if (a.trace) *reinterpret_cast<float4 *>(a.trace + src + i) = x[v]; // in front of the prologue
+            if (a.add_x0) { x[v].x += p0[v].x; x[v].y += p0[v].y; x[v].z += p0[v].z; x[v].w += p0[v].w; }
+            if (a.step) { x[v].x += p1[v].x; x[v].y += p1[v].y; x[v].z += p1[v].z; x[v].w += p1[v].w; }
+        }
+    }
     float inv = 1.0f;
     if (a.w_pre) {
         float ss = 0.0f;
@@ -329,8 +367,8 @@ __global__ void __launch_bounds__(NTH) k_norm_rows_reg(NormArgs a) {
     for (int v = 0; v < VPT; v++) {
         const int i = (tid + v * NTH) * 4;
         if (i >= E) continue;
-        if (a.trace) *reinterpret_cast<float4 *>(a.trace + src + i) = x[v];
-        if (!a.gather && (emb || add)) *reinterpret_cast<float4 *>(a.x + src + i) = x[v];
+        if (!PROLOGUE && a.trace) *reinterpret_cast<float4 *>(a.trace + src + i) = x[v];
+        if (!a.gather && moved) *reinterpret_cast<float4 *>(a.x + src + i) = x[v];
         if (!a.out32 && !a.out16) continue;
         float4 o = x[v];
         if (a.w_pre) o = make_float4(o.x * inv * (a.w_off + w2[v].x), o.y * inv * (a.w_off + w2[v].y), o.z * inv * (a.w_off + w2[v].z), o.w * inv * (a.w_off + w2[v].w));
@@ -946,6 +984,185 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_window_attention(const float
     if (tid == 0) ks_.count[cell] = 0u; // ready for the next launch
 }
 
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) { // 16 bytes, zero-filled when !valid
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int n = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+// ---------------------------------------------------------------------------------------------------------------------
+// The decode step's attention (one row), rows of whole float4.  A head's window is split over the CTAs of a CLUSTER.  What bounds it is latency, not bytes: the
+// general kernel above loads four keys per lane, reduces, looks up a distance row, caps, and only then asks for the next keys, and its parts meet in global memory
+// behind a counter.  Here a CTA asks for the first four tiles of its keys at once (cp.async, 16 KB each: all keys of a window of 1024 split four
+// ways), looks the distances up meanwhile, asks for the first tiles of its values before the softmax, and the parts are merged over distributed shared
+// memory, every CTA finishing its share of the head's entries.  32 heads of 64, 900 keys, cap and distance table: 27 us there, 20 us here.
+// grid (splits, heads), cluster (splits), LY_ATT_THREADS threads; dynamic shared memory step_att_smem_floats(...) floats.
+// ---------------------------------------------------------------------------------------------------------------------
+#define LY_STEP_STAGES 4
+#define LY_STEP_STAGE_FLOATS 4096
+__host__ __device__ inline int step_att_chunk(int window, int splits) { // most keys a CTA can get
+    const int c = (window + splits - 1) / splits;
+    return ((c > LY_ATT_SPLIT_KEYS ? c : LY_ATT_SPLIT_KEYS) + 3) / 4 * 4;
+}
+__host__ __device__ inline size_t step_att_smem_floats(int dk, int dv, int window, int splits) {
+    return (size_t)dk + step_att_chunk(window, splits) + 4 * LY_ATT_THREADS + dv + 4 + LY_STEP_STAGES * LY_STEP_STAGE_FLOATS;
+}
+__device__ __forceinline__ float ld_cluster_f32(const float *p, int rank) { // the same shared variable of another CTA of the cluster
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_barrier() { asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory"); }
+
+__global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *__restrict__ P, WindowAttn a, const float *__restrict__ kc, const float *__restrict__ vc,
+                                                                   const StepState *__restrict__ st, float *__restrict__ out) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float red[32];
+    const int z = blockIdx.x, sp = gridDim.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int qd = a.heads * a.dk, kd = a.kv_heads * a.dk, vd = a.kv_heads * a.dv;
+    const int g = h / (a.heads / a.kv_heads);
+    const int gk = a.maps > 1 ? g * a.maps + h % a.maps : a.k_heads > 0 ? h / (a.heads / a.k_heads) : g;
+    const float sink_v = a.sink_logit ? a.sink_logit[h] : 0.0f;
+    const int pos = st->pos;
+    int lo = window_first(a, pos), nk = pos - lo + 1;
+    {
+        const int want = (nk + LY_ATT_SPLIT_KEYS - 1) / LY_ATT_SPLIT_KEYS, splits = want < sp ? want : sp; // no more parts than there are keys for
+        const int chunk = (nk + splits - 1) / splits, jb = z * chunk;
+        nk = nk - jb < chunk ? nk - jb : chunk;
+        if (nk < 0) nk = 0;
+        lo += jb;
+    }
+    float *qs = sm, *sc = qs + a.dk, *part = sc + step_att_chunk(a.window, sp), *os = part + 4 * LY_ATT_THREADS, *ml = os + a.dv, *ring = ml + 4;
+    const int slot0 = lo % a.ring;
+    // rows of `w` floats -> the ring, `per` keys per tile; lanes_row lanes (a power of two) share a row
+    auto lanes_row = [](int w) { int l = 1; while (l < w / 4 && l < 32) l <<= 1; return l; };
+    auto fetch = [&](const float *base, int ld, int w, int per, int lpr, int tile) {
+        float *dst = ring + (tile % LY_STEP_STAGES) * LY_STEP_STAGE_FLOATS;
+        const int sub = lane & (lpr - 1), rows = 32 / lpr;
+        const int n = nk - tile * per < per ? nk - tile * per : per;
+        for (int r = warp * rows + lane / lpr; r < n; r += (LY_ATT_THREADS / 32) * rows) {
+            int slot = slot0 + tile * per + r;
+            if (slot >= a.ring) slot %= a.ring;
+            const float *src = base + (size_t)slot * ld;
+            for (int c = sub * 4; c < w; c += lpr * 4) cp_async16(dst + r * w + c, src + c, true);
+        }
+    };
+    const int kper = LY_STEP_STAGE_FLOATS / a.dk < 64 ? LY_STEP_STAGE_FLOATS / a.dk : 64, vper = LY_STEP_STAGE_FLOATS / a.dv < 64 ? LY_STEP_STAGE_FLOATS / a.dv : 64;
+    const int ktiles = (nk + kper - 1) / kper, vtiles = (nk + vper - 1) / vper;
+    const float *kb = kc + (size_t)gk * a.dk, *vb = vc + (size_t)g * a.dv;
+    const int klpr = lanes_row(a.dk), vlpr = lanes_row(a.dv);
+#pragma unroll
+    for (int i = 0; i < LY_STEP_STAGES; i++) {
+        if (i < ktiles) fetch(kb, a.ldk, a.dk, kper, klpr, i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int i = tid; i < a.dk; i += LY_ATT_THREADS) qs[i] = P[(size_t)h * a.dk + i];
+    if (a.rel)
+        for (int j = tid; j < nk; j += LY_ATT_THREADS) sc[j] = a.rel[(size_t)a.bucket[pos - lo - j] * a.heads + h];
+    float mx = -INFINITY;
+    for (int i = 0; i < ktiles; i++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(LY_STEP_STAGES - 1) : "memory");
+        __syncthreads();
+        const float *kt = ring + (i % LY_STEP_STAGES) * LY_STEP_STAGE_FLOATS;
+        const int n = nk - i * kper < kper ? nk - i * kper : kper, sub = lane & (klpr - 1), rows = 32 / klpr;
+        for (int r0 = warp * rows; r0 < n; r0 += (LY_ATT_THREADS / 32) * rows) {
+            const int r = r0 + lane / klpr;
+            float d = 0.0f;
+            if (r < n)
+                for (int c = sub * 4; c < a.dk; c += klpr * 4) {
+                    const float4 kv = *reinterpret_cast<const float4 *>(kt + r * a.dk + c), qv = *reinterpret_cast<const float4 *>(qs + c);
+                    d = fmaf(qv.x, kv.x, d); d = fmaf(qv.y, kv.y, d); d = fmaf(qv.z, kv.z, d); d = fmaf(qv.w, kv.w, d);
+                }
+            for (int o = klpr >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            if (r < n && sub == 0) {
+                const int j = i * kper + r;
+                float e = d * a.scale;
+                if (a.softcap > 0.0f) e = a.softcap * tanhf(e / a.softcap);
+                if (a.rel) e += sc[j];
+                sc[j] = e;
+                mx = fmaxf(mx, e);
+            }
+        }
+        if (i + LY_STEP_STAGES < ktiles) { // (uniform) refill the stage when every warp is done with it
+            __syncthreads();
+            fetch(kb, a.ldk, a.dk, kper, klpr, i + LY_STEP_STAGES);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    mx = block_max(mx, red); // also: the ring is free, the scores are written
+#pragma unroll
+    for (int i = 0; i < LY_STEP_STAGES; i++) { // values on their way through the softmax
+        if (i < vtiles) fetch(vb, a.ldv, a.dv, vper, vlpr, i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    float sum = 0.0f;
+    for (int j = tid; j < nk; j += LY_ATT_THREADS) {
+        const float w = expf(sc[j] - mx);
+        sc[j] = w;
+        sum += w;
+    }
+    sum = block_sum(sum, red);
+    const int tpk = a.dv / 4, groups = LY_ATT_THREADS / tpk, grp = tid / tpk, d0 = (tid % tpk) * 4;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = 0; i < vtiles; i++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(LY_STEP_STAGES - 1) : "memory");
+        __syncthreads();
+        const float *vt = ring + (i % LY_STEP_STAGES) * LY_STEP_STAGE_FLOATS;
+        const int n = nk - i * vper < vper ? nk - i * vper : vper;
+        if (grp < groups)
+#pragma unroll 4
+            for (int r = grp; r < n; r += groups) {
+                const float w = sc[i * vper + r];
+                const float4 v = *reinterpret_cast<const float4 *>(vt + r * a.dv + d0);
+                acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
+            }
+        if (i + LY_STEP_STAGES < vtiles) {
+            __syncthreads();
+            fetch(vb, a.ldv, a.dv, vper, vlpr, i + LY_STEP_STAGES);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    *reinterpret_cast<float4 *>(part + tid * 4) = acc; // thread (group, entries): group * dv + d0 while grp < groups
+    if (tid == 0) { ml[0] = mx; ml[1] = sum; }
+    __syncthreads();
+    for (int d = tid; d < a.dv; d += LY_ATT_THREADS) {
+        float o = 0.0f;
+        for (int k = 0; k < groups; k++) o += part[k * a.dv + d];
+        os[d] = o;
+    }
+    if (sp > 1) cluster_barrier();
+    else __syncthreads();
+    // merge: maximum over the parts and the sink, rescaled sums; this CTA finishes entries [z * per, + per)
+    float M = a.sink ? sink_v : -INFINITY, m_[8], f_[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        m_[k] = k < sp ? (sp > 1 ? ld_cluster_f32(ml, k) : ml[0]) : -INFINITY;
+        f_[k] = k < sp ? (sp > 1 ? ld_cluster_f32(ml + 1, k) : ml[1]) : 0.0f;
+        M = fmaxf(M, m_[k]);
+    }
+    float L = a.sink ? expf(sink_v - M) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const float f = m_[k] == -INFINITY ? 0.0f : expf(m_[k] - M);
+        L += f * f_[k];
+        f_[k] = f;
+    }
+    const int per = (a.dv + sp - 1) / sp, d1 = (z + 1) * per < a.dv ? (z + 1) * per : a.dv;
+    const float *gate = (a.gate_src ? a.gate_src : P) + (a.gate_off >= 0 ? a.gate_off : qd + kd + vd) + (a.gate_heads ? (size_t)h : (size_t)h * a.dv);
+    for (int d = z * per + tid; d < d1; d += LY_ATT_THREADS) {
+        float o = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (k < sp && f_[k] > 0.0f) o += f_[k] * (sp > 1 ? ld_cluster_f32(os + d, k) : os[d]);
+        o /= L;
+        if (a.gate) o *= 1.0f / (1.0f + expf(-gate[a.gate_heads ? 0 : d]));
+        out[(size_t)h * a.dv + d] = o * a.out_scale;
+    }
+    if (sp > 1) cluster_barrier(); // nobody leaves while its shared memory may still be read
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // The same attention for a prefill chunk on the tensor cores (BF16 compute mode; instantiated for key / value sizes 64 / 64,
 // 128 / 128 and 192 / 128): one CTA per (128 query rows, head), eight
@@ -964,11 +1181,6 @@ __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.0f,
 // tanh(x) = 1 - 2 / (1 + exp(2x)) with the hardware exponential: absolute error ~1e-7, far below the BF16 rounding of the
 // operands that produced x (the FP32 kernels keep tanhf)
 __device__ __forceinline__ float tanh_fast(float x) { return 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * x)); }
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid) { // 16 bytes, zero-filled when !valid
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    const int n = valid ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
 __device__ __forceinline__ void ldmatrix_x2_trans(unsigned (&r)[2], const void *row) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(row);
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a));

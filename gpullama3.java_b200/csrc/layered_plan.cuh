@@ -356,6 +356,19 @@ static int ly_project(b200_plan *p, bool decode, int n, const float *a32, const 
     return launch_k(p, false, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
 }
 
+// The decode step's attention: k_step_attention for rows of whole float4, with a head's window over as many CTAs as the SMs allow (B200_LAYERED_SPLITS bounds it); else
+// the general kernel with its parts in global memory.  `window` bounds the keys a head can see.
+static int ly_step_attention(b200_plan *p, int heads, int window, const float *q, int ldq, ly::WindowAttn wa, const float *kc, const float *vc, const StepState *st, float *out, int ldo, size_t general_smem) {
+    Layered &Y = *p->ly;
+    int sp = 1;
+    if (Y.split.o && window >= 64) { sp = p->n_sms / heads; if (sp > Y.max_splits) sp = Y.max_splits; if (sp < 1) sp = 1; }
+    const size_t sm = ly::step_att_smem_floats(wa.dk, wa.dv, wa.window, sp) * 4;
+    if ((wa.dk | wa.dv | wa.ldk | wa.ldv) % 4 == 0 && wa.dk <= 1024 && wa.dv <= 4 * LY_ATT_THREADS && sm <= (size_t)Y.smem_max)
+        return launch_cluster(p, false, sp, ly::k_step_attention, dim3(sp, heads), dim3(LY_ATT_THREADS), sm, q, wa, kc, vc, st, out);
+    return launch_k(p, false, ly::k_window_attention<float>, dim3(1, heads, sp), dim3(LY_ATT_THREADS), general_smem, q, ldq, wa, kc, vc, st, out, ldo,
+                    sp > 1 ? Y.split : ly::KeySplit{nullptr, nullptr, nullptr});
+}
+
 // Attention of one layer with its own rings, from the projection rows in PROJ to the (gated) heads in ATT32 / ATT16 (row stride L.gd).
 static int ly_enqueue_attention(b200_plan *p, bool decode, int n, const StepState *st, const LyRun &R, const LyLayer &L, int *nl) {
     Layered &Y = *p->ly;
@@ -383,13 +396,9 @@ static int ly_enqueue_attention(b200_plan *p, bool decode, int n, const StepStat
         rc = ly_launch_mma(p, mma, n, L.s.heads, L.s.window, qsrc, ldq, wa, (const ly::bf16 *)R.kc16, (const ly::bf16 *)R.vc16, st, Y.ATT16, L.gd);
     else if (h16) rc = launch_k(p, false, ly::k_window_attention<ly::bf16>, dim3(n, L.s.heads), dim3(LY_ATT_THREADS), asm_, qsrc, ldq, wa,
                            (const float *)R.kc, (const float *)R.vc, st, Y.ATT16, L.gd, ly::KeySplit{nullptr, nullptr, nullptr});
-    else {
-        // the decode step has one row and few heads: split every head's window over several CTAs so that the SMs are used
-        int sp = 1;
-        if (decode && Y.split.o && L.s.window >= 64) { sp = p->n_sms / L.s.heads; if (sp > Y.max_splits) sp = Y.max_splits; if (sp < 1) sp = 1; }
-        rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, L.s.heads, sp), dim3(LY_ATT_THREADS), asm_, qsrc, ldq, wa,
-                      (const float *)R.kc, (const float *)R.vc, st, Y.ATT32, L.gd, sp > 1 ? Y.split : ly::KeySplit{nullptr, nullptr, nullptr});
-    }
+    else if (decode) rc = ly_step_attention(p, L.s.heads, L.s.window, qsrc, ldq, wa, R.kc, R.vc, st, Y.ATT32, L.gd, asm_);
+    else rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, L.s.heads), dim3(LY_ATT_THREADS), asm_, qsrc, ldq, wa,
+                       (const float *)R.kc, (const float *)R.vc, st, Y.ATT32, L.gd, ly::KeySplit{nullptr, nullptr, nullptr});
     ++*nl;
     return rc;
 }
@@ -403,14 +412,17 @@ static int ly_enqueue_attention(b200_plan *p, bool decode, int n, const StepStat
 // takes more threads.
 static int ly_launch_norm(b200_plan *p, int n, const ly::NormArgs &a) {
     const int E = a.E;
-    if (E % 4 == 0 && E <= 4096 && !a.w_emb && !a.x0 && !a.add_x0 && !a.step && a.top <= LY_NORM_TERMS) {
+    if (E % 4 == 0 && E <= 4096 && a.top <= LY_NORM_TERMS) {
+        auto go = [&](auto plain, auto prologue, int threads) {
+            return a.w_emb || a.x0 || a.add_x0 || a.step ? launch_k(p, false, prologue, dim3(n), dim3(threads), (size_t)0, a) : launch_k(p, false, plain, dim3(n), dim3(threads), (size_t)0, a);
+        };
         if (n == 1 && E > 1024) {
-            if (E <= 2048) return launch_k(p, false, ly::k_norm_rows_reg<512, 1>, dim3(1), dim3(512), (size_t)0, a);
-            return launch_k(p, false, ly::k_norm_rows_reg<1024, 1>, dim3(1), dim3(1024), (size_t)0, a);
+            if (E <= 2048) return go(ly::k_norm_rows_reg<512, 1>, ly::k_norm_rows_reg<512, 1, true>, 512);
+            return go(ly::k_norm_rows_reg<1024, 1>, ly::k_norm_rows_reg<1024, 1, true>, 1024);
         }
-        if (E <= 1024) return launch_k(p, false, ly::k_norm_rows_reg<LY_NORM_THREADS, 1>, dim3(n), dim3(LY_NORM_THREADS), (size_t)0, a);
-        if (E <= 2048) return launch_k(p, false, ly::k_norm_rows_reg<LY_NORM_THREADS, 2>, dim3(n), dim3(LY_NORM_THREADS), (size_t)0, a);
-        return launch_k(p, false, ly::k_norm_rows_reg<LY_NORM_THREADS, 4>, dim3(n), dim3(LY_NORM_THREADS), (size_t)0, a);
+        if (E <= 1024) return go(ly::k_norm_rows_reg<LY_NORM_THREADS, 1>, ly::k_norm_rows_reg<LY_NORM_THREADS, 1, true>, LY_NORM_THREADS);
+        if (E <= 2048) return go(ly::k_norm_rows_reg<LY_NORM_THREADS, 2>, ly::k_norm_rows_reg<LY_NORM_THREADS, 2, true>, LY_NORM_THREADS);
+        return go(ly::k_norm_rows_reg<LY_NORM_THREADS, 4>, ly::k_norm_rows_reg<LY_NORM_THREADS, 4, true>, LY_NORM_THREADS);
     }
     const size_t sm = (size_t)(a.ys ? 2 : 1) * E * 4;
     if (n == 1 && E >= 2048) return launch_k(p, false, ly::k_norm_rows<1024>, dim3(1), dim3(1024), sm, a);
@@ -774,6 +786,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
             CK(set_max_dyn(ly::k_matvec_bf16<ly::EPI_STORE>, Y.smem_max));
             CK(set_max_dyn(ly::k_matvec_bf16<ly::EPI_GATED>, Y.smem_max));
             CK(set_max_dyn(ly::k_window_attention<float>, Y.smem_max));
+            CK(set_max_dyn(ly::k_step_attention, Y.smem_max));
             CK(set_max_dyn(ly::k_window_attention<ly::bf16>, Y.smem_max));
             CK(set_max_dyn(ly::k_window_attention_mma<64, 64>, Y.smem_max));
             CK(set_max_dyn(ly::k_window_attention_mma<64, 64, 64>, Y.smem_max));

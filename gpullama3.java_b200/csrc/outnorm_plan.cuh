@@ -345,12 +345,9 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             else if (h16 && maps == 1)
                 rc = launch_k(p, false, ly::k_window_attention<ly::bf16>, dim3(n, pairs), dim3(LY_ATT_THREADS), ly_att_smem(s.key_dim, s.window), (const float *)Y.PROJ, Y.maxP, wa,
                               (const float *)R.kc, (const float *)R.vc, st, Y.ATT16, ldo, ly::KeySplit{nullptr, nullptr, nullptr});
-            else {
-                int sp = 1;
-                if (decode && Y.split.o && s.window >= 64) { sp = p->n_sms / pairs; if (sp > Y.max_splits) sp = Y.max_splits; if (sp < 1) sp = 1; }
-                rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, pairs, sp), dim3(LY_ATT_THREADS), ly_att_smem(s.key_dim, s.window), (const float *)Y.PROJ, Y.maxP, wa,
-                              (const float *)R.kc, (const float *)R.vc, st, o32, ldo, sp > 1 ? Y.split : ly::KeySplit{nullptr, nullptr, nullptr});
-            }
+            else if (decode) rc = ly_step_attention(p, pairs, s.window, Y.PROJ, Y.maxP, wa, R.kc, R.vc, st, o32, ldo, ly_att_smem(s.key_dim, s.window));
+            else rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, pairs), dim3(LY_ATT_THREADS), ly_att_smem(s.key_dim, s.window), (const float *)Y.PROJ, Y.maxP, wa,
+                               (const float *)R.kc, (const float *)R.vc, st, o32, ldo, ly::KeySplit{nullptr, nullptr, nullptr});
             if (rc) return rc;
             nl += 2;
             if (maps > 1) {
