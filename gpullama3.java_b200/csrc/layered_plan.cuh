@@ -48,7 +48,8 @@ struct LyLayer {
     bool expand = false;                        // BF16 prefill through expanded keys / values and the tensor-core attention kernel
     float *cnorm = nullptr;
     ly::bf16 *w_uq = nullptr;                   // [heads * key_dim][q_rank]: queries out of the normed query latent (qnorm)
-    CUtensorMap m_uq, m_cq, m_qf_c;
+    pg::BMap m_uq;
+    CUtensorMap m_cq, m_qf_c;
     bool tc_uq = false;
     float *router_b = nullptr;
     // matrix memory (B200_MIXER_MLSTM): gate biases; the fused projection is q | k | v | g | i | f, onorm the read-out weight [heads * value_dim]
@@ -59,8 +60,10 @@ struct LyLayer {
     float *ln1_b = nullptr, *ln2_b = nullptr;
     ly::bf16 *w_router = nullptr;
     // TMA descriptors of the tensor-core prefill (BF16 compute mode, shapes the tcgen05 GEMM tiles cover); *_ok = usable
-    CUtensorMap m_proj, m_o, m_gate, m_up, m_down, m_att, m_h;
-    CUtensorMap m_xk_b, m_xv_b, m_xk_c, m_xv_c; // key / value expansion of the BF16 prefill on the tcgen05 GEMM: W_uk, W_uv, FP32 results
+    pg::BMap m_proj, m_o, m_gate, m_up, m_down;
+    CUtensorMap m_att, m_h;
+    pg::BMap m_xk_b, m_xv_b;
+    CUtensorMap m_xk_c, m_xv_c; // key / value expansion of the BF16 prefill on the tcgen05 GEMM: W_uk, W_uv, FP32 results
     bool tc_expand = false;
     CUtensorMap m_moe_gate, m_moe_up, m_moe_down, m_moe_h; // mixture of experts on the tcgen05 GEMM: all experts' matrices in one map each
     bool tc_moe = false;
@@ -83,7 +86,8 @@ struct LyLayer {
     float *gate_bias = nullptr, *lam = nullptr, *x_bias = nullptr, *y_bias = nullptr, *conv_b = nullptr, *ssd_d = nullptr;
     float *correction = nullptr;
     ly::bf16 *w_sgu = nullptr, *w_sdown = nullptr;
-    CUtensorMap m_sgate, m_sup, m_sdown, m_sh;
+    pg::BMap m_sgate, m_sup, m_sdown;
+    CUtensorMap m_sh;
     bool tc_sgu = false, tc_sdown = false;
     // lightning: decays per head.  Attention + scan: ad = the attention's output columns (gd = ad + scan_inner), x_off = first scan column of a projection
     // row ([x | z]), W_x with nx rows (nxp with padding), W_dt, decay exponents; conv_w, conv_b, dt_bias, ssd_d as above
@@ -91,12 +95,13 @@ struct LyLayer {
     bool chunkwise = false; // lightning: BF16 prefill on the tensor cores
     int ad = 0, x_off = 0, nx = 0, nxp = 0;
     ly::bf16 *w_x = nullptr, *w_dt = nullptr;
-    CUtensorMap m_wx, m_u, m_wdt, m_dt16;
+    pg::BMap m_wx, m_wdt;
+    CUtensorMap m_u, m_dt16;
     bool tc_wx = false, tc_wdt = false;
     // per-layer token input
     ly::bf16 *w_sgate = nullptr, *w_sproj = nullptr;
     float *side_norm = nullptr;
-    CUtensorMap m_tsg, m_tsp;
+    pg::BMap m_tsg, m_tsp;
     bool tc_side = false;
 };
 struct LyRun {
@@ -132,7 +137,8 @@ struct Layered {
     int cap_pad = 1; // rows of the activation buffers: cap, padded to whole 256-row GEMM tiles in BF16 mode
     bool tc = false, tc_head = false;
     bool att_mma = true; // BF16 prefill attention on the tensor cores for key/value sizes 64 and 128 (B200_LAYERED_ATT=simt: the FP32 kernel)
-    CUtensorMap m_a, m_head, m_proj_c, m_y_c, m_log_c;
+    pg::BMap m_head;
+    CUtensorMap m_a, m_proj_c, m_y_c, m_log_c;
     // parallel block / latent attention / mixture of experts
     float *final_norm_b = nullptr;
     float *A2_32 = nullptr, *Q = nullptr, *LAT32 = nullptr, *YS = nullptr, *moe_wts = nullptr, *ZR = nullptr;
@@ -187,7 +193,8 @@ struct Layered {
 
 // What ly_project needs to take the tcgen05 route: operand and result descriptors (nullptr = CUDA-core / mma.sync kernels).
 struct LyTc {
-    const CUtensorMap *a = nullptr, *b = nullptr, *b2 = nullptr, *c = nullptr;
+    const pg::BMap *b = nullptr, *b2 = nullptr;
+    const CUtensorMap *a = nullptr, *c = nullptr;
 };
 
 static int ly_vec_f32(b200_plan *p, const b200_tensor *tensors, int nt, const std::string &name, int64_t n, float **dst, bool required = true) {

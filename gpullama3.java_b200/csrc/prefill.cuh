@@ -25,8 +25,9 @@
 #include <vector>
 
 struct PrefillLayerMaps {
-    CUtensorMap qkv, wo, w1, w3, w2; // weight boxes of 128 rows (64 for w1 / w3: the single-CTA gate/up tile is 64 + 64)
-    CUtensorMap w1p, w3p;            // 128-row boxes for the CTA-pair gate/up tile (128 + 128)
+    pg::BMap qkv, wo, w2;
+    CUtensorMap w1, w3; // weight boxes of 128 rows (64 for w1 / w3: the single-CTA gate/up tile is 64 + 64)
+    pg::BMap w1p, w3p;            // 128-row boxes for the CTA-pair gate/up tile (128 + 128)
 };
 
 struct PrefillCtx {

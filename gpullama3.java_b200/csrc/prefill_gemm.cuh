@@ -490,10 +490,25 @@ template <int BN, int STAGES> constexpr size_t smem_bytes_2cta_persist() {
     return (size_t)STAGES * (BM * BK * 2 + (BN / 2) * BK * 2) + 2 * (BM * 32 * 4) + (2 * STAGES + 4) * 8 + 16 + 1024;
 }
 
+// How the columns of one M pair are cut: `wide` tiles of BN columns, then `narrow` tiles of `width` (a multiple of 64) columns.
+// A GEMM of a few rounds over the clusters otherwise ends with a round that is mostly empty: 224 tiles on 74 clusters take four rounds for three of
+// work.  So the rounds that fill every cluster run wide tiles, and a small rest is spread over the clusters in tiles of 64 or 128 columns.  A rest that needs wider
+// tiles than that stays wide: a narrow tile loads as much of A as a wide one, in a round that the loads bound (8192 gated columns as 192-wide tiles: 33.5 us
+// against 31.6).  Measured at 512 rows: 14336 gated columns of K = 4096 113 -> 103 us, 10240 columns 51.4 -> 49.2 us.
+// Narrow tiles fetch B through maps of 32-row boxes.
+struct TileCut { int wide, narrow, width; };
+inline TileCut cut_tiles(int m_pairs, int n_cols, int bn, int clusters) { // n_cols: accumulator columns (gate/up: both), a multiple of bn
+    const int tiles = n_cols / bn, wide = clusters * (m_pairs * tiles / clusters) / m_pairs, left = n_cols - wide * bn; // wide: the tiles of whole rounds
+    for (int w = 64; wide > 0 && left > 0 && w <= 128; w += 64)
+        if ((left + w - 1) / w * m_pairs <= clusters) return TileCut{wide, (left + w - 1) / w, w};
+    return TileCut{tiles, 0, bn};
+}
+
 template <int MODE, int BN, int STAGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
     k_gemm_f16_2cta_persist(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const __grid_constant__ CUtensorMap tma_b2,
-                            const __grid_constant__ CUtensorMap tma_c, void *__restrict__ Cv, int ldc, int m_valid, int K, int m_pairs, int n_tiles, int splits, uint32_t flavor) {
+                            const __grid_constant__ CUtensorMap tma_bn, const __grid_constant__ CUtensorMap tma_b2n, const __grid_constant__ CUtensorMap tma_c,
+                            void *__restrict__ Cv, int ldc, int m_valid, int K, int m_pairs, int n_cols, TileCut cut, int splits, uint32_t flavor) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN / 2) * BK * 2, CST_BYTES = BM * 32 * 4;
@@ -521,34 +536,43 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
     // split-K (GEMM_RESID only: every split reduce-adds its partial product): a work item is (pair tile, k-range); items of one tile are
     // adjacent in the walk so the B tile of neighbouring clusters differs only in k
     const int nk_all = (K + BK - 1) / BK, nk_split = (nk_all + splits - 1) / splits;
-    const int n_clusters = (int)(gridDim.x >> 1), cid = (int)(blockIdx.x >> 1), total = m_pairs * n_tiles * splits;
+    const int n_clusters = (int)(gridDim.x >> 1), cid = (int)(blockIdx.x >> 1), total = m_pairs * (cut.wide + cut.narrow) * splits;
+    auto tile_cols = [&](int nt, int &c0, int &width) { // first accumulator column and width of column tile nt
+        c0 = nt < cut.wide ? nt * BN : cut.wide * BN + (nt - cut.wide) * cut.width;
+        width = nt < cut.wide ? BN : min(cut.width, n_cols - c0);
+    };
 
     if (warp == 0 && lane == 0) {
         // ===== TMA producer (both CTAs) =====
-        const CUtensorMap *bmap = (MODE == GEMM_GATEUP && rank == 1) ? &tma_b2 : &tma_b;
+        const CUtensorMap *bmap = (MODE == GEMM_GATEUP && rank == 1) ? &tma_b2 : &tma_b, *nmap = (MODE == GEMM_GATEUP && rank == 1) ? &tma_b2n : &tma_bn;
         int it = 0; // running k-block counter across tiles: the ring never drains between tiles
         for (int t = cid; t < total; t += n_clusters) {
             const int ks = t % splits, tt = t / splits;
             const int mp = tt % m_pairs, nt = tt / m_pairs;
             const int m0 = mp * 2 * BM + (int)rank * BM;
-            const int n0 = nt * (MODE == GEMM_GATEUP ? BN / 2 : BN);
-            const int brow = MODE == GEMM_GATEUP ? n0 : n0 + (int)rank * (BN / 2);
+            int c0, width;
+            tile_cols(nt, c0, width);
+            const int brow = MODE == GEMM_GATEUP ? c0 / 2 : c0 + (int)rank * (width / 2), bbytes = (width / 2) * BK * 2;
             const int kb0 = ks * nk_split, nk = min(nk_split, nk_all - kb0);
             for (int kb = 0; kb < nk; kb++, it++) {
                 const int st = it % STAGES;
                 mbar_wait(empty0 + 8 * st, ((it / STAGES) & 1) ^ 1);
-                if (rank == 0) mbar_expect_tx(full0 + 8 * st, 2 * (A_BYTES + B_BYTES));
+                if (rank == 0) mbar_expect_tx(full0 + 8 * st, 2 * (A_BYTES + bbytes));
                 tma_load_2d_2sm(s32(sA + st * A_BYTES), &tma_a, (kb0 + kb) * BK, m0, full0 + 8 * st);
-                tma_load_2d_2sm(s32(sB + st * B_BYTES), bmap, (kb0 + kb) * BK, brow, full0 + 8 * st);
+                if (width == BN) tma_load_2d_2sm(s32(sB + st * B_BYTES), bmap, (kb0 + kb) * BK, brow, full0 + 8 * st);
+                else
+                    for (int r = 0; r < width / 2; r += 32) tma_load_2d_2sm(s32(sB + st * B_BYTES + r * BK * 2), nmap, (kb0 + kb) * BK, brow + r, full0 + 8 * st);
             }
         }
     } else if (warp == 1 && lane == 0 && rank == 0) {
         // ===== MMA issuer (leader): accumulator buffer i & 1 =====
-        const uint32_t idesc = umma_idesc_f16(2 * BM, BN) | ((flavor & FLAVOR_BF16) ? UMMA_IDESC_AB_BF16 : 0u);
         int it = 0, i = 0;
         for (int t = cid; t < total; t += n_clusters, i++) {
             const int buf = i & 1;
             const int kb0 = (t % splits) * nk_split, nk = min(nk_split, nk_all - kb0);
+            int c0, width;
+            tile_cols(t / splits / m_pairs, c0, width);
+            const uint32_t idesc = umma_idesc_f16(2 * BM, width) | ((flavor & FLAVOR_BF16) ? UMMA_IDESC_AB_BF16 : 0u);
             mbar_wait(tempty0 + 8 * buf, ((i >> 1) & 1) ^ 1); // both CTAs' epilogues have drained this buffer (first two uses pass at once)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int kb = 0; kb < nk; kb++, it++) {
@@ -571,7 +595,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
             const int tt = t / splits;
             const int mp = tt % m_pairs, nt = tt / m_pairs;
             const int m0 = mp * 2 * BM + (int)rank * BM;
-            const int n0 = nt * (MODE == GEMM_GATEUP ? BN / 2 : BN);
+            int col0, width;
+            tile_cols(nt, col0, width);
+            const int n0 = MODE == GEMM_GATEUP ? col0 / 2 : col0;
             const int row = m0 + q * 32 + lane;
             mbar_wait(tfull0 + 8 * buf, (i >> 1) & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -579,12 +605,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
             if (MODE == GEMM_GATEUP) {
                 __half *C = reinterpret_cast<__half *>(Cv);
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN / 2; c0 += 32) {
+                for (int c0 = 0; c0 < width / 2; c0 += 32) {
                     uint32_t g[32], u[32];
                     tmem_ld32(tlane + (uint32_t)c0, g);
-                    tmem_ld32(tlane + (uint32_t)(BN / 2 + c0), u);
+                    tmem_ld32(tlane + (uint32_t)(width / 2 + c0), u);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (c0 + 32 >= BN / 2) { // last TMEM read of this tile: hand the accumulator back before the (slow) stores
+                    if (c0 + 32 >= width / 2) { // last TMEM read of this tile: hand the accumulator back before the (slow) stores
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
                         if (lane == 0) mbar_arrive_leader(tempty0 + 8 * buf);
@@ -606,11 +632,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
             } else if (MODE == GEMM_ACT) {
                 __nv_bfloat16 *C = reinterpret_cast<__nv_bfloat16 *>(Cv);
 #pragma unroll 1
-                for (int c0 = 0; c0 < BN; c0 += 32) {
+                for (int c0 = 0; c0 < width; c0 += 32) {
                     uint32_t r[32];
                     tmem_ld32(tlane + (uint32_t)c0, r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (c0 + 32 >= BN) { // last TMEM read of this tile
+                    if (c0 + 32 >= width) { // last TMEM read of this tile
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
                         if (lane == 0) mbar_arrive_leader(tempty0 + 8 * buf);
@@ -629,11 +655,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
             } else {
                 const int rloc = q * 32 + lane;
 #pragma unroll 1
-                for (int c = 0; c < BN / 32; c++, chunk++) {
+                for (int c = 0; c < width / 32; c++, chunk++) {
                     uint32_t r[32];
                     tmem_ld32(tlane + (uint32_t)(c * 32), r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (c == BN / 32 - 1) {
+                    if (c == width / 32 - 1) {
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
                         if (lane == 0) mbar_arrive_leader(tempty0 + 8 * buf);
@@ -700,6 +726,13 @@ inline int make_map(CUtensorMap *map, const void *base, uint64_t rows, uint64_t 
     return r == CUDA_SUCCESS ? 0 : -2;
 }
 
+// The B operand of a GEMM: a map for whole tiles and one of 32-row boxes for the narrow tiles of the persistent kernel (same matrix, same swizzle).
+struct BMap : CUtensorMap { CUtensorMap narrow; };
+inline int make_map(BMap *map, const void *base, uint64_t rows, uint64_t K, uint32_t box_rows) {
+    const int rc = make_map(static_cast<CUtensorMap *>(map), base, rows, K, box_rows);
+    return rc ? rc : make_map(&map->narrow, base, rows, K, 32);
+}
+
 // A column block of a wider row-major matrix: K columns of rows that are ld elements apart (ld * 2 bytes a multiple of 16).
 inline int make_map_ld(CUtensorMap *map, const void *base, uint64_t rows, uint64_t K, uint64_t ld, uint32_t box_rows) {
     EncodeTiledFn fn = encode_fn();
@@ -759,7 +792,7 @@ constexpr int GEMM2_STAGES_256_M2 = 4;                    // 4 x (32 KB of A + 1
 
 // Persistent variant (round-2 candidate).  n_sms: SMs of the device; the grid is the largest even number of CTAs <= n_sms.
 template <int MODE, int BN, int STAGES>
-inline int gemm2_persist_launch(const CUtensorMap &a, const CUtensorMap &b, const CUtensorMap &b2, const CUtensorMap &c, void *C, int ldc, int m_valid, int m_tiles,
+inline int gemm2_persist_launch(const CUtensorMap &a, const BMap &b, const BMap &b2, const CUtensorMap &c, void *C, int ldc, int m_valid, int m_tiles,
                                 int n_tiles, int K, int n_sms, cudaStream_t stream, int splits = 1, uint32_t flavor = 0) {
     static bool attr = false;
     if (!attr) {
@@ -773,11 +806,13 @@ inline int gemm2_persist_launch(const CUtensorMap &a, const CUtensorMap &b, cons
         const int nk = (K + BK - 1) / BK, per = (nk + splits - 1) / splits;
         if ((splits - 1) * per >= nk) return -6; // an empty split would publish an unwritten accumulator
     }
-    const int m_pairs = m_tiles / 2, total = m_pairs * n_tiles * splits;
+    const int m_pairs = m_tiles / 2;
     int clusters = n_sms / 2;
+    const TileCut cut = splits > 1 ? TileCut{n_tiles, 0, BN} : cut_tiles(m_pairs, n_tiles * BN, BN, clusters);
+    const int total = m_pairs * (cut.wide + cut.narrow) * splits;
     if (clusters > total) clusters = total;
     if (clusters < 1) return -6;
-    k_gemm_f16_2cta_persist<MODE, BN, STAGES><<<dim3(2 * clusters), 256, smem_bytes_2cta_persist<BN, STAGES>(), stream>>>(a, b, b2, c, C, ldc, m_valid, K, m_pairs, n_tiles, splits, flavor);
+    k_gemm_f16_2cta_persist<MODE, BN, STAGES><<<dim3(2 * clusters), 256, smem_bytes_2cta_persist<BN, STAGES>(), stream>>>(a, b, b2, b.narrow, b2.narrow, c, C, ldc, m_valid, K, m_pairs, n_tiles * BN, cut, splits, flavor);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
 constexpr int GEMM2_PERSIST_STAGES_256 = 5; // 5 x 32 KB of operands + 2 x 16 KB of C staging
@@ -789,7 +824,8 @@ constexpr int GEMM_STAGES = 3, GEMM_STAGES_DEEP = 6;
 // Test/measurement entry: C[M,N] (+)= A[M,K] * B[N,K]^T ; M, N multiples of 128, K multiple of 64.  Device pointers.
 inline int gemm_f16(const __half *A, const __half *B, float *C, int M, int N, int K, int stages, int resid, int two_cta, cudaStream_t stream) {
     if (M % BM || N % BN || K % BK) return -3;
-    CUtensorMap ma, mb, mc;
+    CUtensorMap ma, mc;
+    BMap mb;
     int rc;
     if (two_cta) { // two_cta = pair-tile width (256 or 128)
         const int bn = (two_cta == 512 || two_cta == 1256) ? 256 : two_cta;
