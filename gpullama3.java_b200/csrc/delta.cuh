@@ -42,6 +42,8 @@ struct RopeMixArgs {
 __global__ void __launch_bounds__(ROPE_MIX_THREADS) k_rope_mix_prep(const float *__restrict__ P, int ldp, RopeMixArgs a, const float *__restrict__ bias, float *__restrict__ Q, int ldq,
                                                                     float *__restrict__ kc, float *__restrict__ vc, bf16 *__restrict__ kc16, bf16 *__restrict__ vc16,
                                                                     const StepState *__restrict__ st, int hpc) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float xs[];
     const int r = blockIdx.x, tid = threadIdx.x;
     const int qd = a.heads * a.dk, kd = a.kv_heads * a.dk, vd = a.kv_heads * a.dv;
@@ -118,6 +120,8 @@ __host__ __device__ inline int delta_channels(const DeltaArgs &a) { return 2 * a
 #define DELTA_PREP_THREADS 128
 __global__ void __launch_bounds__(DELTA_PREP_THREADS) k_delta_prep(const float *__restrict__ P, int ldp, DeltaArgs a, float *__restrict__ cstate, float *__restrict__ D, int ldd,
                                                                    const StepState *__restrict__ st) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float row[];
     __shared__ float red[32];
     const int r = blockIdx.x, u = blockIdx.y, tid = threadIdx.x;
@@ -166,6 +170,8 @@ __host__ __device__ inline size_t delta_rule_smem_floats(int dk) { return (size_
 
 __global__ void __launch_bounds__(DELTA_COLS) k_delta_rule(const float *__restrict__ D, int ldd, DeltaArgs a, float *__restrict__ S, int n, float *__restrict__ O, int ldo,
                                                            const StepState *__restrict__ st) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float sm[];
     const int h = blockIdx.x, j0 = blockIdx.y * DELTA_COLS, tid = threadIdx.x, j = j0 + tid;
     const int dk = a.dk, dv = a.dv, g = h / (a.heads / a.kv_heads), C = delta_channels(a);
@@ -235,6 +241,8 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src, bool valid
 template <int R>
 __global__ void __launch_bounds__(DR_THREADS) k_delta_rule_reg(const float *__restrict__ D, int ldd, DeltaArgs a, float *__restrict__ S, int n, float *__restrict__ O, int ldo,
                                                                const StepState *__restrict__ st) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int RP = R > 4 ? R + 4 : R, KR = DR_SLICES * RP; // floats per slice / per token in shared memory
     __shared__ __align__(16) float ks[2][DR_TB][KR], qs[2][DR_TB][KR];
     __shared__ float vs[2][DR_TB][DR_COLS], bd[2][DR_TB][2], os[DR_TB][DR_COLS];
@@ -344,6 +352,8 @@ __host__ __device__ inline size_t delta_coef_floats(int rows, int heads) { retur
 
 // grid (ceil(n / 4), ceil(heads / 4)), 128 threads: a warp per (four tokens, head).  Tokens behind the last one count as beta = 0, decay = 1.
 __global__ void __launch_bounds__(128) k_delta_coef(const float *__restrict__ D, int ldd, DeltaArgs a, int n, float *__restrict__ coef) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int b = blockIdx.x, lane = threadIdx.x & 31, h = blockIdx.y * 4 + (threadIdx.x >> 5);
     if (h >= a.heads) return;
     const int dk = a.dk, g = h / (a.heads / a.kv_heads), C = delta_channels(a), t0 = 4 * b;
@@ -423,6 +433,8 @@ __global__ void __launch_bounds__(DB_THREADS) k_delta_rule_blocks(const float *_
     const int dk = a.dk, dv = a.dv, g = h / (a.heads / a.kv_heads);
     float *Sg = S + ((size_t)h * gridDim.y + tile) * R * DR_THREADS + tid;
     float S0[R], S1[R];
+    pdl_launch_dependents();
+    pdl_wait();
     const bool fresh = st->pos == 0;
     const bool wide = R >= 4 && dk % 4 == 0 && ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(D) & 15) == 0; // rows of whole, aligned 16-byte pieces
     auto stage = [&](int i) { // tokens behind the last one are zero
@@ -588,6 +600,8 @@ struct HeadNormArgs {
 };
 __global__ void __launch_bounds__(256) k_head_norm_gate(const float *__restrict__ O, int ldo, const float *__restrict__ G, int ldg, HeadNormArgs a, float *__restrict__ out32,
                                                         bf16 *__restrict__ out16, int ldout) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, heads = a.heads, dv = a.dv;
     const float eps = a.eps;
     for (int h = blockIdx.y * 8 + warp; h < heads; h += 8 * gridDim.y) {

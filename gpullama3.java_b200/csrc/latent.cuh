@@ -58,6 +58,8 @@ __device__ __forceinline__ float sinusoid_entry(int pos, double f, bool cosine) 
 // One CTA of NTH threads per row (a single wide row takes more threads: more of its loads are in flight)
 template <int NTH>
 __global__ void __launch_bounds__(NTH) k_block_norm_rows(BlockNormArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float row[];
     __shared__ float red[32];
     __shared__ size_t s_row[LY_BLOCK_TERMS]; // offset of a feed-forward result row
@@ -175,6 +177,8 @@ struct LatentArgs {
 // cache16 (nullable): BF16 twin of the cache row.
 __global__ void __launch_bounds__(256) k_latent_prep(float *__restrict__ P, int ldp, LatentArgs a, float *__restrict__ cache, bf16 *__restrict__ cache16, int ring,
                                                      float *__restrict__ Q, bf16 *__restrict__ qu16, const StepState *__restrict__ st) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     const int r = blockIdx.x, tid = threadIdx.x;
     const int pos = st->pos + r, half = a.rope_dims / 2, kw = a.rank + a.dr;
@@ -341,6 +345,8 @@ __device__ __forceinline__ void route_select(float *z, float *sbuf, int experts,
 template <typename IN_T>
 __global__ void __launch_bounds__(128) k_moe_route(const IN_T *__restrict__ X, const bf16 *__restrict__ Wr, int n, int E, int experts, int top, int rows_per_cta,
                                                    int *__restrict__ ids, float *__restrict__ wts, RouteMode m, int extra, float *__restrict__ extra_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool shared_row = rows_per_cta == 1;
@@ -368,6 +374,8 @@ __global__ void __launch_bounds__(128) k_moe_route(const IN_T *__restrict__ X, c
 // The decode step spreads the router's rows over several CTAs (k_matvec_bf16) and selects here: one warp, logits z [experts]
 // in, route_select out.  Dynamic shared memory: 3 * experts floats.
 __global__ void __launch_bounds__(32) k_moe_topk(const float *__restrict__ Z, int experts, int top, int *__restrict__ ids, float *__restrict__ wts, RouteMode m) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float z[];
     const int lane = threadIdx.x;
     for (int e = lane; e < experts; e += 32) z[e] = Z[e];
@@ -381,6 +389,8 @@ __global__ void __launch_bounds__(32) k_moe_topk(const float *__restrict__ Z, in
 // Ids n_real .. experts - 1 are experts without weights (the identity): their slots are sorted like the others but their tiles get group -1.
 __global__ void __launch_bounds__(1024) k_moe_group(const int *__restrict__ ids, int n_slots, int experts, int max_tiles, int *__restrict__ perm,
                                                     int *__restrict__ tile_group, int *__restrict__ tile_row0, int *__restrict__ tile_rows, int n_real) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ int smi[];
     int *count = smi, *offs = smi + experts, *cursor = smi + 2 * experts;
     const int tid = threadIdx.x;
@@ -413,6 +423,8 @@ __global__ void __launch_bounds__(1024) k_moe_group(const int *__restrict__ ids,
 // Expanded keys of a prefill chunk: the rotated shared key part of cached row j (BF16 twin, [.][kw], entries rank ..) goes behind
 // every head's unrotated key in KX [rows][heads * (dk + dr)].
 __global__ void __launch_bounds__(256) k_latent_spread(const bf16 *__restrict__ cache16, int kw, int rank, int dr, int heads, int dk, bf16 *__restrict__ KX, int rows) {
+    pdl_launch_dependents();
+    pdl_wait();
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x, per = (long long)heads * dr;
     if (i >= per * rows) return;
     const int j = (int)(i / per), h = (int)(i % per) / dr, e = (int)(i % per) % dr;
@@ -427,6 +439,8 @@ __global__ void __launch_bounds__(256) k_latent_spread(const bf16 *__restrict__ 
 __global__ void __launch_bounds__(1024) k_moe_group_padded(const int *__restrict__ ids, const float *__restrict__ wts, int n_slots, int experts, int max_tiles,
                                                            int *__restrict__ srt, int *__restrict__ slot_row, float *__restrict__ row_scale, int *__restrict__ tile_group,
                                                            int n_real, int unit_scale) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ int smi[];
     int *count = smi, *offs = smi + experts, *cursor = smi + 2 * experts;
     const int tid = threadIdx.x;
@@ -456,6 +470,8 @@ __global__ void __launch_bounds__(1024) k_moe_group_padded(const int *__restrict
 // Rows of A (one per token) into expert-sorted order: padded row r reads token srt[r] / top; padding rows are zero.  E % 8 == 0.
 __global__ void __launch_bounds__(128) k_moe_gather(const bf16 *__restrict__ A, int E, int top, const int *__restrict__ srt, const int *__restrict__ tile_group,
                                                     bf16 *__restrict__ AS) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int row = blockIdx.x;
     if (tile_group[row >> 7] < 0) return;
     const int slot = srt[row];
@@ -468,6 +484,8 @@ __global__ void __launch_bounds__(128) k_moe_gather(const bf16 *__restrict__ A, 
 // [W_uk c_j | rot r_j] per head and BF16 values.  One CTA per cached row.
 __global__ void __launch_bounds__(256) k_latent_pack(const float *__restrict__ KXF, const float *__restrict__ VXF, const bf16 *__restrict__ cache16, int kw, int rank, int dr,
                                                      int heads, int dk, int dv, bf16 *__restrict__ KX, bf16 *__restrict__ VX) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int j = blockIdx.x, tid = threadIdx.x, DK = dk + dr;
     const float *kf = KXF + (size_t)j * heads * dk, *vf = VXF + (size_t)j * heads * dv;
     bf16 *kx = KX + (size_t)j * heads * DK, *vx = VX + (size_t)j * heads * dv;
@@ -479,6 +497,8 @@ __global__ void __launch_bounds__(256) k_latent_pack(const float *__restrict__ K
 }
 
 __global__ void __launch_bounds__(256) k_softcap(float *__restrict__ x, long long n, float cap) {
+    pdl_launch_dependents();
+    pdl_wait();
     const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
     if (i < n) x[i] = cap * tanhf(x[i] / cap);
 }

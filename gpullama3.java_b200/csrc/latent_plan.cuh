@@ -201,17 +201,17 @@ static int ly_project_view(b200_plan *p, bool decode, int n, const float *a32, c
     if (decode) {
         const int warps = LY_MV_THREADS / 32;
         if (EPI != ly::EPI_GATED && yb == 1 && !mv.group && !mv.mul && !mv.in_scale && ly_few_rows(p, N, K))
-            return launch_k(p, false, ly::k_matvec_row_bf16<EPI == ly::EPI_GATED ? ly::EPI_STORE : EPI>, dim3(N), dim3(LY_MV_THREADS), (size_t)0, W, a32, c32, K, act, mv.tg);
-        return launch_k(p, false, ly::k_matvec_bf16<EPI>, dim3((N + warps - 1) / warps, yb), dim3(LY_MV_THREADS), (size_t)K * 4, W, (const float *)nullptr, a32, c32, N, K, act, mv);
+            return launch_k(p, p->use_pdl, ly::k_matvec_row_bf16<EPI == ly::EPI_GATED ? ly::EPI_STORE : EPI>, dim3(N), dim3(LY_MV_THREADS), (size_t)0, W, a32, c32, K, act, mv.tg);
+        return launch_k(p, p->use_pdl, ly::k_matvec_bf16<EPI>, dim3((N + warps - 1) / warps, yb), dim3(LY_MV_THREADS), (size_t)K * 4, W, (const float *)nullptr, a32, c32, N, K, act, mv);
     }
     dim3 grid((N + 63) / 64, tiles > 0 ? tiles : (n + 63) / 64, zb);
     const float *nb = nullptr;
     if (Y.f32) {
         if (c16) return fail(p, B200_ERR_STATE, "FP32 plans keep FP32 activations");
-        return launch_k(p, false, ly::k_gemm_f32<EPI, float>, grid, dim3(256), (size_t)0, a32, W, nb, c32, n, N, K, ldc, act, gv);
+        return launch_k(p, p->use_pdl, ly::k_gemm_f32<EPI, float>, grid, dim3(256), (size_t)0, a32, W, nb, c32, n, N, K, ldc, act, gv);
     }
-    if (c16) return launch_k(p, false, ly::k_gemm_bf16<EPI, ly::bf16>, grid, dim3(128), (size_t)0, a16, W, nb, c16, n, N, K, ldc, act, gv);
-    return launch_k(p, false, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, nb, c32, n, N, K, ldc, act, gv);
+    if (c16) return launch_k(p, p->use_pdl, ly::k_gemm_bf16<EPI, ly::bf16>, grid, dim3(128), (size_t)0, a16, W, nb, c16, n, N, K, ldc, act, gv);
+    return launch_k(p, p->use_pdl, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, nb, c32, n, N, K, ldc, act, gv);
 }
 
 static ly::BlockNormArgs ly_block_norm_args(const Layered &Y) {
@@ -222,8 +222,8 @@ static ly::BlockNormArgs ly_block_norm_args(const Layered &Y) {
 
 // The row kernel of parallel and layer-norm blocks; a single wide row takes more threads.
 static int ly_launch_block_norm(b200_plan *p, int n, const ly::BlockNormArgs &a) {
-    if (n == 1 && a.E >= 2048) return launch_k(p, false, ly::k_block_norm_rows<1024>, dim3(1), dim3(1024), (size_t)a.E * 4, a);
-    return launch_k(p, false, ly::k_block_norm_rows<LY_NORM_THREADS>, dim3(n), dim3(LY_NORM_THREADS), (size_t)a.E * 4, a);
+    if (n == 1 && a.E >= 2048) return launch_k(p, p->use_pdl, ly::k_block_norm_rows<1024>, dim3(1), dim3(1024), (size_t)a.E * 4, a);
+    return launch_k(p, p->use_pdl, ly::k_block_norm_rows<LY_NORM_THREADS>, dim3(n), dim3(LY_NORM_THREADS), (size_t)a.E * 4, a);
 }
 
 // Latent attention of one layer, from the projection rows in PROJ to the heads' (gated) outputs in ATT32 / ATT16.
@@ -241,7 +241,7 @@ static int ly_enqueue_latent(b200_plan *p, bool decode, int n, const StepState *
     la.heads = s.heads; la.dk = s.key_dim; la.dr = s.rot_dim; la.rank = s.kv_rank; la.q_off = L.q_off; la.kv_off = L.kv_off;
     la.cnorm = L.cnorm; la.cs = L.rope; la.rope_dims = s.rope_dims; la.rope_layout = s.rope_layout; la.eps = Y.c.norm_eps;
     la.q_rank = s.q_rank; la.qnorm = L.qnorm; la.cq32 = h16 ? nullptr : Y.CQ32; la.cq16 = h16 ? Y.CQ16 : nullptr;
-    if ((rc = launch_k(p, false, ly::k_latent_prep, dim3(n, s.q_rank > 0 ? 2 : 1), dim3(256), (size_t)0, Y.PROJ, Y.maxP, la, R.kc, R.own ? R.kc16 : (ly::bf16 *)nullptr, Y.ring, Y.Q,
+    if ((rc = launch_k(p, p->use_pdl, ly::k_latent_prep, dim3(n, s.q_rank > 0 ? 2 : 1), dim3(256), (size_t)0, Y.PROJ, Y.maxP, la, R.kc, R.own ? R.kc16 : (ly::bf16 *)nullptr, Y.ring, Y.Q,
                        h16 && s.q_rank == 0 ? Y.QU16 : (ly::bf16 *)nullptr, st))) return rc;
     ++*nl;
     const float *q32 = Y.PROJ + L.q_off; // query rows: heads x (key size + rotated size), row stride ldq
@@ -271,7 +271,7 @@ static int ly_enqueue_latent(b200_plan *p, bool decode, int n, const StepState *
             int gr = pg::gemm_launch<pg::GEMM_F32, pg::GEMM_STAGES>(O.m_lat, L.m_xk_b, L.m_xk_b, L.m_xk_c, Y.KXF, s.heads * s.key_dim, M, mt, s.heads * s.key_dim / pg::BN, s.kv_rank, p->stream, pg::FLAVOR_BF16);
             if (!gr) gr = pg::gemm_launch<pg::GEMM_F32, pg::GEMM_STAGES>(O.m_lat, L.m_xv_b, L.m_xv_b, L.m_xv_c, Y.VXF, L.gd, M, mt, L.gd / pg::BN, s.kv_rank, p->stream, pg::FLAVOR_BF16);
             if (gr) return fail(p, B200_ERR_CUDA, "tensor-core expansion GEMM launch failed (%d)", gr);
-            if ((rc = launch_k(p, false, ly::k_latent_pack, dim3(M), dim3(256), (size_t)0, (const float *)Y.KXF, (const float *)Y.VXF, (const ly::bf16 *)R.kc16, L.kw, s.kv_rank, s.rot_dim, s.heads,
+            if ((rc = launch_k(p, p->use_pdl, ly::k_latent_pack, dim3(M), dim3(256), (size_t)0, (const float *)Y.KXF, (const float *)Y.VXF, (const ly::bf16 *)R.kc16, L.kw, s.kv_rank, s.rot_dim, s.heads,
                                s.key_dim, s.value_dim, Y.KX16, Y.VX16))) return rc;
         } else {
             ly::GemmView gv{};
@@ -281,7 +281,7 @@ static int ly_enqueue_latent(b200_plan *p, bool decode, int n, const StepState *
             gv2.lda = L.kw;
             if ((rc = ly_project_view<ly::EPI_STORE>(p, false, M, nullptr, R.kc16, L.w_uv, L.gd, s.kv_rank, nullptr, Y.VX16, L.gd, 0, gv2, ly::MvView{}, 1, 1, 0))) return rc;
             const long long cells = (long long)M * s.heads * s.rot_dim;
-            if (cells > 0 && (rc = launch_k(p, false, ly::k_latent_spread, dim3((unsigned)((cells + 255) / 256)), dim3(256), (size_t)0, (const ly::bf16 *)R.kc16, L.kw, s.kv_rank, s.rot_dim,
+            if (cells > 0 && (rc = launch_k(p, p->use_pdl, ly::k_latent_spread, dim3((unsigned)((cells + 255) / 256)), dim3(256), (size_t)0, (const ly::bf16 *)R.kc16, L.kw, s.kv_rank, s.rot_dim,
                                             s.heads, s.key_dim, Y.KX16, M))) return rc;
         }
         wa.heads = wa.kv_heads = s.heads; wa.dk = DK; wa.dv = s.value_dim; wa.ldk = s.heads * DK; wa.ldv = L.gd; wa.gate = s.gate ? 1 : 0;
@@ -301,10 +301,10 @@ static int ly_enqueue_latent(b200_plan *p, bool decode, int n, const StepState *
     // a gate per head commutes with W_uv: it multiplies the latent-space output; a gate per output entry waits for the expanded values
     wa.heads = s.heads; wa.kv_heads = 1; wa.dk = L.kw; wa.dv = s.kv_rank; wa.ldk = wa.ldv = L.kw; wa.gate = s.gate == 2 ? 1 : 0;
     const size_t asm_ = ly_att_smem(wa.dk, wa.window);
-    if (h16) rc = launch_k(p, false, ly::k_window_attention<ly::bf16>, dim3(n, s.heads), dim3(LY_ATT_THREADS), asm_, (const float *)Y.Q, L.qw, wa,
+    if (h16) rc = launch_k(p, p->use_pdl, ly::k_window_attention<ly::bf16>, dim3(n, s.heads), dim3(LY_ATT_THREADS), asm_, (const float *)Y.Q, L.qw, wa,
                            (const float *)R.kc, (const float *)R.kc, st, Y.LAT16, L.lw, ly::KeySplit{nullptr, nullptr, nullptr});
     else if (decode) rc = ly_step_attention(p, s.heads, s.window, Y.Q, L.qw, wa, R.kc, R.kc, st, Y.LAT32, L.lw, asm_);
-    else rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, s.heads), dim3(LY_ATT_THREADS), asm_, (const float *)Y.Q, L.qw, wa,
+    else rc = launch_k(p, p->use_pdl, ly::k_window_attention<float>, dim3(n, s.heads), dim3(LY_ATT_THREADS), asm_, (const float *)Y.Q, L.qw, wa,
                        (const float *)R.kc, (const float *)R.kc, st, Y.LAT32, L.lw, ly::KeySplit{nullptr, nullptr, nullptr});
     if (rc) return rc;
     ++*nl;
@@ -327,13 +327,13 @@ static int ly_enqueue_route(b200_plan *p, bool decode, int n, const LyLayer &L, 
     if (decode) { // one row: the router's rows stream through the multi-CTA matvec, one warp selects
         if ((rc = ly_project<ly::EPI_STORE>(p, true, 1, x32, nullptr, L.w_router, nullptr, scores + extra, E, Y.ZR, nullptr, scores + extra, 0))) return rc;
         *nl += 2;
-        return launch_k(p, false, ly::k_moe_topk, dim3(1), dim3(32), (size_t)3 * scores * 4, (const float *)Y.ZR, scores, top, Y.moe_ids, Y.moe_wts, rm);
+        return launch_k(p, p->use_pdl, ly::k_moe_topk, dim3(1), dim3(32), (size_t)3 * scores * 4, (const float *)Y.ZR, scores, top, Y.moe_ids, Y.moe_wts, rm);
     }
     // a CTA per row: four warps share the row's experts
     const size_t rsm = (size_t)(E + 3 * (scores + extra)) * 4;
     ++*nl;
-    if (!Y.f32) return launch_k(p, false, ly::k_moe_route<ly::bf16>, dim3(n), dim3(128), rsm, x16, (const ly::bf16 *)L.w_router, n, E, scores, top, 1, Y.moe_ids, Y.moe_wts, rm, extra, Y.SGL);
-    return launch_k(p, false, ly::k_moe_route<float>, dim3(n), dim3(128), rsm, x32, (const ly::bf16 *)L.w_router, n, E, scores, top, 1, Y.moe_ids, Y.moe_wts, rm, extra, Y.SGL);
+    if (!Y.f32) return launch_k(p, p->use_pdl, ly::k_moe_route<ly::bf16>, dim3(n), dim3(128), rsm, x16, (const ly::bf16 *)L.w_router, n, E, scores, top, 1, Y.moe_ids, Y.moe_wts, rm, extra, Y.SGL);
+    return launch_k(p, p->use_pdl, ly::k_moe_route<float>, dim3(n), dim3(128), rsm, x32, (const ly::bf16 *)L.w_router, n, E, scores, top, 1, Y.moe_ids, Y.moe_wts, rm, extra, Y.SGL);
 }
 
 // The chosen experts of every row, one result row per slot (row * top + k): *ys, at row (*map)[slot] of it when *map is set.  groups = ids
@@ -350,9 +350,9 @@ static int ly_enqueue_experts(b200_plan *p, bool decode, int n, const LyLayer &L
         // the input) in its epilogue, the down GEMM leaves its results in sorted order and the next row kernel finds a slot's row through slot_row
         int t128 = (n * top + 127) / 128 + X;
         if (t128 > Y.max_tiles128) t128 = Y.max_tiles128;
-        if ((rc = launch_k(p, false, ly::k_moe_group_padded, dim3(1), dim3(1024), (size_t)3 * groups * 4, (const int *)Y.moe_ids, (const float *)Y.moe_wts, n * top, groups, t128, Y.srt, Y.slot_row,
+        if ((rc = launch_k(p, p->use_pdl, ly::k_moe_group_padded, dim3(1), dim3(1024), (size_t)3 * groups * 4, (const int *)Y.moe_ids, (const float *)Y.moe_wts, n * top, groups, t128, Y.srt, Y.slot_row,
                            Y.row_scale, Y.tile_group128, X, scale_input ? 0 : 1))) return rc;
-        if ((rc = launch_k(p, false, ly::k_moe_gather, dim3(t128 * 128), dim3(128), (size_t)0, x16, E, top, (const int *)Y.srt, (const int *)Y.tile_group128, Y.AS16))) return rc;
+        if ((rc = launch_k(p, p->use_pdl, ly::k_moe_gather, dim3(t128 * 128), dim3(128), (size_t)0, x16, E, top, (const int *)Y.srt, (const int *)Y.tile_group128, Y.AS16))) return rc;
         const pg::Grouped g{Y.tile_group128, up_rows, scale_input ? Y.row_scale : (const float *)nullptr};
         int gr;
         if (s.moe_plain)
@@ -371,7 +371,7 @@ static int ly_enqueue_experts(b200_plan *p, bool decode, int n, const LyLayer &L
     if (!decode) {
         tiles = (n * top + 63) / 64 + groups;
         if (tiles > Y.max_tiles) tiles = Y.max_tiles;
-        if ((rc = launch_k(p, false, ly::k_moe_group, dim3(1), dim3(1024), (size_t)3 * groups * 4, (const int *)Y.moe_ids, n * top, groups, tiles, Y.moe_perm, Y.tile_group, Y.tile_row0,
+        if ((rc = launch_k(p, p->use_pdl, ly::k_moe_group, dim3(1), dim3(1024), (size_t)3 * groups * 4, (const int *)Y.moe_ids, n * top, groups, tiles, Y.moe_perm, Y.tile_group, Y.tile_row0,
                            Y.tile_rows, X))) return rc;
         ++*nl;
     }
@@ -441,11 +441,11 @@ static int ly_enqueue_parallel(b200_plan *p, bool decode, int n, const StepState
             if ((rc = ly_project<ly::EPI_STORE>(p, true, 1, Y.A32, nullptr, Y.head, nullptr, Y.c.vocab_size, E, p->logits, nullptr, Y.c.vocab_size, 0))) return rc;
             nl++;
             if (Y.c.logit_softcap > 0.0f) {
-                if ((rc = launch_k(p, false, ly::k_softcap, dim3((Y.c.vocab_size + 255) / 256), dim3(256), (size_t)0, p->logits, (long long)Y.c.vocab_size, Y.c.logit_softcap))) return rc;
+                if ((rc = launch_k(p, p->use_pdl, ly::k_softcap, dim3((Y.c.vocab_size + 255) / 256), dim3(256), (size_t)0, p->logits, (long long)Y.c.vocab_size, Y.c.logit_softcap))) return rc;
                 nl++;
             }
         } else if ((rc = bnorm(false, nullptr, nullptr, nullptr, nullptr))) return rc;
-        if ((rc = launch_k(p, false, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
+        if ((rc = launch_k(p, p->use_pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
                            p->out_ids, with_head ? 1 : 0, (const float *)nullptr, (const int *)nullptr, 0, TraceBuf{nullptr, 0, 0}, p->tp, -1))) return rc;
         nl++;
     } else if ((rc = bnorm(false, nullptr, nullptr, nullptr, nullptr))) return rc;

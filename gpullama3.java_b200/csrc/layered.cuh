@@ -116,6 +116,8 @@ struct NormArgs {
 // its loads are in flight).  Dynamic shared memory: E floats, 2 * E with ys.
 template <int NTH>
 __global__ void __launch_bounds__(NTH) k_norm_rows(NormArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float row[];
     __shared__ float red[32];
     __shared__ size_t s_row[LY_NORM_TERMS];
@@ -253,6 +255,8 @@ __device__ __forceinline__ float dot_row_bf16(const bf16 *__restrict__ w, const 
 // E a multiple of 4, at most 4 * NTH * VPT; top <= LY_NORM_TERMS.  No dynamic shared memory.
 template <int NTH, int VPT, bool PROLOGUE = false>
 __global__ void __launch_bounds__(NTH) k_norm_rows_reg(NormArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32];
     __shared__ size_t s_row[LY_NORM_TERMS];
     __shared__ float s_wt[LY_NORM_TERMS];
@@ -407,6 +411,8 @@ __global__ void __launch_bounds__(LY_MV_THREADS) k_matvec_bf16(const bf16 *__res
                                                               float *__restrict__ y, int N, int K, int act, MvView v_) {
     extern __shared__ __align__(16) float xs[];
     const int b = blockIdx.y;
+    pdl_launch_dependents();
+    pdl_wait();
     if (v_.group && v_.n_groups > 0 && v_.group[b] >= v_.n_groups) return;
     W += (size_t)b * v_.w_bs + (v_.group ? (size_t)v_.group[b] * v_.w_gs : (size_t)0);
     x += (size_t)b * v_.x_bs;
@@ -440,6 +446,8 @@ __global__ void __launch_bounds__(LY_MV_THREADS) k_matvec_row_bf16(const bf16 *_
     __shared__ float red[32];
     const int n = blockIdx.x;
     const bf16 *w = W + (size_t)n * K;
+    pdl_launch_dependents();
+    pdl_wait();
     float acc = 0.0f;
     if ((K & 7) == 0 && (((size_t)W) & 15) == 0 && (((size_t)x) & 15) == 0) {
         int k = threadIdx.x * 8;
@@ -527,6 +535,8 @@ __device__ __forceinline__ float gemm_epilogue(const GemmView &g, float a0, floa
 template <int EPI, typename OUT_T>
 __global__ void __launch_bounds__(256) k_gemm_f32(const float *__restrict__ A, const bf16 *__restrict__ W, const float *__restrict__ bias,
                                                    OUT_T *__restrict__ C, int M, int N, int K, int ldc, int act, GemmView g) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int BM = 64, BN = 64, BK = 16, NB = EPI == EPI_GATED ? 2 : 1;
     __shared__ float As[BK][BM + 4];
     __shared__ float Bs[NB][BK][BN + 4];
@@ -626,6 +636,8 @@ __device__ __forceinline__ void load_tile_bf16(bf16 (*dst)[40], const bf16 *__re
 template <int EPI, typename OUT_T>
 __global__ void __launch_bounds__(128) k_gemm_bf16(const bf16 *__restrict__ A, const bf16 *__restrict__ W, const float *__restrict__ bias,
                                                     OUT_T *__restrict__ C, int M, int N, int K, int ldc, int act, GemmView gv) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int NB = EPI == EPI_GATED ? 2 : 1;
     __shared__ __align__(16) bf16 As[64][40];
     __shared__ __align__(16) bf16 Bs[NB][64][40];
@@ -745,6 +757,8 @@ __device__ __forceinline__ void rope_pair_index(int i, int dims, int layout, int
 template <int NTH>
 __global__ void __launch_bounds__(NTH) k_qk_prep(float *__restrict__ P, int ldp, WindowAttn a, const float *__restrict__ bias, float *__restrict__ kc,
                                                  float *__restrict__ vc, bf16 *__restrict__ kc16, bf16 *__restrict__ vc16, const StepState *__restrict__ st) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float red[32], redk[32];
     const int r = blockIdx.x, tid = threadIdx.x;
     const int qd = a.heads * a.dk, kd = a.kv_heads * a.dk, vd = a.kv_heads * a.dv;
@@ -830,6 +844,8 @@ template <typename OUT_T>
 __global__ void __launch_bounds__(LY_ATT_THREADS) k_window_attention(const float *__restrict__ P, int ldp, WindowAttn a, const float *__restrict__ kc,
                                                                      const float *__restrict__ vc, const StepState *__restrict__ st,
                                                                      OUT_T *__restrict__ out, int ldo, KeySplit ks_) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float sm[];
     __shared__ float red[32];
     __shared__ int s_last;
@@ -1020,6 +1036,8 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *
     extern __shared__ __align__(16) float sm[];
     __shared__ float red[32];
     const int z = blockIdx.x, sp = gridDim.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_launch_dependents();
+    pdl_wait();
     const int qd = a.heads * a.dk, kd = a.kv_heads * a.dk, vd = a.kv_heads * a.dv;
     const int g = h / (a.heads / a.kv_heads);
     const int gk = a.maps > 1 ? g * a.maps + h % a.maps : a.k_heads > 0 ? h / (a.heads / a.k_heads) : g;
@@ -1190,6 +1208,8 @@ template <int DK, int DV, int BM = LY_ATT_MMA_ROWS>
 __global__ void __launch_bounds__(BM * 2) k_window_attention_mma(const float *__restrict__ P, int ldp, WindowAttn a, const bf16 *__restrict__ kc16,
                                                                              const bf16 *__restrict__ vc16, const StepState *__restrict__ st, int n,
                                                                              bf16 *__restrict__ out, int ldo, float *__restrict__ out32 = nullptr) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int LY_ATT_MMA_THREADS = BM * 2;
     constexpr int QT = BM * (DK + 8) * 2, KT = 64 * (DK + 8) * 2, VT = 64 * (DV + 8) * 2; // bytes of the Q tile, one K tile, one V tile

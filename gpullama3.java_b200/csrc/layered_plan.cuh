@@ -162,6 +162,7 @@ struct Layered {
     float w_off = 1.0f;   // what the norm kernels add to a norm weight (sandwich: weights are deviations from one)
     bool prenorm = false;
     float *emb_norm = nullptr;
+    bool pdl = false;     // prefill launches are programmatic
     float *DCO = nullptr; // coefficients of the delta rule per four rows and head (k_delta_coef)
     float *DLT = nullptr, *DO = nullptr; // prepared q | k | v | beta | decay rows and read-out rows of a delta layer, [cap][...]
     int maxD = 0, maxDO = 0, cring = 0, max_taps = 0;
@@ -287,8 +288,8 @@ static int ly_launch_mma(b200_plan *p, int kind, int n, int heads, int window, c
     const int rows = tall ? LY_ATT_MMA_ROWS : 64;
     const dim3 grid((n + rows - 1) / rows, heads), block(rows * 2);
 #define LY_MMA_CASE(K, DK, DV) \
-    if (kind == K) return tall ? launch_k(p, false, ly::k_window_attention_mma<DK, DV>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32) \
-                               : launch_k(p, false, ly::k_window_attention_mma<DK, DV, 64>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32);
+    if (kind == K) return tall ? launch_k(p, p->use_pdl, ly::k_window_attention_mma<DK, DV>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32) \
+                               : launch_k(p, p->use_pdl, ly::k_window_attention_mma<DK, DV, 64>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32);
     LY_MMA_CASE(1, 64, 64)
     LY_MMA_CASE(2, 128, 128)
     LY_MMA_CASE(3, 192, 128)
@@ -331,8 +332,8 @@ static int ly_project(b200_plan *p, bool decode, int n, const float *a32, const 
         const int warps = LY_MV_THREADS / 32;
         int grid = (N + warps - 1) / warps;
         if (EPI != ly::EPI_GATED && !bias && ly_few_rows(p, N, K))
-            return launch_k(p, false, ly::k_matvec_row_bf16<EPI == ly::EPI_GATED ? ly::EPI_STORE : EPI>, dim3(N), dim3(LY_MV_THREADS), (size_t)0, W, a32, c32, K, act, ly::TokenGate{});
-        return launch_k(p, false, ly::k_matvec_bf16<EPI>, dim3(grid), dim3(LY_MV_THREADS), (size_t)K * 4, W, bias, a32, c32, N, K, act, ly::MvView{});
+            return launch_k(p, p->use_pdl, ly::k_matvec_row_bf16<EPI == ly::EPI_GATED ? ly::EPI_STORE : EPI>, dim3(N), dim3(LY_MV_THREADS), (size_t)0, W, a32, c32, K, act, ly::TokenGate{});
+        return launch_k(p, p->use_pdl, ly::k_matvec_bf16<EPI>, dim3(grid), dim3(LY_MV_THREADS), (size_t)K * 4, W, bias, a32, c32, N, K, act, ly::MvView{});
     }
     if (tc && tc->a && !Y.f32) {
         const int mt2 = (n + 255) / 256 * 2;
@@ -358,9 +359,9 @@ static int ly_project(b200_plan *p, bool decode, int n, const float *a32, const 
         return rc ? fail(p, B200_ERR_CUDA, "tensor-core GEMM launch failed (%d)", rc) : B200_OK;
     }
     dim3 grid((N + 63) / 64, (n + 63) / 64);
-    if (Y.f32) return launch_k(p, false, ly::k_gemm_f32<EPI, float>, grid, dim3(256), (size_t)0, a32, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
-    if (c16) return launch_k(p, false, ly::k_gemm_bf16<EPI, ly::bf16>, grid, dim3(128), (size_t)0, a16, W, bias, c16, n, N, K, ldc, act, ly::GemmView{});
-    return launch_k(p, false, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
+    if (Y.f32) return launch_k(p, p->use_pdl, ly::k_gemm_f32<EPI, float>, grid, dim3(256), (size_t)0, a32, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
+    if (c16) return launch_k(p, p->use_pdl, ly::k_gemm_bf16<EPI, ly::bf16>, grid, dim3(128), (size_t)0, a16, W, bias, c16, n, N, K, ldc, act, ly::GemmView{});
+    return launch_k(p, p->use_pdl, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
 }
 
 // The decode step's attention: k_step_attention for rows of whole float4, with a head's window over as many CTAs as the SMs allow (B200_LAYERED_SPLITS bounds it); else
@@ -371,8 +372,8 @@ static int ly_step_attention(b200_plan *p, int heads, int window, const float *q
     if (Y.split.o && window >= 64) { sp = p->n_sms / heads; if (sp > Y.max_splits) sp = Y.max_splits; if (sp < 1) sp = 1; }
     const size_t sm = ly::step_att_smem_floats(wa.dk, wa.dv, wa.window, sp) * 4;
     if ((wa.dk | wa.dv | wa.ldk | wa.ldv) % 4 == 0 && wa.dk <= 1024 && wa.dv <= 4 * LY_ATT_THREADS && sm <= (size_t)Y.smem_max)
-        return launch_cluster(p, false, sp, ly::k_step_attention, dim3(sp, heads), dim3(LY_ATT_THREADS), sm, q, wa, kc, vc, st, out);
-    return launch_k(p, false, ly::k_window_attention<float>, dim3(1, heads, sp), dim3(LY_ATT_THREADS), general_smem, q, ldq, wa, kc, vc, st, out, ldo,
+        return launch_cluster(p, p->use_pdl, sp, ly::k_step_attention, dim3(sp, heads), dim3(LY_ATT_THREADS), sm, q, wa, kc, vc, st, out);
+    return launch_k(p, p->use_pdl, ly::k_window_attention<float>, dim3(1, heads, sp), dim3(LY_ATT_THREADS), general_smem, q, ldq, wa, kc, vc, st, out, ldo,
                     sp > 1 ? Y.split : ly::KeySplit{nullptr, nullptr, nullptr});
 }
 
@@ -390,21 +391,21 @@ static int ly_enqueue_attention(b200_plan *p, bool decode, int n, const StepStat
         ra.cs = L.rope; ra.temp = L.temp; ra.talk = L.talk; ra.value_from_key = L.s.value_from_key; ra.ring = Y.ring;
         qsrc = Y.Q; ldq = L.s.heads * L.dk_eff;
         const int hpc = decode ? 1 : ROPE_MIX_HEADS; // one row: a CTA per head; a chunk: several heads share the rotation of the row
-        rc = launch_k(p, false, ly::k_rope_mix_prep, dim3(n, (L.s.heads + hpc - 1) / hpc + 1), dim3(ROPE_MIX_THREADS), (size_t)(L.qd > L.kd ? L.qd : L.kd) * 4, (const float *)Y.PROJ, Y.maxP, ra,
+        rc = launch_k(p, p->use_pdl, ly::k_rope_mix_prep, dim3(n, (L.s.heads + hpc - 1) / hpc + 1), dim3(ROPE_MIX_THREADS), (size_t)(L.qd > L.kd ? L.qd : L.kd) * 4, (const float *)Y.PROJ, Y.maxP, ra,
                       (const float *)L.b_proj, Y.Q, ldq, R.kc, R.vc, R.kc16, R.vc16, st, hpc);
     } else
-        rc = n == 1 && L.qd + L.kd >= 1024 ? launch_k(p, false, ly::k_qk_prep<1024>, dim3(1), dim3(1024), (size_t)0, Y.PROJ, Y.maxP, wa, (const float *)L.b_proj, R.kc, R.vc, R.kc16, R.vc16, st)
-           : launch_k(p, false, ly::k_qk_prep<256>, dim3(n), dim3(256), (size_t)0, Y.PROJ, Y.maxP, wa, (const float *)L.b_proj, R.kc, R.vc, R.kc16, R.vc16, st);
+        rc = n == 1 && L.qd + L.kd >= 1024 ? launch_k(p, p->use_pdl, ly::k_qk_prep<1024>, dim3(1), dim3(1024), (size_t)0, Y.PROJ, Y.maxP, wa, (const float *)L.b_proj, R.kc, R.vc, R.kc16, R.vc16, st)
+           : launch_k(p, p->use_pdl, ly::k_qk_prep<256>, dim3(n), dim3(256), (size_t)0, Y.PROJ, Y.maxP, wa, (const float *)L.b_proj, R.kc, R.vc, R.kc16, R.vc16, st);
     if (rc) return rc;
     ++*nl;
     const size_t asm_ = ly_att_smem(L.s, Y.ring);
     const int mma = ly_mma_kind(L.mixprep ? L.dk_eff : L.s.key_dim, L.s.value_dim);
     if (h16 && R.kc16 && mma)
         rc = ly_launch_mma(p, mma, n, L.s.heads, L.s.window, qsrc, ldq, wa, (const ly::bf16 *)R.kc16, (const ly::bf16 *)R.vc16, st, Y.ATT16, L.gd);
-    else if (h16) rc = launch_k(p, false, ly::k_window_attention<ly::bf16>, dim3(n, L.s.heads), dim3(LY_ATT_THREADS), asm_, qsrc, ldq, wa,
+    else if (h16) rc = launch_k(p, p->use_pdl, ly::k_window_attention<ly::bf16>, dim3(n, L.s.heads), dim3(LY_ATT_THREADS), asm_, qsrc, ldq, wa,
                            (const float *)R.kc, (const float *)R.vc, st, Y.ATT16, L.gd, ly::KeySplit{nullptr, nullptr, nullptr});
     else if (decode) rc = ly_step_attention(p, L.s.heads, L.s.window, qsrc, ldq, wa, R.kc, R.vc, st, Y.ATT32, L.gd, asm_);
-    else rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, L.s.heads), dim3(LY_ATT_THREADS), asm_, qsrc, ldq, wa,
+    else rc = launch_k(p, p->use_pdl, ly::k_window_attention<float>, dim3(n, L.s.heads), dim3(LY_ATT_THREADS), asm_, qsrc, ldq, wa,
                        (const float *)R.kc, (const float *)R.vc, st, Y.ATT32, L.gd, ly::KeySplit{nullptr, nullptr, nullptr});
     ++*nl;
     return rc;
@@ -421,7 +422,7 @@ static int ly_launch_norm(b200_plan *p, int n, const ly::NormArgs &a) {
     const int E = a.E;
     if (E % 4 == 0 && E <= 4096 && a.top <= LY_NORM_TERMS) {
         auto go = [&](auto plain, auto prologue, int threads) {
-            return a.w_emb || a.x0 || a.add_x0 || a.step ? launch_k(p, false, prologue, dim3(n), dim3(threads), (size_t)0, a) : launch_k(p, false, plain, dim3(n), dim3(threads), (size_t)0, a);
+            return a.w_emb || a.x0 || a.add_x0 || a.step ? launch_k(p, p->use_pdl, prologue, dim3(n), dim3(threads), (size_t)0, a) : launch_k(p, p->use_pdl, plain, dim3(n), dim3(threads), (size_t)0, a);
         };
         if (n == 1 && E > 1024) {
             if (E <= 2048) return go(ly::k_norm_rows_reg<512, 1>, ly::k_norm_rows_reg<512, 1, true>, 512);
@@ -432,8 +433,8 @@ static int ly_launch_norm(b200_plan *p, int n, const ly::NormArgs &a) {
         return go(ly::k_norm_rows_reg<LY_NORM_THREADS, 4>, ly::k_norm_rows_reg<LY_NORM_THREADS, 4, true>, LY_NORM_THREADS);
     }
     const size_t sm = (size_t)(a.ys ? 2 : 1) * E * 4;
-    if (n == 1 && E >= 2048) return launch_k(p, false, ly::k_norm_rows<1024>, dim3(1), dim3(1024), sm, a);
-    return launch_k(p, false, ly::k_norm_rows<LY_NORM_THREADS>, dim3(n), dim3(LY_NORM_THREADS), sm, a);
+    if (n == 1 && E >= 2048) return launch_k(p, p->use_pdl, ly::k_norm_rows<1024>, dim3(1), dim3(1024), sm, a);
+    return launch_k(p, p->use_pdl, ly::k_norm_rows<LY_NORM_THREADS>, dim3(n), dim3(LY_NORM_THREADS), sm, a);
 }
 
 const int LY_DELTA_BLOCK_ROWS = 3; // the decode step's single row (and two) stay with the token-by-token kernel: it needs no coefficients
@@ -488,12 +489,12 @@ static int ly_enqueue(b200_plan *p, bool decode, int n, const StepState *st, con
             da.heads = L.s.heads; da.kv_heads = L.s.kv_heads; da.dk = L.s.key_dim; da.dv = L.s.value_dim; da.taps = L.s.conv_taps; da.cring = Y.cring;
             da.conv_w = L.conv_w; da.a_log = L.a_log; da.dt_bias = L.dt_bias; da.unit_eps = 1e-6f;
             const int dmax = L.s.key_dim > L.s.value_dim ? L.s.key_dim : L.s.value_dim;
-            if ((rc = launch_k(p, false, ly::k_delta_prep, dim3(n, 2 * L.s.kv_heads + L.s.heads + 1), dim3(DELTA_PREP_THREADS), (size_t)dmax * 4, (const float *)Y.PROJ, Y.maxP, da, R.cstate,
+            if ((rc = launch_k(p, p->use_pdl, ly::k_delta_prep, dim3(n, 2 * L.s.kv_heads + L.s.heads + 1), dim3(DELTA_PREP_THREADS), (size_t)dmax * 4, (const float *)Y.PROJ, Y.maxP, da, R.cstate,
                                Y.DLT, Y.maxD, st))) return rc;
             const dim3 rgrid(L.s.heads, (L.s.value_dim + DR_COLS - 1) / DR_COLS), rblock(DR_THREADS);
             const int reg = ly::delta_reg_rows(L.s.key_dim);
             if (reg && n >= LY_DELTA_BLOCK_ROWS) {
-                if ((rc = launch_k(p, false, ly::k_delta_coef, dim3((n + 3) / 4, (L.s.heads + 3) / 4), dim3(128), (size_t)0, (const float *)Y.DLT, Y.maxD, da, n, Y.DCO))) return rc;
+                if ((rc = launch_k(p, p->use_pdl, ly::k_delta_coef, dim3((n + 3) / 4, (L.s.heads + 3) / 4), dim3(128), (size_t)0, (const float *)Y.DLT, Y.maxD, da, n, Y.DCO))) return rc;
                 nl++;
                 auto go = [&](auto kern) { return launch_k(p, false, kern, rgrid, dim3(DB_THREADS), (size_t)0, (const float *)Y.DLT, Y.maxD, da, (const float *)Y.DCO, R.S, n, Y.DO, Y.maxDO, st); };
                 rc = reg == 1 ? go(ly::k_delta_rule_blocks<1>) : reg == 2 ? go(ly::k_delta_rule_blocks<2>) : reg == 4 ? go(ly::k_delta_rule_blocks<4>) : go(ly::k_delta_rule_blocks<8>);
@@ -509,7 +510,7 @@ static int ly_enqueue(b200_plan *p, bool decode, int n, const StepState *st, con
             }
             if (rc) return rc;
             const ly::HeadNormArgs ha{L.onorm, 0, 0, nullptr, L.s.heads, L.s.value_dim, Y.c.norm_eps};
-            if ((rc = launch_k(p, false, ly::k_head_norm_gate, dim3(n), dim3(256), (size_t)0, (const float *)Y.DO, Y.maxDO, (const float *)(Y.PROJ + L.dC + 2 * L.s.heads), Y.maxP, ha,
+            if ((rc = launch_k(p, p->use_pdl, ly::k_head_norm_gate, dim3(n), dim3(256), (size_t)0, (const float *)Y.DO, Y.maxDO, (const float *)(Y.PROJ + L.dC + 2 * L.s.heads), Y.maxP, ha,
                                h16 ? (float *)nullptr : Y.ATT32, h16 ? Y.ATT16 : (ly::bf16 *)nullptr, L.gd))) return rc;
             nl += 3;
         } else if (L.s.mixer == B200_MIXER_LIGHTNING) {
@@ -554,7 +555,7 @@ static int ly_enqueue(b200_plan *p, bool decode, int n, const StepState *st, con
             if ((rc = ly_project<ly::EPI_STORE>(p, true, 1, Y.A32, nullptr, Y.head, nullptr, Y.c.vocab_size, E, p->logits, nullptr, Y.c.vocab_size, 0))) return rc;
             nl++;
         } else if ((rc = norm(false, false, nullptr, nullptr))) return rc;
-        if ((rc = launch_k(p, false, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
+        if ((rc = launch_k(p, p->use_pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
                            p->out_ids, with_head ? 1 : 0, (const float *)nullptr, (const int *)nullptr, 0, TraceBuf{nullptr, 0, 0}, p->tp, -1))) return rc;
         nl++;
     } else if ((rc = norm(false, false, nullptr, nullptr))) return rc;
@@ -1080,6 +1081,13 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
         CK(cudaEventCreateWithFlags(&Y.ev_fork, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&Y.ev_join, cudaEventDisableTiming));
     }
+    {   // Programmatic dependent launch in prefill chunks: every kernel of a layered plan waits for its predecessor before it touches anything, so the next launch
+        // can be on its way during the current one (1.5 - 3.5 % of a 512-row chunk).  Not in the decode graph (370 -> 400 us a step: a kernel that becomes
+        // resident early is spread unevenly over the SMs, and there every kernel is one short wave), not for the delta rule (a CTA per SM) and not for plans whose
+        // mixers fork into a second stream.
+        const char *e = getenv("B200_PDL");
+        Y.pdl = !Y.branch && !(e && e[0] == '0');
+    }
     if (c.side_dim > 0) {
         if ((rc = dalloc(p, &Y.SIDE32, rows32 * c.side_dim * 4))) return rc;
         if (!Y.f32 && ((rc = dalloc(p, &Y.SIDE16, cap * c.side_dim * 2)) || (rc = dalloc(p, &Y.SIDEF, cap * Y.side_pad * 4)))) return rc;
@@ -1203,7 +1211,10 @@ static int ly_batch(b200_plan *p, const int32_t *tokens, int n, int start_pos, c
     CK(cudaMemcpyAsync(Y.st_pf, h, sizeof(StepState), cudaMemcpyHostToDevice, p->stream));
     CK(cudaEventRecord(p->ev0, p->stream));
     Y.pf_pos = start_pos;
-    if ((rc = ly_enqueue(p, false, n, Y.st_pf, Y.tok, false, trace_out ? Y.trace : nullptr, &p->launches_prefill))) return rc;
+    p->use_pdl = Y.pdl;
+    rc = ly_enqueue(p, false, n, Y.st_pf, Y.tok, false, trace_out ? Y.trace : nullptr, &p->launches_prefill);
+    p->use_pdl = false;
+    if (rc) return rc;
     CK(cudaEventRecord(p->ev1, p->stream));
     CK(cudaStreamSynchronize(p->stream)); // h_ids / h_st are reused below
     CK(cudaEventElapsedTime(&p->prefill_ms, p->ev0, p->ev1));
@@ -1215,7 +1226,7 @@ static int ly_batch(b200_plan *p, const int32_t *tokens, int n, int start_pos, c
             ly::OutNormArgs a = ly_outnorm_args(Y, m);
             a.w_out = Y.final_norm; a.gather = Y.rows; a.st = Y.st_pf;
             a.out32 = Y.f32 ? Y.A32 : nullptr; a.out16 = Y.f32 ? nullptr : Y.A16;
-            if ((rc = launch_k(p, false, ly::k_outnorm_rows<LY_NORM_THREADS>, dim3(m), dim3(LY_NORM_THREADS), (size_t)2 * E * 4, a))) return rc;
+            if ((rc = launch_k(p, p->use_pdl, ly::k_outnorm_rows<LY_NORM_THREADS>, dim3(m), dim3(LY_NORM_THREADS), (size_t)2 * E * 4, a))) return rc;
         } else if (Y.c.block == B200_BLOCK_PARALLEL || Y.c.block == B200_BLOCK_LAYERNORM) {
             ly::BlockNormArgs a = ly_block_norm_args(Y);
             a.w1 = Y.final_norm; a.b1 = Y.final_norm_b; a.gather = Y.rows;
@@ -1231,7 +1242,7 @@ static int ly_batch(b200_plan *p, const int32_t *tokens, int n, int start_pos, c
         if (Y.tc_head) { t_head.a = &Y.m_a; t_head.b = &Y.m_head; t_head.c = &Y.m_log_c; }
         if ((rc = ly_project<ly::EPI_STORE>(p, false, m, Y.A32, Y.A16, Y.head, nullptr, V, E, Y.LOG, nullptr, V, 0, &t_head))) return rc;
         if (Y.c.logit_softcap > 0.0f &&
-            (rc = launch_k(p, false, ly::k_softcap, dim3((unsigned)(((size_t)m * V + 255) / 256)), dim3(256), (size_t)0, Y.LOG, (long long)m * V, Y.c.logit_softcap))) return rc;
+            (rc = launch_k(p, p->use_pdl, ly::k_softcap, dim3((unsigned)(((size_t)m * V + 255) / 256)), dim3(256), (size_t)0, Y.LOG, (long long)m * V, Y.c.logit_softcap))) return rc;
         CK(cudaMemcpyAsync(logits_out + (size_t)r0 * V, Y.LOG, (size_t)m * V * 4, cudaMemcpyDeviceToHost, p->stream));
         CK(cudaStreamSynchronize(p->stream));
     }

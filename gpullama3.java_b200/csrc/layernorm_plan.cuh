@@ -125,19 +125,19 @@ static int ly_enqueue_mlstm(b200_plan *p, bool decode, int n, const StepState *s
     const dim3 grid(s.heads, ly::mlstm_tiles(s.key_dim, s.value_dim)), block(MLSTM_THREADS);
     const float *P = Y.PROJ;
     switch (ly::mlstm_reg_rows(s.key_dim)) {
-    case 1: rc = launch_k(p, false, ly::k_mlstm_scan<1>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 2: rc = launch_k(p, false, ly::k_mlstm_scan<2>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 4: rc = launch_k(p, false, ly::k_mlstm_scan<4>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 8: rc = launch_k(p, false, ly::k_mlstm_scan<8>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 16: rc = launch_k(p, false, ly::k_mlstm_scan<16>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 32: rc = launch_k(p, false, ly::k_mlstm_scan<32>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    default: rc = launch_k(p, false, ly::k_mlstm_scan_any, grid, dim3(256), (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO);
+    case 1: rc = launch_k(p, p->use_pdl, ly::k_mlstm_scan<1>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 2: rc = launch_k(p, p->use_pdl, ly::k_mlstm_scan<2>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 4: rc = launch_k(p, p->use_pdl, ly::k_mlstm_scan<4>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 8: rc = launch_k(p, p->use_pdl, ly::k_mlstm_scan<8>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 16: rc = launch_k(p, p->use_pdl, ly::k_mlstm_scan<16>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 32: rc = launch_k(p, p->use_pdl, ly::k_mlstm_scan<32>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    default: rc = launch_k(p, p->use_pdl, ly::k_mlstm_scan_any, grid, dim3(256), (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO);
     }
     if (rc) return rc;
     const ly::HeadNormArgs ha{L.onorm, s.value_dim, 1, Y.DO + L.gd, s.heads, s.value_dim, Y.c.norm_eps};
     *nl += 2;
     // one row: eight heads per CTA, a warp each; a chunk has CTAs enough with one per row
-    return launch_k(p, false, ly::k_head_norm_gate, dim3(n, decode ? (s.heads + 7) / 8 : 1), dim3(256), (size_t)0, (const float *)Y.DO, Y.maxDO, (const float *)(Y.PROJ + L.g_off), Y.maxP, ha,
+    return launch_k(p, p->use_pdl, ly::k_head_norm_gate, dim3(n, decode ? (s.heads + 7) / 8 : 1), dim3(256), (size_t)0, (const float *)Y.DO, Y.maxDO, (const float *)(Y.PROJ + L.g_off), Y.maxP, ha,
                     h16 ? (float *)nullptr : Y.ATT32, h16 ? Y.ATT16 : (ly::bf16 *)nullptr, L.gd);
 }
 
@@ -206,11 +206,11 @@ static int ly_enqueue_layernorm(b200_plan *p, bool decode, int n, const StepStat
             if ((rc = ly_project<ly::EPI_STORE>(p, true, 1, Y.A32, nullptr, Y.head, nullptr, Y.c.vocab_size, E, p->logits, nullptr, Y.c.vocab_size, 0))) return rc;
             nl++;
             if (Y.c.logit_softcap > 0.0f) {
-                if ((rc = launch_k(p, false, ly::k_softcap, dim3((Y.c.vocab_size + 255) / 256), dim3(256), (size_t)0, p->logits, (long long)Y.c.vocab_size, Y.c.logit_softcap))) return rc;
+                if ((rc = launch_k(p, p->use_pdl, ly::k_softcap, dim3((Y.c.vocab_size + 255) / 256), dim3(256), (size_t)0, p->logits, (long long)Y.c.vocab_size, Y.c.logit_softcap))) return rc;
                 nl++;
             }
         }
-        if ((rc = launch_k(p, false, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
+        if ((rc = launch_k(p, p->use_pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
                            p->out_ids, with_head ? 1 : 0, (const float *)nullptr, (const int *)nullptr, 0, TraceBuf{nullptr, 0, 0}, p->tp, -1))) return rc;
         nl++;
     } else if ((rc = row(false, nullptr))) return rc;

@@ -34,6 +34,8 @@ __device__ __forceinline__ float siluf_(float z) { return z / (1.0f + expf(-z));
 template <int R>
 __global__ void __launch_bounds__(LIGHT_THREADS) k_lightning_scan(const float *__restrict__ P, int ldp, LightningArgs a, float *__restrict__ S, int n, const StepState *__restrict__ st,
                                                                   float *__restrict__ Y, int ldy) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int RW = R * 16, TB = R >= 32 ? 4 : R >= 16 ? 8 : 16, LB = TB * RW / LIGHT_THREADS;
     __shared__ __align__(16) float ks[2][TB][RW], qs[2][TB][RW];
     __shared__ float vs[2][TB][LIGHT_COLS];
@@ -163,6 +165,8 @@ __device__ __forceinline__ void split_bf16(float x, float y, unsigned &hi, unsig
 template <int DK, int COLS>
 __global__ void __launch_bounds__(4 * COLS) k_lightning_chunk(const bf16 *__restrict__ QKV, int ld, LightningArgs a, float *__restrict__ S, int n, const StepState *__restrict__ st,
                                                                 float *__restrict__ Y, int ldy) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) unsigned char lsm[];
     constexpr int T = LC_TOKENS, QW = DK + 8, VW = COLS + 8, LC_THREADS = 4 * COLS, LC_COLS = COLS;
     typedef bf16 QRow[QW];

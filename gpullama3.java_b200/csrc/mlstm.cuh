@@ -40,6 +40,8 @@ __device__ __forceinline__ float logsigmoidf_(float z) { return fminf(z, 0.0f) -
 template <int R>
 __global__ void __launch_bounds__(MLSTM_THREADS) k_mlstm_scan(const float *__restrict__ P, int ldp, MlstmArgs a, float *__restrict__ S, int n, const StepState *__restrict__ st,
                                                               float *__restrict__ Y, int ldy) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int RW = R * 16, TB = MLSTM_TB_OF(R);
     __shared__ __align__(16) float ks[2][TB][RW], qs[2][TB][RW];
     __shared__ float vs[2][TB][MLSTM_COLS], gs[2][2][16];
@@ -177,6 +179,8 @@ __global__ void __launch_bounds__(MLSTM_THREADS) k_mlstm_scan(const float *__res
 // [dk][dv + 1], then [head][tile] running maxima.
 __global__ void __launch_bounds__(256) k_mlstm_scan_any(const float *__restrict__ P, int ldp, MlstmArgs a, float *__restrict__ S, int n, const StepState *__restrict__ st,
                                                         float *__restrict__ Y, int ldy) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float part[8][33];
     const int h = blockIdx.x, tid = threadIdx.x, c = tid & 31, sl = tid >> 5, W = a.dv + 1, col = blockIdx.y * 32 + c;
     const bool live = col < W;

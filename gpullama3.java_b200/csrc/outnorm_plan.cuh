@@ -301,8 +301,8 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
         pend = ly_outnorm_args(Y, n);
         nl++;
         // a single row is one CTA: more threads keep more of its loads in flight
-        if (n == 1 && E >= 2048) return launch_k(p, false, ly::k_outnorm_rows<1024>, dim3(1), dim3(1024), (size_t)2 * E * 4, a);
-        return launch_k(p, false, ly::k_outnorm_rows<LY_NORM_THREADS>, dim3(n), dim3(LY_NORM_THREADS), (size_t)2 * E * 4, a);
+        if (n == 1 && E >= 2048) return launch_k(p, p->use_pdl, ly::k_outnorm_rows<1024>, dim3(1), dim3(1024), (size_t)2 * E * 4, a);
+        return launch_k(p, p->use_pdl, ly::k_outnorm_rows<LY_NORM_THREADS>, dim3(n), dim3(LY_NORM_THREADS), (size_t)2 * E * 4, a);
     };
     for (size_t r = 0; r < Y.runs.size(); r++) {
         const LyRun &R = Y.runs[r];
@@ -313,7 +313,7 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
         const bool inline_shift = n == 1 || !L.shift;
         if ((rc = post(n == 1 ? L.shift : nullptr, R.prev, nullptr, inline_shift))) return rc;
         if (!inline_shift) {
-            if ((rc = launch_k(p, false, ly::k_shift_rows, dim3(n), dim3(256), (size_t)0, (const float *)Y.X, E, (const float *)L.shift, (const float *)R.prev, st,
+            if ((rc = launch_k(p, p->use_pdl, ly::k_shift_rows, dim3(n), dim3(256), (size_t)0, (const float *)Y.X, E, (const float *)L.shift, (const float *)R.prev, st,
                                h16 ? (float *)nullptr : Y.A32, h16 ? Y.A16 : (ly::bf16 *)nullptr))) return rc;
             nl++;
         }
@@ -331,7 +331,7 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             ly::SliceNormRopeArgs sa{};
             sa.q_slices = pairs; sa.k_slices = s.kv_heads * maps; sa.dk = s.key_dim; sa.v_width = L.vd; sa.has_kv = R.own ? 1 : 0;
             sa.qnorm = L.qnorm; sa.knorm = L.knorm; sa.cs = L.rope; sa.rope_dims = s.rope_dims; sa.rope_layout = s.rope_layout; sa.eps = Y.c.norm_eps; sa.ring = Y.ring;
-            if ((rc = launch_k(p, false, ly::k_slice_norm_rope, dim3(n), dim3(256), (size_t)0, Y.PROJ, Y.maxP, sa, R.kc, R.vc, R.own ? R.kc16 : (ly::bf16 *)nullptr,
+            if ((rc = launch_k(p, p->use_pdl, ly::k_slice_norm_rope, dim3(n), dim3(256), (size_t)0, Y.PROJ, Y.maxP, sa, R.kc, R.vc, R.own ? R.kc16 : (ly::bf16 *)nullptr,
                                R.own ? R.vc16 : (ly::bf16 *)nullptr, st))) return rc;
             ly::WindowAttn wa{};
             wa.heads = pairs; wa.kv_heads = s.kv_heads; wa.dk = s.key_dim; wa.dv = s.value_dim; wa.window = s.window; wa.ring = Y.ring;
@@ -343,15 +343,15 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             if (h16 && R.kc16 && kind)
                 rc = ly_launch_mma(p, kind, n, pairs, s.window, Y.PROJ, Y.maxP, wa, (const ly::bf16 *)R.kc16, (const ly::bf16 *)R.vc16, st, Y.ATT16, ldo, maps > 1 ? Y.DO : (float *)nullptr);
             else if (h16 && maps == 1)
-                rc = launch_k(p, false, ly::k_window_attention<ly::bf16>, dim3(n, pairs), dim3(LY_ATT_THREADS), ly_att_smem(s.key_dim, s.window), (const float *)Y.PROJ, Y.maxP, wa,
+                rc = launch_k(p, p->use_pdl, ly::k_window_attention<ly::bf16>, dim3(n, pairs), dim3(LY_ATT_THREADS), ly_att_smem(s.key_dim, s.window), (const float *)Y.PROJ, Y.maxP, wa,
                               (const float *)R.kc, (const float *)R.vc, st, Y.ATT16, ldo, ly::KeySplit{nullptr, nullptr, nullptr});
             else if (decode) rc = ly_step_attention(p, pairs, s.window, Y.PROJ, Y.maxP, wa, R.kc, R.vc, st, o32, ldo, ly_att_smem(s.key_dim, s.window));
-            else rc = launch_k(p, false, ly::k_window_attention<float>, dim3(n, pairs), dim3(LY_ATT_THREADS), ly_att_smem(s.key_dim, s.window), (const float *)Y.PROJ, Y.maxP, wa,
+            else rc = launch_k(p, p->use_pdl, ly::k_window_attention<float>, dim3(n, pairs), dim3(LY_ATT_THREADS), ly_att_smem(s.key_dim, s.window), (const float *)Y.PROJ, Y.maxP, wa,
                                (const float *)R.kc, (const float *)R.vc, st, o32, ldo, ly::KeySplit{nullptr, nullptr, nullptr});
             if (rc) return rc;
             nl += 2;
             if (maps > 1) {
-                if ((rc = launch_k(p, false, ly::k_diff_combine, dim3(n), dim3(256), (size_t)0, (const float *)Y.DO, ldo, s.heads, s.value_dim, L.diff_lambda, 1.0f - s.diff_init, Y.c.norm_eps,
+                if ((rc = launch_k(p, p->use_pdl, ly::k_diff_combine, dim3(n), dim3(256), (size_t)0, (const float *)Y.DO, ldo, s.heads, s.value_dim, L.diff_lambda, 1.0f - s.diff_init, Y.c.norm_eps,
                                    att32, att16, L.gd))) return rc;
                 nl++;
             }
@@ -359,7 +359,7 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             const int W = L.qd, nb = s.heads, bs = s.value_dim;
             ly::ConvArgs ca{};
             ca.C = W; ca.taps = s.conv_taps; ca.cring = Y.cring; ca.w = L.conv_w; ca.bias_in = L.x_bias; ca.bias_out = L.conv_b; ca.silu = 0;
-            if ((rc = launch_k(p, false, ly::k_conv_rows, dim3((n + LY_CONV_ROWS - 1) / LY_CONV_ROWS, (W + 255) / 256), dim3(256), (size_t)0, (const float *)Y.PROJ, Y.maxP, 0, ca, R.cstate, Y.DLT, Y.maxD,
+            if ((rc = launch_k(p, p->use_pdl, ly::k_conv_rows, dim3((n + LY_CONV_ROWS - 1) / LY_CONV_ROWS, (W + 255) / 256), dim3(256), (size_t)0, (const float *)Y.PROJ, Y.maxP, 0, ca, R.cstate, Y.DLT, Y.maxD,
                                h16 ? Y.U16 : (ly::bf16 *)nullptr, Y.maxD, st, n))) return rc;
             { // gate logits of every block: [r | i] rows of the block's stacked matrix times the block's channels
                 ly::GemmView gv{};
@@ -371,9 +371,9 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             ly::RglruArgs ra{};
             ra.W = W; ra.blocks = nb; ra.gate_bias = L.gate_bias; ra.lam = L.lam; ra.y_bias = L.y_bias;
             // a chunk: 16 channels x up to 32 row groups per CTA (the last group may be short, never empty rows in between); few rows: 32 channels, one group
-            if (n >= 64) rc = launch_k(p, false, ly::k_rglru_scan<16, RGLRU_MAX_GROUPS>, dim3((W + 15) / 16), dim3(16 * RGLRU_MAX_GROUPS), (size_t)0, (const float *)Y.DLT, Y.maxD, (const float *)Y.Q, Y.maxQ,
+            if (n >= 64) rc = launch_k(p, p->use_pdl, ly::k_rglru_scan<16, RGLRU_MAX_GROUPS>, dim3((W + 15) / 16), dim3(16 * RGLRU_MAX_GROUPS), (size_t)0, (const float *)Y.DLT, Y.maxD, (const float *)Y.Q, Y.maxQ,
                                        (const float *)(Y.PROJ + W), Y.maxP, ra, R.S, n, st, att32, att16, L.gd);
-            else rc = launch_k(p, false, ly::k_rglru_scan<32, 1>, dim3((W + 31) / 32), dim3(32), (size_t)0, (const float *)Y.DLT, Y.maxD, (const float *)Y.Q, Y.maxQ,
+            else rc = launch_k(p, p->use_pdl, ly::k_rglru_scan<32, 1>, dim3((W + 31) / 32), dim3(32), (size_t)0, (const float *)Y.DLT, Y.maxD, (const float *)Y.Q, Y.maxQ,
                                (const float *)(Y.PROJ + W), Y.maxP, ra, R.S, n, st, att32, att16, L.gd);
             if (rc) return rc;
             nl += 3;
@@ -381,21 +381,21 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             const int inner = L.gd, gn = s.kv_heads * s.key_dim;
             ly::ConvArgs ca{};
             ca.C = L.dC; ca.taps = s.conv_taps; ca.cring = Y.cring; ca.w = L.conv_w; ca.bias_in = nullptr; ca.bias_out = L.conv_b; ca.silu = 1;
-            if ((rc = launch_k(p, false, ly::k_conv_rows, dim3((n + LY_CONV_ROWS - 1) / LY_CONV_ROWS, (L.dC + 255) / 256), dim3(256), (size_t)0, (const float *)Y.PROJ, Y.maxP, inner, ca, R.cstate, Y.DLT, Y.maxD,
+            if ((rc = launch_k(p, p->use_pdl, ly::k_conv_rows, dim3((n + LY_CONV_ROWS - 1) / LY_CONV_ROWS, (L.dC + 255) / 256), dim3(256), (size_t)0, (const float *)Y.PROJ, Y.maxP, inner, ca, R.cstate, Y.DLT, Y.maxD,
                                (ly::bf16 *)nullptr, 0, st, n))) return rc;
             ly::SsdArgs sa{};
             sa.heads = s.heads; sa.groups = s.kv_heads; sa.N = s.key_dim; sa.P = s.value_dim; sa.a_log = L.a_log; sa.dt_bias = L.dt_bias; sa.D = L.ssd_d;
             const dim3 grid(s.heads, (s.value_dim + SSD_COLS - 1) / SSD_COLS), block(SSD_THREADS);
             const float *dt = Y.PROJ + 2 * inner + 2 * gn;
             switch (ly::ssd_reg_rows(s.key_dim)) {
-            case 1: rc = launch_k(p, false, ly::k_ssd_scan<1>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
-            case 2: rc = launch_k(p, false, ly::k_ssd_scan<2>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
-            case 4: rc = launch_k(p, false, ly::k_ssd_scan<4>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
-            case 8: rc = launch_k(p, false, ly::k_ssd_scan<8>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
-            default: rc = launch_k(p, false, ly::k_ssd_scan<16>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO);
+            case 1: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<1>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
+            case 2: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<2>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
+            case 4: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<4>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
+            case 8: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<8>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
+            default: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<16>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO);
             }
             if (rc) return rc;
-            if ((rc = launch_k(p, false, ly::k_gated_group_norm, dim3(n), dim3(n == 1 && inner >= 2048 ? 1024 : 256), (size_t)inner * 4, (const float *)Y.DO, Y.maxDO, (const float *)Y.PROJ, Y.maxP, (const float *)L.onorm, inner,
+            if ((rc = launch_k(p, p->use_pdl, ly::k_gated_group_norm, dim3(n), dim3(n == 1 && inner >= 2048 ? 1024 : 256), (size_t)inner * 4, (const float *)Y.DO, Y.maxDO, (const float *)Y.PROJ, Y.maxP, (const float *)L.onorm, inner,
                                s.mixer_norm_groups, Y.c.norm_eps, 0, att32, att16, L.gd))) return rc;
             nl += 3;
         }
@@ -413,7 +413,7 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
                 if (Y.tc && h16 && L.tc_gu) { // tcgen05 product into the FP32 projection buffer, then the activation into the next operand
                     LyTc t_up; t_up.a = &Y.m_a; t_up.b = &L.m_up; t_up.c = &Y.m_proj_c;
                     if ((rc = ly_project<ly::EPI_STORE>(p, false, n, nullptr, Y.A16, L.w_gu, nullptr, F, E, Y.PROJ, nullptr, Y.maxP, 0, &t_up))) return rc;
-                    if ((rc = launch_k(p, false, ly::k_act_rows, dim3(n), dim3(256), (size_t)0, (const float *)Y.PROJ, Y.maxP, F, s.ff_act, Y.H16, F, ly::TokenGate{}))) return rc;
+                    if ((rc = launch_k(p, p->use_pdl, ly::k_act_rows, dim3(n), dim3(256), (size_t)0, (const float *)Y.PROJ, Y.maxP, F, s.ff_act, Y.H16, F, ly::TokenGate{}))) return rc;
                     nl += 2;
                 } else {
                     if ((rc = ly_project<ly::EPI_ACT>(p, decode, n, x32, Y.A16, L.w_gu, nullptr, F, E, Y.H32, h16 ? Y.H16 : nullptr, F, s.ff_act))) return rc;
@@ -455,7 +455,7 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             if ((rc = ly_project<ly::EPI_STORE>(p, true, 1, Y.A32, nullptr, Y.head, nullptr, Y.c.vocab_size, E, p->logits, nullptr, Y.c.vocab_size, 0))) return rc;
             nl++;
         } else if ((rc = post(nullptr, nullptr, nullptr, false))) return rc;
-        if ((rc = launch_k(p, false, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
+        if ((rc = launch_k(p, p->use_pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
                            p->out_ids, with_head ? 1 : 0, (const float *)nullptr, (const int *)nullptr, 0, TraceBuf{nullptr, 0, 0}, p->tp, -1))) return rc;
         nl++;
     } else if ((rc = post(nullptr, nullptr, nullptr, false))) return rc;

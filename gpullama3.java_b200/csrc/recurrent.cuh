@@ -100,6 +100,8 @@ __device__ __forceinline__ void group_inv_rms(const float *v, int E, int groups,
 // One CTA of NTH threads per row.  Dynamic shared memory: 2 * E floats.
 template <int NTH>
 __global__ void __launch_bounds__(NTH, 1) k_outnorm_rows(OutNormArgs a) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float smo[];
     __shared__ float red[32];
     __shared__ float inv[LY_OUTNORM_MAX_GROUPS];
@@ -223,6 +225,8 @@ __global__ void __launch_bounds__(NTH, 1) k_outnorm_rows(OutNormArgs a) {
 // `prev` (kept by an earlier call), zeros at position 0.  grid (n), 256 threads.
 __global__ void __launch_bounds__(256) k_shift_rows(const float *__restrict__ x, int E, const float *__restrict__ shift, const float *__restrict__ prev,
                                                     const StepState *__restrict__ st, float *__restrict__ out32, bf16 *__restrict__ out16) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.x;
     const bool zero = r == 0 && st->pos == 0;
     const float *p = r > 0 ? x + (size_t)(r - 1) * E : prev;
@@ -236,6 +240,8 @@ __global__ void __launch_bounds__(256) k_shift_rows(const float *__restrict__ x,
 
 // Activation over FP32 rows: out[r][i] = act(in[r * ldi + i]) (times the entry of the row's token, with a table), i < F.  grid (n), 256 threads.
 __global__ void __launch_bounds__(256) k_act_rows(const float *__restrict__ in, int ldi, int F, int act, bf16 *__restrict__ out16, int ldo, TokenGate tg) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.x;
     for (int i = threadIdx.x; i < F; i += 256) {
         float v = act_apply(act, in[(size_t)r * ldi + i]);
@@ -261,6 +267,8 @@ struct ConvArgs {
 #define LY_CONV_ROWS 4 // consecutive rows of a channel per thread: their loads are independent and in flight together
 __global__ void __launch_bounds__(256) k_conv_rows(const float *__restrict__ P, int ldp, int c_off, ConvArgs a, float *__restrict__ cstate, float *__restrict__ out32, int ldo,
                                                    bf16 *__restrict__ out16, int ldo16, const StepState *__restrict__ st, int n) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r0 = blockIdx.x * LY_CONV_ROWS, c = blockIdx.y * 256 + threadIdx.x;
     if (c >= a.C) return;
     const float bi = a.bias_in ? a.bias_in[c] : 0.0f, bo = a.bias_out ? a.bias_out[c] : 0.0f;
@@ -330,6 +338,8 @@ template <int CW, int MAXG> // MAXG = 1: the one-group form only (a launch of CW
 __global__ void __launch_bounds__(CW * MAXG) k_rglru_scan(const float *__restrict__ U, int ldu, const float *__restrict__ G, int ldg, const float *__restrict__ PY, int ldp,
                                                                       RglruArgs a, float *__restrict__ S, int n, const StepState *__restrict__ st, float *__restrict__ out32,
                                                                       bf16 *__restrict__ out16, int ldo) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float cA[MAXG][CW], cB[MAXG][CW];
     const int cl = threadIdx.x % CW, g = threadIdx.x / CW, c = blockIdx.x * CW + cl, groups = blockDim.x / CW;
     const bool live = c < a.W;
@@ -459,6 +469,8 @@ __device__ __forceinline__ void ssd_rows(const float *tile, int slice, float (&v
 template <int R>
 __global__ void __launch_bounds__(SSD_THREADS) k_ssd_scan(const float *__restrict__ XBC, int ldx, const float *__restrict__ DT, int lddt, SsdArgs a, float *__restrict__ S, int n,
                                                           const StepState *__restrict__ st, float *__restrict__ Y, int ldy) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int RW = R * 16;                  // staged state rows per token (rows beyond N are zero)
     constexpr int SSD_TB = SSD_TB_OF(R);
     constexpr int LB = SSD_TB * R / 16;         // elements of a batch's B (or C) tile per thread
@@ -555,6 +567,8 @@ __global__ void __launch_bounds__(SSD_THREADS) k_ssd_scan(const float *__restric
 // One CTA per row (any multiple of 32 threads), dynamic shared memory: n_in floats.
 __global__ void __launch_bounds__(1024) k_gated_group_norm(const float *__restrict__ Yv, int ldy, const float *__restrict__ Z, int ldz, const float *__restrict__ w, int n_in,
                                                           int groups, float eps, int sigmoid_after, float *__restrict__ out32, bf16 *__restrict__ out16, int ldo) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) float gv[];
     __shared__ float red[32];
     __shared__ float inv[LY_OUTNORM_MAX_GROUPS];
@@ -592,6 +606,8 @@ struct SliceNormRopeArgs {
 };
 __global__ void __launch_bounds__(256) k_slice_norm_rope(float *__restrict__ P, int ldp, SliceNormRopeArgs a, float *__restrict__ kc, float *__restrict__ vc, bf16 *__restrict__ kc16,
                                                          bf16 *__restrict__ vc16, const StepState *__restrict__ st) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int pos = st->pos + r, half = a.rope_dims / 2, slot = pos % a.ring;
     const int kd = a.k_slices * a.dk, qd = a.q_slices * a.dk;
@@ -636,6 +652,8 @@ __global__ void __launch_bounds__(256) k_slice_norm_rope(float *__restrict__ P, 
 // over the head's dv values times out_scale.  One CTA per row, a warp per head.
 __global__ void __launch_bounds__(256) k_diff_combine(const float *__restrict__ A, int lda, int heads, int dv, float lambda, float out_scale, float eps, float *__restrict__ out32,
                                                       bf16 *__restrict__ out16, int ldo) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int h = warp; h < heads; h += 8) {
         const float *a1 = A + (size_t)r * lda + (size_t)h * 2 * dv, *a2 = a1 + dv;

@@ -228,31 +228,31 @@ static int ly_enqueue_lightning(b200_plan *p, bool decode, int n, const StepStat
     const float *P = Y.PROJ;
     if (h16 && L.chunkwise && n >= LC_CHUNK_MIN) {
         const int w = 2 * L.qd + L.vd;
-        if ((rc = launch_k(p, false, ly::k_act_rows, dim3(n), dim3(256), (size_t)0, P, Y.maxP, w, (int)ly::ACT_SILU, Y.LQ16, w, ly::TokenGate{}))) return rc;
+        if ((rc = launch_k(p, p->use_pdl, ly::k_act_rows, dim3(n), dim3(256), (size_t)0, P, Y.maxP, w, (int)ly::ACT_SILU, Y.LQ16, w, ly::TokenGate{}))) return rc;
         const bool wide = s.heads * ((s.value_dim + 63) / 64) >= p->n_sms;
         const int cols = wide ? 64 : 32;
         const dim3 cgrid(s.heads, (s.value_dim + cols - 1) / cols), cblock(4 * cols);
         const ly::bf16 *qkv = Y.LQ16;
 #define LY_CHUNK_CASE(DK) \
-        if (s.key_dim == DK) rc = wide ? launch_k(p, false, ly::k_lightning_chunk<DK, 64>, cgrid, cblock, ly::lightning_chunk_smem<DK, 64>(), qkv, w, a, R.S, n, st, Y.DO, Y.maxDO) \
-                                       : launch_k(p, false, ly::k_lightning_chunk<DK, 32>, cgrid, cblock, ly::lightning_chunk_smem<DK, 32>(), qkv, w, a, R.S, n, st, Y.DO, Y.maxDO);
+        if (s.key_dim == DK) rc = wide ? launch_k(p, p->use_pdl, ly::k_lightning_chunk<DK, 64>, cgrid, cblock, ly::lightning_chunk_smem<DK, 64>(), qkv, w, a, R.S, n, st, Y.DO, Y.maxDO) \
+                                       : launch_k(p, p->use_pdl, ly::k_lightning_chunk<DK, 32>, cgrid, cblock, ly::lightning_chunk_smem<DK, 32>(), qkv, w, a, R.S, n, st, Y.DO, Y.maxDO);
         LY_CHUNK_CASE(32)
         LY_CHUNK_CASE(64)
         LY_CHUNK_CASE(128)
 #undef LY_CHUNK_CASE
         ++*nl;
     } else switch (ly::lightning_reg_rows(s.key_dim)) {
-    case 1: rc = launch_k(p, false, ly::k_lightning_scan<1>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 2: rc = launch_k(p, false, ly::k_lightning_scan<2>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 4: rc = launch_k(p, false, ly::k_lightning_scan<4>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 8: rc = launch_k(p, false, ly::k_lightning_scan<8>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    case 16: rc = launch_k(p, false, ly::k_lightning_scan<16>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
-    default: rc = launch_k(p, false, ly::k_lightning_scan<32>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO);
+    case 1: rc = launch_k(p, p->use_pdl, ly::k_lightning_scan<1>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 2: rc = launch_k(p, p->use_pdl, ly::k_lightning_scan<2>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 4: rc = launch_k(p, p->use_pdl, ly::k_lightning_scan<4>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 8: rc = launch_k(p, p->use_pdl, ly::k_lightning_scan<8>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    case 16: rc = launch_k(p, p->use_pdl, ly::k_lightning_scan<16>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO); break;
+    default: rc = launch_k(p, p->use_pdl, ly::k_lightning_scan<32>, grid, block, (size_t)0, P, Y.maxP, a, R.S, n, st, Y.DO, Y.maxDO);
     }
     if (rc) return rc;
     *nl += 2;
     // one statistic over all heads
-    return launch_k(p, false, ly::k_gated_group_norm, dim3(n), dim3(n == 1 && L.gd >= 2048 ? 1024 : 256), (size_t)L.gd * 4, (const float *)Y.DO, Y.maxDO, (const float *)(Y.PROJ + 2 * L.qd + L.vd), Y.maxP,
+    return launch_k(p, p->use_pdl, ly::k_gated_group_norm, dim3(n), dim3(n == 1 && L.gd >= 2048 ? 1024 : 256), (size_t)L.gd * 4, (const float *)Y.DO, Y.maxDO, (const float *)(Y.PROJ + 2 * L.qd + L.vd), Y.maxP,
                     (const float *)L.onorm, L.gd, 1, Y.c.norm_eps, 1, h16 ? (float *)nullptr : Y.ATT32, h16 ? Y.ATT16 : (ly::bf16 *)nullptr, L.gd);
 }
 
@@ -265,7 +265,7 @@ static int ly_enqueue_selective(b200_plan *p, bool decode, int n, const StepStat
     int rc;
     ly::ConvArgs ca{};
     ca.C = I; ca.taps = s.conv_taps; ca.cring = Y.cring; ca.w = L.conv_w; ca.bias_out = L.conv_b; ca.silu = 1;
-    if ((rc = launch_k(p, false, ly::k_conv_rows, dim3((n + LY_CONV_ROWS - 1) / LY_CONV_ROWS, (I + 255) / 256), dim3(256), (size_t)0, (const float *)Y.PROJ, Y.maxP, L.x_off, ca, R.cstate, Y.DLT, Y.maxD,
+    if ((rc = launch_k(p, p->use_pdl, ly::k_conv_rows, dim3((n + LY_CONV_ROWS - 1) / LY_CONV_ROWS, (I + 255) / 256), dim3(256), (size_t)0, (const float *)Y.PROJ, Y.maxP, L.x_off, ca, R.cstate, Y.DLT, Y.maxD,
                        h16 ? Y.U16 : (ly::bf16 *)nullptr, Y.maxD, st, n))) return rc;
     if (h16 && Y.tc && L.tc_wx) {
         LyTc t; t.a = &L.m_u; t.b = &L.m_wx; t.c = &Y.m_xp_c;
@@ -280,7 +280,7 @@ static int ly_enqueue_selective(b200_plan *p, bool decode, int n, const StepStat
     if (!one) { // step sizes of the chunk; a single row's are computed inside the scan
         ly::GemmView gv{};
         if (h16) {
-            if ((rc = launch_k(p, false, ly::k_act_rows, dim3(n), dim3(256), (size_t)0, (const float *)Y.XP, Y.maxX, Rk, (int)ly::ACT_NONE, Y.DT16, Rk, ly::TokenGate{}))) return rc;
+            if ((rc = launch_k(p, p->use_pdl, ly::k_act_rows, dim3(n), dim3(256), (size_t)0, (const float *)Y.XP, Y.maxX, Rk, (int)ly::ACT_NONE, Y.DT16, Rk, ly::TokenGate{}))) return rc;
             ++*nl;
         }
         ++*nl;
@@ -304,16 +304,16 @@ static int ly_enqueue_selective(b200_plan *p, bool decode, int n, const StepStat
     ly::bf16 *o16 = h16 ? Y.ATT16 + L.ad : nullptr;
     const int rr = ly::sel_reg_rows(N);
     if (lpc > SEL_LANES) {
-        if (rr == 8) return launch_k(p, false, ly::k_selective_scan<32, 8>, grid, block, ly::sel_smem(32, 8), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
-        return launch_k(p, false, ly::k_selective_scan<32, 16>, grid, block, ly::sel_smem(32, 16), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
+        if (rr == 8) return launch_k(p, p->use_pdl, ly::k_selective_scan<32, 8>, grid, block, ly::sel_smem(32, 8), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
+        return launch_k(p, p->use_pdl, ly::k_selective_scan<32, 16>, grid, block, ly::sel_smem(32, 16), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
     }
     switch (rr) {
-    case 1: return launch_k(p, false, ly::k_selective_scan<SEL_LANES, 1>, grid, block, ly::sel_smem(SEL_LANES, 1), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
-    case 2: return launch_k(p, false, ly::k_selective_scan<SEL_LANES, 2>, grid, block, ly::sel_smem(SEL_LANES, 2), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
-    case 4: return launch_k(p, false, ly::k_selective_scan<SEL_LANES, 4>, grid, block, ly::sel_smem(SEL_LANES, 4), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
-    case 8: return launch_k(p, false, ly::k_selective_scan<SEL_LANES, 8>, grid, block, ly::sel_smem(SEL_LANES, 8), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
-    case 16: return launch_k(p, false, ly::k_selective_scan<SEL_LANES, 16>, grid, block, ly::sel_smem(SEL_LANES, 16), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
-    default: return launch_k(p, false, ly::k_selective_scan<SEL_LANES, 32>, grid, block, ly::sel_smem(SEL_LANES, 32), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
+    case 1: return launch_k(p, p->use_pdl, ly::k_selective_scan<SEL_LANES, 1>, grid, block, ly::sel_smem(SEL_LANES, 1), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
+    case 2: return launch_k(p, p->use_pdl, ly::k_selective_scan<SEL_LANES, 2>, grid, block, ly::sel_smem(SEL_LANES, 2), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
+    case 4: return launch_k(p, p->use_pdl, ly::k_selective_scan<SEL_LANES, 4>, grid, block, ly::sel_smem(SEL_LANES, 4), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
+    case 8: return launch_k(p, p->use_pdl, ly::k_selective_scan<SEL_LANES, 8>, grid, block, ly::sel_smem(SEL_LANES, 8), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
+    case 16: return launch_k(p, p->use_pdl, ly::k_selective_scan<SEL_LANES, 16>, grid, block, ly::sel_smem(SEL_LANES, 16), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
+    default: return launch_k(p, p->use_pdl, ly::k_selective_scan<SEL_LANES, 32>, grid, block, ly::sel_smem(SEL_LANES, 32), U, Y.maxD, PX, Y.maxX, DT, Y.maxQ, Z, Y.maxP, a, R.S, n, st, o32, o16, L.gd);
     }
 }
 
@@ -362,7 +362,7 @@ static int ly_enqueue_side(b200_plan *p, bool decode, int n, const StepState *st
         LyTc t, t2;
         t.a = &Y.m_a; t.b = &L.m_tsg; t.c = &Y.m_sidef_c;
         if ((rc = ly_project<ly::EPI_STORE>(p, false, n, nullptr, Y.A16, L.w_sgate, nullptr, Y.side_pad, E, Y.SIDEF, nullptr, Y.side_pad, 0, &t))) return rc;
-        if ((rc = launch_k(p, false, ly::k_act_rows, dim3(n), dim3(256), (size_t)0, (const float *)Y.SIDEF, Y.side_pad, D, (int)ly::ACT_GELU_TANH, Y.SIDE16, D, tg))) return rc;
+        if ((rc = launch_k(p, p->use_pdl, ly::k_act_rows, dim3(n), dim3(256), (size_t)0, (const float *)Y.SIDEF, Y.side_pad, D, (int)ly::ACT_GELU_TANH, Y.SIDE16, D, tg))) return rc;
         t2.a = &Y.m_side; t2.b = &L.m_tsp; t2.c = &Y.m_y_c;
         ++*nl;
         return ly_project<ly::EPI_STORE>(p, false, n, nullptr, Y.SIDE16, L.w_sproj, nullptr, E, D, Y.Y, nullptr, E, 0, &t2);

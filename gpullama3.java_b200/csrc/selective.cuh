@@ -86,6 +86,8 @@ template <int LPC, int R>
 __global__ void __launch_bounds__(SEL_BLOCK) k_selective_scan(const float *__restrict__ U, int ldu, const float *__restrict__ PX, int ldx, const float *__restrict__ DT, int lddt,
                                                                 const float *__restrict__ Z, int ldz, SelScanArgs a, float *__restrict__ S, int n, const StepState *__restrict__ st,
                                                                 float *__restrict__ out32, bf16 *__restrict__ out16, int ldo) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int CH = SEL_THREADS / LPC, RW = LPC * R, TB = sel_tb(LPC), RP = (R + 1) / 2;
     extern __shared__ __align__(16) float selm[];
     typedef float CRow[CH];
