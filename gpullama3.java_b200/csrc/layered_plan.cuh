@@ -377,6 +377,19 @@ static int ly_step_attention(b200_plan *p, int heads, int window, const float *q
                     sp > 1 ? Y.split : ly::KeySplit{nullptr, nullptr, nullptr});
 }
 
+// k_qk_prep_reg for rows of whole, aligned float4 without rotation and of at most 8192 entries of q | k | v, else k_qk_prep; a single row takes more threads
+static int ly_launch_qk_prep(b200_plan *p, int n, const LyLayer &L, const LyRun &R, const ly::WindowAttn &wa, const StepState *st) {
+    Layered &Y = *p->ly;
+    auto go = [&](auto kern, int threads) {
+        return launch_k(p, p->use_pdl, kern, dim3(n), dim3(threads), (size_t)0, Y.PROJ, Y.maxP, wa, (const float *)L.b_proj, R.kc, R.vc, R.kc16, R.vc16, st);
+    };
+    const int all = L.qd + L.kd + L.vd;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(wa.qnorm) | reinterpret_cast<uintptr_t>(wa.knorm) | reinterpret_cast<uintptr_t>((const float *)L.b_proj)) & 15) == 0;
+    if (wa.rope_dims == 0 && (L.qd | L.kd | L.vd | Y.maxP) % 4 == 0 && all <= 8192 && aligned)
+        return n == 1 && all > 2048 ? go(ly::k_qk_prep_reg<1024, 2>, 1024) : all <= 4096 ? go(ly::k_qk_prep_reg<256, 4>, 256) : go(ly::k_qk_prep_reg<512, 4>, 512);
+    return n == 1 && L.qd + L.kd >= 1024 ? go(ly::k_qk_prep<1024>, 1024) : go(ly::k_qk_prep<256>, 256);
+}
+
 // Attention of one layer with its own rings, from the projection rows in PROJ to the (gated) heads in ATT32 / ATT16 (row stride L.gd).
 static int ly_enqueue_attention(b200_plan *p, bool decode, int n, const StepState *st, const LyRun &R, const LyLayer &L, int *nl) {
     Layered &Y = *p->ly;
@@ -394,8 +407,7 @@ static int ly_enqueue_attention(b200_plan *p, bool decode, int n, const StepStat
         rc = launch_k(p, p->use_pdl, ly::k_rope_mix_prep, dim3(n, (L.s.heads + hpc - 1) / hpc + 1), dim3(ROPE_MIX_THREADS), (size_t)(L.qd > L.kd ? L.qd : L.kd) * 4, (const float *)Y.PROJ, Y.maxP, ra,
                       (const float *)L.b_proj, Y.Q, ldq, R.kc, R.vc, R.kc16, R.vc16, st, hpc);
     } else
-        rc = n == 1 && L.qd + L.kd >= 1024 ? launch_k(p, p->use_pdl, ly::k_qk_prep<1024>, dim3(1), dim3(1024), (size_t)0, Y.PROJ, Y.maxP, wa, (const float *)L.b_proj, R.kc, R.vc, R.kc16, R.vc16, st)
-           : launch_k(p, p->use_pdl, ly::k_qk_prep<256>, dim3(n), dim3(256), (size_t)0, Y.PROJ, Y.maxP, wa, (const float *)L.b_proj, R.kc, R.vc, R.kc16, R.vc16, st);
+        rc = ly_launch_qk_prep(p, n, L, R, wa, st);
     if (rc) return rc;
     ++*nl;
     const size_t asm_ = ly_att_smem(L.s, Y.ring);

@@ -68,3 +68,13 @@ def test_argmax(pkg, vocab):
             assert am == int(np.argmax(lg))
     finally:
         plan.free()
+
+
+# q | k | v of a row in registers (k_qk_prep_reg): 2048, 4096 and 8192 entries, one step more, which takes the next kernel or the general one
+@pytest.mark.parametrize("heads,kv,dk,dv", [(14, 1, 128, 128), (14, 1, 128, 132), (16, 8, 128, 128), (16, 8, 128, 132), (48, 8, 128, 128), (48, 8, 128, 132)])
+def test_projection_rows(pkg, heads, kv, dk, dv):
+    S = pkg.synth
+    cfg = S.pibidra_config(64, 96, [S.pibidra_layer(heads, kv, dk, dv, 12, None)])
+    w = S.pibidra_weights(cfg, heads, bias_rows=4)
+    got, ref = decode_behind(pkg, cfg, w, 20, 3, 8)
+    assert_rows(got, ref, TOL_DECODE)
