@@ -18,6 +18,9 @@
 // apart modulo 128 so the row groups of a warp hit different banks.
 //   SF_GATEUP: half of the warp's row slots are ffn_gate rows, the other half the same rows of ffn_up; SwiGLU (InferenceCore.java:150-158)
 //   is applied in the epilogue, so w1, w3 and the SwiGLU kernel of the round-1 FP16 graph collapse into one launch.
+// What set the pace of a warp was not the copies but the work around them: positions computed with four divisions an item, and eight loads at a time in front of
+// their products (48 registers, by the compiler's choice).  With positions carried along, sixteen loads ahead and up to 128 registers, steps of two layers at
+// position 8 went from 326 to 246 us (8B), 151 to 108 us (1B); three layers of 1536 columns 156 to 118 us.
 // PDL: the rings are filled before griddepcontrol.wait (weights are immutable); x, and out in SF_RESID, are touched only after it.
 #pragma once
 #include "stream_matvec.cuh"
@@ -89,7 +92,7 @@ __device__ __forceinline__ unsigned f16x2_flush_subnormals(unsigned w) { // both
 
 // E > 0: the RMSNorm of the activation happens here too (fused_norm.cuh); E == 0: x is finished.
 template <int L, int MODE, int E = 0>
-__global__ void __launch_bounds__(SF_THREADS) k_stream_matvec_f16(SfArgs a) {
+__global__ void __launch_bounds__(SF_THREADS, 2) k_stream_matvec_f16(SfArgs a) {
     constexpr int LPR = L / 2;         // lanes per row (a lane owns chains 2u and 2u+1)
     constexpr int RW = 32 / LPR;       // row slots per warp
     constexpr int MR = MODE == SF_GATEUP ? RW / 2 : RW; // matrix rows per warp step
@@ -111,18 +114,23 @@ __global__ void __launch_bounds__(SF_THREADS) k_stream_matvec_f16(SfArgs a) {
     const size_t row_bytes = (size_t)a.cols * 2;
     const unsigned long long pol = l2_policy_evict_first();
 
-    auto issue = [&](int k) { // lane 0 only
-        const int st = k % S, gi = k / nseg, s = k - gi * nseg;
-        const size_t row0 = (size_t)(gw + gi * G) * MR;
-        const unsigned bar = bar0 + 8u * st;
+    // Positions of the next stage to fetch and to consume are carried along: computed from the item number (four divisions an item) they, not the copies,
+    // set the pace of a warp.
+    int f_k = 0, f_st = 0, f_s = 0;
+    size_t f_off = (size_t)gw * MR * row_bytes; // bytes from the first row slot's matrix
+    const size_t f_next = (size_t)(G * MR - 1) * row_bytes; // from the end of a row to the warp's next group
+    auto issue = [&]() { // lane 0 only
+        const unsigned bar = bar0 + 8u * f_st, dst = ring_u + f_st * stage_b;
         mbar_expect_tx(bar, RW * (unsigned)seg * 2u);
 #pragma unroll
         for (int r = 0; r < RW; r++) {
-            const __half *m = (MODE == SF_GATEUP && r >= MR) ? a.w1 : a.w0;
-            const size_t row = row0 + (MODE == SF_GATEUP ? r % MR : r);
-            bulk_g2s_evict_first(ring_u + st * stage_b + r * row_b, reinterpret_cast<const unsigned char *>(m) + row * row_bytes + (size_t)s * seg * 2,
-                                 (unsigned)seg * 2u, bar, pol);
+            const unsigned char *m = reinterpret_cast<const unsigned char *>(MODE == SF_GATEUP && r >= MR ? a.w1 : a.w0);
+            bulk_g2s_evict_first(dst + r * row_b, m + (MODE == SF_GATEUP ? r % MR : r) * row_bytes + f_off, (unsigned)seg * 2u, bar, pol);
         }
+        f_k++;
+        f_off += (unsigned)seg * 2u;
+        if (++f_s == nseg) { f_s = 0; f_off += f_next; }
+        if (++f_st == S) f_st = 0;
     };
 
     if (lane == 0) {
@@ -133,7 +141,7 @@ __global__ void __launch_bounds__(SF_THREADS) k_stream_matvec_f16(SfArgs a) {
     trace_entry(a.tr);
     pdl_launch_dependents();
     if (lane == 0)
-        for (int k = 0; k < S && k < n_items; k++) issue(k);
+        while (f_k < S && f_k < n_items) issue();
     constexpr bool W_EARLY = E > 0 && E <= 16;
     float nw[E > 0 ? E : 1];
     if constexpr (W_EARLY) norm_weights<E>(a.norm, a.cols, nw, tid); // immutable: on their way while the kernel in front still runs
@@ -161,29 +169,41 @@ __global__ void __launch_bounds__(SF_THREADS) k_stream_matvec_f16(SfArgs a) {
     float acc0 = 0.0f, acc1 = 0.0f; // chains 2u and 2u+1 of row slot r
     float best = -INFINITY;          // (a lane's rows ascend, so a strict comparison keeps the first maximum)
     int best_i = 0x7fffffff;
+    int st = 0, sg = 0;
+    unsigned phase = 0;
+    size_t row = (size_t)gw * MR + (MODE == SF_GATEUP ? r % MR : r);
     for (int k = 0; k < n_items; k++) {
-        const int st = k % S, gi = k / nseg, s = k - gi * nseg;
-        mbar_wait(bar0 + 8u * st, (unsigned)(k / S) & 1u);
+        mbar_wait(bar0 + 8u * st, phase);
         const unsigned *wr = reinterpret_cast<const unsigned *>(ring + st * stage_b + r * row_b) + u; // half2 (L j + 2u, L j + 2u + 1)
-        const float2 *xs = reinterpret_cast<const float2 *>(sx + s * seg) + u;
-#pragma unroll 8
-        for (int j = 0; j < seg / L; j++) {
-            const unsigned w2 = f16x2_flush_subnormals(wr[j * LPR]);
-            const float2 xv = xs[j * LPR];
-            const __half2 h2 = *reinterpret_cast<const __half2 *>(&w2);
-            acc0 = fmaf(__low2float(h2), xv.x, acc0);
-            acc1 = fmaf(__high2float(h2), xv.y, acc1);
+        const float2 *xs = reinterpret_cast<const float2 *>(sx + sg * seg) + u;
+#pragma unroll 1
+        for (int j = 0; j < seg / L; j += 16) { // (seg is a multiple of 256) sixteen loads ahead of the chain of products
+            unsigned w[16];
+            float2 xv[16];
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                w[i] = wr[(j + i) * LPR];
+                xv[i] = xs[(j + i) * LPR];
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                const unsigned w2 = f16x2_flush_subnormals(w[i]);
+                const __half2 h2 = *reinterpret_cast<const __half2 *>(&w2);
+                acc0 = fmaf(__low2float(h2), xv[i].x, acc0);
+                acc1 = fmaf(__high2float(h2), xv[i].y, acc1);
+            }
         }
         __syncwarp(); // every lane has consumed the stage: lane 0 may overwrite it
-        if (lane == 0 && k + S < n_items) issue(k + S);
-        if (s == nseg - 1) {
+        if (lane == 0 && f_k < n_items) issue();
+        if (++st == S) { st = 0; phase ^= 1u; }
+        if (++sg == nseg) {
+            sg = 0;
             float result = 0.0f; // reduceLanes(ADD): ascending lanes from the identity
 #pragma unroll
             for (int q = 0; q < LPR; q++) {
                 result = __fadd_rn(result, __shfl_sync(0xffffffffu, acc0, r * LPR + q));
                 result = __fadd_rn(result, __shfl_sync(0xffffffffu, acc1, r * LPR + q));
             }
-            const size_t row = (size_t)(gw + gi * G) * MR + (MODE == SF_GATEUP ? r % MR : r);
             if (MODE == SF_GATEUP) {
                 const float up = __shfl_sync(0xffffffffu, result, ((r + MR) % RW) * LPR);
                 if (r < MR && u == 0) a.out[row] = swiglu(result, up);
@@ -192,6 +212,7 @@ __global__ void __launch_bounds__(SF_THREADS) k_stream_matvec_f16(SfArgs a) {
                 if (MODE == SF_STORE && result > best) { best = result; best_i = (int)row; }
             }
             acc0 = acc1 = 0.0f;
+            row += (size_t)G * MR;
         }
     }
     if (MODE == SF_STORE && a.part_val) { // uniform over the grid
