@@ -499,7 +499,8 @@ template <typename F> int by_norm_terms(int dim, F &&f) { // f(integral_constant
 }
 template <typename... KA, typename... A> int launch_cluster(b200_plan *p, bool pdl, int cluster, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args);
 // Widest row whose norm the FP16 streaming matvecs compute themselves.  They run two CTAs per SM, which share its issue slots during the norm, and the norm's
-// scratch takes stages from their rings: measured on two layers at position 8 (rows of 1536: three), separate -> inside: dim 1536 188 -> 160 us, 2048 160 -> 152, 3072 208 -> 200, 4096 325 -> 344.
+// scratch takes stages from their rings.  Measured at position 8, separate -> inside: three layers of 1536 entries 188 -> 160 us, two of 2048 160 -> 152,
+// two of 3072 208 -> 200; two of 4096 342 -> 344, where the launch is kept.
 const int SF_NORM_MAX_DIM = 3072;
 int sf_grid(const b200_plan *p, int rows, int cols, bool gateup, bool norm) { // CTAs of an FP16 streaming launch
     const int lanes = p->cfg.fp16_lanes;

@@ -200,7 +200,7 @@ class B200MasterPlan:
         return self._native.prefill_info()
 
     # -Dllama.cudaGraphs-style switch of the decode implementation (both bit-identical): "graph" = one CUDA graph of
-    # ~7 kernels per layer, "persistent" = one persistent kernel per token (csrc/decode_persistent.cuh)
+    # 5 to 7 kernels per layer, "persistent" = one persistent kernel per token (csrc/decode_persistent.cuh)
     DECODE_GRAPH, DECODE_PERSISTENT = 0, 1
 
     def set_decode_mode(self, mode):
