@@ -826,13 +826,15 @@ __global__ void __launch_bounds__(NTH) k_qk_prep(float *__restrict__ P, int ldp,
 }
 
 // The same without rotation, for rows of whole float4: every entry of q | k | v is read once, all loads of a thread in flight together, and stays in registers over
-// the one reduction.  k_qk_prep is bound by its chain of three dependent passes, not by bytes.  q 4096, k 1024, v 1024: one row 8.4 -> 5.6 us, 512 rows 15.5 -> 10.4 us.
-template <int NTH, int VPT>
+// the one reduction.  The squares are added as k_qk_prep adds them, SUMMERS threads with every SUMMERS-th entry each (through shared memory), so the results have
+// its bits: sums in another order moved the BF16 roundings of everything behind them.  k_qk_prep is bound by its chain of three dependent passes, not by bytes.  q 4096, k 1024, v 1024: one row 8.4 -> 5.6 us, 512 rows 15.5 -> 10.4 us.
+template <int NTH, int VPT, int SUMMERS>
 __global__ void __launch_bounds__(NTH) k_qk_prep_reg(float *__restrict__ P, int ldp, WindowAttn a, const float *__restrict__ bias, float *__restrict__ kc, float *__restrict__ vc,
                                                      bf16 *__restrict__ kc16, bf16 *__restrict__ vc16, const StepState *__restrict__ st) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ float red[32], redk[32];
+    __shared__ __align__(16) float qk[4 * NTH * VPT];
     const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const int q4 = a.heads * a.dk / 4, k4 = a.kv_heads * a.dk / 4, all = q4 + k4 + a.kv_heads * a.dv / 4;
     float4 *row = reinterpret_cast<float4 *>(P + (size_t)r * ldp);
@@ -858,13 +860,16 @@ __global__ void __launch_bounds__(NTH) k_qk_prep_reg(float *__restrict__ P, int 
         }
     float qinv = 1.0f, kinv = 1.0f;
     if (a.qnorm || a.knorm) { // both sums in one reduction
-        float sq = 0.0f, sk = 0.0f;
 #pragma unroll
-        for (int u = 0; u < VPT; u++) {
-            const int e = tid + u * NTH;
-            const float s2 = fmaf(x[u].x, x[u].x, x[u].y * x[u].y) + fmaf(x[u].z, x[u].z, x[u].w * x[u].w);
-            if (e < q4) sq += s2;
-            else if (e < q4 + k4) sk += s2;
+        for (int u = 0; u < VPT; u++)
+            if (tid + u * NTH < q4 + k4) reinterpret_cast<float4 *>(qk)[tid + u * NTH] = x[u];
+        __syncthreads();
+        float sq = 0.0f, sk = 0.0f;
+        if (tid < SUMMERS) {
+#pragma unroll 8
+            for (int i = tid; i < 4 * q4; i += SUMMERS) sq = fmaf(qk[i], qk[i], sq);
+#pragma unroll 4
+            for (int i = tid; i < 4 * k4; i += SUMMERS) sk = fmaf(qk[4 * q4 + i], qk[4 * q4 + i], sk);
         }
         sq = warp_sum(sq);
         sk = warp_sum(sk);

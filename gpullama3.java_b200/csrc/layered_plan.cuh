@@ -137,6 +137,7 @@ struct Layered {
     int cap_pad = 1; // rows of the activation buffers: cap, padded to whole 256-row GEMM tiles in BF16 mode
     bool tc = false, tc_head = false;
     bool att_mma = true; // BF16 prefill attention on the tensor cores for key/value sizes 64 and 128 (B200_LAYERED_ATT=simt: the FP32 kernel)
+    bool prep_reg = true; // projection rows in registers (B200_LAYERED_PREP=general: k_qk_prep for every row; the results are the same)
     pg::BMap m_head;
     CUtensorMap m_a, m_proj_c, m_y_c, m_log_c;
     // parallel block / latent attention / mixture of experts
@@ -377,17 +378,19 @@ static int ly_step_attention(b200_plan *p, int heads, int window, const float *q
                     sp > 1 ? Y.split : ly::KeySplit{nullptr, nullptr, nullptr});
 }
 
-// k_qk_prep_reg for rows of whole, aligned float4 without rotation and of at most 8192 entries of q | k | v, else k_qk_prep; a single row takes more threads
+// k_qk_prep_reg for rows of whole, aligned float4 without rotation and of at most 8192 entries of q | k | v, else k_qk_prep, with the same sums; a single row
+// takes more threads
 static int ly_launch_qk_prep(b200_plan *p, int n, const LyLayer &L, const LyRun &R, const ly::WindowAttn &wa, const StepState *st) {
     Layered &Y = *p->ly;
     auto go = [&](auto kern, int threads) {
         return launch_k(p, p->use_pdl, kern, dim3(n), dim3(threads), (size_t)0, Y.PROJ, Y.maxP, wa, (const float *)L.b_proj, R.kc, R.vc, R.kc16, R.vc16, st);
     };
     const int all = L.qd + L.kd + L.vd;
+    const bool single = n == 1 && L.qd + L.kd >= 1024;
     const bool aligned = ((reinterpret_cast<uintptr_t>(wa.qnorm) | reinterpret_cast<uintptr_t>(wa.knorm) | reinterpret_cast<uintptr_t>((const float *)L.b_proj)) & 15) == 0;
-    if (wa.rope_dims == 0 && (L.qd | L.kd | L.vd | Y.maxP) % 4 == 0 && all <= 8192 && aligned)
-        return n == 1 && all > 2048 ? go(ly::k_qk_prep_reg<1024, 2>, 1024) : all <= 4096 ? go(ly::k_qk_prep_reg<256, 4>, 256) : go(ly::k_qk_prep_reg<512, 4>, 512);
-    return n == 1 && L.qd + L.kd >= 1024 ? go(ly::k_qk_prep<1024>, 1024) : go(ly::k_qk_prep<256>, 256);
+    if (Y.prep_reg && wa.rope_dims == 0 && (L.qd | L.kd | L.vd | Y.maxP) % 4 == 0 && all <= 8192 && aligned)
+        return single ? go(ly::k_qk_prep_reg<1024, 2, 1024>, 1024) : all <= 4096 ? go(ly::k_qk_prep_reg<256, 4, 256>, 256) : go(ly::k_qk_prep_reg<512, 4, 256>, 512);
+    return single ? go(ly::k_qk_prep<1024>, 1024) : go(ly::k_qk_prep<256>, 256);
 }
 
 // Attention of one layer with its own rings, from the projection rows in PROJ to the (gated) heads in ATT32 / ATT16 (row stride L.gd).
@@ -679,6 +682,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
     Y.has_loop = c.loop_times >= 0;
     if (Y.c.block == B200_BLOCK_PARALLEL && !(Y.c.residual_mult == Y.c.residual_mult)) return fail(p, B200_ERR_BAD_ARG, "residual multiplier is not a number");
     { const char *e = getenv("B200_LAYERED_ATT"); Y.att_mma = !(e && e[0] == 's'); }
+    { const char *e = getenv("B200_LAYERED_PREP"); Y.prep_reg = !(e && e[0] == 'g'); }
     if (Y.has_loop && (c.loop_start < 0 || c.loop_stop > c.n_layers || c.loop_start > c.loop_stop)) return fail(p, B200_ERR_BAD_ARG, "loop [%d, %d) outside the %d layers", c.loop_start, c.loop_stop, c.n_layers);
     const int E = c.width;
     // the fields of b200_config the shared entry points read
