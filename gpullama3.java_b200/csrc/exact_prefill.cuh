@@ -52,12 +52,17 @@ __device__ __forceinline__ xp_f2 xp_mul2(xp_f2 a, xp_f2 b) {
 
 // ---- RMSNorm + Q8_0 quantisation of one token's row (InferenceCore.rmsnorm, InferenceCore.java:39-48) ------------------------------
 // One CTA per token, E entries per thread in registers, the sum of squares by seqsum3.cuh (a literal chain by one thread, the rows of a chunk side by
-// side, took 22 us at dim 4096).  EMBED: the row is gathered from the embedding table first.  The last token's quantised row also goes to the
-// single-token buffers (xq1, xs1).
+// side, took 22 us at dim 4096).  EMBED: the row is gathered from the embedding table first.
+// The single-token buffers: every kernel leaves the last token's results there too, in the order of that token's own step (the attention's quantised output and the
+// norms' share xq / xs), so that a read-back behind the chunk finds what it finds behind single steps.
+struct XpLast {
+    int8_t *xq, *hq;
+    float *xs, *hs, *hb;
+};
 struct XpSync { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
 template <bool EMBED, int E>
 __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const int *__restrict__ tok, DevMat emb, const float *__restrict__ w, float eps, int dim,
-                                                 int8_t *__restrict__ AQ, float *__restrict__ AS, int lds, int8_t *__restrict__ xq1, float *__restrict__ xs1) {
+                                                 int8_t *__restrict__ AQ, float *__restrict__ AS, int lds, XpLast out1) {
     __shared__ __align__(16) float sq[256 * E];
     __shared__ SeqSum3Scratch scratch;
     constexpr int TPB = 32 / E; // threads of a quantisation block
@@ -107,11 +112,11 @@ __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const in
             p |= ((unsigned)__float2int_rz(__fadd_rn(s, copysignf(0.5f, s))) & 0xffu) << (8 * u);
         }
         *reinterpret_cast<unsigned *>(AQ + (size_t)b * dim + base + k) = p;
-        if (last) *reinterpret_cast<unsigned *>(xq1 + base + k) = p;
+        if (last) *reinterpret_cast<unsigned *>(out1.xq + base + k) = p;
     }
     if (tid % TPB == 0) {
         AS[(size_t)(base / 32) * lds + b] = as;
-        if (last) xs1[base / 32] = as;
+        if (last) out1.xs[base / 32] = as;
     }
 }
 
@@ -141,7 +146,7 @@ template <int NJ> struct XpTile {
 
 template <int MODE, int NJ>
 __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(TileMat W, const int8_t *__restrict__ AQ, const float *__restrict__ AS, int lds, int n, float *__restrict__ out, int ldo,
-                                                        int8_t *__restrict__ HQ, float *__restrict__ HS, float *__restrict__ hb1) {
+                                                        int8_t *__restrict__ HQ, float *__restrict__ HS, XpLast last) {
     using T = XpTile<NJ>;
     constexpr int TOK = T::TOK, MI = NJ >= 4 ? 2 : 1, NW = NJ / MI; // a warp's tile: 16 MI rows x 8 NW tokens
     extern __shared__ __align__(128) unsigned char smraw[];
@@ -309,7 +314,11 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(TileMat W, const int8
             const int q = quant_block_lane(v, as);
             HQ[(size_t)(tok0 + t) * hidden + blockIdx.x * 32 + lane] = (int8_t)q;
             if (lane == 0) HS[(size_t)blockIdx.x * lds + tok0 + t] = as;
-            if (tok0 + t == n - 1) hb1[blockIdx.x * 32 + lane] = v;
+            if (tok0 + t == n - 1) {
+                last.hb[blockIdx.x * 32 + lane] = v;
+                last.hq[blockIdx.x * 32 + lane] = (int8_t)q;
+                if (lane == 0) last.hs[blockIdx.x] = as;
+            }
         }
         return;
     }
@@ -388,7 +397,7 @@ __host__ __device__ inline size_t xp_att_smem_bytes(int hs, int qt, int nt, bool
 }
 template <int HS, int QI, int XP_ATT_THREADS>
 __global__ void __launch_bounds__(XP_ATT_THREADS) k_xp_attention(const float *__restrict__ QKV, const float *__restrict__ kc, const float *__restrict__ vc, int n_heads, int n_kv_heads,
-                                                                 int n, int start_pos, float sqrt_hs, int8_t *__restrict__ AQ, float *__restrict__ AS, int lds, float *scratch) {
+                                                                 int n, int start_pos, float sqrt_hs, int8_t *__restrict__ AQ, float *__restrict__ AS, int lds, float *scratch, XpLast last) {
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = HS + 4, QG = XP_ATT_THREADS / 32, QT = QG * QI;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -564,6 +573,10 @@ __global__ void __launch_bounds__(XP_ATT_THREADS) k_xp_attention(const float *__
             const int q = quant_block_lane(sq[r * LD + blk * 32 + lane], as);
             AQ[(size_t)(q0 + r) * qd + h * HS + blk * 32 + lane] = (int8_t)q;
             if (lane == 0) AS[(size_t)(h * (HS / 32) + blk) * lds + q0 + r] = as;
+            if (q0 + r == n - 1) {
+                last.xq[h * HS + blk * 32 + lane] = (int8_t)q;
+                if (lane == 0) last.xs[h * (HS / 32) + blk] = as;
+            }
         }
     }
 }

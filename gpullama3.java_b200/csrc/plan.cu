@@ -1248,14 +1248,16 @@ int exact_prefill_init(b200_plan *p) {
     return B200_OK;
 }
 
+XpLast xp_last(const b200_plan *p) { return XpLast{p->xq, p->hq, p->xs, p->hs, p->hb}; }
+
 template <int MODE>
-int xp_gemm(b200_plan *p, const TileMat &W, const int8_t *aq, const float *as, int n, float *out, int ldo, int8_t *hq, float *hs, float *hb1) {
+int xp_gemm(b200_plan *p, const TileMat &W, const int8_t *aq, const float *as, int n, float *out, int ldo, int8_t *hq, float *hs) {
     const int mt = (W.rows + XP_ROWS - 1) / XP_ROWS;
     auto go = [&](auto nj) -> int {
         constexpr int NJ = decltype(nj)::value;
         auto kern = k_xp_gemm<MODE, NJ>;
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<NJ>::BYTES));
-        kern<<<dim3(mt, (n + 8 * NJ - 1) / (8 * NJ)), XP_THREADS, XpTile<NJ>::BYTES, p->stream>>>(W, aq, as, p->xp.rows, n, out, ldo, hq, hs, hb1);
+        kern<<<dim3(mt, (n + 8 * NJ - 1) / (8 * NJ)), XP_THREADS, XpTile<NJ>::BYTES, p->stream>>>(W, aq, as, p->xp.rows, n, out, ldo, hq, hs, xp_last(p));
         CK(cudaGetLastError());
         return B200_OK;
     };
@@ -1279,8 +1281,8 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     auto norm = [&](bool embed, const float *w) {
         return by_norm_terms(g.dim, [&](auto e_c) -> int {
             constexpr int E = decltype(e_c)::value;
-            if (embed) k_xp_norm<true, E><<<n, 256, 0, p->stream>>>(c.X, p->prefill.tok, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
-            else k_xp_norm<false, E><<<n, 256, 0, p->stream>>>(c.X, nullptr, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, p->xq, p->xs);
+            if (embed) k_xp_norm<true, E><<<n, 256, 0, p->stream>>>(c.X, p->prefill.tok, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, xp_last(p));
+            else k_xp_norm<false, E><<<n, 256, 0, p->stream>>>(c.X, nullptr, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, xp_last(p));
             CK(cudaGetLastError());
             return B200_OK;
         });
@@ -1299,7 +1301,7 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
                     if ((size_t)ctas > slots) ctas = (int)slots;
                 }
                 CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
-                kern<<<ctas, threads, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, c.AS, c.rows, scratch ? c.scratch : nullptr);
+                kern<<<ctas, threads, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, c.AS, c.rows, scratch ? c.scratch : nullptr, xp_last(p));
                 CK(cudaGetLastError());
                 return B200_OK;
             };
@@ -1314,16 +1316,16 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
         int rc;
         if ((rc = norm(l == 0, L.attn_norm))) return rc;
-        if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, c.AQ, c.AS, n, c.QKV, nqkv, nullptr, nullptr, nullptr))) return rc;
+        if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, c.AQ, c.AS, n, c.QKV, nqkv, nullptr, nullptr))) return rc;
         k_xp_rope_kv<<<n, 256, rope_smem, p->stream>>>(c.QKV, kc, vc, g.head_size, g.n_heads, g.n_kv_heads, p->kflags, L.q_norm, L.k_norm, g.rms_norm_eps, p->rope_cr, p->rope_ci, start_pos);
         CK(cudaGetLastError());
         if ((rc = attention(kc, vc))) return rc;
-        if ((rc = xp_gemm<XP_RESID>(p, L.two, c.AQ, c.AS, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, L.two, c.AQ, c.AS, n, c.X, g.dim, nullptr, nullptr))) return rc;
         if ((rc = norm(false, L.ffn_norm))) return rc;
-        if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, c.AQ, c.AS, n, nullptr, 0, c.HQ, c.HS, p->hb))) return rc;
-        if ((rc = xp_gemm<XP_RESID>(p, L.tw2, c.HQ, c.HS, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
+        if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, c.AQ, c.AS, n, nullptr, 0, c.HQ, c.HS))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, L.tw2, c.HQ, c.HS, n, c.X, g.dim, nullptr, nullptr))) return rc;
     }
-    // the single-token buffers hold what the last token's own step would have left there
+    // the single-token buffers hold what the last token's own step would have left there (the others: XpLast)
     CK(cudaMemcpyAsync(p->x, c.X + (size_t)(n - 1) * g.dim, (size_t)g.dim * 4, cudaMemcpyDeviceToDevice, p->stream));
     CK(cudaMemcpyAsync(p->qkv, c.QKV + (size_t)(n - 1) * nqkv, (size_t)nqkv * 4, cudaMemcpyDeviceToDevice, p->stream));
     return B200_OK;
