@@ -186,6 +186,21 @@ template <typename T> int dalloc(b200_plan *p, T **ptr, size_t n_bytes) {
     return B200_OK;
 }
 
+// Buffers that a plan can do without: `alloc` allocates them with dalloc.  Where the device has no room the ones already made are given back and the plan goes on
+// without any (*done = false); every other error is returned.
+template <typename F> int alloc_optional(b200_plan *p, bool *done, F &&alloc) {
+    const size_t n = p->allocs.size();
+    const int64_t bytes = p->bytes;
+    const int rc = alloc();
+    *done = rc == B200_OK;
+    if (rc != B200_ERR_OOM) return rc;
+    for (; p->allocs.size() > n; p->allocs.pop_back()) cudaFree(p->allocs.back());
+    p->bytes = bytes;
+    p->err.clear();
+    cudaGetLastError(); // the failed allocation's
+    return B200_OK;
+}
+
 void par_memcpy(void *dst, const void *src, size_t n, int threads) {
     if (threads <= 1 || n < (size_t)(4u << 20)) { memcpy(dst, src, n); return; }
     std::vector<std::thread> th;
@@ -1195,8 +1210,10 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
     if (3 * c.head_size + c.context_length > ATT_SMEM_FLOATS_MAX) { // long context: score rows in global memory
         if ((rc = dalloc(p, &p->att_scratch, (size_t)p->nh_l * att_row_stride(c.context_length) * 4))) return rc;
     }
-    if (att_cluster(c.head_size, c.context_length) > 1) {
-        if ((rc = dalloc(p, &p->att_rows, (size_t)p->nh_l * (att_row_stride(c.context_length) + 8) * 4))) return rc;
+    if (att_cluster(c.head_size, c.context_length) > 1) { // (without them every position runs the graph with a CTA per head)
+        bool done;
+        if ((rc = alloc_optional(p, &done, [&] { return dalloc(p, &p->att_rows, (size_t)p->nh_l * (att_row_stride(c.context_length) + 8) * 4); }))) return rc;
+        if (!done) p->att_rows = nullptr;
     }
     if ((rc = set_smem_attrs(p))) return rc;
     if (c.tp_size > 1) { CK(cudaStreamSynchronize(p->stream)); return B200_OK; } // graphs are captured by b200_tp_attach
@@ -1220,11 +1237,26 @@ template <typename F> int xp_by_head_size(int hs, F &&f) { // f(integral_constan
 const size_t XP_SMEM_MAX = 220 * 1024;
 const size_t XP_SCRATCH_MAX = (size_t)256 << 20;
 
-// Buffers of one chunk.  Plans off the streaming path (row-major weights) and tensor-parallel ones keep the token-by-token graph.
+int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide);
+// Buffers of one chunk.  Plans off the streaming path (row-major weights) and tensor-parallel ones keep the token-by-token graph, and so do plans that these buffers
+// have no room beside.  A chunk is never longer than the context, whatever the batch size.
 int exact_prefill_init(b200_plan *p) {
     const b200_config &g = p->cfg;
     if (!p->use_stream || g.tp_size > 1 || p->wtype != B200_GGML_Q8_0) return B200_OK;
-    const int rows = (p->prefill_batch + 63) / 64 * 64, nqkv = p->qd + 2 * p->kvd, wide = p->qd > g.dim ? p->qd : g.dim;
+    const int chunk = p->prefill_batch < g.context_length ? p->prefill_batch : g.context_length;
+    const int rows = (chunk + 63) / 64 * 64, nqkv = p->qd + 2 * p->kvd, wide = p->qd > g.dim ? p->qd : g.dim;
+    int *const tok = p->prefill.tok;
+    bool done;
+    int rc = alloc_optional(p, &done, [&]() -> int { return exact_prefill_alloc(p, rows, nqkv, wide); });
+    if (rc) return rc;
+    if (!done) {
+        p->xp = {};
+        p->prefill.tok = tok;
+    }
+    return B200_OK;
+}
+int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide) {
+    const b200_config &g = p->cfg;
     int rc;
     if ((rc = dalloc(p, &p->xp.X, (size_t)rows * g.dim * 4))) return rc;
     if ((rc = dalloc(p, &p->xp.QKV, (size_t)rows * nqkv * 4))) return rc;
