@@ -99,7 +99,7 @@ struct b200_plan {
     int *h_ids = nullptr;      // pinned, seq_cap
 
     cudaGraphExec_t g_decode = nullptr, g_prefill = nullptr, g_trace = nullptr; // the multi-kernel decode graph (round 1)
-    cudaGraphExec_t g_decode_deep = nullptr, g_prefill_deep = nullptr; // the same with clusters in the attention: positions from ATT_SPLIT on (null: not for this plan)
+    cudaGraphExec_t g_decode_deep = nullptr, g_prefill_deep = nullptr, g_trace_deep = nullptr; // the same with clusters in the attention: positions from ATT_SPLIT on (null: not for this plan)
     cudaGraphExec_t g_pdecode = nullptr, g_pprefill = nullptr, g_ptrace = nullptr; // one persistent kernel per token (decode_persistent.cuh)
     unsigned long long *trace_rec = nullptr;
     int decode_mode = B200_DECODE_GRAPH; // which of the two the forward entry points launch
@@ -869,6 +869,7 @@ int capture_all(b200_plan *p) {
     if (p->use_stream || p->use_f16_stream) {
         if ((rc = dalloc(p, &p->trace_rec, (size_t)(p->launches_decode + 8) * 32))) return rc;
         if ((rc = capture(p, true, &p->g_trace, nullptr, true))) return rc;
+        if (p->att_rows && (rc = capture(p, true, &p->g_trace_deep, nullptr, true, false, true))) return rc;
     }
     if ((rc = pd_prepare(p))) return rc;
     if (p->pd_ok) {
@@ -2037,7 +2038,7 @@ int b200_trace_decode(b200_plan *p, int32_t token, int32_t position, uint64_t *r
     for (int i = 0; i < n; i++) { init[i * 4] = 0; init[i * 4 + 1] = ~0ull; init[i * 4 + 2] = 0; init[i * 4 + 3] = 0; }
     CK(cudaMemcpyAsync(p->trace_rec, init.data(), init.size() * 8, cudaMemcpyHostToDevice, p->stream));
     if ((rc = set_state(p, token, position, 0, 0))) return rc;
-    CK(cudaGraphLaunch(p->g_trace, p->stream));
+    CK(cudaGraphLaunch(position >= ATT_SPLIT && p->g_trace_deep ? p->g_trace_deep : p->g_trace, p->stream)); // the kernels that a step at this position runs
     CK(cudaStreamSynchronize(p->stream));
     int m = n < cap ? n : cap;
     CK(cudaMemcpy(records, p->trace_rec, (size_t)m * 32, cudaMemcpyDeviceToHost));
@@ -2188,6 +2189,7 @@ void b200_plan_free(b200_plan *p) {
     if (p->g_decode_deep) cudaGraphExecDestroy(p->g_decode_deep);
     if (p->g_prefill_deep) cudaGraphExecDestroy(p->g_prefill_deep);
     if (p->g_trace) cudaGraphExecDestroy(p->g_trace);
+    if (p->g_trace_deep) cudaGraphExecDestroy(p->g_trace_deep);
     if (p->g_pdecode) cudaGraphExecDestroy(p->g_pdecode);
     if (p->g_pprefill) cudaGraphExecDestroy(p->g_pprefill);
     if (p->g_ptrace) cudaGraphExecDestroy(p->g_ptrace);

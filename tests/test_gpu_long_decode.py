@@ -46,3 +46,25 @@ def test_head_size_256(pkg, orc, tmp_path):
     shape = S.Shape("llama", 512, 512, 1, 2, 1, 256, 512, False, 500000.0, 1e-5)
     model = pkg.loader.model_from_tensors(shape, Q8, S.build_tensors_fast(shape, Q8, seed=3), 300)
     run(pkg, orc, model, [127, 128, 131, 290], 64)
+
+
+def test_trace_runs_the_step_s_kernels(pkg, make_model):
+    """The traced copy of the step shows the attention that the step runs: shared by a cluster from 128 positions on, where a head's 900 keys take one CTA several
+    times as long."""
+    plan = pkg.B200MasterPlan(make_model("tiny-qwen3", pkg.gguf.GGMLType.Q8_0, ctx=1000), prefill_batch_size=512)
+    toks = np.random.default_rng(1).integers(0, 640, 900).astype(np.int32)
+    for p in range(0, 900, 300):
+        plan.forward_batch_prefill(toks[p:p + 300], p)
+
+    def attention_us(at):
+        best = 1e9
+        for _ in range(5):
+            rec = plan._native.trace_decode(7, at).astype(np.int64)
+            best = min(best, min((x - w) / 1e3 for k, _, w, x in rec if k == 4))
+        return best
+
+    deep, single = attention_us(900), attention_us(127)
+    traced = plan.read_buffer("logits", 640).view(np.uint32)
+    assert np.array_equal(traced, plan.forward_decode(7, 127)[0].view(np.uint32))
+    plan.free()
+    assert deep < 3 * single, (deep, single)  # a CTA per head: about 5 times the 128-key step's
