@@ -577,7 +577,6 @@ int launch_cluster(b200_plan *p, bool pdl, int cluster, void (*kern)(KA...), dim
     return B200_OK;
 }
 
-const size_t SMV_SMEM_BUDGET_MAX = 96 * 1024;
 // Debug/tuning knobs, read ONCE per plan (b200_plan_create), never inside a launch helper.
 void read_knobs(b200_plan *p) {
     const char *e = getenv("B200_SMV_BUDGET_KB");   // force a shallow ring
@@ -611,7 +610,8 @@ template <int MODE>
 int launch_stream(b200_plan *p, const TileMat &W, const int8_t *xq, const float *xs, float *out, int8_t *hq, float *hs, bool argmax = false,
                   TraceBuf tr = TraceBuf{nullptr, 0, 0}, int wait_slot = -1, unsigned wait_op = 0, int out_slot = -1, unsigned out_op = 0,
                   int row_base = 0, const NormIn *norm = nullptr) {
-    SmvSmem L = smv_layout(W.cols, W.seg, smv_budget(p, W.cols), norm != nullptr);
+    const SmvSmem L = smv_layout(W.cols, W.seg, smv_budget(p, W.cols), norm != nullptr);
+    if (L.stages < 1) return fail(p, B200_ERR_UNSUPPORTED, "B200_SMV_BUDGET_KB leaves no stage for rows of %d", W.cols);
     SmvArgs a{};
     a.W = W; a.xq = xq; a.xs = xs; a.out = out; a.hq = hq; a.hs = hs; a.blk_cnt = p->blk_cnt;
     a.part_val = argmax ? p->part_val : nullptr;

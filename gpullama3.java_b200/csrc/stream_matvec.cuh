@@ -22,6 +22,7 @@
 #define SMV_CONSUMER_WARPS 8
 #define SMV_THREADS ((SMV_CONSUMER_WARPS + 1) * 32)
 #define SMV_MAX_STAGES 16
+const size_t SMV_SMEM_BUDGET_MAX = 96 * 1024; // shared memory of a CTA: two of them, of neighbouring launches, fit an SM
 #define SMV_HVALS 512 // capacity (hidden units per CTA) of the gate/up epilogue buffer
 
 enum { SMV_STORE = 0, SMV_RESID = 1, SMV_GATEUP = 2 };
@@ -60,6 +61,8 @@ __host__ __device__ inline SmvSmem smv_layout(int cols, int seg, size_t budget, 
     L.off_hvals = o; o += SMV_HVALS * 4; // GATEUP: this CTA's swiglu outputs; STORE+argmax: per-warp candidates
     o = (o + 127) & ~(size_t)127;
     L.off_ring = o;
+    // a budget below the most (B200_SMV_BUDGET_KB, a shallow ring) bounds the ring as it does without the norm, whose squares come on top of it
+    if (budget < SMV_SMEM_BUDGET_MAX && sq > terms) budget = budget + (sq - terms) < SMV_SMEM_BUDGET_MAX ? budget + (sq - terms) : SMV_SMEM_BUDGET_MAX;
     long room = (long)budget - (long)o;
     int s = room > 0 ? (int)(room / L.stage_bytes) : 0;
     if (s > SMV_MAX_STAGES) s = SMV_MAX_STAGES;

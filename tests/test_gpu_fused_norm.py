@@ -55,3 +55,29 @@ def check(pkg, orc, dim, quant):
         got, _ = plan.forward_decode(tok, pos)
         assert np.array_equal(got.view(np.uint32), np.asarray(om.forward(tok, pos), dtype=np.float32).view(np.uint32)), pos
     plan.free()
+
+
+# a shallow ring (B200_SMV_BUDGET_KB) is as deep as without the norm: its squares come on top of the budget.  Rows of 4128 to 8192 entries had no stage left at 48 KB.
+@pytest.mark.parametrize("dim,kb", [(2080, 40), (4288, 40), (4288, 48), (8192, 48), (8192, 64)])
+def test_q8_small_budget(pkg, monkeypatch, dim, kb):
+    S, Q8 = pkg.synth, pkg.gguf.GGMLType.Q8_0
+    shape = S.Shape("qwen3", dim, 512, 1, 4, 2, 64, 512, True, 1000000.0, 1e-6)
+    model = pkg.loader.model_from_tensors(shape, Q8, S.build_tensors_fast(shape, Q8, seed=dim), 8)
+
+    def logits():
+        plan = pkg.B200MasterPlan(model)
+        try:
+            return [plan.forward_decode(tok, pos)[0].view(np.uint32) for pos, tok in enumerate((3, 77))]
+        finally:
+            plan.free()
+
+    want = logits()
+    monkeypatch.setenv("B200_SMV_BUDGET_KB", str(kb))
+    for a, b in zip(want, logits()):
+        assert np.array_equal(a, b)
+
+
+def test_q8_budget_without_a_stage_is_refused(pkg, monkeypatch, make_model):
+    monkeypatch.setenv("B200_SMV_BUDGET_KB", "1")
+    with pytest.raises(Exception, match="leaves no stage"):
+        pkg.B200MasterPlan(make_model("tiny-llama", pkg.gguf.GGMLType.Q8_0, ctx=8))
