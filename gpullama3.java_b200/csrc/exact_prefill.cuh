@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(XP_ATT_THREADS) k_xp_attention(const float *__
 #pragma unroll
             for (int ps = 0; ps < PV_PASSES; ps++) {
                 const int w = tid + ps * XP_ATT_THREADS, g = w / DG, dg = w % DG;
-                if (w < QG * DG) {
+                if (w < QG * DG && g * QI < rows) { // (a group behind the last row sees positions that its score rows have no room for)
                     const float *a0 = S + (size_t)(g * QI) * stride + t0;
                     const int full = start_pos + q0 + g * QI + 1 - t0; // positions of this tile that the group's first row sees
                     if (full >= XP_KT) { // ... all of them: so do the later rows
