@@ -1239,11 +1239,13 @@ const size_t XP_SMEM_MAX = 220 * 1024;
 const size_t XP_SCRATCH_MAX = (size_t)256 << 20;
 
 int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide);
+size_t xp_rope_smem_bytes(const b200_config &g) { return (size_t)(g.n_heads + g.n_kv_heads) * (g.head_size + 1) * 4; } // k_xp_rope_kv: a token's query and key heads
+
 // Buffers of one chunk.  Plans off the streaming path (row-major weights) and tensor-parallel ones keep the token-by-token graph, and so do plans that these buffers
-// have no room beside.  A chunk is never longer than the context, whatever the batch size.
+// have no room beside and plans whose rows of query and key heads are wider than shared memory.  A chunk is never longer than the context, whatever the batch size.
 int exact_prefill_init(b200_plan *p) {
     const b200_config &g = p->cfg;
-    if (!p->use_stream || g.tp_size > 1 || p->wtype != B200_GGML_Q8_0) return B200_OK;
+    if (!p->use_stream || g.tp_size > 1 || p->wtype != B200_GGML_Q8_0 || xp_rope_smem_bytes(g) > XP_SMEM_MAX) return B200_OK;
     const int chunk = p->prefill_batch < g.context_length ? p->prefill_batch : g.context_length;
     const int rows = (chunk + 63) / 64 * 64, nqkv = p->qd + 2 * p->kvd, wide = p->qd > g.dim ? p->qd : g.dim;
     int *const tok = p->prefill.tok;
@@ -1309,7 +1311,7 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     auto &c = p->xp;
     const int nqkv = p->qd + 2 * p->kvd;
     const size_t ctx_kv = (size_t)g.context_length * p->kvd;
-    const size_t rope_smem = (size_t)(g.n_heads + g.n_kv_heads) * (g.head_size + 1) * 4;
+    const size_t rope_smem = xp_rope_smem_bytes(g);
     CK(cudaFuncSetAttribute(k_xp_rope_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
     auto norm = [&](bool embed, const float *w) {
         return by_norm_terms(g.dim, [&](auto e_c) -> int {
