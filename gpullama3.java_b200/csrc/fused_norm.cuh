@@ -23,7 +23,7 @@ struct NormIn { // x == nullptr: the kernel takes a finished activation
     float *xs, *xb;
 };
 // Terms per thread of the 256: a power of two, so that a quantisation block of 32 is 32 / E neighbouring lanes.
-__host__ __device__ inline int norm_terms(int dim) { return dim <= 1024 ? 4 : dim <= 2048 ? 8 : dim <= 4096 ? 16 : 32; }
+__host__ __device__ constexpr int norm_terms(int dim) { return dim <= 1024 ? 4 : dim <= 2048 ? 8 : dim <= 4096 ? 16 : 32; }
 
 // Threads [0, 256); tid * E is the thread's first entry.  Returns the scale in every thread and the entries in x; sq: 256 * E floats of shared memory.
 // w (immutable) is requested before the wait for the kernel in front when the registers allow it.

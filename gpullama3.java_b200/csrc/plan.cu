@@ -504,19 +504,21 @@ template <int MODE> int launch_matvec_f16(b200_plan *p, const DevMat &m, const f
 
 // FP16 plans on the streaming path (stream_matvec_f16.cuh); m2 = ffn_up for SF_GATEUP.
 template <typename... KA, typename... A> int launch_k(b200_plan *p, bool pdl, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args);
-template <typename F> int by_norm_terms(int dim, F &&f) { // f(integral_constant<entries per thread>) (fused_norm.cuh)
+template <int MOST = 32, typename F> int by_norm_terms(int dim, F &&f) { // f(integral_constant<entries per thread, at most MOST>) (fused_norm.cuh)
     switch (norm_terms(dim)) {
     case 4: return f(std::integral_constant<int, 4>());
     case 8: return f(std::integral_constant<int, 8>());
     case 16: return f(std::integral_constant<int, 16>());
-    default: return f(std::integral_constant<int, 32>());
+    default: return f(std::integral_constant<int, MOST>());
     }
 }
 template <typename... KA, typename... A> int launch_cluster(b200_plan *p, bool pdl, int cluster, void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, A... args);
 // Widest row whose norm the FP16 streaming matvecs compute themselves.  They run two CTAs per SM, which share its issue slots during the norm, and the norm's
-// scratch takes stages from their rings.  Measured at position 8, separate -> inside: three layers of 1536 entries 188 -> 160 us, two of 2048 160 -> 152,
-// two of 3072 208 -> 200; two of 4096 342 -> 344, where the launch is kept.
-const int SF_NORM_MAX_DIM = 3072;
+// scratch takes stages from their rings.  Measured at position 8, separate -> inside: three layers of 1024 entries 173 -> 136 us, of 1536 221 -> 165, two of 2048
+// 173 -> 136, of 3072 223 -> 198, of 4096 296 -> 276; beyond 4096, where a thread has 32 entries, the launch is kept: 5120 421 -> 433, 6144 534 -> 543,
+// 8192 765 -> 780.
+const int SF_NORM_MAX_DIM = 4096, SF_NORM_MAX_TERMS = 16;
+static_assert(SF_NORM_MAX_TERMS == norm_terms(SF_NORM_MAX_DIM), "entries per thread of the widest row");
 int sf_grid(const b200_plan *p, int rows, int cols, bool gateup, bool norm) { // CTAs of an FP16 streaming launch
     const int lanes = p->cfg.fp16_lanes;
     const SfLayout L = sf_layout(rows, cols, lanes, gateup, norm);
@@ -542,7 +544,7 @@ template <int MODE> int launch_stream_f16(b200_plan *p, const DevMat &m, const D
         return launch_k(p, p->use_pdl, k_stream_matvec_f16<8, MODE, E>, dim3(grid), dim3(SF_THREADS), L.total, a);
     };
     if constexpr (MODE != SF_RESID)
-        if (norm) return by_norm_terms(m.cols, go);
+        if (norm) return by_norm_terms<SF_NORM_MAX_TERMS>(m.cols, go);
     return go(std::integral_constant<int, 0>());
 }
 
@@ -935,10 +937,12 @@ int set_smem_attrs(b200_plan *p) {
             constexpr int E = decltype(e_c)::value;
             CK(cudaFuncSetAttribute(k_stream_matvec_q8<SMV_STORE, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMV_SMEM_BUDGET_MAX));
             CK(cudaFuncSetAttribute(k_stream_matvec_q8<SMV_GATEUP, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMV_SMEM_BUDGET_MAX));
-            CK(set_max_dyn(k_stream_matvec_f16<16, SF_STORE, E>, maxdyn));
-            CK(set_max_dyn(k_stream_matvec_f16<16, SF_GATEUP, E>, maxdyn));
-            CK(set_max_dyn(k_stream_matvec_f16<8, SF_STORE, E>, maxdyn));
-            CK(set_max_dyn(k_stream_matvec_f16<8, SF_GATEUP, E>, maxdyn));
+            if constexpr (E <= SF_NORM_MAX_TERMS) {
+                CK(set_max_dyn(k_stream_matvec_f16<16, SF_STORE, E>, maxdyn));
+                CK(set_max_dyn(k_stream_matvec_f16<16, SF_GATEUP, E>, maxdyn));
+                CK(set_max_dyn(k_stream_matvec_f16<8, SF_STORE, E>, maxdyn));
+                CK(set_max_dyn(k_stream_matvec_f16<8, SF_GATEUP, E>, maxdyn));
+            }
             return B200_OK;
         });
         if (rc) return rc;

@@ -42,7 +42,7 @@ def test_q8_widths(pkg, orc, dim):
 
 
 @pytest.mark.parametrize("dim", [256, 1024, 1280, 2048, 2304, 4096, 4352, 8192])
-def test_f16_widths(pkg, orc, dim):
+def test_f16_widths(pkg, orc, dim):  # inside the matvecs up to 4096, a launch of its own beyond
     check(pkg, orc, dim, pkg.gguf.GGMLType.F16)
 
 
