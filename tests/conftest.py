@@ -11,7 +11,7 @@ import __graft_entry__ as ge  # noqa: E402
 
 
 def pytest_configure(config):
-    config.addinivalue_line("markers", "gpu: needs a real B200 (run with -m gpu under gpurun)")
+    config.addinivalue_line("markers", "gpu: needs a real B200 (run with -m gpu)")
 
 
 @pytest.fixture(scope="session")

@@ -57,7 +57,8 @@ def test_geometries(pkg, shape, n):
     check(pkg, model, toks, [n], n)
 
 
-# score rows of long contexts live in global memory: a chunk right behind a long cache, and the cache rows that fill shared memory exactly
+# chunks behind a long cache; four heads take the 8-token attention tile, whose score rows of 2093 keys still fit shared memory (test_gpu_exact_prefill_long.py has
+# those in global memory)
 @pytest.mark.parametrize("shape", ["tiny-llama", "tiny-qwen3"])
 def test_long_context(pkg, make_model, shape):
     chunks = [512] * 4 + [40, 5]

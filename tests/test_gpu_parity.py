@@ -258,9 +258,10 @@ def test_long_context_score_row_in_global_memory(pkg, orc, make_model):
                                                   ("tiny-phi3", "Q8_0", 704, "graph"), ("tiny-llama", "F16", 704, "graph"),
                                                   ("tiny-llama", "Q8_0", 20000, "graph"), ("tiny-qwen3", "Q8_0", 20000, "persistent")])
 def test_deep_context_bit_exact(pkg, orc, make_model, shape, quant, ctx, mode):
-    """Depth: 700 positions.  Past 128 keys the attention kernel's score and weighted-sum loops run several software-pipelined passes
-    (next pass's K / V rows in flight during the current chain), from 512 keys on the softmax sum is the exact parallel accumulator, the
-    K/V rows are bulk-prefetched into L2 ahead of the dependency wait; with a 20000-token context the score row lives in global memory.
+    """Depth: 700 positions.  Graph: from 128 keys on a cluster of CTAs shares a head (test_gpu_deep_head32.py: heads of 32 entries, which keep a
+    CTA per head).  Persistent: past 128 keys the score and weighted-sum loops run several software-pipelined passes (next pass's K / V rows in
+    flight during the current chain), from 512 keys on the softmax sum is the exact parallel accumulator; with a 20000-token context the
+    score row lives in global memory.
     Logits are compared on both sides of every switch-over (127|128|129 keys, 255|256|257, 511|512|513, ...) and at the end; the KV cache
     of all 700 positions must be bit-equal.  Head sizes 64 (Llama), 128 (Qwen3: q/k norm, NeoX), 96 (Phi-3)."""
     m = make_model(shape, getattr(pkg.gguf.GGMLType, quant), ctx)

@@ -1,6 +1,6 @@
 """Host-side logic of the tensor-parallel path, on CPU: the row-sharding plan and the rank-ordered
 handle exchange over a world_size-2 gloo group (the device side is exercised by tools/tp_check.py
-under `gpurun --gpus 2`)."""
+on two GPUs)."""
 import os
 import socket
 import sys
