@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py -- Llama-3-8B Q8_0 single-stream decode (tg) on B200, the BASELINE.json headline.
+"""bench.py -- Llama-3-8B Q8_0 single-stream decode (tg) on B200, the reference's headline workload.
 
 A "step" is one single-token decode forward (all layers + lm_head + on-device argmax) at a
 growing KV position, on the LlamaBench synthetic token stream (`new Random(42).nextInt(vocab)`,
@@ -16,10 +16,10 @@ LlamaBench.java:188-193) over a seeded synthetic GGUF-layout model of the real L
                roofline.other_kernels; traffic = measured DRAM bytes per launch from the committed ncu capture
   cpu_baseline the oracle (CPU restatement of the reference's onGPU=false path) on this box's
                host cores, bounded sample
-  parity       in the same run: greedy ids of the first steps GPU == oracle, max|dlogit| of step 0
-               (BASELINE.md section 3); a mismatch exits non-zero
+  parity       in the same run: greedy ids of the first steps GPU == oracle, max|dlogit| of step 0;
+               a mismatch exits non-zero
 `--impl reference` times only that CPU restatement (the reference itself needs a JDK + TornadoVM,
-neither is installable here; see DESIGN.md).
+neither is installable here).
 """
 from __future__ import annotations
 
@@ -63,7 +63,7 @@ def tensor_peak():
 
 
 def prefill_leg(pkg, lb, local: int, n: int, reps: int):
-    """BASELINE config 3: Llama-3-8B FP16, --batch-prefill-size 512, pp512 from depth 0 (LlamaBench `pp`
+    """Llama-3-8B FP16, --batch-prefill-size 512, pp512 from depth 0 (LlamaBench `pp`
     semantics: forward only, no logits).  Tensor-core path: TMA + tcgen05 GEMMs, csrc/prefill*.cuh."""
     shape = pkg.synth.SHAPES[WORKLOAD]
     F16 = pkg.gguf.GGMLType.F16
@@ -590,7 +590,7 @@ class ClockSampler:
 
 
 def algorithmic_bytes_per_token(shape, quant_q8: bool, ctx_avg_pos: float) -> dict:
-    """matmul weights read once + F32 norm weights + FP32 KV reads."""
+    """Matmul weights read once + F32 norm weights + FP32 KV reads."""
     elems = shape.matmul_elements()
     w = elems // 32 * 34 if quant_q8 else elems * 2
     norms = (2 * shape.n_layers + 1) * shape.dim * 4
@@ -627,7 +627,7 @@ def cpu_leg(orc, model, tokens, budget_s: float, max_tokens: int):
 
 
 def parity_gate(plan, tokens, ref, want_logits: bool):
-    """the GPU path on the same tokens/positions the oracle just ran.  Teacher-forced (LlamaBench's
+    """The GPU path on the same tokens/positions the oracle just ran.  Teacher-forced (LlamaBench's
     token stream), so every step is an independent check of logits -> argmax at a growing KV depth."""
     plan.kv_reset()
     n = len(ref["ids"])
@@ -657,11 +657,11 @@ def main():
     ap.add_argument("--no-cpu", action="store_true", help="skip the cpu_baseline leg (profiling runs)")
     ap.add_argument("--no-pp", action="store_true", help="skip the pp512 tensor-core prefill leg")
     ap.add_argument("--decode-mode", default="default", choices=["default", "persistent", "graph"],
-                    help="decode implementation: one persistent kernel per token, or the round-1 CUDA graph of ~7 kernels per layer")
+                    help="decode implementation: one persistent kernel per token, or the CUDA graph of 5 to 7 kernels per layer")
     ap.add_argument("--quant", default="q8_0", choices=["q8_0", "f16"], help="weight type of the synthetic model (f16: the exact lane-order FP16 matvec path, graph mode)")
     ap.add_argument("--depth", type=int, default=-1, help="LlamaBench -d: KV positions filled before the timed steps (default: the warm-up steps)")
     ap.add_argument("--workload", default=WORKLOAD, choices=["llama-3-8b", "llama-3-70b", "llama-3.2-1b", "qwen3-4b"],
-                    help="shape of the synthetic model (default: the BASELINE headline, Llama-3-8B; 70B is BASELINE config 5, meant for --gpus 2/4/8)")
+                    help="shape of the synthetic model (default: the headline workload, Llama-3-8B; 70B is meant for --gpus 2/4/8)")
     ap.add_argument("--compare", default=None, choices=["pibidra", "latusun", "lerosun", "dinuzen", "kegasun", "zulesun"],
                     help="instead of the headline workload: decode and prefill throughput of a layered design beside its closest existing model "
                          "at equal sizes (pibidra: the FP16 Qwen3 plan; latusun, lerosun: the Pibidra plan; dinuzen: the Lerosun plan; kegasun: the Latusun and the Dinuzen plan; zulesun: the Dinuzen and the Kegasun plan), with per-kernel rooflines; one JSON line")
@@ -847,7 +847,7 @@ def main():
             dist.broadcast_object_list([len(ref["ids"])], src=0)
         line["parity"] = parity_gate(plan, tokens, ref, want_logits=world == 1)
     plan.free()
-    if not args.no_pp and world == 1 and WORKLOAD == "llama-3-8b" and QUANT == "q8_0":  # BASELINE config 3 is the 8B FP16 model
+    if not args.no_pp and world == 1 and WORKLOAD == "llama-3-8b" and QUANT == "q8_0":  # the prompt benchmark is of the 8B FP16 model
         del model, plan
         line["pp512"] = prefill_leg(pkg, lb, local, 512, 5)
     print(json.dumps(line))

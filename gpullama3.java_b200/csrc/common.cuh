@@ -1,7 +1,7 @@
 // common.cuh -- shared device helpers for libb200llama (sm_100a only).
 //
 // Numerics contract: every kernel reproduces the float evaluation order of the reference's
-// CPU path (see DESIGN.md "Exactness").  The translation unit is compiled with -fmad=false
+// CPU path.  The translation unit is compiled with -fmad=false
 // and, belt and braces, all order-sensitive arithmetic uses the __f*_rn intrinsics, which
 // the compiler never contracts or reassociates.
 #pragma once

@@ -1,7 +1,7 @@
 // decode_kernels.cuh -- single-token decode kernels (Q8_0 and FP16 weights), bit-exact with the
 // reference's CPU path.  One CUDA graph strings them together per token (plan.cu).
 //
-// Replaces (reference kernel inventory):
+// Replaces (the reference's kernels):
 //   k_rmsnorm_quant  <- reductionOneBlockWithLayer + reductionOneBlock2WithLayer / mapContextWithQuantize
 //                       (TransformerComputeKernelsLayered.java:387-454) + convertQ8_0toFP32 embedding
 //   k_matvec_q8      <- fusedQKVMatmulQ8 / matrixVectorGenericWithResidualQ8_0Byte / matrixVectorGenericQ8Byte
@@ -43,7 +43,7 @@ __device__ __forceinline__ float emb_get(const DevMat &e, int token, int i) {
 #define NORM_THREADS SEQSUM_THREADS
 static_assert(SEQSUM_THREADS == SEQSUM2_THREADS, "both accumulators run on the whole norm CTA");
 __host__ __device__ inline int norm_padded(int dim) { return (dim + SEQSUM2_THREADS - 1) / SEQSUM2_THREADS * SEQSUM2_THREADS; }
-// V2 = seqsum2.cuh (three scans + a short serial walk), otherwise the round-1 accumulator seqsum.cuh
+// V2 = seqsum2.cuh (three scans + a short serial walk), otherwise seqsum.cuh
 __host__ __device__ inline size_t norm_smem_bytes(int dim, bool v2) {
     return v2 ? (size_t)norm_padded(dim) * 4 + 16 + seqsum2_scratch_bytes() : (size_t)dim * 4 + 16 + seqsum_scratch_bytes(dim);
 }
@@ -52,7 +52,7 @@ template <bool EMBED, bool V2>
 __global__ void __launch_bounds__(NORM_THREADS, 1) k_rmsnorm_quant(float *__restrict__ x, const StepState *__restrict__ st,
                                                                DevMat emb, const float *__restrict__ w, float eps, int dim,
                                                                int8_t *__restrict__ xq, float *__restrict__ xs,
-                                                               float *__restrict__ xb, long long *__restrict__ prof, TraceBuf tr, TpCtx tp, int tp_wait_op) {
+                                                               float *__restrict__ xb, long long *__restrict__ prof, TraceBuf tr) {
     // One CTA of 1024 threads.  Under PDL this CTA only has to fit next to ONE streaming-matvec CTA
     // (the following matvec's CTA for this SM simply starts a little later).
     extern __shared__ __align__(16) float sm[];
@@ -66,10 +66,6 @@ __global__ void __launch_bounds__(NORM_THREADS, 1) k_rmsnorm_quant(float *__rest
     pdl_wait();
     trace_mark(tr, 2);
     if (prof) t1 = clock64();
-    if (tp.n > 1 && tp_wait_op >= 0) { // x is gathered from all ranks: wait for their slices
-        if (tid == 0) tp_wait(tp, TP_SLOT_X, tp_seq(tp, (unsigned)tp_wait_op));
-        __syncthreads();
-    }
     int token = 0;
     if (EMBED) token = st->token;
     for (int i = tid; i < dim; i += NORM_THREADS) {
@@ -416,7 +412,8 @@ __global__ void k_swiglu(float *__restrict__ hb, const float *__restrict__ hb2, 
 //             itself; the row lives in global memory (L2) and is handed over at two cluster barriers.
 //   output    a CTA owns 32 elements of the head: one warp walks the positions (one dependent add each: 4 cycles per position, the bound of this part),
 //             the others stage V rows and the quotients ahead of it.
-// Decode step of two layers of the 8B geometry at position 3000: 562 us with a CTA per head, 316 us so; the dependent adds alone are 6.3 us a layer.
+// Decode step of two layers of the 8B geometry at position 3000: 562 us with a CTA per head, 316 us so (277 us since the norms run inside the
+// matvecs); the dependent adds alone are 6.3 us a layer.
 #define ATT_SPLIT 128
 #define ATT_KW 8           // scoring warps of a CTA
 #define ATT_KSTAGES 4      // stages of a scoring warp's ring

@@ -1,5 +1,5 @@
 // decode_persistent.cuh -- ONE persistent kernel per decoded token (sm_100a), replacing the 227 dependent launches of
-// the round-1 decode graph (and, in the reference, TornadoVMMasterPlanSingleToken.tornadoVMForwardDecode's N+2 TaskGraph
+// the multi-kernel decode graph (and, in the reference, TornadoVMMasterPlanSingleToken.tornadoVMForwardDecode's N+2 TaskGraph
 // executions, TornadoVMMasterPlanSingleToken.java:68-95).  The arithmetic of every phase is the bit-exact CPU order of
 // decode_kernels.cuh / stream_matvec.cuh (InferenceCore.java:50-172, 565-697); what this file adds is the orchestration:
 //
@@ -34,7 +34,7 @@
 #define PD_CT (PD_WARPS * 32)           // consumer threads
 #define PD_THREADS (PD_CT + 32)         // + the producer warp
 #define PD_MAX_STAGES 32
-#define PD_TIMEOUT_NS 4000000000ull    // 4 s: far beyond any legitimate wait, well under gpurun's limits
+#define PD_TIMEOUT_NS 4000000000ull    // 4 s: far beyond any legitimate wait
 #define PD_STAMPS 20                    // trace stamps per layer and CTA (0-9 phases, 10-15 inside the attn norm / the attention)
 
 enum { PD_S_QKV = 0, PD_S_ATT = 1, PD_S_WO = 2, PD_S_GU = 3, PD_S_W2 = 4, PD_S_LM = 5, PD_S_ARG = 6, PD_S_SLOTS = 8,

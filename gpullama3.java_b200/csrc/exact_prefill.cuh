@@ -7,7 +7,7 @@
 //   AQ <- Q8_0(rmsnorm(X) * w)                 k_xp_norm       a CTA per token
 //   QKV <- AQ [Wq;Wk;Wv]^T                     k_xp_gemm<XP_STORE>
 //   q, k <- (Qwen3 head norm,) rotation; k, v -> cache     k_xp_rope_kv
-//   AQ <- Q8_0(softmax(q k^T / sqrt(hs)) v)    k_xp_attention  a CTA per (32 or 8 tokens, head)
+//   AQ <- Q8_0(softmax(q k^T / sqrt(hs)) v)    k_xp_attention  a CTA per (64, 32 or 8 tokens, head)
 //   X += AQ Wo^T                               k_xp_gemm<XP_RESID>
 //   AQ <- Q8_0(rmsnorm(X) * w)                 k_xp_norm
 //   HQ <- Q8_0(silu(AQ W1^T) * (AQ W3^T))      k_xp_gemm<XP_GATEUP>
@@ -128,12 +128,12 @@ __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const in
 // exact subtraction replaces the conversion; the subtraction and the products are issued two values at a time (f32x2).  The ordered add is a scalar
 // __fadd_rn: a packed add behind a packed product comes out as one fused operation (measured: results differ in the last bits), the scalar one never.
 // Half of the row tiles take the conversion instruction after all: it runs beside the FP32 pipe (2799 -> 2746 us for the 512-token prompt above).
+// Bound by latency, not by a pipe: the gate/up product of 512 tokens takes 41.5 cycles of a scheduler per (16 x 8 tile, block), of which the FP32 operations need 16;
+// issue slots are used in 58 % of the cycles, the FMA pipe in 38 %.  128 registers allow four warps a scheduler, and a block's ldmatrix, mma, conversion, products and
+// ordered add follow one another in each.
 // A CTA is 4 warps: 64 weight rows (16 groups of the tile-major layout) x 8 * NJ tokens; with 32 tokens and more a warp owns 32 rows and half of the tokens
 // (every B fragment and activation scale serves two row tiles), else 16 rows and all of them.  Three stages of 128 columns come in by cp.async; rows of 128 bytes are swizzled in 16-byte chunks so that ldmatrix is conflict-free.
 // NJ (tokens per tile) is the largest that still gives every SM a CTA: a chunk of a few tokens is bound by the length of the column chain.
-#ifndef XP_CVT
-#define XP_CVT 1
-#endif
 #define XP_STAGES 3
 #define XP_ROWS 64
 #define XP_THREADS 128
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(TileMat W, const int8
 #pragma unroll
                     for (int i = 0; i < MI; i++) {
                         // one row tile turns its integers to floats by the subtraction above, the other by conversions: they run beside the FP32 pipe
-                        const bool cvt = XP_CVT && i == 1;
+                        const bool cvt = i == 1;
                         int d0, d1, d2, d3;
                         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                                      : "=r"(d0), "=r"(d1), "=r"(d2), "=r"(d3)

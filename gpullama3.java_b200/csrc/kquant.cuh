@@ -1,5 +1,5 @@
 // kquant.cuh -- load-time re-quantisation of K-quant tensors (Q4_K / Q5_K / Q6_K) to Q8_0 ON THE DEVICE, inside the upload pipeline
-// (SURVEY 8(f) N4).  The reference does this on the host, one element at a time, while loading
+// The reference does this on the host, one element at a time, while loading
 // (ModelLoader.dequantizeToQ8_0TornadoTensor, model/loader/ModelLoader.java:173-224); here the K-quant bytes cross PCIe as they are
 // (4.5-6.6 bits per weight instead of 8.5) and one thread per 32-element block produces the GGUF Q8_0 block the repack kernels expect.
 // Byte-identical to the reference's output:

@@ -1098,7 +1098,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
         CK(cudaEventCreateWithFlags(&Y.ev_join, cudaEventDisableTiming));
     }
     {   // Programmatic dependent launch in prefill chunks: every kernel of a layered plan waits for its predecessor before it touches anything, so the next launch
-        // can be on its way during the current one (1.5 - 3.5 % of a 512-row chunk).  Not in the decode graph (370 -> 400 us a step: a kernel that becomes
+        // can be on its way during the current one (1.5 - 3.5 % of a 512-row chunk).  Not in the decode graph (371 us a step became 400 to 484 in the variants tried: a kernel that becomes
         // resident early is spread unevenly over the SMs, and there every kernel is one short wave), not for the delta rule (a CTA per SM) and not for plans whose
         // mixers fork into a second stream.
         const char *e = getenv("B200_PDL");

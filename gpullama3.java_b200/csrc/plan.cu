@@ -34,7 +34,7 @@ struct LayerW {
 
 } // namespace
 
-// Weight upload pipeline (SURVEY 8f N1; replaces the reference's lazy FIRST_EXECUTION copy-in, LlamaQ8_0FFNLayers.java:122-132,
+// Weight upload pipeline (replaces the reference's lazy FIRST_EXECUTION copy-in, LlamaQ8_0FFNLayers.java:122-132,
 // timed by TornadoVMMasterPlanSingleToken.java:51-54): pageable/mmapped host bytes -> pinned double buffer (several host
 // threads) -> async H2D on a copy stream -> device staging (double buffered) -> repack kernel on the plan's stream.  The host
 // copy of chunk i+1, the DMA of chunk i and the repack of the previous matrix overlap; nothing synchronises per matrix.
@@ -98,7 +98,7 @@ struct b200_plan {
     StepState *h_st = nullptr; // pinned
     int *h_ids = nullptr;      // pinned, seq_cap
 
-    cudaGraphExec_t g_decode = nullptr, g_prefill = nullptr, g_trace = nullptr; // the multi-kernel decode graph (round 1)
+    cudaGraphExec_t g_decode = nullptr, g_prefill = nullptr, g_trace = nullptr; // the multi-kernel decode graph
     cudaGraphExec_t g_decode_deep = nullptr, g_prefill_deep = nullptr, g_trace_deep = nullptr; // the same with clusters in the attention: positions from ATT_SPLIT on (null: not for this plan)
     cudaGraphExec_t g_pdecode = nullptr, g_pprefill = nullptr, g_ptrace = nullptr; // one persistent kernel per token (decode_persistent.cuh)
     unsigned long long *trace_rec = nullptr;
@@ -216,7 +216,7 @@ void par_memcpy(void *dst, const void *src, size_t n, int threads) {
 
 int up_init(b200_plan *p, size_t dst_bytes) {
     Uploader &u = p->up;
-    const char *e = getenv("B200_UPLOAD_SYNC"); // =1: the round-1 path (one blocking copy + synchronize per matrix)
+    const char *e = getenv("B200_UPLOAD_SYNC"); // =1: the simple path (one blocking copy + synchronize per matrix)
     if (e && e[0] == '1') return B200_OK;
     const char *t = getenv("B200_UPLOAD_THREADS");
     u.threads = t ? atoi(t) : 4;
@@ -672,9 +672,9 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
     float *xbf = q8 ? nullptr : p->xb;
     const size_t ctx_kv = (size_t)c.context_length * p->kvd_l;
     const int rank = p->tp.rank;
-    auto norm = [&](bool embed, const float *w, int wait_op) {
+    auto norm = [&](bool embed, const float *w) {
         auto go = [&](auto kern) {
-            return launch_k(p, pdl, kern, dim3(1), dim3(NORM_THREADS), norm_smem, p->x, (const StepState *)p->st, p->emb, w, c.rms_norm_eps, c.dim, xq, xs, xbf, (long long *)nullptr, TR(1), p->tp, wait_op);
+            return launch_k(p, pdl, kern, dim3(1), dim3(NORM_THREADS), norm_smem, p->x, (const StepState *)p->st, p->emb, w, c.rms_norm_eps, c.dim, xq, xs, xbf, (long long *)nullptr, TR(1));
         };
         if (p->norm_v2) return embed ? go(k_rmsnorm_quant<true, true>) : go(k_rmsnorm_quant<false, true>);
         return embed ? go(k_rmsnorm_quant<true, false>) : go(k_rmsnorm_quant<false, false>);
@@ -685,7 +685,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         // TP flag epochs inside one forward: op = 4*l + {0: attention out, 1: x after Wo, 2: hb, 3: x after W2}
         const NormIn nin = norm_in(p, l == 0, L.attn_norm), nff = norm_in(p, false, L.ffn_norm);
         if (!fused) {
-            if ((rc = norm(l == 0, L.attn_norm, -1))) return rc;
+            if ((rc = norm(l == 0, L.attn_norm))) return rc;
             n++;
         }
         const int x_slot = tpar && l ? TP_SLOT_X : -1;
@@ -718,7 +718,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         else rc = launch_matvec_f16<MODE_RESID>(p, L.wo, p->xb, p->x);
         if (rc) return rc; n++;
         if (!fused) {
-            if ((rc = norm(false, L.ffn_norm, -1))) return rc;
+            if ((rc = norm(false, L.ffn_norm))) return rc;
             n++;
         }
         if (st) {
@@ -746,7 +746,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         int rc;
         const NormIn nout = norm_in(p, false, p->out_norm);
         if (!fused) {
-            if ((rc = norm(false, p->out_norm, -1))) return rc;
+            if ((rc = norm(false, p->out_norm))) return rc;
             n++;
         }
         if (st) rc = launch_stream<SMV_STORE>(p, p->tout, nullptr, nullptr, p->logits, nullptr, nullptr, true, TR(8), tpar ? TP_SLOT_X : -1, last_x_op, -1, 0, rank * p->voc_l, &nout);
@@ -1009,7 +1009,7 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
         p->use_stream = want && p->wtype == B200_GGML_Q8_0 && stream_shape_ok(p->qd_l + 2 * p->kvd_l, c.dim) && stream_shape_ok(p->dim_l, p->qd) &&
                         stream_shape_ok(2 * p->hid_l, c.dim) && stream_shape_ok(p->dim_l, c.hidden_dim) && stream_shape_ok(p->voc_l, c.dim) &&
                         gateup_fits(p->hid_l, p->n_sms);
-        const char *e3 = getenv("B200_F16_STREAM"); // FP16 plans: 0 = the round-1 k_matvec_f16 launches
+        const char *e3 = getenv("B200_F16_STREAM"); // FP16 plans: 0 = the k_matvec_f16 launches
         p->sf_norm = c.dim <= SF_NORM_MAX_DIM;
         p->use_f16_stream = !(e3 && e3[0] == '0') && p->wtype == B200_GGML_F16 && c.tp_size == 1 && sf_layout(p->qd + 2 * p->kvd, c.dim, c.fp16_lanes, false, p->sf_norm).ok &&
                             sf_layout(c.dim, p->qd, c.fp16_lanes, false, false).ok && sf_layout(c.hidden_dim, c.dim, c.fp16_lanes, true, p->sf_norm).ok &&
@@ -1033,7 +1033,7 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
         stage_bytes *= 2;
     }
     const auto t_up0 = std::chrono::steady_clock::now();
-    if ((rc = up_init(p, stage_bytes))) return rc; // pipelined upload (B200_UPLOAD_SYNC=1: the blocking round-1 path)
+    if ((rc = up_init(p, stage_bytes))) return rc; // pipelined upload (B200_UPLOAD_SYNC=1: the blocking path)
     if (!p->up.on && (p->wtype == B200_GGML_Q8_0 || eff_type(emb->ggml_type) == B200_GGML_Q8_0)) CK(cudaMalloc(&stage, stage_bytes));
     struct StageGuard { void *s; b200_plan *pl; ~StageGuard() { if (s) cudaFree(s); up_destroy(pl); } } guard{stage, p};
 
@@ -1422,7 +1422,7 @@ int prefill_init(b200_plan *p) {
         const char *e2 = getenv("B200_GEMM_PERSIST"); // persistent CTA-pair kernel (double-buffered TMEM) for QKV and gate/up: validated on the
         c.persist = !(e2 && e2[0] == '0');
         const char *e3 = getenv("B200_GEMM_PERSIST_RESID"); // =1: Wo / W2 through the persistent kernel too (split-K folded into its work list); experimental
-        c.persist_resid = c.persist && e3 && e3[0] == '1';            // GPU in round 2 (tests/test_gpu_prefill.py, profiles/r2_run1_first_green.log); =0 selects the one-tile kernels
+        c.persist_resid = c.persist && e3 && e3[0] == '1';            // GPU (tests/test_gpu_prefill.py, profiles/r2_run1_first_green.log); =0 selects the one-tile kernels
     }
     if (!ok) { c.why = "cuTensorMapEncodeTiled rejected a tensor map"; return B200_OK; }
     if (g.head_size == 128) {
@@ -1511,7 +1511,7 @@ int prefill_forward(b200_plan *p, int n, int start_pos, int *launches) {
         const PrefillLayerMaps &m = c.maps[l];
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
         k_pf_rmsnorm_f16<<<n, 256, 0, s>>>(c.X, L.attn_norm, g.rms_norm_eps, g.dim, c.A16); nl++;
-        if (c.pair && c.persist) { // round-2 candidate, B200_GEMM_PERSIST=1
+        if (c.pair && c.persist) { // B200_GEMM_PERSIST=0: the one-tile kernels
             if (pg::gemm2_persist_launch<pg::GEMM_F32, 256, pg::GEMM2_PERSIST_STAGES_256>(c.mA, m.qkv, m.qkv, c.mQKV, c.QKV, nqkv, n, mt2, nqkv / 256, g.dim, p->n_sms, s)) return fail(p, B200_ERR_CUDA, "QKV GEMM launch failed");
         } else if (c.pair) {
             if (pg::gemm2_launch<pg::GEMM_F32, 256, pg::GEMM2_STAGES_256>(c.mA, m.qkv, m.qkv, c.mQKV, c.QKV, nqkv, n, mt2, nqkv / 256, g.dim, s)) return fail(p, B200_ERR_CUDA, "QKV GEMM launch failed");
@@ -1549,7 +1549,7 @@ int prefill_forward(b200_plan *p, int n, int start_pos, int *launches) {
             return fail(p, B200_ERR_CUDA, "Wo GEMM launch failed");
         nl++;
         k_pf_rmsnorm_f16<<<n, 256, 0, s>>>(c.X, L.ffn_norm, g.rms_norm_eps, g.dim, c.A16); nl++;
-        if (c.pair && c.persist) { // round-2 candidate, B200_GEMM_PERSIST=1
+        if (c.pair && c.persist) { // B200_GEMM_PERSIST=0: the one-tile kernels
             if (pg::gemm2_persist_launch<pg::GEMM_GATEUP, 256, pg::GEMM2_PERSIST_STAGES_256>(c.mA, m.w1p, m.w3p, c.mX, c.H16, g.hidden_dim, n, mt2, g.hidden_dim / 128, g.dim, p->n_sms, s)) return fail(p, B200_ERR_CUDA, "gate/up GEMM launch failed");
         } else if (c.pair) {
             if (wide ? pg::gemm2_launch<pg::GEMM_GATEUP, 256, pg::GEMM2_STAGES_256_M2, 2>(c.mA, m.w1p, m.w3p, c.mX, c.H16, g.hidden_dim, n, mt4, g.hidden_dim / 128, g.dim, s)
@@ -2063,9 +2063,9 @@ int b200_profile_norm(b200_plan *p, int64_t *cycles4) {
     const bool q8 = p->wtype == B200_GGML_Q8_0;
     for (int i = 0; i < 3; i++)
         if (p->norm_v2) k_rmsnorm_quant<false, true><<<1, NORM_THREADS, norm_smem, p->stream>>>(p->x, p->st, p->emb, p->layers[0].attn_norm, c.rms_norm_eps, c.dim,
-                                                                 q8 ? p->xq : nullptr, q8 ? p->xs : nullptr, q8 ? nullptr : p->xb, d, TraceBuf{nullptr, 0, 0}, p->tp, -1);
+                                                                 q8 ? p->xq : nullptr, q8 ? p->xs : nullptr, q8 ? nullptr : p->xb, d, TraceBuf{nullptr, 0, 0});
         else k_rmsnorm_quant<false, false><<<1, NORM_THREADS, norm_smem, p->stream>>>(p->x, p->st, p->emb, p->layers[0].attn_norm, c.rms_norm_eps, c.dim,
-                                                                 q8 ? p->xq : nullptr, q8 ? p->xs : nullptr, q8 ? nullptr : p->xb, d, TraceBuf{nullptr, 0, 0}, p->tp, -1);
+                                                                 q8 ? p->xq : nullptr, q8 ? p->xs : nullptr, q8 ? nullptr : p->xb, d, TraceBuf{nullptr, 0, 0});
     cudaError_t e = cudaStreamSynchronize(p->stream);
     long long h[16] = {0};
     if (e == cudaSuccess) e = cudaMemcpy(h, d, 128, cudaMemcpyDeviceToHost);
@@ -2083,7 +2083,7 @@ static int run_seqsum_hook(const float *terms, int32_t n, int threads, float *ou
     if (cudaMalloc(&o, 16) != cudaSuccess) { cudaFree(d); return B200_ERR_OOM; }
     cudaError_t e = cudaMemcpy(d, terms, (size_t)n * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
-        if (threads == 0) { // round-1 accumulator (seqsum.cuh)
+        if (threads == 0) { // seqsum.cuh
             const size_t smem = (size_t)((n + 31) & ~31) * 4 + seqsum_scratch_bytes((n + 31) & ~31);
             e = cudaFuncSetAttribute(k_test_seqsum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e == cudaSuccess) k_test_seqsum<<<1, NORM_THREADS, smem>>>(d, n, o, reinterpret_cast<int *>(o) + 1);

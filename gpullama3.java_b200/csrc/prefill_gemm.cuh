@@ -474,7 +474,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(256, 1)
 }
 
 // =====================================================================================================
-// The CTA-pair GEMM as a PERSISTENT kernel (default for the QKV and gate/up GEMMs since round 2; B200_GEMM_PERSIST=0 disables).  One cluster per TPC walks tiles t = cluster + i * clusters (M pair tiles fastest, so neighbouring
+// The CTA-pair GEMM as a PERSISTENT kernel (default for the QKV and gate/up GEMMs; B200_GEMM_PERSIST=0 disables).  One cluster per TPC walks tiles t = cluster + i * clusters (M pair tiles fastest, so neighbouring
 // clusters share a weight tile in L2); the accumulator is double buffered in TMEM (2 x BN columns), so while the four
 // epilogue warps drain tile i the MMA thread already accumulates tile i+1 and the producers are loading tile i+2 --
 // prologue, pipeline fill and epilogue no longer sit on the critical path of every tile (they are ~25 % of a K = 4096 tile
@@ -790,7 +790,7 @@ inline int gemm2_launch(const CUtensorMap &a, const CUtensorMap &b, const CUtens
 constexpr int GEMM2_STAGES_256 = 6, GEMM2_STAGES_128 = 8; // 192 KB of operand ring per CTA either way
 constexpr int GEMM2_STAGES_256_M2 = 4;                    // 4 x (32 KB of A + 16 KB of B)
 
-// Persistent variant (round-2 candidate).  n_sms: SMs of the device; the grid is the largest even number of CTAs <= n_sms.
+// Persistent variant.  n_sms: SMs of the device; the grid is the largest even number of CTAs <= n_sms.
 template <int MODE, int BN, int STAGES>
 inline int gemm2_persist_launch(const CUtensorMap &a, const BMap &b, const BMap &b2, const CUtensorMap &c, void *C, int ldc, int m_valid, int m_tiles,
                                 int n_tiles, int K, int n_sms, cudaStream_t stream, int splits = 1, uint32_t flavor = 0) {
@@ -833,7 +833,7 @@ inline int gemm_f16(const __half *A, const __half *B, float *C, int M, int N, in
         if ((rc = make_map(&ma, A, (uint64_t)M, (uint64_t)K, BM))) return rc;
         if ((rc = make_map(&mb, B, (uint64_t)N, (uint64_t)K, bn / 2))) return rc;
         if ((rc = make_map_c(&mc, C, (uint64_t)M, (uint64_t)N))) return rc;
-        if (two_cta == 1256) { // persistent CTA-pair kernel, 256-wide pair tiles (round-2 candidate)
+        if (two_cta == 1256) { // persistent CTA-pair kernel, 256-wide pair tiles
             int dev = 0, sms = 148;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

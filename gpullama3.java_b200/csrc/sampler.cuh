@@ -1,4 +1,4 @@
-// sampler.cuh -- device-side temperature / top-p sampler (SURVEY.md 8f N3): the reference copies the whole logits row to the
+// sampler.cuh -- device-side temperature / top-p sampler: the reference copies the whole logits row to the
 // host whenever temperature > 0 and samples there (Sampler.selectSampler, inference/sampler/Sampler.java:74-122;
 // CategoricalSampler.java:28-40; ToppSampler.java:62-156); here only the sampled id (4 bytes) leaves the GPU.
 //

@@ -1,8 +1,8 @@
-// seqsum2.cuh -- the exact sequential-sum accumulator of the decode path's RMSNorms (round 2; the algorithm is validated on
+// seqsum2.cuh -- the exact sequential-sum accumulator of the decode path's RMSNorms (the algorithm is validated on
 // the CPU by tools/seqsum2/proto.c, on the GPU by tools/seqsum2/harness.cu and tests/test_gpu_parity.py).
 //
 // Same contract as block_seqsum_exact (seqsum.cuh): the bit-exact value of  s = 0; for (i) s = s + t[i]  for non-negative
-// float terms (InferenceCore.rmsnorm's accumulator, InferenceCore.java:39-48), evaluated by one CTA.  Where the round-1
+// float terms (InferenceCore.rmsnorm's accumulator, InferenceCore.java:39-48), evaluated by one CTA.  Where the first
 // kernel works in 32-term groups with per-warp ordered composition, entry lists and a literal first quarter (~16 us at
 // n = 4096, a third of the decode step), this version is three block-wide scans and a ~25-item serial walk:
 //   1. float prefix P over per-thread sums (E consecutive terms per thread)            -> predicted binade per thread

@@ -1,5 +1,5 @@
-// stream_matvec_f16.cuh -- FP16-weight matvec of the decode step on per-warp bulk-copy rings (FP16 plans, SURVEY 8(a) a4/a6/a9/a10,
-// BASELINE configs 1 and 3).  Bit-exact with FP16FloatTensor.vectorDot (FP16FloatTensor.java:62-110) for an L-lane species, like
+// stream_matvec_f16.cuh -- FP16-weight matvec of the decode step on per-warp bulk-copy rings (FP16
+// plans).  Bit-exact with FP16FloatTensor.vectorDot (FP16FloatTensor.java:62-110) for an L-lane species, like
 // k_matvec_f16 (decode_kernels.cuh) which stays as the fallback for odd shapes and the scalar (L = 0) order:
 //   * per output row L independent chains  acc_c = fma(w[L j + c], x[L j + c], acc_c), j ascending   (FloatVector.fma: fused),
 //   * reduceLanes(ADD) in ascending lane order starting from the identity,
@@ -17,7 +17,7 @@
 // 3.0 TB/s on the 1 GB classifier, issue-bound; profiles/r2_run8_f16_stream_kquants.log).  The rows of a stage are SF_ROW_PAD bytes
 // apart modulo 128 so the row groups of a warp hit different banks.
 //   SF_GATEUP: half of the warp's row slots are ffn_gate rows, the other half the same rows of ffn_up; SwiGLU (InferenceCore.java:150-158)
-//   is applied in the epilogue, so w1, w3 and the SwiGLU kernel of the round-1 FP16 graph collapse into one launch.
+//   is applied in the epilogue, so w1, w3 and the SwiGLU kernel collapse into one launch.
 // What set the pace of a warp was not the copies but the work around them: positions computed with four divisions an item, and eight loads at a time in front of
 // their products (48 registers, by the compiler's choice).  With positions carried along, sixteen loads ahead and up to 128 registers, steps of two layers at
 // position 8 went from 326 to 246 us (8B), 151 to 108 us (1B); three layers of 1536 columns 156 to 118 us.

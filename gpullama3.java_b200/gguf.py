@@ -5,8 +5,8 @@ Wire format the hot path consumes.  Mirrors the reference parser
 tensor-data offset) and ``tensor/GGUF.java:105-137`` (one mapping of the tensor-data
 section, per-tensor slices), plus ``tensor/GGMLType.java:5-20`` (block sizes:
 Q8_0 = 34 bytes / 32 elements).  The writer has no reference counterpart: it exists
-because no real checkpoints are available offline and every BASELINE config runs on
-seeded synthetic GGUF files (SURVEY.md section 8d).
+because no real checkpoints are available offline and every benchmark configuration runs on
+seeded synthetic GGUF files.
 """
 from __future__ import annotations
 

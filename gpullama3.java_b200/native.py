@@ -132,7 +132,7 @@ def _raise(code: int, msg: str):
 
 
 def test_seqsum(terms, want_info: bool = False, threads: int = 0):
-    """threads = 0: the round-1 accumulator (seqsum.cuh); 1024 / 256: seqsum2.cuh in the norm kernel's / persistent kernel's form; 3: seqsum3.cuh."""
+    """threads = 0: the first accumulator (seqsum.cuh); 1024 / 256: seqsum2.cuh in the norm kernel's / persistent kernel's form; 3: seqsum3.cuh."""
     t = np.ascontiguousarray(terms, dtype=np.float32)
     out = C.c_float(0)
     info = (C.c_int32 * 2)()

@@ -1,5 +1,5 @@
-"""Seeded synthetic GGUF models in the BASELINE shapes (no real checkpoints are available
-offline; SURVEY.md section 8d).  Tensor names/types are exactly what the reference loaders
+"""Seeded synthetic GGUF models in the benchmark shapes (no real checkpoints are available
+offline).  Tensor names/types are exactly what the reference loaders
 expect (``model/loader/LlamaModelLoader.java:78-99``, ``Qwen3ModelLoader.java:98-124``):
 norm weights F32, matrices and the embedding table in the model quantisation, metadata keys
 per ``LlamaModelLoader.java:47-63`` / ``Qwen3ModelLoader.java:48-74``.
@@ -37,7 +37,7 @@ class Shape:
         return self.n_kv_heads * self.head_size
 
     def matmul_elements(self) -> int:
-        """Weight elements streamed per decoded token (SURVEY.md 8d)."""
+        """Weight elements streamed per decoded token."""
         per_layer = 2 * self.q_dim * self.dim + 2 * self.kv_dim * self.dim + 3 * self.hidden * self.dim
         return self.n_layers * per_layer + self.vocab * self.dim
 
@@ -59,11 +59,11 @@ SHAPES = {
     "small-llama": Shape("llama", 1536, 4096, 3, 12, 4, 128, 4096, False, 500000.0, 1e-5),
     # the real Llama-3-8B layer geometry (7 column segments in the down projection, 4 KB rows) with 2 layers / small vocab
     "mid-llama": Shape("llama", 4096, 14336, 2, 32, 8, 128, 8192, False, 500000.0, 1e-5),
-    # 2-layer cuts of the other BASELINE geometries (parity tests at the real row/segment shapes, small vocabulary)
+    # 2-layer cuts of the other benchmark geometries (parity tests at the real row/segment shapes, small vocabulary)
     "mid-qwen3-4b": Shape("qwen3", 2560, 9728, 2, 32, 8, 128, 8192, True, 1000000.0, 1e-6, 40960),
     "mid-llama-1b": Shape("llama", 2048, 8192, 2, 32, 8, 64, 8192, True, 500000.0, 1e-5, 131072),
     "mid-llama-70b": Shape("llama", 8192, 28672, 2, 64, 8, 128, 8192, False, 500000.0, 1e-5),
-    # BASELINE.json shapes
+    # the shapes of the benchmarked models
     "llama-3.2-1b": Shape("llama", 2048, 8192, 16, 32, 8, 64, 128256, True, 500000.0, 1e-5, 131072),
     "llama-3-8b": Shape("llama", 4096, 14336, 32, 32, 8, 128, 128256, False, 500000.0, 1e-5),
     "qwen3-4b": Shape("qwen3", 2560, 9728, 36, 32, 8, 128, 151936, True, 1000000.0, 1e-6, 40960),

@@ -1,6 +1,6 @@
 /* b200tok.h -- C ABI of the native byte-level BPE tokenizer (gpullama3.java_b200/csrc/tokenizer.cpp -> libb200tok.so).
  *
- * the host-side tokenizer of the reference, natively.  Replaces, for the Llama-3 and Qwen3 GGUF
+ * The host-side tokenizer of the reference, natively.  Replaces, for the Llama-3 and Qwen3 GGUF
  * vocabularies, tokenizer/LlamaTokenizer.java:30-269 and tokenizer/Qwen3Tokenizer.java:20-352 (encode / encodeOrdinary /
  * encodeChunk / decode), keeping their observable behaviour token for token -- including that the pre-tokenisation
  * pattern is applied to the byte-mapped text and that merge priority is the merged token's id (see

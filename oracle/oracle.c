@@ -22,7 +22,7 @@
  *   the only fused operations in the reference are the explicit
  *   FloatVector.fma calls in FP16FloatTensor.vectorDot, restated with fmaf().
  *
- * Pinned host-dependent choices (see DESIGN.md "Oracle pins"):
+ * Pinned host-dependent choices:
  *   - FP16 vector dot lane count: `lanes` in the model config (16 = 512-bit
  *     species, 8 = 256-bit, 0 = llama.VectorBitSize=0 scalar path).
  *   - FloatVector.reduceLanes(ADD) order: ascending lane order (JDK 21 C2
@@ -454,7 +454,7 @@ void oracle_quantize_q8_0(const float *x, int64_t n, uint8_t *out) {
 }
 
 /* ================================================================================================================
- * K-quants (SURVEY 8f N4): the reference's accelerator path never computes with Q4_K/Q5_K/Q6_K -- ModelLoader.loadTornadoTensor
+ * K-quants: the reference's accelerator path never computes with Q4_K/Q5_K/Q6_K -- ModelLoader.loadTornadoTensor
  * (model/loader/ModelLoader.java:163) re-quantises such tensors to Q8_0 at load time (dequantizeToQ8_0TornadoTensor, :173-224) and
  * AbstractModelLoader.java:45-59 reports the model as Q8_0.  Restated here: the element read of each format (getFloat of
  * tensor/standard/Q4_KFloatTensor.java:90-120, Q5_KFloatTensor.java:84-122, Q6_KFloatTensor.java:64-116; float products evaluated left
@@ -539,7 +539,7 @@ void oracle_kquant_to_q8_0(int type, const uint8_t *src, int64_t n, uint8_t *dst
 }
 
 /* ================================================================================================================
- * Sampler (SURVEY 8f N3): Sampler.selectSampler (inference/sampler/Sampler.java:74-122), CategoricalSampler.java:28-40,
+ * Sampler: Sampler.selectSampler (inference/sampler/Sampler.java:74-122), CategoricalSampler.java:28-40,
  * ToppSampler.java:26-156.  Temperature 0 -> FloatTensor.argmax; otherwise logits / temperature, softmaxInPlace, then
  * either the categorical walk or the top-p heap.  PARITY UNPINNED (no JDK here): the uniform numbers come from
  * RandomGeneratorFactory.getDefault() = L32X64MixRandom, restated below from the published LXM algorithm (Steele & Vigna,
