@@ -371,9 +371,9 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             ly::RglruArgs ra{};
             ra.W = W; ra.blocks = nb; ra.gate_bias = L.gate_bias; ra.lam = L.lam; ra.y_bias = L.y_bias;
             // a chunk: 16 channels x up to 32 row groups per CTA (the last group may be short, never empty rows in between); few rows: 32 channels, one group
-            if (n >= 64) rc = launch_k(p, p->use_pdl, ly::k_rglru_scan<16, RGLRU_MAX_GROUPS>, dim3((W + 15) / 16), dim3(16 * RGLRU_MAX_GROUPS), (size_t)0, (const float *)Y.DLT, Y.maxD, (const float *)Y.Q, Y.maxQ,
+            if (n >= 64) rc = launch_k(p, false, ly::k_rglru_scan<16, RGLRU_MAX_GROUPS>, dim3((W + 15) / 16), dim3(16 * RGLRU_MAX_GROUPS), (size_t)0, (const float *)Y.DLT, Y.maxD, (const float *)Y.Q, Y.maxQ,
                                        (const float *)(Y.PROJ + W), Y.maxP, ra, R.S, n, st, att32, att16, L.gd);
-            else rc = launch_k(p, p->use_pdl, ly::k_rglru_scan<32, 1>, dim3((W + 31) / 32), dim3(32), (size_t)0, (const float *)Y.DLT, Y.maxD, (const float *)Y.Q, Y.maxQ,
+            else rc = launch_k(p, false, ly::k_rglru_scan<32, 1>, dim3((W + 31) / 32), dim3(32), (size_t)0, (const float *)Y.DLT, Y.maxD, (const float *)Y.Q, Y.maxQ,
                                (const float *)(Y.PROJ + W), Y.maxP, ra, R.S, n, st, att32, att16, L.gd);
             if (rc) return rc;
             nl += 3;
@@ -388,11 +388,11 @@ static int ly_enqueue_outnorm(b200_plan *p, bool decode, int n, const StepState 
             const dim3 grid(s.heads, (s.value_dim + SSD_COLS - 1) / SSD_COLS), block(SSD_THREADS);
             const float *dt = Y.PROJ + 2 * inner + 2 * gn;
             switch (ly::ssd_reg_rows(s.key_dim)) {
-            case 1: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<1>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
-            case 2: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<2>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
-            case 4: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<4>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
-            case 8: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<8>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
-            default: rc = launch_k(p, p->use_pdl, ly::k_ssd_scan<16>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO);
+            case 1: rc = launch_k(p, false, ly::k_ssd_scan<1>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
+            case 2: rc = launch_k(p, false, ly::k_ssd_scan<2>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
+            case 4: rc = launch_k(p, false, ly::k_ssd_scan<4>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
+            case 8: rc = launch_k(p, false, ly::k_ssd_scan<8>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO); break;
+            default: rc = launch_k(p, false, ly::k_ssd_scan<16>, grid, block, (size_t)0, (const float *)Y.DLT, Y.maxD, dt, Y.maxP, sa, R.S, n, st, Y.DO, Y.maxDO);
             }
             if (rc) return rc;
             if ((rc = launch_k(p, p->use_pdl, ly::k_gated_group_norm, dim3(n), dim3(n == 1 && inner >= 2048 ? 1024 : 256), (size_t)inner * 4, (const float *)Y.DO, Y.maxDO, (const float *)Y.PROJ, Y.maxP, (const float *)L.onorm, inner,
