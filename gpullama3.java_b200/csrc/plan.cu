@@ -563,7 +563,7 @@ int launch_cluster(b200_plan *p, bool pdl, int cluster, void (*kern)(KA...), dim
     cfg.stream = p->stream;
     cudaLaunchAttribute attr[2];
     int n = 0;
-    if (pdl && (size_t)grid.x * grid.y * grid.z <= 4096) { // (a launch of many waves gains nothing and pays for the wait in every CTA)
+    if (pdl) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n++].val.programmaticStreamSerializationAllowed = 1;
     }
