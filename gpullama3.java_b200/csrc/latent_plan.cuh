@@ -208,10 +208,10 @@ static int ly_project_view(b200_plan *p, bool decode, int n, const float *a32, c
     const float *nb = nullptr;
     if (Y.f32) {
         if (c16) return fail(p, B200_ERR_STATE, "FP32 plans keep FP32 activations");
-        return launch_k(p, p->use_pdl, ly::k_gemm_f32<EPI, float>, grid, dim3(256), (size_t)0, a32, W, nb, c32, n, N, K, ldc, act, gv);
+        return launch_k(p, false, ly::k_gemm_f32<EPI, float>, grid, dim3(256), (size_t)0, a32, W, nb, c32, n, N, K, ldc, act, gv);
     }
-    if (c16) return launch_k(p, p->use_pdl, ly::k_gemm_bf16<EPI, ly::bf16>, grid, dim3(128), (size_t)0, a16, W, nb, c16, n, N, K, ldc, act, gv);
-    return launch_k(p, p->use_pdl, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, nb, c32, n, N, K, ldc, act, gv);
+    if (c16) return launch_k(p, false, ly::k_gemm_bf16<EPI, ly::bf16>, grid, dim3(128), (size_t)0, a16, W, nb, c16, n, N, K, ldc, act, gv);
+    return launch_k(p, false, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, nb, c32, n, N, K, ldc, act, gv);
 }
 
 static ly::BlockNormArgs ly_block_norm_args(const Layered &Y) {

@@ -289,8 +289,8 @@ static int ly_launch_mma(b200_plan *p, int kind, int n, int heads, int window, c
     const int rows = tall ? LY_ATT_MMA_ROWS : 64;
     const dim3 grid((n + rows - 1) / rows, heads), block(rows * 2);
 #define LY_MMA_CASE(K, DK, DV) \
-    if (kind == K) return tall ? launch_k(p, p->use_pdl, ly::k_window_attention_mma<DK, DV>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32) \
-                               : launch_k(p, p->use_pdl, ly::k_window_attention_mma<DK, DV, 64>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32);
+    if (kind == K) return tall ? launch_k(p, false, ly::k_window_attention_mma<DK, DV>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32) \
+                               : launch_k(p, false, ly::k_window_attention_mma<DK, DV, 64>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32);
     LY_MMA_CASE(1, 64, 64)
     LY_MMA_CASE(2, 128, 128)
     LY_MMA_CASE(3, 192, 128)
@@ -360,9 +360,9 @@ static int ly_project(b200_plan *p, bool decode, int n, const float *a32, const 
         return rc ? fail(p, B200_ERR_CUDA, "tensor-core GEMM launch failed (%d)", rc) : B200_OK;
     }
     dim3 grid((N + 63) / 64, (n + 63) / 64);
-    if (Y.f32) return launch_k(p, p->use_pdl, ly::k_gemm_f32<EPI, float>, grid, dim3(256), (size_t)0, a32, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
-    if (c16) return launch_k(p, p->use_pdl, ly::k_gemm_bf16<EPI, ly::bf16>, grid, dim3(128), (size_t)0, a16, W, bias, c16, n, N, K, ldc, act, ly::GemmView{});
-    return launch_k(p, p->use_pdl, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
+    if (Y.f32) return launch_k(p, false, ly::k_gemm_f32<EPI, float>, grid, dim3(256), (size_t)0, a32, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
+    if (c16) return launch_k(p, false, ly::k_gemm_bf16<EPI, ly::bf16>, grid, dim3(128), (size_t)0, a16, W, bias, c16, n, N, K, ldc, act, ly::GemmView{});
+    return launch_k(p, false, ly::k_gemm_bf16<EPI, float>, grid, dim3(128), (size_t)0, a16, W, bias, c32, n, N, K, ldc, act, ly::GemmView{});
 }
 
 // The decode step's attention: k_step_attention for rows of whole float4, with a head's window over as many CTAs as the SMs allow (B200_LAYERED_SPLITS bounds it); else
@@ -1099,9 +1099,11 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
     }
     {   // Programmatic dependent launch in prefill chunks: every kernel of a layered plan waits for its predecessor before it touches anything, so the next launch
         // can be on its way during the current one (1.5 - 3.5 % of a 512-row chunk).  Not in the decode graph (371 us a step became 400 to 484 in the variants tried: a kernel that becomes
-        // resident early is spread unevenly over the SMs, and there every kernel is one short wave), not for the delta rule, the SSD and the RG-LRU scan (up to a CTA per SM, which
-        // runs for the whole chunk: 512 rows of a model with two SSD layers and an RG-LRU layer took 1340 us with both scans programmatic, 1237 with the RG-LRU scan alone, 1226
-        // with neither, 1261 without any programmatic launch) and not for plans whose mixers fork into a second stream.
+        // resident early is spread unevenly over the SMs, and there every kernel is one short wave), not for kernels whose CTAs fill the SMs for long: the delta rule, the SSD and the
+        // RG-LRU scan (512 rows of a model with two SSD layers and an RG-LRU layer took 1340 us with both scans programmatic, 1237 with the RG-LRU scan alone, 1226 with neither, 1261
+        // without any programmatic launch), the GEMMs off the tcgen05 path (FP32 mode, 512 rows of two layers of 1024: 5476 -> 4518 us, 4564 without any programmatic launch; BF16,
+        // width 1000: 968 -> 955) and the mma.sync attention (974 -> 948 behind those GEMMs; 790 and 793 behind tcgen05 GEMMs, within noise).  And not for plans whose
+        // mixers fork into a second stream.
         const char *e = getenv("B200_PDL");
         Y.pdl = !Y.branch && !(e && e[0] == '0');
     }
