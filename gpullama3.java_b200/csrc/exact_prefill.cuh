@@ -13,18 +13,16 @@
 //   HQ <- Q8_0(silu(AQ W1^T) * (AQ W3^T))      k_xp_gemm<XP_GATEUP>
 //   X += HQ W2^T                               k_xp_gemm<XP_RESID>
 //
-// Measured on two layers of the 8B geometry, 512 tokens and the decode step behind them: 109.8 ms token by token, 2.68 ms here; two layers of the 4B
-// Qwen3 geometry, 36 tokens: 5.36 ms and 0.54 ms.
+// Measured on two layers of the 8B geometry, 512 tokens and the decode step behind them: 109.8 ms token by token, 2.25 ms here; two layers of the 4B
+// Qwen3 geometry, 36 tokens: 5.36 ms and 0.52 ms.
 #pragma once
+#include "prefill_gemm.cuh"
 #include "stream_matvec.cuh"
 
 enum { XP_STORE = 0, XP_RESID = 1, XP_GATEUP = 2 };
 
 __device__ __forceinline__ void xp_cp16(unsigned dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void xp_cp8(unsigned dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void xp_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void xp_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -39,14 +37,14 @@ __device__ __forceinline__ xp_f2 xp_pack(float a, float b) {
     return r;
 }
 __device__ __forceinline__ void xp_unpack(xp_f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ xp_f2 xp_add2(xp_f2 a, xp_f2 b) {
-    xp_f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 __device__ __forceinline__ xp_f2 xp_mul2(xp_f2 a, xp_f2 b) {
     xp_f2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ xp_f2 xp_fma2(xp_f2 a, xp_f2 b, xp_f2 c) {
+    xp_f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
 
@@ -122,155 +120,138 @@ __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const in
 
 // ---- the product -----------------------------------------------------------------------------------------------------------------
 // out[token][row] = sum over 32-blocks, strictly in block order, of (float)isum * (wScale * aScale)   (Q8_0FloatTensor.java:90-123).
-// isum of a block is one mma.sync.m16n8k32 (int8, exact).  The tensor pipe is not what bounds this: every (row, token, block) costs four
-// FP32 operations (int to float, scale product, term, ordered add), the order of the adds is fixed, and those run on the CUDA cores.  So: the
-// accumulator of each mma starts at the integer 0x4B400000, whose bit pattern plus isum IS the float 12582912 + isum (|isum| <= 520,192), and one
-// exact subtraction replaces the conversion; the subtraction and the products are issued two values at a time (f32x2).  The ordered add is a scalar
-// __fadd_rn: a packed add behind a packed product comes out as one fused operation (measured: results differ in the last bits), the scalar one never.
-// Half of the row tiles take the conversion instruction after all: it runs beside the FP32 pipe (2799 -> 2746 us for the 512-token prompt above).
-// Bound by latency, not by a pipe: the gate/up product of 512 tokens takes 41.5 cycles of a scheduler per (16 x 8 tile, block), of which the FP32 operations need 16;
-// issue slots are used in 58 % of the cycles, the FMA pipe in 38 %.  128 registers allow four warps a scheduler, and a block's ldmatrix, mma, conversion, products and
-// ordered add follow one another in each.
+// isum of a block is one mma.sync.m16n8k32 (int8, exact).  The tensor pipe is not what bounds this: every (row, token, block) costs a conversion, two
+// products and an ordered add, and those run on the CUDA cores, two values at a time (f32x2).  The ordered add is fma(acc, 1, term), which rounds like the
+// add: a packed add behind a packed product comes out as ONE fused operation (measured; also where the 1 is a constant of the kernel, so it is an argument).
+// Integers are converted by the conversion instruction: accumulators that start at 0x4B400000 and a subtraction cost four register moves for every mma (gate/up
+// product 411 against 392 us).  Gate/up of 512 tokens, 8B layer: 560 us with scalar adds and cp.async fetches by all threads, 392 us so (FMA pipe 50 %, issue slots
+// 64 %; 19 warp instructions per 16 x 8 tile and block, 15 of them the arithmetic and its operands); Wo + W2 341 -> 281 us, QKV 121 -> 90 us.
+// tcgen05.mma.kind::i8 does not pay here: a sum is read back after every 32 columns, so each block costs a round trip product - barrier - tcgen05.ld - barrier; with 2 to
+// 4 accumulator buffers, a warp each for loads and products and up to 24 warps on the sums it took 410 us (32-token tiles) to 494 us.
 // A CTA is 4 warps: 64 weight rows (16 groups of the tile-major layout) x 8 * NJ tokens; with 32 tokens and more a warp owns 32 rows and half of the tokens
-// (every B fragment and activation scale serves two row tiles), else 16 rows and all of them.  Three stages of 128 columns come in by cp.async; rows of 128 bytes are swizzled in 16-byte chunks so that ldmatrix is conflict-free.
-// NJ (tokens per tile) is the largest that still gives every SM a CTA: a chunk of a few tokens is bound by the length of the column chain.
+// (every B fragment and activation scale serves two row tiles), else 16 rows and all of them.  Three stages of 128 columns come in by TMA (thread 0 issues: weights and
+// their scales straight out of the tile-major layout by a 4-D map), rows of 128 bytes swizzled so that ldmatrix is conflict-free.
 #define XP_STAGES 3
 #define XP_ROWS 64
 #define XP_THREADS 128
+#define XP_SPINS (1 << 22)
+struct XpMaps { CUtensorMap q, s; }; // quants; scales
 template <int NJ> struct XpTile {
     static constexpr int TOK = 8 * NJ;
-    static constexpr int A_Q = 0, A_S = XP_ROWS * 128, B_Q = A_S + XP_ROWS * 8, B_S = B_Q + TOK * 128, STAGE = (B_S + 4 * TOK * 4 + 127) & ~127;
+    static constexpr int A_Q = 0, B_Q = XP_ROWS * 128, A_S = B_Q + TOK * 128, B_S = A_S + XP_ROWS * 16, BYTES_IN = B_S + 4 * TOK * 4, STAGE = (BYTES_IN + 1023) & ~1023;
     static constexpr int HV = 33 * TOK * 4; // gate/up: the tile's 32 hidden units (+ 1: no bank conflicts) per token
-    static constexpr int BYTES = XP_STAGES * STAGE > HV ? XP_STAGES * STAGE : HV;
+    static constexpr int BYTES = 1024 + XP_STAGES * STAGE + 16 * XP_STAGES;
 };
+__device__ __forceinline__ bool xp_wait(unsigned bar, unsigned parity) { // bounded: false = given up
+    unsigned ok = 0;
+    for (int i = 0; i < XP_SPINS && !ok; i++)
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void xp_load4(unsigned dst, const CUtensorMap *map, int x, int seg, int group, unsigned bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst), "l"(map), "r"(x), "r"(0), "r"(seg),
+                 "r"(group), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ xp_f2 xp_lds64(unsigned a) {
+    xp_f2 r;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(r) : "r"(a));
+    return r;
+}
 
 template <int MODE, int NJ>
-__global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(TileMat W, const int8_t *__restrict__ AQ, const float *__restrict__ AS, int lds, int n, float *__restrict__ out, int ldo,
-                                                        int8_t *__restrict__ HQ, float *__restrict__ HS, XpLast last) {
+__global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant__ XpMaps map_w, const __grid_constant__ XpMaps map_a, TileMat W, int lds, int n, float *__restrict__ out, int ldo,
+                                                        int8_t *__restrict__ HQ, float *__restrict__ HS, XpLast last, float one_f, unsigned *err) {
     using T = XpTile<NJ>;
     constexpr int TOK = T::TOK, MI = NJ >= 4 ? 2 : 1, NW = NJ / MI; // a warp's tile: 16 MI rows x 8 NW tokens
-    extern __shared__ __align__(128) unsigned char smraw[];
-    const unsigned smb = smem_u32(smraw);
+    extern __shared__ unsigned char smraw[];
+    unsigned char *const ring = reinterpret_cast<unsigned char *>(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023); // (the swizzle is by address)
+    const unsigned smb = smem_u32(ring), full0 = smb + XP_STAGES * T::STAGE, empty0 = full0 + 8 * XP_STAGES;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row0 = blockIdx.x * XP_ROWS, tok0 = blockIdx.y * TOK;
     const int nbs = W.seg >> 5, cps = (nbs + 3) >> 2, n_chunks = W.nseg * cps; // blocks per segment, chunks of <= 4 blocks per segment
-
-    // what this thread fetches of a stage: A chunks c = tid + 128 u -> row c / 8, 16-byte piece c % 8 (4 of them)
-    const int piece = tid & 7;
-    const unsigned char *arow[4];
-    unsigned adst[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const int r = (tid >> 3) + 16 * u;
-        const int row = min(row0 + r, W.rows - 1);
-        arow[u] = W.base + ((size_t)(row >> 2) * W.nseg * 4 + (row & 3)) * (size_t)W.unit_bytes;
-        adst[u] = T::A_Q + r * 128 + ((piece ^ (r & 7)) << 4);
-    }
-    const int srow = min(row0 + (tid & 63), W.rows - 1);
-    const unsigned char *asrc = W.base + ((size_t)(srow >> 2) * W.nseg * 4 + (srow & 3)) * (size_t)W.unit_bytes + W.seg;
-    constexpr int BU = (TOK + 15) / 16;
-    const int8_t *brow[BU];
-    unsigned bdst[BU];
-#pragma unroll
-    for (int u = 0; u < BU; u++) {
-        const int t = (tid >> 3) + 16 * u;
-        brow[u] = AQ + (size_t)(tok0 + t) * W.cols + piece * 16; // (TOK == 8: rows 8 .. 15 belong to nobody and are not fetched)
-        bdst[u] = T::B_Q + t * 128 + ((piece ^ (t & 7)) << 4);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++) arow[u] += piece * 16;
-    const float *bsrc = AS + (size_t)((tid - 64) / (TOK / 4)) * lds + tok0 + (tid - 64) % (TOK / 4) * 4; // scales of block (tid - 64) / (TOK / 4) of a stage
-    const unsigned seg_step = 4u * (unsigned)W.unit_bytes;
-    unsigned a_off = 0, s_off = 0, b_off = 0, f_c = 0, seg_off = 0; // byte offsets of the next chunk: weights, weight scales, activations; chunk in the segment
-    size_t bs_off = 0;                                              // activation scales (floats)
-
-    auto fetch = [&](int stage) {
-        const int blocks = min(4, nbs - 4 * (int)f_c);
-        const unsigned s = smb + stage * T::STAGE;
-        if (piece < 2 * blocks) {
-#pragma unroll
-            for (int u = 0; u < 4; u++) xp_cp16(s + adst[u], arow[u] + a_off);
-#pragma unroll
-            for (int u = 0; u < BU; u++)
-                if (TOK >= 16 || (tid >> 3) < TOK) xp_cp16(s + bdst[u], brow[u] + b_off);
-        }
-        if (tid < 64) xp_cp8(s + T::A_S + tid * 8, asrc + s_off); // the scale area of a unit is padded to 16 bytes
-        else if (tid - 64 < blocks * (TOK / 4)) xp_cp16(s + T::B_S + (tid - 64) * 16, bsrc + bs_off);
-        a_off += 128; s_off += 8;
-        b_off += 32 * blocks;
-        bs_off += (size_t)blocks * lds;
-        if (++f_c == (unsigned)cps) { f_c = 0; seg_off += seg_step; a_off = s_off = seg_off; }
+    int f_seg = 0, f_c = 0, f_stage = 0; // (thread 0) the next chunk to fetch
+    auto fetch = [&]() {
+        const unsigned s = smb + f_stage * T::STAGE, bar = full0 + 8 * f_stage;
+        mbar_expect_tx(bar, T::BYTES_IN);
+        xp_load4(s + T::A_Q, &map_w.q, 128 * f_c, f_seg, row0 >> 2, bar);
+        pg::tma_load_2d(s + T::B_Q, &map_a.q, f_seg * W.seg + 128 * f_c, tok0, bar);
+        xp_load4(s + T::A_S, &map_w.s, W.seg + ((8 * f_c) & ~15), f_seg, row0 >> 2, bar); // 8 scales of a row, 16 bytes
+        pg::tma_load_2d(s + T::B_S, &map_a.s, tok0, f_seg * nbs + 4 * f_c, bar);
+        if (++f_c == cps) { f_c = 0; f_seg++; }
+        if (++f_stage == XP_STAGES) f_stage = 0;
     };
-#pragma unroll
-    for (int s = 0; s < XP_STAGES - 1; s++) {
-        if (s < n_chunks) fetch(s);
-        xp_cp_commit();
+    if (tid == 0) {
+        for (int s = 0; s < XP_STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, XP_THREADS / 32); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int s = 0; s < XP_STAGES && s < n_chunks; s++) fetch();
     }
+    __syncthreads();
 
-    float acc[MI][NW][2][2]; // [row tile][token tile][row lane/4 | row lane/4 + 8][token 2 (lane % 4) | + 1]
+    xp_f2 acc[MI][NW][2]; // [row tile][token tile][row lane/4 | row lane/4 + 8], tokens 2 (lane % 4), + 1
 #pragma unroll
     for (int i = 0; i < MI; i++)
 #pragma unroll
-        for (int j = 0; j < NW; j++) acc[i][j][0][0] = acc[i][j][0][1] = acc[i][j][1][0] = acc[i][j][1][1] = 0.0f;
-    const xp_f2 minus_magic = xp_pack(-12582912.0f, -12582912.0f);
+        for (int j = 0; j < NW; j++) acc[i][j][0] = acc[i][j][1] = 0ull;
+    const xp_f2 one = xp_pack(one_f, one_f);
     const int wrow = (warp % (4 / MI)) * 16 * MI, wtok = (warp / (4 / MI)) * 8 * NW; // the warp's first row and token in the tile
     const int ar = wrow + (lane & 15), ap = lane >> 4;                              // ldmatrix: A row, 16-byte half
     const int bt = wtok + (NW > 1 ? ((lane >> 4) << 3) + (lane & 7) : (lane & 7)), bp = (lane >> 3) & 1; // B token (of 16), half
-    int stage = 0, c_in_seg = 0;
-    for (int c = 0; c < n_chunks; c++) {
-        xp_cp_wait<XP_STAGES - 2>();
-        __syncthreads();
-        {
-            int fs = stage + XP_STAGES - 1;
-            if (fs >= XP_STAGES) fs -= XP_STAGES;
-            if (c + XP_STAGES - 1 < n_chunks) fetch(fs);
-            xp_cp_commit();
-        }
+    const unsigned a_base = T::A_Q + ar * 128, b_base = T::B_Q + bt * 128, as_base = T::B_S + (wtok + 2 * (lane & 3)) * 4, ws_base = T::A_S + (wrow + (lane >> 2)) * 16;
+    int stage = 0, c_in_seg = 0, c = 0;
+    unsigned ph = 0;
+    bool ok = true;
+    for (; c < n_chunks; c++) {
+        if (!(ok = __all_sync(0xffffffffu, xp_wait(full0 + 8 * stage, ph)))) break;
         const unsigned s = smb + stage * T::STAGE;
-        const unsigned char *sp = smraw + stage * T::STAGE;
-        uint2 ws[MI][2];
+        __half2 ws[MI][2][2]; // scales of blocks {0, 1}, {2, 3}
 #pragma unroll
         for (int i = 0; i < MI; i++)
 #pragma unroll
-            for (int h = 0; h < 2; h++) ws[i][h] = *reinterpret_cast<const uint2 *>(sp + T::A_S + (wrow + 16 * i + 8 * h + (lane >> 2)) * 8);
+            for (int h = 0; h < 2; h++) {
+                const xp_f2 v = xp_lds64(s + ws_base + (16 * i + 8 * h) * 16 + 8 * (c_in_seg & 1));
+                const unsigned lo = (unsigned)v, hi = (unsigned)(v >> 32);
+                ws[i][h][0] = *reinterpret_cast<const __half2 *>(&lo);
+                ws[i][h][1] = *reinterpret_cast<const __half2 *>(&hi);
+            }
         const int blocks = min(4, nbs - 4 * c_in_seg);
-        auto block = [&](int k) {
+        auto block = [&](const int k) {
             unsigned a[MI][4];
             xp_f2 wp[MI][2];
 #pragma unroll
             for (int i = 0; i < MI; i++) {
-                xp_ldsm4(a[i], s + T::A_Q + (ar + 16 * i) * 128 + (((2 * k + ap) ^ (ar & 7)) << 4));
+                xp_ldsm4(a[i], s + a_base + i * 2048 + (((2 * k + ap) ^ (ar & 7)) << 4));
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const unsigned hw = k < 2 ? ws[i][h].x : ws[i][h].y;
-                    const float w = __half2float(__ushort_as_half((unsigned short)(k & 1 ? hw >> 16 : hw & 0xffffu)));
+                    const float w = k & 1 ? __high2float(ws[i][h][k >> 1]) : __low2float(ws[i][h][k >> 1]);
                     wp[i][h] = xp_pack(w, w);
                 }
             }
 #pragma unroll
             for (int j = 0; j < NW; j += 2) {
                 unsigned b[4]; // two token tiles (NW == 1: the second one is the first again)
-                const int t = bt + j * 8;
-                xp_ldsm4(b, s + T::B_Q + t * 128 + (((2 * k + bp) ^ (t & 7)) << 4));
+                xp_ldsm4(b, s + b_base + j * 1024 + (((2 * k + bp) ^ (bt & 7)) << 4));
 #pragma unroll
                 for (int jj = 0; jj < (NW > 1 ? 2 : 1); jj++) {
-                    const xp_f2 as = *reinterpret_cast<const xp_f2 *>(sp + T::B_S + (k * TOK + wtok + (j + jj) * 8 + 2 * (lane & 3)) * 4);
+                    const xp_f2 as = xp_lds64(s + as_base + (k * TOK + (j + jj) * 8) * 4);
 #pragma unroll
                     for (int i = 0; i < MI; i++) {
-                        // one row tile turns its integers to floats by the subtraction above, the other by conversions: they run beside the FP32 pipe
-                        const bool cvt = i == 1;
                         int d0, d1, d2, d3;
                         asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                                      : "=r"(d0), "=r"(d1), "=r"(d2), "=r"(d3)
-                                     : "r"(a[i][0]), "r"(a[i][1]), "r"(a[i][2]), "r"(a[i][3]), "r"(b[2 * jj]), "r"(b[2 * jj + 1]), "r"(cvt ? 0 : 0x4B400000));
-                        const xp_f2 f0 = cvt ? xp_pack((float)d0, (float)d1) : xp_add2(xp_pack(__int_as_float(d0), __int_as_float(d1)), minus_magic);
-                        const xp_f2 f1 = cvt ? xp_pack((float)d2, (float)d3) : xp_add2(xp_pack(__int_as_float(d2), __int_as_float(d3)), minus_magic);
-                        float t0, t1, t2, t3;
-                        xp_unpack(xp_mul2(f0, xp_mul2(wp[i][0], as)), t0, t1);
-                        xp_unpack(xp_mul2(f1, xp_mul2(wp[i][1], as)), t2, t3);
-                        float(&ac)[2][2] = acc[i][j + jj];
-                        ac[0][0] = __fadd_rn(ac[0][0], t0); ac[0][1] = __fadd_rn(ac[0][1], t1);
-                        ac[1][0] = __fadd_rn(ac[1][0], t2); ac[1][1] = __fadd_rn(ac[1][1], t3);
+                                     : "r"(a[i][0]), "r"(a[i][1]), "r"(a[i][2]), "r"(a[i][3]), "r"(b[2 * jj]), "r"(b[2 * jj + 1]), "r"(0));
+                        const xp_f2 f0 = xp_pack((float)d0, (float)d1), f1 = xp_pack((float)d2, (float)d3);
+                        xp_f2(&ac)[2] = acc[i][j + jj];
+                        ac[0] = xp_fma2(ac[0], one, xp_mul2(f0, xp_mul2(wp[i][0], as)));
+                        ac[1] = xp_fma2(ac[1], one, xp_mul2(f1, xp_mul2(wp[i][1], as)));
                     }
                 }
             }
@@ -283,28 +264,36 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(TileMat W, const int8
             for (int k = 0; k < 3; k++)
                 if (k < blocks) block(k);
         }
-        if (++stage == XP_STAGES) stage = 0;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty0 + 8 * stage);
+        if (tid == 0 && c + XP_STAGES < n_chunks) { // the stage goes to the chunk after the next two, once every warp is done with it
+            ok = xp_wait(empty0 + 8 * stage, ph);
+            if (ok) fetch();
+        }
+        if (++stage == XP_STAGES) { stage = 0; ph ^= 1u; }
         if (++c_in_seg == cps) c_in_seg = 0;
+    }
+    if (!ok && lane == 0) { // (a wait gave up: the host is told, and nothing leaves with its copies in flight)
+        *reinterpret_cast<volatile unsigned *>(err) = 200u;
+        for (int q = c; q < n_chunks && q < c + XP_STAGES; q++) xp_wait(full0 + 8 * (q % XP_STAGES), (q / XP_STAGES) & 1);
     }
 
     const int r0 = wrow + (lane >> 2), t0 = wtok + 2 * (lane & 3);
     if (MODE == XP_GATEUP) { // rows of a group: gate 2G, gate 2G + 1, up 2G, up 2G + 1; the CTA's 64 rows are one 32-unit block of the hidden row
-        xp_cp_wait<0>();
-        __syncthreads();
-        float *hv = reinterpret_cast<float *>(smraw);
+        __syncthreads(); // (every fetch has landed: a warp is here behind its last chunk)
+        float *hv = reinterpret_cast<float *>(ring);
 #pragma unroll
         for (int i = 0; i < MI; i++)
 #pragma unroll
             for (int j = 0; j < NW; j++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    const float g0 = acc[i][j][h][0], g1 = acc[i][j][h][1];
-                    const float u0 = __shfl_down_sync(0xffffffffu, g0, 8), u1 = __shfl_down_sync(0xffffffffu, g1, 8);
-                    if (!((lane >> 2) & 2)) {
-                        const int row = r0 + 16 * i + 8 * h, unit = (row >> 2) * 2 + (row & 1), t = t0 + j * 8;
-                        hv[t * 33 + unit] = swiglu_exact(g0, u0);
-                        hv[(t + 1) * 33 + unit] = swiglu_exact(g1, u1);
-                    }
+                    float v0, v1; // lanes with a gate row finish the first token, those with its up row the second
+                    xp_unpack(acc[i][j][h], v0, v1);
+                    const bool up = (lane >> 2) & 2;
+                    const float o = __shfl_xor_sync(0xffffffffu, up ? v0 : v1, 8);
+                    const int row = r0 + 16 * i + 8 * h, unit = (row >> 2) * 2 + (row & 1), t = t0 + j * 8 + (up ? 1 : 0);
+                    hv[t * 33 + unit] = swiglu_exact(up ? o : v0, up ? v1 : o);
                 }
         __syncthreads();
         const int hidden = W.rows >> 1;
@@ -329,13 +318,42 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(TileMat W, const int8
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int row = row0 + r0 + 16 * i + 8 * h, t = tok0 + t0 + j * 8;
-                const float v0 = acc[i][j][h][0], v1 = acc[i][j][h][1];
+                float v0, v1;
+                xp_unpack(acc[i][j][h], v0, v1);
                 if (row < W.rows) {
                     float *o = out + (size_t)t * ldo + row;
                     if (t < n) o[0] = MODE == XP_RESID ? __fadd_rn(o[0], v0) : v0;
                     if (t + 1 < n) o[ldo] = MODE == XP_RESID ? __fadd_rn(o[ldo], v1) : v1;
                 }
             }
+}
+
+// The tile-major matrix as {column of a segment, slot of a group, segment, group}: a box is 128 bytes of quants, or 16 of scales, of one segment in 16 groups =
+// 64 rows.  Behind the segment's last column a box of quants holds scales: blocks that are not multiplied.
+inline int xp_map_weights(XpMaps *maps, const TileMat &W) {
+    pg::EncodeTiledFn fn = pg::encode_fn();
+    if (!fn) return -1;
+    cuuint64_t dims[4] = {(cuuint64_t)W.unit_bytes, 4, (cuuint64_t)W.nseg, (cuuint64_t)(W.rows / 4)};
+    cuuint64_t strides[3] = {(cuuint64_t)W.unit_bytes, (cuuint64_t)W.unit_bytes * 4, (cuuint64_t)W.unit_bytes * 4 * W.nseg};
+    cuuint32_t box[4] = {128, 4, 1, XP_ROWS / 4}, sbox[4] = {16, 4, 1, XP_ROWS / 4}, estr[4] = {1, 1, 1, 1};
+    void *base = const_cast<unsigned char *>(W.base);
+    const CUresult q = fn(&maps->q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult s = fn(&maps->s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base, dims, strides, sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return q == CUDA_SUCCESS && s == CUDA_SUCCESS ? 0 : -2;
+}
+// int8 activations [rows][cols] and their scales [blocks][rows]: boxes of 128 columns x the tile's tokens, and of the tile's tokens x 4 blocks
+inline int xp_map_acts(XpMaps *maps, const int8_t *q, const float *s, int rows, int cols, int nt) {
+    pg::EncodeTiledFn fn = pg::encode_fn();
+    if (!fn) return -1;
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols}, sdims[2] = {(cuuint64_t)rows, (cuuint64_t)cols / 32}, sstrides[1] = {(cuuint64_t)rows * 4};
+    cuuint32_t box[2] = {128, (cuuint32_t)nt}, sbox[2] = {(cuuint32_t)nt, 4}, estr[2] = {1, 1};
+    const CUresult rq = fn(&maps->q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t *>(q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult rs = fn(&maps->s, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(s), sdims, sstrides, sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return rq == CUDA_SUCCESS && rs == CUDA_SUCCESS ? 0 : -2;
 }
 
 // ---- head norm, rotation, cache rows of one token (k_attention's prologue for a whole row) ------------------------------------------

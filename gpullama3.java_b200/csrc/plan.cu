@@ -18,6 +18,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <chrono>
 #include <string>
 #include <thread>
@@ -134,6 +135,9 @@ struct b200_plan {
         int8_t *AQ = nullptr, *HQ = nullptr;
         float *scratch = nullptr; // score rows of contexts whose rows do not fit shared memory
         size_t scratch_bytes = 0;
+        struct Maps { XpMaps qkv, wo, gu, w2; }; // a layer's weights
+        std::vector<Maps> maps;
+        XpMaps mA[4], mATT[4], mH[4]; // activations in tiles of 8, 16, 32, 64 tokens: AQ with rows of dim and of the query width, HQ
     } xp;
     // persistent decode kernel
     bool pd_ok = false;           // the plan fits the kernel's restrictions
@@ -1283,6 +1287,17 @@ int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide) {
         if ((rc = dalloc(p, &p->xp.scratch, want))) return rc;
         p->xp.scratch_bytes = want;
     }
+    bool ok = true;
+    for (int i = 0; ok && i < 4; i++)
+        ok = xp_map_acts(&p->xp.mA[i], p->xp.AQ, p->xp.AS, rows, g.dim, 8 << i) == 0 && xp_map_acts(&p->xp.mATT[i], p->xp.AQ, p->xp.AS, rows, p->qd, 8 << i) == 0 &&
+             xp_map_acts(&p->xp.mH[i], p->xp.HQ, p->xp.HS, rows, g.hidden_dim, 8 << i) == 0;
+    p->xp.maps.resize(g.n_layers);
+    for (int l = 0; ok && l < g.n_layers; l++) {
+        const LayerW &L = p->layers[l];
+        auto &m = p->xp.maps[l];
+        ok = xp_map_weights(&m.qkv, L.tqkv) == 0 && xp_map_weights(&m.wo, L.two) == 0 && xp_map_weights(&m.gu, L.tgu) == 0 && xp_map_weights(&m.w2, L.tw2) == 0;
+    }
+    if (!ok) return fail(p, B200_ERR_CUDA, "cuTensorMapEncodeTiled rejected a tensor map of the batched exact prefill");
     p->xp.rows = rows;
     return B200_OK;
 }
@@ -1290,23 +1305,33 @@ int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide) {
 XpLast xp_last(const b200_plan *p) { return XpLast{p->xq, p->hq, p->xs, p->hs, p->hb}; }
 
 template <int MODE>
-int xp_gemm(b200_plan *p, const TileMat &W, const int8_t *aq, const float *as, int n, float *out, int ldo, int8_t *hq, float *hs) {
+int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps (&ma)[4], int n, float *out, int ldo, int8_t *hq, float *hs) {
     const int mt = (W.rows + XP_ROWS - 1) / XP_ROWS;
     auto go = [&](auto nj) -> int {
         constexpr int NJ = decltype(nj)::value;
         auto kern = k_xp_gemm<MODE, NJ>;
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<NJ>::BYTES));
-        kern<<<dim3(mt, (n + 8 * NJ - 1) / (8 * NJ)), XP_THREADS, XpTile<NJ>::BYTES, p->stream>>>(W, aq, as, p->xp.rows, n, out, ldo, hq, hs, xp_last(p));
+        kern<<<dim3(mt, (n + 8 * NJ - 1) / (8 * NJ)), XP_THREADS, XpTile<NJ>::BYTES, p->stream>>>(mw, ma[NJ == 8 ? 3 : NJ == 4 ? 2 : NJ - 1], W, p->xp.rows, n, out, ldo, hq, hs, xp_last(p), 1.0f, p->d_err);
         CK(cudaGetLastError());
         return B200_OK;
     };
-    // the largest token tile that leaves no SM without a CTA (and is not mostly padding): a wider tile reads a weight fewer times, a narrower one
-    // shortens the chain of a column block
-    auto fits = [&](int tok) { return (tok == 8 || n > tok / 2) && (tok == 8 || mt * ((n + tok - 1) / tok) >= p->n_sms); };
-    if (fits(64)) return go(std::integral_constant<int, 8>());
-    if (fits(32)) return go(std::integral_constant<int, 4>());
-    if (fits(16)) return go(std::integral_constant<int, 2>());
-    return go(std::integral_constant<int, 1>());
+    // The token tile with the least time by this model: an SM works its CTAs off at `share` each, but no faster than the chain of one CTA, which the others
+    // lengthen a little (both in ns per column block, measured at 1 - 28 CTAs per SM, 36 - 512 tokens, 4B and 8B layers).  A wide tile has the cheaper token, a
+    // narrow one the shorter chain and the evener spread: Wo and W2 of the 4B layer at 200 tokens 62.4 us in tiles of 64, 47.5 of 32, 45.9 of 16, 69.7 of 8.
+    static const struct { int tok; float chain, share; } tiles[4] = {{64, 240.f, 120.f}, {32, 185.f, 75.f}, {16, 150.f, 46.f}, {8, 140.f, 35.f}};
+    int best = 0;
+    float least = 0.f;
+    for (int i = 0; i < 4; i++) {
+        const int ctas = mt * ((n + tiles[i].tok - 1) / tiles[i].tok), per_sm = (ctas + p->n_sms - 1) / p->n_sms;
+        const float t = std::max(per_sm * tiles[i].share, tiles[i].chain + (per_sm - 1) * tiles[i].share / 3.f);
+        if (i == 0 || t < least) { best = i; least = t; }
+    }
+    switch (best) {
+    case 0: return go(std::integral_constant<int, 8>());
+    case 1: return go(std::integral_constant<int, 4>());
+    case 2: return go(std::integral_constant<int, 2>());
+    default: return go(std::integral_constant<int, 1>());
+    }
 }
 
 // n tokens already in prefill.tok (device), positions start_pos .. start_pos + n - 1
@@ -1352,17 +1377,18 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     };
     for (int l = 0; l < g.n_layers; l++) {
         const LayerW &L = p->layers[l];
+        const auto &m = c.maps[l];
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
         int rc;
         if ((rc = norm(l == 0, L.attn_norm))) return rc;
-        if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, c.AQ, c.AS, n, c.QKV, nqkv, nullptr, nullptr))) return rc;
+        if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, m.qkv, c.mA, n, c.QKV, nqkv, nullptr, nullptr))) return rc;
         k_xp_rope_kv<<<n, 256, rope_smem, p->stream>>>(c.QKV, kc, vc, g.head_size, g.n_heads, g.n_kv_heads, p->kflags, L.q_norm, L.k_norm, g.rms_norm_eps, p->rope_cr, p->rope_ci, start_pos);
         CK(cudaGetLastError());
         if ((rc = attention(kc, vc))) return rc;
-        if ((rc = xp_gemm<XP_RESID>(p, L.two, c.AQ, c.AS, n, c.X, g.dim, nullptr, nullptr))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, L.two, m.wo, c.mATT, n, c.X, g.dim, nullptr, nullptr))) return rc;
         if ((rc = norm(false, L.ffn_norm))) return rc;
-        if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, c.AQ, c.AS, n, nullptr, 0, c.HQ, c.HS))) return rc;
-        if ((rc = xp_gemm<XP_RESID>(p, L.tw2, c.HQ, c.HS, n, c.X, g.dim, nullptr, nullptr))) return rc;
+        if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, m.gu, c.mA, n, nullptr, 0, c.HQ, c.HS))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, L.tw2, m.w2, c.mH, n, c.X, g.dim, nullptr, nullptr))) return rc;
     }
     // the single-token buffers hold what the last token's own step would have left there (the others: XpLast)
     CK(cudaMemcpyAsync(p->x, c.X + (size_t)(n - 1) * g.dim, (size_t)g.dim * 4, cudaMemcpyDeviceToDevice, p->stream));
@@ -1590,8 +1616,8 @@ cudaGraphExec_t prefill_graph(b200_plan *p, int pos) {
 int check_device_error(b200_plan *p) {
     if (p->h_err && *reinterpret_cast<volatile unsigned *>(p->h_err)) {
         const unsigned code = *reinterpret_cast<volatile unsigned *>(p->h_err);
-        return fail(p, B200_ERR_STATE, "a device-side wait timed out (code %u: 1+phase of the persistent decode kernel, 100+slot of a tensor-parallel flag): a peer "
-                                       "rank is missing or the ranks' call sequences diverged; the plan must be freed", code);
+        return fail(p, B200_ERR_STATE, "a device-side wait timed out (code %u: 1+phase of the persistent decode kernel, 100+slot of a tensor-parallel flag, 200 the "
+                                       "batched exact prefill's operand ring): a peer rank is missing or the ranks' call sequences diverged; the plan must be freed", code);
     }
     return B200_OK;
 }
@@ -1761,7 +1787,7 @@ int b200_forward_batch_prefill(b200_plan *p, const int32_t *tokens, int32_t n, i
         int rc2 = exact_prefill(p, n, start_pos);
         if (rc2) return rc2;
         CK(cudaStreamSynchronize(p->stream));
-        return B200_OK;
+        return check_device_error(p);
     }
     CK(cudaMemcpyAsync(p->seq_tokens, p->h_ids, (size_t)n * 4, cudaMemcpyHostToDevice, p->stream));
     int rc;
