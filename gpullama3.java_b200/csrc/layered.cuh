@@ -1255,41 +1255,69 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// The same attention for a prefill chunk on the tensor cores (BF16 compute mode; instantiated for key / value sizes 64 / 64,
-// 128 / 128 and 192 / 128): one CTA per (128 query rows, head), eight
-// warps of 16 rows (two warps per scheduler: a lone warp cannot hide the latency of its own dependent instructions).  Keys and values come from the BF16 twin rows of the ring (written by k_qk_prep next to the FP32 rows the
-// decode step reads): key tiles of 64 positions travel global -> shared with cp.async, double buffered, so the copy of tile
-// i + 1 overlaps the mma.sync m16n8k16 work on tile i; V fragments are read with ldmatrix.trans.  Scores, cap, distance bias,
-// mask and the ONLINE softmax stay in FP32 registers.  The sink is the initial state of the running softmax: maximum 0,
-// denominator exp(0) = 1, no value.  Dynamic shared memory: att_mma_smem_bytes<DK, DV>(window).
+// The same attention for a prefill chunk on the tensor cores (BF16 compute mode; instances: ly_mma_kind): a CTA per (64 or 128 query rows, head), a warp per 16
+// rows.  Keys and values come from the BF16 twin rows of the ring (written by k_qk_prep next to the FP32 rows the decode step reads): key tiles of 64 positions travel
+// global -> shared with cp.async, double buffered, so the copy of tile i + 1 overlaps the mma.sync m16n8k16 work on tile i.  Scores, cap, distance bias, mask and the
+// ONLINE softmax stay in FP32 registers, in units of log2.  The sink is the initial state of the running softmax: maximum z, denominator exp(z - z), no value.
+// Bound by the latency of few warps (one or two per scheduler: 512 rows are only 1024 warps of 16 rows at 32 heads), so what counts is a warp's instructions and its
+// dependent chains: the eight score tiles of a step advance side by side with 16 keys per ldmatrix (one after the other, their sums wait for each other), only
+// tiles that a row does not wholly see are masked, a lane's column of the copies is fixed, exponentials are the hardware's, the accumulator is rescaled only when a
+// maximum moved, and the loads of queries, distances and gates are in flight together.  2058 warp instructions per (16 rows, 64 keys) at key size 192 before.
+// Where the tiles do not fill the SMs, the CTAs of a cluster share a tile's keys and merge over distributed shared memory.  512 rows: 32 heads of 128 with cap and
+// distances 50 -> 35 us, 32 heads of 64 30 -> 24, 16 heads of 192 / 128 36 -> 24, of 256 / 128 38 -> 24.  Dynamic shared memory: att_mma_smem_bytes<DK, DV>(rows, window).
 // ---------------------------------------------------------------------------------------------------------------------
 #define LY_ATT_MMA_ROWS 128 // query rows per CTA: eight warps of 16 rows share every key tile (launches of few CTAs: 64 rows, four warps, so that more SMs work)
-template <int DK, int DV> __host__ __device__ constexpr size_t att_mma_smem_bytes(int window) { // for the taller tile; the other one needs less
-    return (size_t)(LY_ATT_MMA_ROWS * (DK + 8) * 2) + (size_t)(64 * (DK + 8) * 2) * 2 + (size_t)(64 * (DV + 8) * 2) * 2 + (size_t)window * 4;
+template <int DK, int DV> __host__ __device__ constexpr size_t att_mma_smem_bytes(int rows, int window) { // two stages of keys and values, the queries first in the second one; distances
+    const size_t stage = (size_t)64 * (DK + 8) * 2 + (size_t)64 * (DV + 8) * 2, q = (size_t)rows * (DK + 8) * 2;
+    return stage + (stage > q ? stage : q) + (size_t)window * 4;
 }
 // 1 / (1 + exp(-x)) with the hardware exponential and division: relative error ~1e-6, far below the BF16 rounding of the gated result
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
-// tanh(x) = 1 - 2 / (1 + exp(2x)) with the hardware exponential: absolute error ~1e-7, far below the BF16 rounding of the
-// operands that produced x (the FP32 kernels keep tanhf)
-__device__ __forceinline__ float tanh_fast(float x) { return 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * x)); }
 __device__ __forceinline__ void ldmatrix_x2_trans(unsigned (&r)[2], const void *row) {
     const unsigned a = (unsigned)__cvta_generic_to_shared(row);
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a));
 }
 
+#define LOG2E 1.4426950408889634f
+// The hardware's 2^x and 1 / x, subnormals to zero: an exponential and a division without them take three instructions more each
+__device__ __forceinline__ float exp2_fast(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], unsigned a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(unsigned (&r)[4], unsigned a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ float4 ld_cluster_f32x4(const float4 *p, int rank) {
+    unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r) : "memory");
+    return v;
+}
+
 template <int DK, int DV, int BM = LY_ATT_MMA_ROWS>
 __global__ void __launch_bounds__(BM * 2) k_window_attention_mma(const float *__restrict__ P, int ldp, WindowAttn a, const bf16 *__restrict__ kc16,
                                                                              const bf16 *__restrict__ vc16, const StepState *__restrict__ st, int n,
-                                                                             bf16 *__restrict__ out, int ldo, float *__restrict__ out32 = nullptr) {
+                                                                             bf16 *__restrict__ out, int ldo, float *__restrict__ out32, int parts) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int LY_ATT_MMA_THREADS = BM * 2;
-    constexpr int QT = BM * (DK + 8) * 2, KT = 64 * (DK + 8) * 2, VT = 64 * (DV + 8) * 2; // bytes of the Q tile, one K tile, one V tile
-    bf16(*Qs)[DK + 8] = reinterpret_cast<bf16(*)[DK + 8]>(smraw);
-    float *sbias = reinterpret_cast<float *>(smraw + QT + 2 * KT + 2 * VT);
+    constexpr int QT = BM * (DK + 8) * 2, KT = 64 * (DK + 8) * 2, VT = 64 * (DV + 8) * 2, ST = KT + VT; // bytes of the Q tile, one K tile, one V tile, a stage
+    bf16(*Qs)[DK + 8] = reinterpret_cast<bf16(*)[DK + 8]>(smraw + ST);                                  // until it is in registers
+    float *sbias = reinterpret_cast<float *>(smraw + ST + (ST > QT ? ST : QT));
+    const int part = blockIdx.x % parts;                                                                // which CTA of the cluster this is
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int h = blockIdx.y, r0 = blockIdx.x * BM;
+    const int h = blockIdx.y, r0 = ((int)(gridDim.x / parts) - 1 - (int)(blockIdx.x / parts)) * BM; // the latest rows (the most keys) first
     const int kd = a.ldk, vd = a.ldv, qd = a.heads * DK; // row strides of the BF16 twin rings = those of the FP32 rings
     const int kvh = h / (a.heads / a.kv_heads);
     const int kh = a.maps > 1 ? kvh * a.maps + h % a.maps : a.k_heads > 0 ? h / (a.heads / a.k_heads) : kvh;
@@ -1297,39 +1325,58 @@ __global__ void __launch_bounds__(BM * 2) k_window_attention_mma(const float *__
     const int pos0 = st->pos;
     const int rows = n - r0 < BM ? n - r0 : BM;
     const int q_lo = pos0 + r0, q_hi = pos0 + r0 + rows - 1;
-    const int k_lo = window_first(a, q_lo);
+    const int k_lo = window_first(a, q_lo), k_first = k_lo + 64 * part; // the parts take the key tiles in turn
+    // 64 rows of W elements -> shared memory, rows behind the last position zero; a power of two of lanes per row keeps a lane's column fixed
+    auto load_rows = [&](auto w_c, unsigned dst, const bf16 *src, int ld, int kt0, int slot0) {
+        constexpr int W = decltype(w_c)::value, LPR = W <= 32 ? 4 : W <= 64 ? 8 : W <= 128 ? 16 : 32, RPP = LY_ATT_MMA_THREADS / LPR; // lanes per row, rows per pass
+        const int c = (lane % LPR) * 8, rr = tid / LPR;
+        if (W % (8 * LPR) && c >= W) return;
+#pragma unroll
+        for (int u = 0; u < 64 / RPP; u++) {
+            const int r = rr + u * RPP;
+            const bool ok = kt0 + r <= q_hi;
+            int sl = slot0 + r;
+            if (sl >= a.ring) sl = a.ring >= 64 ? sl - a.ring : sl % a.ring;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (r * (W + 8) + c) * 2), "l"(src + (ok ? (size_t)sl * ld + c : 0)), "r"(ok ? 16 : 0) : "memory");
+        }
+    };
+    const unsigned smb = (unsigned)__cvta_generic_to_shared(smraw);
     auto load_tile = [&](int buf, int kt0) {
-        bf16(*Kd)[DK + 8] = reinterpret_cast<bf16(*)[DK + 8]>(smraw + QT + buf * KT);
-        bf16(*Vd)[DV + 8] = reinterpret_cast<bf16(*)[DV + 8]>(smraw + QT + 2 * KT + buf * VT);
         const int slot0 = kt0 % a.ring; // one division per tile; rows wrap by subtraction (by division only in rings below 64 slots)
-        for (int e = tid; e < 64 * (DK / 8); e += LY_ATT_MMA_THREADS) {
-            const int r = e / (DK / 8), c = (e % (DK / 8)) * 8;
-            const bool ok = kt0 + r <= q_hi;
-            int sl = slot0 + r;
-            if (sl >= a.ring) sl = a.ring >= 64 ? sl - a.ring : sl % a.ring;
-            cp_async16(&Kd[r][c], kc16 + (ok ? (size_t)sl * kd + (size_t)kh * DK + c : 0), ok);
-        }
-        for (int e = tid; e < 64 * (DV / 8); e += LY_ATT_MMA_THREADS) {
-            const int r = e / (DV / 8), c = (e % (DV / 8)) * 8;
-            const bool ok = kt0 + r <= q_hi;
-            int sl = slot0 + r;
-            if (sl >= a.ring) sl = a.ring >= 64 ? sl - a.ring : sl % a.ring;
-            cp_async16(&Vd[r][c], vc16 + (ok ? (size_t)sl * vd + (size_t)kvh * DV + c : 0), ok);
-        }
+        load_rows(std::integral_constant<int, DK>(), smb + buf * ST, kc16 + (size_t)kh * DK, kd, kt0, slot0);
+        load_rows(std::integral_constant<int, DV>(), smb + buf * ST + KT, vc16 + (size_t)kvh * DV, vd, kt0, slot0);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    load_tile(0, k_lo);
+    if (k_first <= q_hi) load_tile(0, k_first);
     // distance -> bias of this head, for the distances this tile of rows can see
-    {
-        const int dmax = q_hi - k_lo + 1 < a.window ? q_hi - k_lo + 1 : a.window;
-        for (int d = tid; d < dmax; d += LY_ATT_MMA_THREADS) sbias[d] = a.rel ? a.rel[(size_t)a.bucket[d] * a.heads + h] : 0.0f;
-    }
+    const int dmax = q_hi - k_lo + 1 < a.window ? q_hi - k_lo + 1 : a.window;
+    if (a.rel)
+        for (int d0 = tid; d0 < dmax; d0 += 4 * LY_ATT_MMA_THREADS) { // four look-ups (two dependent loads each) side by side
+            int row[4];
+            float v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) row[u] = __ldg(a.bucket + min(d0 + u * LY_ATT_MMA_THREADS, dmax - 1));
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = __ldg(a.rel + (size_t)row[u] * a.heads + h);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (d0 + u * LY_ATT_MMA_THREADS < dmax) sbias[d0 + u * LY_ATT_MMA_THREADS] = v[u] * LOG2E;
+        }
     // Q tile -> BF16
-    for (int e = tid; e < BM * (DK / 4); e += LY_ATT_MMA_THREADS) {
-        const int r = e / (DK / 4), c = (e % (DK / 4)) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < rows) v = *reinterpret_cast<const float4 *>(P + (size_t)(r0 + r) * ldp + (size_t)h * DK + c);
-        *reinterpret_cast<uint2 *>(&Qs[r][c]) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    constexpr int QB = DK / 8 <= 16 ? DK / 8 : DK / 16; // loads of a thread in flight (DK / 8 in all)
+#pragma unroll 1
+    for (int e0 = tid; e0 < BM * (DK / 4); e0 += QB * LY_ATT_MMA_THREADS) {
+        float4 v[QB];
+#pragma unroll
+        for (int u = 0; u < QB; u++) {
+            const int e = e0 + u * LY_ATT_MMA_THREADS, r = e / (DK / 4), c = (e % (DK / 4)) * 4;
+            v[u] = r < rows ? __ldg(reinterpret_cast<const float4 *>(P + (size_t)(r0 + r) * ldp + (size_t)h * DK + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < QB; u++) {
+            const int e = e0 + u * LY_ATT_MMA_THREADS, r = e / (DK / 4), c = (e % (DK / 4)) * 4;
+            *reinterpret_cast<uint2 *>(&Qs[r][c]) = make_uint2(pack_bf16(v[u].x, v[u].y), pack_bf16(v[u].z, v[u].w));
+        }
     }
     __syncthreads();
     unsigned qf[DK / 16][4];
@@ -1343,59 +1390,92 @@ __global__ void __launch_bounds__(BM * 2) k_window_attention_mma(const float *__
             qf[kk][3] = *reinterpret_cast<const unsigned *>(&Qs[r + 8][kk * 16 + 2 * t + 8]);
         }
     }
+    __syncthreads(); // the queries make room for the second stage
     float o[DV / 8][4];
 #pragma unroll
     for (int j = 0; j < DV / 8; j++)
 #pragma unroll
         for (int e = 0; e < 4; e++) o[j][e] = 0.0f;
     float mrow[2], lrow[2];
-    mrow[0] = mrow[1] = a.sink ? sink_v : -INFINITY; // the sink: a running softmax that starts at (maximum z, denominator exp(z - z))
-    lrow[0] = lrow[1] = a.sink ? 1.0f : 0.0f;
+    mrow[0] = mrow[1] = a.sink && part == 0 ? sink_v * LOG2E : -INFINITY; // the sink: a running softmax that starts at (maximum z, denominator exp(z - z))
+    lrow[0] = lrow[1] = a.sink && part == 0 ? 1.0f : 0.0f;
     const int prow[2] = {pos0 + r0 + warp * 16 + g, pos0 + r0 + warp * 16 + g + 8}; // positions of this thread's two rows
     const bool vrow[2] = {warp * 16 + g < rows, warp * 16 + g + 8 < rows};
     const int w_lo = pos0 + r0 + warp * 16, w_hi = w_lo + 15; // positions of this warp's rows
     const int w_first = window_first(a, w_lo);                // first key any of them sees
-    const int c_first[2] = {a.chunked ? window_first(a, prow[0]) : 0, a.chunked ? window_first(a, prow[1]) : 0};
-    const float inv_cap = a.softcap > 0.0f ? 1.0f / a.softcap : 0.0f;
+    // keys [k_from, k_from + k_span] that this thread's rows see (none: a span of zero keys behind every position)
+    int k_from[2];
+    unsigned k_span[2];
+#pragma unroll
+    for (int rr = 0; rr < 2; rr++) {
+        const int first = window_first(a, prow[rr]);
+        k_from[rr] = vrow[rr] ? first : 0x7fffffff;
+        k_span[rr] = vrow[rr] ? (unsigned)(prow[rr] - first) : 0u;
+    }
+    // Scores in units of log2: scale, or cap * tanh(scale / cap * x) = cap - 2 cap / (1 + 2^(2 log2(e) scale / cap * x))
+    const float k_scale = a.softcap > 0.0f ? 2.0f * LOG2E * a.scale / a.softcap : a.scale * LOG2E, k_cap = a.softcap * LOG2E, k_cap2 = -2.0f * k_cap;
     int buf = 0;
-    for (int kt0 = k_lo; kt0 <= q_hi; kt0 += 64, buf ^= 1) {
-        if (kt0 + 64 <= q_hi) {
-            load_tile(buf ^ 1, kt0 + 64); // the other buffer was released by the barrier that ended the previous iteration
+    const int step = 64 * parts, w_last_first = window_first(a, w_hi); // first key that the warp's last row sees
+    const bool w_whole = warp * 16 + 16 <= rows;
+    for (int kt0 = k_first; kt0 <= q_hi; kt0 += step, buf ^= 1) {
+        if (kt0 + step <= q_hi) {
+            load_tile(buf ^ 1, kt0 + step); // the other buffer was released by the barrier that ended the previous iteration
             asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         // a warp whose rows see no key of this tile (all later, or all beyond the window) skips the arithmetic
         if (kt0 <= w_hi && kt0 + 63 >= w_first) {
-            bf16(*Ks)[DK + 8] = reinterpret_cast<bf16(*)[DK + 8]>(smraw + QT + buf * KT);
-            bf16(*Vs)[DV + 8] = reinterpret_cast<bf16(*)[DV + 8]>(smraw + QT + 2 * KT + buf * VT);
-            // S = Q K^T for this warp's 16 rows x 64 keys
+            const unsigned ks = smb + buf * ST, vs = ks + KT;
+            // S = Q K^T for this warp's 16 rows x 64 keys: the eight sums of a step are independent, 16 keys per ldmatrix
             float sc[8][4];
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
+            for (int j = 0; j < 8; j++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) sc[j][e] = 0.0f;
+            const unsigned krow = ks + (((lane & 7) + ((lane >> 4) << 3)) * (DK + 8) + (((lane >> 3) & 1) << 3)) * 2;
 #pragma unroll
-                for (int kk = 0; kk < DK / 16; kk++) {
-                    unsigned bfr[2];
-                    bfr[0] = *reinterpret_cast<const unsigned *>(&Ks[j * 8 + g][kk * 16 + 2 * t]);
-                    bfr[1] = *reinterpret_cast<const unsigned *>(&Ks[j * 8 + g][kk * 16 + 2 * t + 8]);
-                    mma_bf16_16816(sc[j], qf[kk], bfr);
+            for (int kk = 0; kk < DK / 16; kk++)
+#pragma unroll
+                for (int j = 0; j < 8; j += 2) {
+                    unsigned b4[4];
+                    ldmatrix_x4(b4, krow + (j * 8 * (DK + 8) + kk * 16) * 2);
+                    const unsigned b0[2] = {b4[0], b4[1]}, b1[2] = {b4[2], b4[3]};
+                    mma_bf16_16816(sc[j], qf[kk], b0);
+                    mma_bf16_16816(sc[j + 1], qf[kk], b1);
                 }
+            // cap, bias, mask (only where a row does not see the whole tile); tile maximum per row
+            const bool whole = w_whole && kt0 + 63 <= w_lo && kt0 >= w_last_first;
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) sc[j][e] *= k_scale;
+            if (a.softcap > 0.0f) {
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) sc[j][e] = fmaf(k_cap2, rcp_fast(1.0f + exp2_fast(sc[j][e])), k_cap);
             }
-            // cap, bias, mask; tile maximum per row
+            if (a.rel) {
+                const int d_top = dmax - 1, d0 = prow[0] - kt0 - 2 * t;
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) // (a distance that is masked below reads any entry)
+                        sc[j][e] += sbias[min(max(d0 + 8 * (e >> 1) - 8 * j - (e & 1), 0), d_top)];
+            }
+            if (!whole) {
+                const unsigned p0 = (unsigned)(kt0 + 2 * t - k_from[0]), p1 = (unsigned)(kt0 + 2 * t - k_from[1]);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if ((e < 2 ? p0 : p1) + (unsigned)(8 * j + (e & 1)) > k_span[e >> 1]) sc[j][e] = -INFINITY;
+            }
             float tmax[2] = {-INFINITY, -INFINITY};
 #pragma unroll
             for (int j = 0; j < 8; j++)
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int rr = e >> 1, pj = kt0 + j * 8 + 2 * t + (e & 1), dist = prow[rr] - pj;
-                    float v = sc[j][e] * a.scale;
-                    if (a.softcap > 0.0f) v = a.softcap * tanh_fast(v * inv_cap);
-                    if (vrow[rr] && dist >= 0 && dist < a.window && pj >= c_first[rr]) v += sbias[dist];
-                    else v = -INFINITY;
-                    sc[j][e] = v;
-                    tmax[rr] = fmaxf(tmax[rr], v);
-                }
+                for (int e = 0; e < 4; e++) tmax[e >> 1] = fmaxf(tmax[e >> 1], sc[j][e]);
             float corr[2], muse[2];
 #pragma unroll
             for (int rr = 0; rr < 2; rr++) {
@@ -1403,7 +1483,7 @@ __global__ void __launch_bounds__(BM * 2) k_window_attention_mma(const float *__
                 tmax[rr] = fmaxf(tmax[rr], __shfl_xor_sync(0xffffffffu, tmax[rr], 2));
                 const float mnew = fmaxf(mrow[rr], tmax[rr]);
                 muse[rr] = mnew == -INFINITY ? 0.0f : mnew;
-                corr[rr] = mrow[rr] == -INFINITY ? 0.0f : __expf(mrow[rr] - muse[rr]);
+                corr[rr] = exp2_fast(mrow[rr] - muse[rr]); // (2^-inf = 0)
                 mrow[rr] = mnew;
                 lrow[rr] *= corr[rr];
             }
@@ -1412,7 +1492,7 @@ __global__ void __launch_bounds__(BM * 2) k_window_attention_mma(const float *__
             for (int j = 0; j < 8; j++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const float pv = __expf(sc[j][e] - muse[e >> 1]); // exp(-inf) = 0 for masked entries
+                    const float pv = exp2_fast(sc[j][e] - muse[e >> 1]); // 2^-inf = 0 for masked entries
                     sc[j][e] = pv;
                     psum[e >> 1] += pv;
                 }
@@ -1422,9 +1502,11 @@ __global__ void __launch_bounds__(BM * 2) k_window_attention_mma(const float *__
                 psum[rr] += __shfl_xor_sync(0xffffffffu, psum[rr], 2);
                 lrow[rr] += psum[rr];
             }
+            if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) { // (no new maximum: nothing to rescale)
 #pragma unroll
-            for (int j = 0; j < DV / 8; j++) {
-                o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1];
+                for (int j = 0; j < DV / 8; j++) {
+                    o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1];
+                }
             }
             // O += P V: the score fragments are the A operand as they stand; V[key][d] becomes the B operand through ldmatrix.trans
 #pragma unroll
@@ -1435,37 +1517,85 @@ __global__ void __launch_bounds__(BM * 2) k_window_attention_mma(const float *__
                 pf[2] = pack_bf16(sc[2 * kk + 1][0], sc[2 * kk + 1][1]);
                 pf[3] = pack_bf16(sc[2 * kk + 1][2], sc[2 * kk + 1][3]);
 #pragma unroll
-                for (int j = 0; j < DV / 8; j++) {
-                    unsigned bfr[2];
-                    ldmatrix_x2_trans(bfr, &Vs[kk * 16 + (lane & 15)][j * 8]);
-                    mma_bf16_16816(o[j], pf, bfr);
+                for (int j = 0; j < DV / 8; j += 2) {
+                    unsigned b4[4];
+                    ldmatrix_x4_trans(b4, vs + ((kk * 16 + (lane & 15)) * (DV + 8) + j * 8 + ((lane >> 4) << 3)) * 2);
+                    const unsigned b0[2] = {b4[0], b4[1]}, b1[2] = {b4[2], b4[3]};
+                    mma_bf16_16816(o[j], pf, b0);
+                    mma_bf16_16816(o[j + 1], pf, b1);
                 }
             }
         }
         __syncthreads(); // every warp is done with this buffer before the next iteration's copy lands in it
     }
-    // normalise, gate, store
+    // The parts meet over distributed shared memory: a part leaves its sums and (maximum, denominator) in place of its tiles, and every part finishes its share of
+    // the columns.
+    int j_lo = 0, j_hi = DV / 8;
+    if (parts > 1) {
+        constexpr int NT = LY_ATT_MMA_THREADS;
+        static_assert((size_t)NT * (DV / 8) * 16 + NT * 16 <= 2 * (size_t)ST, "the sums take the tiles' place");
+        float4 *so = reinterpret_cast<float4 *>(smraw), *sml = so + NT * (DV / 8);
+#pragma unroll
+        for (int j = 0; j < DV / 8; j++) so[j * NT + tid] = make_float4(o[j][0], o[j][1], o[j][2], o[j][3]);
+        sml[tid] = make_float4(mrow[0], mrow[1], lrow[0], lrow[1]);
+        cluster_barrier();
+        float M[2] = {mrow[0], mrow[1]}, L[2] = {0.0f, 0.0f};
+        for (int k = 0; k < parts; k++) {
+            const float4 ml = ld_cluster_f32x4(sml + tid, k);
+            M[0] = fmaxf(M[0], ml.x); M[1] = fmaxf(M[1], ml.y);
+        }
+        const int share = (DV / 8 + parts - 1) / parts;
+        j_lo = part * share;
+        j_hi = j_lo + share < DV / 8 ? j_lo + share : DV / 8;
+#pragma unroll
+        for (int j = 0; j < DV / 8; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
+        for (int k = 0; k < parts; k++) {
+            const float4 ml = ld_cluster_f32x4(sml + tid, k);
+            const float f0 = ml.x == -INFINITY ? 0.0f : exp2_fast(ml.x - M[0]), f1 = ml.y == -INFINITY ? 0.0f : exp2_fast(ml.y - M[1]);
+            L[0] += f0 * ml.z; L[1] += f1 * ml.w;
+#pragma unroll
+            for (int j = 0; j < DV / 8; j++)
+                if (j >= j_lo && j < j_hi) {
+                    const float4 v = ld_cluster_f32x4(so + j * NT + tid, k);
+                    o[j][0] += f0 * v.x; o[j][1] += f0 * v.y; o[j][2] += f1 * v.z; o[j][3] += f1 * v.w;
+                }
+        }
+        lrow[0] = L[0]; lrow[1] = L[1];
+        cluster_barrier(); // nobody leaves while its shared memory may still be read
+    }
+    // normalise, gate, store: the gates of both rows are asked for together
+    const bool entries = a.gate && !a.gate_heads;
+    auto gate_row = [&](int rr) {
+        const int r = r0 + warp * 16 + g + rr * 8;
+        return (a.gate_src ? a.gate_src + (size_t)r * a.gate_ld : P + (size_t)r * ldp) + (a.gate_off >= 0 ? a.gate_off : qd + kd + vd) + (a.gate_heads ? (size_t)h : (size_t)h * DV);
+    };
+    float2 gv[2][DV / 8];
+    float ghead[2] = {1.0f, 1.0f};
+#pragma unroll
+    for (int rr = 0; rr < 2; rr++) {
+        if (!a.gate || !vrow[rr]) continue;
+        const float *gate = gate_row(rr);
+        if (!entries) ghead[rr] = gate[0];
+        else {
+#pragma unroll
+            for (int j = 0; j < DV / 8; j++)
+                if (j >= j_lo && j < j_hi) gv[rr][j] = __ldg(reinterpret_cast<const float2 *>(gate + j * 8 + 2 * t));
+        }
+    }
 #pragma unroll
     for (int rr = 0; rr < 2; rr++) {
         if (!vrow[rr]) continue;
         const int r = r0 + warp * 16 + g + rr * 8;
-        const float inv = lrow[rr] > 0.0f ? a.out_scale / lrow[rr] : 0.0f;
-        const float *gate = (a.gate_src ? a.gate_src + (size_t)r * a.gate_ld : P + (size_t)r * ldp) + (a.gate_off >= 0 ? a.gate_off : qd + kd + vd) +
-                            (a.gate_heads ? (size_t)h : (size_t)h * DV);
-        const float ghead = a.gate && a.gate_heads ? 1.0f / (1.0f + expf(-gate[0])) : 1.0f;
-        const bool entries = a.gate && !a.gate_heads;
-        float2 gv[DV / 8]; // a gate per output entry: the row's loads are in flight together
-        if (entries) {
-#pragma unroll
-            for (int j = 0; j < DV / 8; j++) gv[j] = __ldg(reinterpret_cast<const float2 *>(gate + j * 8 + 2 * t));
-        }
+        float inv = lrow[rr] > 0.0f ? a.out_scale / lrow[rr] : 0.0f;
+        if (a.gate && a.gate_heads) inv *= 1.0f / (1.0f + expf(-ghead[rr]));
 #pragma unroll
         for (int j = 0; j < DV / 8; j++) {
+            if (j < j_lo || j >= j_hi) continue;
             const int d = j * 8 + 2 * t;
-            float v0 = o[j][2 * rr] * inv * ghead, v1 = o[j][2 * rr + 1] * inv * ghead;
+            float v0 = o[j][2 * rr] * inv, v1 = o[j][2 * rr + 1] * inv;
             if (entries) {
-                v0 *= sigmoid_fast(gv[j].x);
-                v1 *= sigmoid_fast(gv[j].y);
+                v0 *= sigmoid_fast(gv[rr][j].x);
+                v1 *= sigmoid_fast(gv[rr][j].y);
             }
             if (out32) *reinterpret_cast<float2 *>(out32 + (size_t)r * ldo + (size_t)h * DV + d) = make_float2(v0, v1); // FP32 results (what a later subtraction reads)
             else *reinterpret_cast<unsigned *>(out + (size_t)r * ldo + (size_t)h * DV + d) = pack_bf16(v0, v1);

@@ -277,20 +277,24 @@ static size_t ly_att_smem(const b200_layer_spec &s, int ring) {
 static int ly_mma_kind(int dk, int dv) {
     return dk == 64 && dv == 64 ? 1 : dk == 128 && dv == 128 ? 2 : dk == 192 && dv == 128 ? 3 : dk == 128 && dv == 64 ? 4 : dk == 256 && dv == 128 ? 5 : dk == 64 && dv == 32 ? 6 : 0;
 }
-static size_t ly_mma_smem(int kind, int window) {
-    return kind == 1 ? ly::att_mma_smem_bytes<64, 64>(window) : kind == 2 ? ly::att_mma_smem_bytes<128, 128>(window) : kind == 3 ? ly::att_mma_smem_bytes<192, 128>(window)
-         : kind == 4 ? ly::att_mma_smem_bytes<128, 64>(window) : kind == 5 ? ly::att_mma_smem_bytes<256, 128>(window) : ly::att_mma_smem_bytes<64, 32>(window);
+static size_t ly_mma_smem(int kind, int window, int rows = LY_ATT_MMA_ROWS) {
+    return kind == 1 ? ly::att_mma_smem_bytes<64, 64>(rows, window) : kind == 2 ? ly::att_mma_smem_bytes<128, 128>(rows, window) : kind == 3 ? ly::att_mma_smem_bytes<192, 128>(rows, window)
+         : kind == 4 ? ly::att_mma_smem_bytes<128, 64>(rows, window) : kind == 5 ? ly::att_mma_smem_bytes<256, 128>(rows, window) : ly::att_mma_smem_bytes<64, 32>(rows, window);
 }
 static int ly_launch_mma(b200_plan *p, int kind, int n, int heads, int window, const float *P, int ldp, const ly::WindowAttn &wa, const ly::bf16 *k16, const ly::bf16 *v16,
                          const StepState *st, ly::bf16 *out, int ldo, float *out32 = nullptr) {
-    const size_t sm = ly_mma_smem(kind, window);
     // few tall tiles leave SMs idle: half as many rows per CTA then
     const bool tall = (n + LY_ATT_MMA_ROWS - 1) / LY_ATT_MMA_ROWS * heads >= p->n_sms;
-    const int rows = tall ? LY_ATT_MMA_ROWS : 64;
-    const dim3 grid((n + rows - 1) / rows, heads), block(rows * 2);
+    const int rows = tall ? LY_ATT_MMA_ROWS : 64, tiles = (n + rows - 1) / rows;
+    // A CTA per SM or less: two CTAs share a tile's keys and every SM has twice the warps (512 rows, 16 heads: 31.0 -> 24.6 us at key size 192, 30.1 -> 24.4 at
+    // 256; with more tiles than SMs it costs: 34.2 -> 39.6 us at 32 heads; a few keys are not worth the merge: 100 rows 17.5 -> 18.2 us)
+    const int keys = p->ly->pf_pos + n < window + rows ? p->ly->pf_pos + n : window + rows;
+    const int parts = tiles * heads <= p->n_sms && keys > 128 ? 2 : 1;
+    const size_t sm = ly_mma_smem(kind, window, rows);
+    const dim3 grid(tiles * parts, heads), block(rows * 2);
 #define LY_MMA_CASE(K, DK, DV) \
-    if (kind == K) return tall ? launch_k(p, false, ly::k_window_attention_mma<DK, DV>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32) \
-                               : launch_k(p, false, ly::k_window_attention_mma<DK, DV, 64>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32);
+    if (kind == K) return tall ? launch_cluster(p, false, parts, ly::k_window_attention_mma<DK, DV>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32, parts) \
+                               : launch_cluster(p, false, parts, ly::k_window_attention_mma<DK, DV, 64>, grid, block, sm, P, ldp, wa, k16, v16, st, n, out, ldo, out32, parts);
     LY_MMA_CASE(1, 64, 64)
     LY_MMA_CASE(2, 128, 128)
     LY_MMA_CASE(3, 192, 128)
