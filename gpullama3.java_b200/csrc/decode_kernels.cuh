@@ -848,7 +848,7 @@ __device__ __forceinline__ void argmax_merge(float &v, int &i, float ov, int oi)
 __global__ void __launch_bounds__(1024) k_argmax_advance(const float *__restrict__ logits, int vocab, StepState *st,
                                                         const int *__restrict__ seq_tokens, int *__restrict__ out_ids,
                                                         int do_argmax, const float *__restrict__ part_val,
-                                                        const int *__restrict__ part_idx, int n_part, TraceBuf tr, TpCtx tp, int tp_wait_x_op) {
+                                                        const int *__restrict__ part_idx, int n_part, TraceBuf tr, TpCtx tp, int tp_wait_x_op, int *__restrict__ id_copy) {
     __shared__ float sv[32];
     __shared__ int si[32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -937,6 +937,7 @@ __global__ void __launch_bounds__(1024) k_argmax_advance(const float *__restrict
     if (tid == 0) {
         int step = st->step;
         if (do_argmax && out_ids) out_ids[step] = best_i;
+        if (do_argmax && id_copy) *id_copy = best_i; // behind the logits: one copy brings both to the host
         int next = step + 1;
         if (st->feedback && do_argmax) st->token = best_i;
         else if (next < st->n_seq) st->token = seq_tokens[next];

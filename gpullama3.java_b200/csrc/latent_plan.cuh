@@ -446,7 +446,7 @@ static int ly_enqueue_parallel(b200_plan *p, bool decode, int n, const StepState
             }
         } else if ((rc = bnorm(false, nullptr, nullptr, nullptr, nullptr))) return rc;
         if ((rc = launch_k(p, p->use_pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
-                           p->out_ids, with_head ? 1 : 0, (const float *)nullptr, (const int *)nullptr, 0, TraceBuf{nullptr, 0, 0}, p->tp, -1))) return rc;
+                           p->out_ids, with_head ? 1 : 0, (const float *)nullptr, (const int *)nullptr, 0, TraceBuf{nullptr, 0, 0}, p->tp, -1, id_behind_logits(p)))) return rc;
         nl++;
     } else if ((rc = bnorm(false, nullptr, nullptr, nullptr, nullptr))) return rc;
     if (launches) *launches = nl;

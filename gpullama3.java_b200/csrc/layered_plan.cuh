@@ -128,7 +128,7 @@ struct Layered {
     bool f32 = false, has_loop = false;
     float *X = nullptr, *X0 = nullptr, *Y = nullptr, *PROJ = nullptr, *A32 = nullptr, *ATT32 = nullptr, *H32 = nullptr, *LOG = nullptr;
     ly::bf16 *A16 = nullptr, *ATT16 = nullptr, *H16 = nullptr;
-    int *tok = nullptr, *rows = nullptr;
+    int *tok = nullptr, *rows = nullptr, *h_rows = nullptr; // (h_rows: pinned)
     StepState *st_pf = nullptr;
     float *trace = nullptr; // [runs][cap][width], allocated on first use
     int smem_max = 0;
@@ -261,6 +261,7 @@ static void ly_free(b200_plan *p) {
         if (p->ly->ev_fork) cudaEventDestroy(p->ly->ev_fork);
         if (p->ly->ev_join) cudaEventDestroy(p->ly->ev_join);
         if (p->ly->branch) cudaStreamDestroy(p->ly->branch);
+        if (p->ly->h_rows) cudaFreeHost(p->ly->h_rows);
     }
     delete p->ly;
     p->ly = nullptr;
@@ -575,7 +576,7 @@ static int ly_enqueue(b200_plan *p, bool decode, int n, const StepState *st, con
             nl++;
         } else if ((rc = norm(false, false, nullptr, nullptr))) return rc;
         if ((rc = launch_k(p, p->use_pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, Y.c.vocab_size, p->st, (const int *)p->seq_tokens,
-                           p->out_ids, with_head ? 1 : 0, (const float *)nullptr, (const int *)nullptr, 0, TraceBuf{nullptr, 0, 0}, p->tp, -1))) return rc;
+                           p->out_ids, with_head ? 1 : 0, (const float *)nullptr, (const int *)nullptr, 0, TraceBuf{nullptr, 0, 0}, p->tp, -1, id_behind_logits(p)))) return rc;
         nl++;
     } else if ((rc = norm(false, false, nullptr, nullptr))) return rc;
     if (launches) *launches = nl;
@@ -1175,6 +1176,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
     if ((rc = dalloc(p, &Y.LOG, (size_t)(Y.f32 ? Y.logit_rows : 256) * c.vocab_size * 4))) return rc;
     if ((rc = dalloc(p, &Y.tok, cap * 4))) return rc;
     if ((rc = dalloc(p, &Y.rows, cap * 4))) return rc;
+    CK(cudaMallocHost(&Y.h_rows, cap * 4));
     {
         const char *e = getenv("B200_LAYERED_SPLITS");
         if (e && atoi(e) >= 1) Y.max_splits = atoi(e) > 8 ? 8 : atoi(e);
@@ -1191,8 +1193,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
     if ((rc = dalloc(p, &Y.st_pf, sizeof(StepState)))) return rc;
     CK(cudaMemset(Y.st_pf, 0, sizeof(StepState)));
     // what the shared single-token entry points use
-    if ((rc = dalloc(p, &p->logits, (size_t)sampler_padded(c.vocab_size) * 4))) return rc;
-    CK(cudaMemset(p->logits, 0, (size_t)sampler_padded(c.vocab_size) * 4));
+    if ((rc = logits_alloc(p, c.vocab_size))) return rc;
     if ((rc = dalloc(p, &p->smp_indices, (size_t)c.vocab_size * 4))) return rc;
     if ((rc = dalloc(p, &p->smp_out, 8 * 4))) return rc;
     p->seq_cap = (c.context_length > Y.cap ? c.context_length : Y.cap) + 8;
@@ -1239,12 +1240,11 @@ static int ly_batch(b200_plan *p, const int32_t *tokens, int n, int start_pos, c
     p->use_pdl = false;
     if (rc) return rc;
     CK(cudaEventRecord(p->ev1, p->stream));
-    CK(cudaStreamSynchronize(p->stream)); // h_ids / h_st are reused below
-    CK(cudaEventElapsedTime(&p->prefill_ms, p->ev0, p->ev1));
+    if (n_rows == 0) CK(cudaStreamSynchronize(p->stream)); // (else behind the rows' logits: a wait here left the GPU idle for 17 us)
     for (int r0 = 0; r0 < n_rows; r0 += Y.logit_rows) {
         const int m = n_rows - r0 < Y.logit_rows ? n_rows - r0 : Y.logit_rows;
-        memcpy(p->h_ids, rows + r0, (size_t)m * 4);
-        CK(cudaMemcpyAsync(Y.rows, p->h_ids, (size_t)m * 4, cudaMemcpyHostToDevice, p->stream));
+        memcpy(Y.h_rows, rows + r0, (size_t)m * 4); // (not h_ids: the chunk's tokens may still be on their way)
+        CK(cudaMemcpyAsync(Y.rows, Y.h_rows, (size_t)m * 4, cudaMemcpyHostToDevice, p->stream));
         if (Y.outnorm) {
             ly::OutNormArgs a = ly_outnorm_args(Y, m);
             a.w_out = Y.final_norm; a.gather = Y.rows; a.st = Y.st_pf;
@@ -1269,6 +1269,7 @@ static int ly_batch(b200_plan *p, const int32_t *tokens, int n, int start_pos, c
         CK(cudaMemcpyAsync(logits_out + (size_t)r0 * V, Y.LOG, (size_t)m * V * 4, cudaMemcpyDeviceToHost, p->stream));
         CK(cudaStreamSynchronize(p->stream));
     }
+    CK(cudaEventElapsedTime(&p->prefill_ms, p->ev0, p->ev1));
     if (trace_out)
         for (size_t r = 0; r < Y.runs.size(); r++)
             CK(cudaMemcpy(trace_out + r * (size_t)n * E, Y.trace + r * (size_t)Y.cap * E, (size_t)n * E * 4, cudaMemcpyDeviceToHost));

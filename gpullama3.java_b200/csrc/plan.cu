@@ -98,6 +98,8 @@ struct b200_plan {
     int seq_cap = 0;
     StepState *h_st = nullptr; // pinned
     int *h_ids = nullptr;      // pinned, seq_cap
+    float *h_logits = nullptr; // pinned copy of the logits, their pad and the greedy token (logits_alloc)
+    size_t logits_words = 0;
 
     cudaGraphExec_t g_decode = nullptr, g_prefill = nullptr, g_trace = nullptr; // the multi-kernel decode graph
     cudaGraphExec_t g_decode_deep = nullptr, g_prefill_deep = nullptr, g_trace_deep = nullptr; // the same with clusters in the attention: positions from ATT_SPLIT on (null: not for this plan)
@@ -660,6 +662,19 @@ size_t att_smem_bytes(int head_size, int ctx, bool scratch, int cluster = 1) {
 
 int att_row_stride(int ctx) { return (ctx + PD_CT - 1) / PD_CT * PD_CT; } // score rows in global memory: whole accumulator chunks
 
+// The logits, the sampler's pad (zeros: its exact sum runs over whole thread chunks) and one word more: the greedy token of a step, so that ONE copy, to pinned memory,
+// brings the host both (two copies, the second one to pageable memory, cost a step 6 us more: each waits for the one in front and is set up by itself).
+int logits_alloc(b200_plan *p, int vocab) {
+    const size_t words = (size_t)sampler_padded(vocab) + 1;
+    int rc;
+    if ((rc = dalloc(p, &p->logits, words * 4))) return rc;
+    CK(cudaMemset(p->logits, 0, words * 4));
+    CK(cudaMallocHost(&p->h_logits, words * 4));
+    p->logits_words = words;
+    return B200_OK;
+}
+int *id_behind_logits(const b200_plan *p) { return reinterpret_cast<int *>(p->logits + p->logits_words - 1); }
+
 // Enqueue one single-token forward on p->stream (captured into a CUDA graph at creation).
 // with_logits=false is the prefill variant (InferenceCoreBatchPrefillDecode.java:166-167).
 int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = false, bool deep = false) {
@@ -763,7 +778,7 @@ int enqueue_forward(b200_plan *p, bool with_logits, int *launches, bool trace = 
         int rc;
         if ((rc = launch_k(p, pdl, k_argmax_advance, dim3(1), dim3(1024), (size_t)0, (const float *)p->logits, c.vocab_size, p->st, (const int *)p->seq_tokens, p->out_ids, with_logits ? 1 : 0,
                            (const float *)(st || sf ? p->part_val : nullptr), (const int *)(st || sf ? p->part_idx : nullptr),
-                           sf ? sf_grid(p, c.vocab_size, c.dim, false, p->sf_norm) : p->n_sms, TR(9), p->tp, with_logits ? -1 : last_x_op))) return rc;
+                           sf ? sf_grid(p, c.vocab_size, c.dim, false, p->sf_norm) : p->n_sms, TR(9), p->tp, with_logits ? -1 : last_x_op, id_behind_logits(p)))) return rc;
         n++;
     }
     if (launches) *launches = n;
@@ -1177,7 +1192,7 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
     if ((rc = dalloc(p, &p->qkv, (size_t)(p->qd_l + 2 * p->kvd_l) * 4))) return rc;
     if ((rc = dalloc(p, &p->hb, (size_t)c.hidden_dim * 4))) return rc;
     if ((rc = dalloc(p, &p->hb2, (size_t)c.hidden_dim * 4))) return rc;
-    if ((rc = dalloc(p, &p->logits, (size_t)sampler_padded(c.vocab_size) * 4))) return rc; // zero pad: the sampler's exact sum runs over whole thread chunks
+    if ((rc = logits_alloc(p, c.vocab_size))) return rc;
     if ((rc = dalloc(p, &p->xq, (size_t)big))) return rc;
     if ((rc = dalloc(p, &p->xs, (size_t)(big / 32) * 4))) return rc;
     if (c.tp_size > 1) {
@@ -1196,7 +1211,6 @@ int build(b200_plan *p, const b200_tensor *tensors, int n_tensors) {
     if ((rc = dalloc(p, &p->value_cache, kv_bytes))) return rc;
     CK(cudaMemset(p->key_cache, 0, kv_bytes));
     CK(cudaMemset(p->value_cache, 0, kv_bytes));
-    CK(cudaMemset(p->logits, 0, (size_t)sampler_padded(c.vocab_size) * 4));
     if ((rc = dalloc(p, &p->smp_indices, (size_t)c.vocab_size * 4))) return rc;
     if ((rc = dalloc(p, &p->smp_out, 8 * 4))) return rc;
     p->seq_cap = c.context_length + 8;
@@ -1709,11 +1723,13 @@ int b200_forward_decode(b200_plan *p, int32_t token, int32_t position, float *lo
     CK(cudaSetDevice(p->device));
     if ((rc = set_state(p, token, position, 0, 0))) return rc;
     CK(cudaGraphLaunch(decode_graph(p, position), p->stream));
-    if (argmax) CK(cudaMemcpyAsync(p->h_ids, p->out_ids, 4, cudaMemcpyDeviceToHost, p->stream));
-    if (logits) CK(cudaMemcpyAsync(logits, p->logits, (size_t)p->cfg.vocab_size * 4, cudaMemcpyDeviceToHost, p->stream));
+    const bool id_apart = !logits || (p->decode_mode == B200_DECODE_PERSISTENT && p->g_pdecode); // (the persistent kernel leaves its token in out_ids only)
+    if (argmax && id_apart) CK(cudaMemcpyAsync(p->h_ids, p->out_ids, 4, cudaMemcpyDeviceToHost, p->stream));
+    if (logits) CK(cudaMemcpyAsync(p->h_logits, p->logits, p->logits_words * 4, cudaMemcpyDeviceToHost, p->stream));
     CK(cudaStreamSynchronize(p->stream));
     if ((rc = check_device_error(p))) return rc;
-    if (argmax) *argmax = p->h_ids[0];
+    if (logits) memcpy(logits, p->h_logits, (size_t)p->cfg.vocab_size * 4);
+    if (argmax) *argmax = id_apart ? p->h_ids[0] : reinterpret_cast<const int *>(p->h_logits)[p->logits_words - 1];
     return B200_OK;
 }
 
@@ -2230,6 +2246,7 @@ void b200_plan_free(b200_plan *p) {
     for (void *d : p->allocs) cudaFree(d);
     if (p->h_st) cudaFreeHost(p->h_st);
     if (p->h_ids) cudaFreeHost(p->h_ids);
+    if (p->h_logits) cudaFreeHost(p->h_logits);
     if (p->ev0) cudaEventDestroy(p->ev0);
     if (p->ev1) cudaEventDestroy(p->ev1);
     if (p->stream) cudaStreamDestroy(p->stream);
