@@ -1083,7 +1083,8 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool vali
 // general kernel above loads four keys per lane, reduces, looks up a distance row, caps, and only then asks for the next keys, and its parts meet in global memory
 // behind a counter.  Here a CTA asks for the first four tiles of its keys at once (cp.async, 16 KB each: all keys of a window of 1024 split four
 // ways), looks the distances up meanwhile, asks for the first tiles of its values before the softmax, and the parts are merged over distributed shared
-// memory, every CTA finishing its share of the head's entries.  32 heads of 64, 900 keys, cap and distance table: 27 us there, 20 us here.
+// memory, every CTA finishing its share of the head's entries.  Lanes that share a row take four of them at a time (U; one where a stage holds no more than a row per
+// group).  32 heads of 64, 900 keys, cap and distance table: 27 us there, 17 us with one row at a time, 13 us with four; 32 heads of 128, 2000 keys: 56 and 38 us.
 // grid (splits, heads), cluster (splits), LY_ATT_THREADS threads; dynamic shared memory step_att_smem_floats(...) floats.
 // ---------------------------------------------------------------------------------------------------------------------
 #define LY_STEP_STAGES 4
@@ -1104,6 +1105,7 @@ __device__ __forceinline__ float ld_cluster_f32(const float *p, int rank) { // t
 }
 __device__ __forceinline__ void cluster_barrier() { asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory"); }
 
+template <int U> // rows of a lane group at a time
 __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *__restrict__ P, WindowAttn a, const float *__restrict__ kc, const float *__restrict__ vc,
                                                                    const StepState *__restrict__ st, float *__restrict__ out) {
     extern __shared__ __align__(16) float sm[];
@@ -1157,23 +1159,36 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *
         __syncthreads();
         const float *kt = ring + (i % LY_STEP_STAGES) * LY_STEP_STAGE_FLOATS;
         const int n = nk - i * kper < kper ? nk - i * kper : kper, sub = lane & (klpr - 1), rows = 32 / klpr;
-        for (int r0 = warp * rows; r0 < n; r0 += (LY_ATT_THREADS / 32) * rows) {
-            const int r = r0 + lane / klpr;
-            float d = 0.0f;
-            if (r < n)
-                for (int c = sub * 4; c < a.dk; c += klpr * 4) {
-                    const float4 kv = *reinterpret_cast<const float4 *>(kt + r * a.dk + c), qv = *reinterpret_cast<const float4 *>(qs + c);
-                    d = fmaf(qv.x, kv.x, d); d = fmaf(qv.y, kv.y, d); d = fmaf(qv.z, kv.z, d); d = fmaf(qv.w, kv.w, d);
-                }
-            for (int o = klpr >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            if (r < n && sub == 0) {
-                const int j = i * kper + r;
-                float e = d * a.scale;
-                if (a.softcap > 0.0f) e = a.softcap * tanhf(e / a.softcap);
-                if (a.rel) e += sc[j];
-                sc[j] = e;
-                mx = fmaxf(mx, e);
+        const int hop = (LY_ATT_THREADS / 32) * rows;
+        for (int w0 = warp * rows; w0 < n; w0 += U * hop) { // (their chains of products, shuffles and cap run side by side)
+            const int r0 = w0 + lane / klpr;
+            float d[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) d[u] = 0.0f;
+            for (int c = sub * 4; c < a.dk; c += klpr * 4) {
+                const float4 qv = *reinterpret_cast<const float4 *>(qs + c);
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (r0 + u * hop < n) {
+                        const float4 kv = *reinterpret_cast<const float4 *>(kt + (r0 + u * hop) * a.dk + c);
+                        d[u] = fmaf(qv.x, kv.x, d[u]); d[u] = fmaf(qv.y, kv.y, d[u]); d[u] = fmaf(qv.z, kv.z, d[u]); d[u] = fmaf(qv.w, kv.w, d[u]);
+                    }
             }
+            for (int o = klpr >> 1; o > 0; o >>= 1)
+#pragma unroll
+                for (int u = 0; u < U; u++) d[u] += __shfl_xor_sync(0xffffffffu, d[u], o);
+            for (int u = sub; u < U; u += klpr) // the group's lanes finish a row each
+                if (r0 + u * hop < n) {
+                    const int j = i * kper + r0 + u * hop;
+                    float e = d[0];
+#pragma unroll
+                    for (int k = 1; k < U; k++) e = u == k ? d[k] : e;
+                    e *= a.scale;
+                    if (a.softcap > 0.0f) e = a.softcap * tanhf(e / a.softcap);
+                    if (a.rel) e += sc[j];
+                    sc[j] = e;
+                    mx = fmaxf(mx, e);
+                }
         }
         if (i + LY_STEP_STAGES < ktiles) { // (uniform) refill the stage when every warp is done with it
             __syncthreads();
