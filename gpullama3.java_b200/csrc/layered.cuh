@@ -439,6 +439,81 @@ __global__ void __launch_bounds__(LY_MV_THREADS) k_matvec_bf16(const bf16 *__res
     }
 }
 
+// The same as a stream: a CTA loads the activation once and its warps walk many rows, eight 128-bit loads of a lane (2048 columns) in flight while the eight before them
+// are multiplied; the activation lies in shared memory as two rows of float4 so that neighbouring lanes read neighbouring 16 bytes.  What bounds it is HBM; the kernel
+// above starts thousands of CTAs that each wait for the activation, then for four loads at a time, and adds in one chain.
+// K a multiple of 8, W / x and their offsets of 16 bytes.  Dynamic shared memory: K floats.
+template <int EPI>
+__global__ void __launch_bounds__(LY_MV_THREADS, 2) k_matvec_stream_bf16(const bf16 *__restrict__ W, const float *__restrict__ bias, const float *__restrict__ x,
+                                                                        float *__restrict__ y, int N, int K, int act, MvView v_) {
+    extern __shared__ __align__(16) float xs[];
+    constexpr int R = EPI == EPI_GATED ? 2 : 1, LOADS = 8, SEG = LOADS * 256;
+    const int b = blockIdx.y;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (v_.group && v_.n_groups > 0 && v_.group[b] >= v_.n_groups) return;
+    W += (size_t)b * v_.w_bs + (v_.group ? (size_t)v_.group[b] * v_.w_gs : (size_t)0);
+    x += (size_t)b * v_.x_bs;
+    y += (size_t)b * v_.y_bs;
+    const int lane = threadIdx.x & 31, nw = gridDim.x * (LY_MV_THREADS / 32), n0 = blockIdx.x * (LY_MV_THREADS / 32) + (threadIdx.x >> 5);
+    const int segs = (K + SEG - 1) / SEG, per_item = R * segs, units = n0 < N ? ((N - 1 - n0) / nw + 1) * per_item : 0; // a unit: one segment of one row
+    int l_n = n0, l_r = 0, l_s = 0; // the next unit to load
+    auto load = [&](int4 (&q)[LOADS]) {
+        const bf16 *w = W + (size_t)(l_n + l_r * N) * K + l_s * SEG + lane * 8;
+        const int left = K - l_s * SEG - lane * 8;
+#pragma unroll
+        for (int u = 0; u < LOADS; u++) q[u] = u * 256 < left ? ldg128_stream(w + u * 256) : make_int4(0, 0, 0, 0);
+        if (++l_s == segs) { l_s = 0; if (++l_r == R) { l_r = 0; l_n += nw; } }
+    };
+    int4 q0[LOADS], q1[LOADS];
+    if (units > 0) load(q0);
+    float4 *x0 = reinterpret_cast<float4 *>(xs), *x1 = x0 + K / 8;
+    for (int i = threadIdx.x; i < K / 8; i += LY_MV_THREADS) {
+        x0[i] = *reinterpret_cast<const float4 *>(x + 8 * i);
+        x1[i] = *reinterpret_cast<const float4 *>(x + 8 * i + 4);
+    }
+    const float sc = v_.in_scale ? v_.in_scale[b] : 1.0f;
+    __syncthreads();
+    int n = n0, r = 0, sg = 0;
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, first = 0.0f;
+    auto multiply = [&](const int4 (&q)[LOADS]) {
+#pragma unroll
+        for (int u = 0; u < LOADS; u++) {
+            const int c = sg * (SEG / 8) + u * 32 + lane;
+            if (sg * SEG + u * 256 >= K) break; // (uniform)
+            const float4 a0 = x0[c < K / 8 ? c : 0], a1 = x1[c < K / 8 ? c : 0]; // (behind the row the weights are zero)
+            acc[0] = fmaf(bf_lo((unsigned)q[u].x), a0.x, acc[0]); acc[1] = fmaf(bf_hi((unsigned)q[u].x), a0.y, acc[1]);
+            acc[2] = fmaf(bf_lo((unsigned)q[u].y), a0.z, acc[2]); acc[3] = fmaf(bf_hi((unsigned)q[u].y), a0.w, acc[3]);
+            acc[0] = fmaf(bf_lo((unsigned)q[u].z), a1.x, acc[0]); acc[1] = fmaf(bf_hi((unsigned)q[u].z), a1.y, acc[1]);
+            acc[2] = fmaf(bf_lo((unsigned)q[u].w), a1.z, acc[2]); acc[3] = fmaf(bf_hi((unsigned)q[u].w), a1.w, acc[3]);
+        }
+        if (++sg < segs) return;
+        sg = 0;
+        float v = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
+        acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
+        if (R == 2 && r == 0) { first = v; r = 1; return; }
+        r = 0;
+        if (EPI == EPI_GATED) v = act_apply(act, first * sc) * (v * sc);
+        else if (EPI == EPI_ACT) {
+            if (bias) v += bias[n];
+            v = act_apply(act, v);
+            if (v_.tg.table) v *= token_gate(v_.tg, 0, n);
+        } else {
+            if (bias) v += bias[n];
+            if (v_.mul) v *= 1.0f / (1.0f + expf(-v_.mul[(size_t)b * v_.y_bs + n]));
+        }
+        if (lane == 0) y[n] = v;
+        n += nw;
+    };
+    for (int u = 0; u < units; u += 2) {
+        if (u + 1 < units) load(q1);
+        multiply(q0);
+        if (u + 1 >= units) break;
+        if (u + 2 < units) load(q0);
+        multiply(q1);
+    }
+}
+
 // The same for matrices of FEW rows (a router, the step / state parameters of a scan, a narrow gate): a CTA per row, so that the reduction width is
 // spread over all its warps instead of one.  grid (N), LY_MV_THREADS threads; plain and EPI_ACT results.
 template <int EPI>

@@ -327,6 +327,20 @@ static ly::WindowAttn ly_attn_args(const Layered &Y, const LyLayer &L) {
 // A decode projection with a warp per row would occupy less than half of the SMs and every warp walk a long row: a CTA per row then.
 static bool ly_few_rows(const b200_plan *p, int N, int K) { return (N + LY_MV_THREADS / 32 - 1) / (LY_MV_THREADS / 32) * 2 < p->n_sms && K >= 1024; }
 
+// A decode projection: the streaming kernel where its loads are aligned and rows are long enough for them, two CTAs an SM; else a warp per row.  Warp per row ->
+// stream, us: 2048 x 8192 12.2 -> 9.3, 2048 x 2048 5.1 -> 4.0, 4096 x 14336 25.8 -> 23.8, 32768 x 2048 28.0 -> 26.5, gated pairs 14336 x 4096 44.1 -> 42.0.  Gated pairs of
+// shorter rows stay: their few rows a warp spread unevenly over the stream's warps (8192 x 2048 13.6 -> 15.2, 4096 x 1024 6.2 -> 6.8).
+template <int EPI>
+static int ly_matvec(b200_plan *p, const ly::bf16 *W, const float *bias, const float *x, float *y, int N, int K, int act, const ly::MvView &v, int yb) {
+    const int warps = LY_MV_THREADS / 32, ctas = (N + warps - 1) / warps;
+    auto whole = [](const void *q) { return ((uintptr_t)q & 15) == 0; };
+    if (K >= (EPI == ly::EPI_GATED ? 4096 : 1024) && K % 8 == 0 && whole(W) && whole(x) && v.w_bs % 8 == 0 && v.w_gs % 8 == 0 && v.x_bs % 4 == 0 && (size_t)K * 4 <= (size_t)100 * 1024) {
+        const int most = (2 * p->n_sms + yb - 1) / yb;
+        return launch_k(p, p->use_pdl, ly::k_matvec_stream_bf16<EPI>, dim3(ctas < most ? ctas : most, yb), dim3(LY_MV_THREADS), (size_t)K * 4, W, bias, x, y, N, K, act, v);
+    }
+    return launch_k(p, p->use_pdl, ly::k_matvec_bf16<EPI>, dim3(ctas, yb), dim3(LY_MV_THREADS), (size_t)K * 4, W, bias, x, y, N, K, act, v);
+}
+
 // C[n][N] = A[n][K] W^T with the epilogue EPI; decode (n == 1 through the graph) streams the rows, prefill takes a GEMM:
 // the persistent CTA-pair tcgen05 kernel (256-wide tiles) or the single-CTA one (128-wide) of prefill_gemm.cuh when the
 // shape fits and the plan computes in BF16, else the any-shape kernels of layered.cuh.
@@ -335,11 +349,9 @@ static int ly_project(b200_plan *p, bool decode, int n, const float *a32, const 
                       float *c32, ly::bf16 *c16, int ldc, int act, const LyTc *tc = nullptr) {
     Layered &Y = *p->ly;
     if (decode) {
-        const int warps = LY_MV_THREADS / 32;
-        int grid = (N + warps - 1) / warps;
         if (EPI != ly::EPI_GATED && !bias && ly_few_rows(p, N, K))
             return launch_k(p, p->use_pdl, ly::k_matvec_row_bf16<EPI == ly::EPI_GATED ? ly::EPI_STORE : EPI>, dim3(N), dim3(LY_MV_THREADS), (size_t)0, W, a32, c32, K, act, ly::TokenGate{});
-        return launch_k(p, p->use_pdl, ly::k_matvec_bf16<EPI>, dim3(grid), dim3(LY_MV_THREADS), (size_t)K * 4, W, bias, a32, c32, N, K, act, ly::MvView{});
+        return ly_matvec<EPI>(p, W, bias, a32, c32, N, K, act, ly::MvView{}, 1);
     }
     if (tc && tc->a && !Y.f32) {
         const int mt2 = (n + 255) / 256 * 2;
@@ -814,7 +826,9 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
             CK(set_max_dyn(ly::k_moe_route<float>, Y.smem_max));
             CK(set_max_dyn(ly::k_moe_route<ly::bf16>, Y.smem_max));
             CK(set_max_dyn(ly::k_matvec_bf16<ly::EPI_STORE>, Y.smem_max));
+            CK(set_max_dyn(ly::k_matvec_stream_bf16<ly::EPI_STORE>, Y.smem_max));
             CK(set_max_dyn(ly::k_matvec_bf16<ly::EPI_GATED>, Y.smem_max));
+            CK(set_max_dyn(ly::k_matvec_stream_bf16<ly::EPI_GATED>, Y.smem_max));
             CK(set_max_dyn(ly::k_window_attention<float>, Y.smem_max));
             CK(set_max_dyn(ly::k_step_attention<1>, Y.smem_max));
             CK(set_max_dyn(ly::k_step_attention<4>, Y.smem_max));
@@ -850,6 +864,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
             CK(set_max_dyn(ly::k_outnorm_rows<1024>, Y.smem_max));
             CK(set_max_dyn(ly::k_gated_group_norm, Y.smem_max));
             CK(set_max_dyn(ly::k_matvec_bf16<ly::EPI_ACT>, Y.smem_max));
+            CK(set_max_dyn(ly::k_matvec_stream_bf16<ly::EPI_ACT>, Y.smem_max));
             attrs = true;
         }
     }
