@@ -9,6 +9,7 @@
 //   * k_norm_rows_reg   the same with the row in registers, for the shapes and steps that allow it;
 //   * k_matvec_bf16     decode projection: BF16 weight rows streamed with 128-bit loads, FP32 activation and accumulator,
 //                       bias or gated-activation epilogue (gelu_tanh(g) * u);
+//   * k_matvec_stream_bf16  the same for rows of 1024 columns and more: two CTAs an SM, loads ahead of the products;
 //   * k_matvec_row_bf16 the same for matrices of few rows: a CTA per row;
 //   * k_gemm_f32 / k_gemm_bf16   prefill projections for any M, N, K: true FP32 on the CUDA cores, or BF16 operands on the
 //                       tensor cores (mma.sync m16n8k16, FP32 accumulation), same epilogues;
