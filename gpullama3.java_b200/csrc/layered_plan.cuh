@@ -278,9 +278,16 @@ static size_t ly_att_smem(const b200_layer_spec &s, int ring) {
 static int ly_mma_kind(int dk, int dv) {
     return dk == 64 && dv == 64 ? 1 : dk == 128 && dv == 128 ? 2 : dk == 192 && dv == 128 ? 3 : dk == 128 && dv == 64 ? 4 : dk == 256 && dv == 128 ? 5 : dk == 64 && dv == 32 ? 6 : 0;
 }
-static size_t ly_mma_smem(int kind, int window, int rows = LY_ATT_MMA_ROWS) {
+static size_t ly_mma_smem(int kind, int window, int rows) {
     return kind == 1 ? ly::att_mma_smem_bytes<64, 64>(rows, window) : kind == 2 ? ly::att_mma_smem_bytes<128, 128>(rows, window) : kind == 3 ? ly::att_mma_smem_bytes<192, 128>(rows, window)
          : kind == 4 ? ly::att_mma_smem_bytes<128, 64>(rows, window) : kind == 5 ? ly::att_mma_smem_bytes<256, 128>(rows, window) : ly::att_mma_smem_bytes<64, 32>(rows, window);
+}
+// Does a layer attend on the tensor cores, that is with BF16 queries, keys and values?  Up to the window whose distances fit shared memory beside 128 queries and two stages
+// of keys and values, 32000 positions at key and value size 128.  The kernel itself needs less (its queries make room for the second stage), but a layer with
+// a wider window has its scores and sums in FP32, in the general kernel, and a smaller footprint is no reason to round its operands.
+static bool ly_mma_fits(const Layered &Y, int dk, int dv, int window) {
+    const size_t tiles = (size_t)((LY_ATT_MMA_ROWS + 128) * (dk + 8) + 128 * (dv + 8)) * 2;
+    return ly_mma_kind(dk, dv) && tiles + (size_t)window * 4 <= (size_t)Y.smem_max;
 }
 static int ly_launch_mma(b200_plan *p, int kind, int n, int heads, int window, const float *P, int ldp, const ly::WindowAttn &wa, const ly::bf16 *k16, const ly::bf16 *v16,
                          const StepState *st, ly::bf16 *out, int ldo, float *out32 = nullptr) {
@@ -874,8 +881,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
         for (LyLayer &L : Y.layers) {
             if (L.s.mixer != B200_MIXER_LATENT_ATTENTION) continue;
             const int DK = L.s.key_dim + L.s.rot_dim;
-            const int kind = ly_mma_kind(DK, L.s.value_dim);
-            L.expand = kind && ly_mma_smem(kind, L.s.window) <= (size_t)Y.smem_max && (L.s.gate != 1 || L.g_off % 2 == 0) && L.s.key_dim % 8 == 0;
+            L.expand = ly_mma_fits(Y, DK, L.s.value_dim, L.s.window) && (L.s.gate != 1 || L.g_off % 2 == 0) && L.s.key_dim % 8 == 0;
             if (L.expand) {
                 if (L.s.heads * DK > Y.maxKX) Y.maxKX = L.s.heads * DK;
                 if (L.gd > Y.maxVX) Y.maxVX = L.gd;
@@ -1081,9 +1087,8 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
         if ((rc = dalloc(p, &R.vc, (size_t)Y.ring * L.vd * 4))) return rc;
         CK(cudaMemset(R.kc, 0, (size_t)Y.ring * L.kd * 4));
         CK(cudaMemset(R.vc, 0, (size_t)Y.ring * L.vd * 4));
-        // tensor-core prefill attention: BF16 plans, key = value size 64 or 128, a window whose tiles fit shared memory
-        const int kind = ly_mma_kind(L.mixprep ? L.dk_eff : L.s.key_dim, L.s.value_dim);
-        if (!Y.f32 && Y.att_mma && Y.cap > 1 && kind && ly_mma_smem(kind, L.s.window) <= (size_t)Y.smem_max && Y.maxP % 4 == 0 && L.gd % 2 == 0) {
+        // tensor-core prefill attention: BF16 plans, key and value sizes of an instance, a window up to the limit
+        if (!Y.f32 && Y.att_mma && Y.cap > 1 && ly_mma_fits(Y, L.mixprep ? L.dk_eff : L.s.key_dim, L.s.value_dim, L.s.window) && Y.maxP % 4 == 0 && L.gd % 2 == 0) {
             if ((rc = dalloc(p, &R.kc16, (size_t)Y.ring * L.kd * 2))) return rc;
             if ((rc = dalloc(p, &R.vc16, (size_t)Y.ring * L.vd * 2))) return rc;
             CK(cudaMemset(R.kc16, 0, (size_t)Y.ring * L.kd * 2));

@@ -243,8 +243,7 @@ static int ly_outnorm_run(b200_plan *p, LyRun &R, const LyLayer &L) {
         if ((rc = dalloc(p, &R.kc, (size_t)Y.ring * L.kd * 4)) || (rc = dalloc(p, &R.vc, (size_t)Y.ring * L.vd * 4))) return rc;
         CK(cudaMemset(R.kc, 0, (size_t)Y.ring * L.kd * 4));
         CK(cudaMemset(R.vc, 0, (size_t)Y.ring * L.vd * 4));
-        const int kind = ly_mma_kind(s.key_dim, s.value_dim);
-        if (!Y.f32 && Y.att_mma && Y.cap > 1 && kind && ly_mma_smem(kind, s.window) <= (size_t)Y.smem_max && Y.maxP % 4 == 0) {
+        if (!Y.f32 && Y.att_mma && Y.cap > 1 && ly_mma_fits(Y, s.key_dim, s.value_dim, s.window) && Y.maxP % 4 == 0) {
             if ((rc = dalloc(p, &R.kc16, (size_t)Y.ring * L.kd * 2)) || (rc = dalloc(p, &R.vc16, (size_t)Y.ring * L.vd * 2))) return rc;
             CK(cudaMemset(R.kc16, 0, (size_t)Y.ring * L.kd * 2));
             CK(cudaMemset(R.vc16, 0, (size_t)Y.ring * L.vd * 2));
