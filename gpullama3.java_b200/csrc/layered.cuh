@@ -443,7 +443,9 @@ __global__ void __launch_bounds__(LY_MV_THREADS) k_matvec_bf16(const bf16 *__res
 // The same as a stream: a CTA loads the activation once and its warps walk many rows, eight 128-bit loads of a lane (2048 columns) in flight while the eight before them
 // are multiplied; the activation lies in shared memory as two rows of float4 so that neighbouring lanes read neighbouring 16 bytes.  What bounds it is HBM; the kernel
 // above starts thousands of CTAs that each wait for the activation, then for four loads at a time, and adds in one chain.
-// K a multiple of 8, W / x and their offsets of 16 bytes.  Dynamic shared memory: K floats.
+// K a multiple of 8, W / x and their offsets of 16 bytes.  Dynamic shared memory: mv_stream_floats(K) floats: the activation is followed by zeros up to a warp's whole
+// load, so that a lane behind the row multiplies zero by zero and not by an entry, which may be infinite.
+__host__ __device__ constexpr int mv_stream_floats(int K) { return (K + 255) / 256 * 256; }
 template <int EPI>
 __global__ void __launch_bounds__(LY_MV_THREADS, 2) k_matvec_stream_bf16(const bf16 *__restrict__ W, const float *__restrict__ bias, const float *__restrict__ x,
                                                                         float *__restrict__ y, int N, int K, int act, MvView v_) {
@@ -468,10 +470,11 @@ __global__ void __launch_bounds__(LY_MV_THREADS, 2) k_matvec_stream_bf16(const b
     };
     int4 q0[LOADS], q1[LOADS];
     if (units > 0) load(q0);
-    float4 *x0 = reinterpret_cast<float4 *>(xs), *x1 = x0 + K / 8;
-    for (int i = threadIdx.x; i < K / 8; i += LY_MV_THREADS) {
-        x0[i] = *reinterpret_cast<const float4 *>(x + 8 * i);
-        x1[i] = *reinterpret_cast<const float4 *>(x + 8 * i + 4);
+    float4 *x0 = reinterpret_cast<float4 *>(xs), *x1 = x0 + mv_stream_floats(K) / 8;
+    for (int i = threadIdx.x; i < mv_stream_floats(K) / 8; i += LY_MV_THREADS) {
+        const bool in = i < K / 8;
+        x0[i] = in ? *reinterpret_cast<const float4 *>(x + 8 * i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        x1[i] = in ? *reinterpret_cast<const float4 *>(x + 8 * i + 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
     const float sc = v_.in_scale ? v_.in_scale[b] : 1.0f;
     __syncthreads();
@@ -482,7 +485,7 @@ __global__ void __launch_bounds__(LY_MV_THREADS, 2) k_matvec_stream_bf16(const b
         for (int u = 0; u < LOADS; u++) {
             const int c = sg * (SEG / 8) + u * 32 + lane;
             if (sg * SEG + u * 256 >= K) break; // (uniform)
-            const float4 a0 = x0[c < K / 8 ? c : 0], a1 = x1[c < K / 8 ? c : 0]; // (behind the row the weights are zero)
+            const float4 a0 = x0[c], a1 = x1[c];
             acc[0] = fmaf(bf_lo((unsigned)q[u].x), a0.x, acc[0]); acc[1] = fmaf(bf_hi((unsigned)q[u].x), a0.y, acc[1]);
             acc[2] = fmaf(bf_lo((unsigned)q[u].y), a0.z, acc[2]); acc[3] = fmaf(bf_hi((unsigned)q[u].y), a0.w, acc[3]);
             acc[0] = fmaf(bf_lo((unsigned)q[u].z), a1.x, acc[0]); acc[1] = fmaf(bf_hi((unsigned)q[u].z), a1.y, acc[1]);

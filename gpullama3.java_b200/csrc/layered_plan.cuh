@@ -341,9 +341,9 @@ template <int EPI>
 static int ly_matvec(b200_plan *p, const ly::bf16 *W, const float *bias, const float *x, float *y, int N, int K, int act, const ly::MvView &v, int yb) {
     const int warps = LY_MV_THREADS / 32, ctas = (N + warps - 1) / warps;
     auto whole = [](const void *q) { return ((uintptr_t)q & 15) == 0; };
-    if (K >= (EPI == ly::EPI_GATED ? 4096 : 1024) && K % 8 == 0 && whole(W) && whole(x) && v.w_bs % 8 == 0 && v.w_gs % 8 == 0 && v.x_bs % 4 == 0 && (size_t)K * 4 <= (size_t)100 * 1024) {
+    if (K >= (EPI == ly::EPI_GATED ? 4096 : 1024) && K % 8 == 0 && whole(W) && whole(x) && v.w_bs % 8 == 0 && v.w_gs % 8 == 0 && v.x_bs % 4 == 0 && K <= 25600) { // (two CTAs' activations of 100 KB an SM)
         const int most = (2 * p->n_sms + yb - 1) / yb;
-        return launch_k(p, p->use_pdl, ly::k_matvec_stream_bf16<EPI>, dim3(ctas < most ? ctas : most, yb), dim3(LY_MV_THREADS), (size_t)K * 4, W, bias, x, y, N, K, act, v);
+        return launch_k(p, p->use_pdl, ly::k_matvec_stream_bf16<EPI>, dim3(ctas < most ? ctas : most, yb), dim3(LY_MV_THREADS), (size_t)ly::mv_stream_floats(K) * 4, W, bias, x, y, N, K, act, v);
     }
     return launch_k(p, p->use_pdl, ly::k_matvec_bf16<EPI>, dim3(ctas, yb), dim3(LY_MV_THREADS), (size_t)K * 4, W, bias, x, y, N, K, act, v);
 }

@@ -23,3 +23,19 @@ def test_projections(pkg, width, ff, vocab):
         assert_rows(np.stack([plan.forward_decode(t, i)[0] for i, t in enumerate(toks)]), ref, TOL_DECODE)
     finally:
         plan.free()
+
+
+# An infinite first entry of the activation is infinite in every result and in no other way: lanes of a warp's last load that lie behind the row (1032, 2504 columns) take part in
+# no product.  1016 columns keep a warp per row, 1280 have no such lanes.
+@pytest.mark.parametrize("width", [1016, 1032, 1280, 2504])
+def test_infinite_activation(pkg, width):
+    S, vocab = pkg.synth, 2500
+    cfg = S.pibidra_config(width, vocab, [S.pibidra_layer(2, 1, 16, 24, 8, 64)])
+    w = S.pibidra_weights(cfg, width, bias_rows=8)
+    w["embed"][:, 0] = 50.0
+    w["final.norm"][0] = 3e38
+    w["head"][:, 0] = np.where(np.arange(vocab) % 3 == 0, -1.0, 1.0)
+    plan = make_plan(pkg, cfg, w, ctx=16, batch=1)
+    logits = plan.forward_decode(7, 0)[0]
+    plan.free()
+    assert np.array_equal(logits, np.where(np.arange(vocab) % 3 == 0, -np.inf, np.inf).astype(np.float32))
