@@ -128,7 +128,7 @@ struct Layered {
     bool f32 = false, has_loop = false;
     float *X = nullptr, *X0 = nullptr, *Y = nullptr, *PROJ = nullptr, *A32 = nullptr, *ATT32 = nullptr, *H32 = nullptr, *LOG = nullptr;
     ly::bf16 *A16 = nullptr, *ATT16 = nullptr, *H16 = nullptr;
-    int *tok = nullptr, *rows = nullptr, *h_rows = nullptr; // (h_rows: pinned)
+    int *tok = nullptr, *rows = nullptr, *h_rows = nullptr; // (h_rows: pinned, may be null)
     StepState *st_pf = nullptr;
     float *trace = nullptr; // [runs][cap][width], allocated on first use
     int smem_max = 0;
@@ -1198,7 +1198,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
     if ((rc = dalloc(p, &Y.LOG, (size_t)(Y.f32 ? Y.logit_rows : 256) * c.vocab_size * 4))) return rc;
     if ((rc = dalloc(p, &Y.tok, cap * 4))) return rc;
     if ((rc = dalloc(p, &Y.rows, cap * 4))) return rc;
-    CK(cudaMallocHost(&Y.h_rows, cap * 4));
+    if ((rc = pinned_optional(p, &Y.h_rows, cap * 4))) return rc;
     {
         const char *e = getenv("B200_LAYERED_SPLITS");
         if (e && atoi(e) >= 1) Y.max_splits = atoi(e) > 8 ? 8 : atoi(e);
@@ -1262,11 +1262,12 @@ static int ly_batch(b200_plan *p, const int32_t *tokens, int n, int start_pos, c
     p->use_pdl = false;
     if (rc) return rc;
     CK(cudaEventRecord(p->ev1, p->stream));
-    if (n_rows == 0) CK(cudaStreamSynchronize(p->stream)); // (else behind the rows' logits: a wait here left the GPU idle for 17 us)
+    int *const h_rows = Y.h_rows ? Y.h_rows : p->h_ids; // (not h_ids where that can be helped: the chunk's tokens may still be on their way)
+    if (n_rows == 0 || h_rows == p->h_ids) CK(cudaStreamSynchronize(p->stream)); // (else behind the rows' logits: a wait here left the GPU idle for 17 us)
     for (int r0 = 0; r0 < n_rows; r0 += Y.logit_rows) {
         const int m = n_rows - r0 < Y.logit_rows ? n_rows - r0 : Y.logit_rows;
-        memcpy(Y.h_rows, rows + r0, (size_t)m * 4); // (not h_ids: the chunk's tokens may still be on their way)
-        CK(cudaMemcpyAsync(Y.rows, Y.h_rows, (size_t)m * 4, cudaMemcpyHostToDevice, p->stream));
+        memcpy(h_rows, rows + r0, (size_t)m * 4);
+        CK(cudaMemcpyAsync(Y.rows, h_rows, (size_t)m * 4, cudaMemcpyHostToDevice, p->stream));
         if (Y.outnorm) {
             ly::OutNormArgs a = ly_outnorm_args(Y, m);
             a.w_out = Y.final_norm; a.gather = Y.rows; a.st = Y.st_pf;

@@ -98,7 +98,7 @@ struct b200_plan {
     int seq_cap = 0;
     StepState *h_st = nullptr; // pinned
     int *h_ids = nullptr;      // pinned, seq_cap
-    float *h_logits = nullptr; // pinned copy of the logits, their pad and the greedy token (logits_alloc)
+    float *h_logits = nullptr; // pinned copy of the logits, their pad and the greedy token (logits_alloc; may be null)
     size_t logits_words = 0;
 
     cudaGraphExec_t g_decode = nullptr, g_prefill = nullptr, g_trace = nullptr; // the multi-kernel decode graph
@@ -203,6 +203,22 @@ template <typename F> int alloc_optional(b200_plan *p, bool *done, F &&alloc) {
     for (; p->allocs.size() > n; p->allocs.pop_back()) cudaFree(p->allocs.back());
     p->bytes = bytes;
     p->err.clear();
+    cudaGetLastError(); // the failed allocation's
+    return B200_OK;
+}
+
+// What the tests of a plan's fallbacks refuse: B200_TEST_REFUSE holds the names of the optional steps of a plan's creation that fail as where the driver refuses them.
+bool refused(const char *step) {
+    const char *e = getenv("B200_TEST_REFUSE");
+    return e && strstr(e, step);
+}
+// Pinned host memory that only makes a plan faster: null where the system has none left.
+template <typename T> int pinned_optional(b200_plan *p, T **ptr, size_t n_bytes) {
+    *ptr = nullptr;
+    const cudaError_t e = refused("pinned") ? cudaErrorMemoryAllocation : cudaMallocHost((void **)ptr, n_bytes);
+    if (e == cudaSuccess) return B200_OK;
+    *ptr = nullptr;
+    if (e != cudaErrorMemoryAllocation) CK(e);
     cudaGetLastError(); // the failed allocation's
     return B200_OK;
 }
@@ -669,15 +685,15 @@ int logits_alloc(b200_plan *p, int vocab) {
     int rc;
     if ((rc = dalloc(p, &p->logits, words * 4))) return rc;
     CK(cudaMemset(p->logits, 0, words * 4));
-    CK(cudaMallocHost(&p->h_logits, words * 4));
     p->logits_words = words;
-    return B200_OK;
+    return pinned_optional(p, &p->h_logits, words * 4);
 }
 // A caller's pinned buffer takes a long row without the copy on the host: a second small copy for the token (3 us) against a host copy of the row.  Step of a toy model
 // into a pinned buffer, us, through h_logits / direct: 8192 entries 91.5 / 93.1, 24576 106.7 / 105.6, 32768 109.5 / 107.0, 128256 178 / 162.  (Pageable ones: 180 / 193 at
 // 128256, the driver copies through its own pinned memory.)  Asked while the step runs.
 #define LOGITS_DIRECT_MIN 24576
 bool logits_direct(const b200_plan *p, const float *logits) {
+    if (!p->h_logits) return true; // (a plan without pinned memory)
     if (p->cfg.vocab_size < LOGITS_DIRECT_MIN) return false;
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, logits) == cudaSuccess) return a.type == cudaMemoryTypeHost;
