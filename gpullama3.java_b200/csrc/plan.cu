@@ -140,6 +140,8 @@ struct b200_plan {
         struct Maps { XpMaps qkv, wo, gu, w2; }; // a layer's weights
         std::vector<Maps> maps;
         XpMaps mA[4], mATT[4], mH[4]; // activations in tiles of 8, 16, 32, 64 tokens: AQ with rows of dim and of the query width, HQ
+        int64_t chunks = 0;           // multiplied at once so far
+        std::string why;              // rows == 0: why not
     } xp;
     // persistent decode kernel
     bool pd_ok = false;           // the plan fits the kernel's restrictions
@@ -192,16 +194,17 @@ template <typename T> int dalloc(b200_plan *p, T **ptr, size_t n_bytes) {
     return B200_OK;
 }
 
-// Buffers that a plan can do without: `alloc` allocates them with dalloc.  Where the device has no room the ones already made are given back and the plan goes on
-// without any (*done = false); every other error is returned.
-template <typename F> int alloc_optional(b200_plan *p, bool *done, F &&alloc) {
+// Buffers that a plan can do without: `alloc` allocates them with dalloc.  Where the device has no room, or its driver does not support what they are for, the ones
+// already made are given back and the plan goes on without any (*done = false, the reason in *why); every other error is returned.
+template <typename F> int alloc_optional(b200_plan *p, bool *done, F &&alloc, std::string *why = nullptr) {
     const size_t n = p->allocs.size();
     const int64_t bytes = p->bytes;
     const int rc = alloc();
     *done = rc == B200_OK;
-    if (rc != B200_ERR_OOM) return rc;
+    if (rc != B200_ERR_OOM && rc != B200_ERR_UNSUPPORTED) return rc;
     for (; p->allocs.size() > n; p->allocs.pop_back()) cudaFree(p->allocs.back());
     p->bytes = bytes;
+    if (why) *why = p->err;
     p->err.clear();
     cudaGetLastError(); // the failed allocation's
     return B200_OK;
@@ -1291,18 +1294,22 @@ int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide);
 size_t xp_rope_smem_bytes(const b200_config &g) { return (size_t)(g.n_heads + g.n_kv_heads) * (g.head_size + 1) * 4; } // k_xp_rope_kv: a token's query and key heads
 
 // Buffers of one chunk.  Plans off the streaming path (row-major weights) and tensor-parallel ones keep the token-by-token graph, and so do plans that these buffers
-// have no room beside and plans whose rows of query and key heads are wider than shared memory.  A chunk is never longer than the context, whatever the batch size.
+// have no room beside, plans whose rows of query and key heads are wider than shared memory and plans whose tensor maps the driver does not make: b200_exact_prefill_info
+// says which.  A chunk is never longer than the context, whatever the batch size.
 int exact_prefill_init(b200_plan *p) {
     const b200_config &g = p->cfg;
-    if (!p->use_stream || g.tp_size > 1 || p->wtype != B200_GGML_Q8_0 || xp_rope_smem_bytes(g) > XP_SMEM_MAX) return B200_OK;
+    if (p->wtype != B200_GGML_Q8_0 || !p->use_stream || g.tp_size > 1) { p->xp.why = "the plan's weights are not Q8_0 on the streaming path"; return B200_OK; }
+    if (xp_rope_smem_bytes(g) > XP_SMEM_MAX) { p->xp.why = "a token's query and key heads are wider than shared memory"; return B200_OK; }
     const int chunk = p->prefill_batch < g.context_length ? p->prefill_batch : g.context_length;
     const int rows = (chunk + 63) / 64 * 64, nqkv = p->qd + 2 * p->kvd, wide = p->qd > g.dim ? p->qd : g.dim;
     int *const tok = p->prefill.tok;
     bool done;
-    int rc = alloc_optional(p, &done, [&]() -> int { return exact_prefill_alloc(p, rows, nqkv, wide); });
+    std::string why;
+    int rc = alloc_optional(p, &done, [&]() -> int { return exact_prefill_alloc(p, rows, nqkv, wide); }, &why);
     if (rc) return rc;
     if (!done) {
         p->xp = {};
+        p->xp.why = why;
         p->prefill.tok = tok;
     }
     return B200_OK;
@@ -1328,7 +1335,7 @@ int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide) {
         if ((rc = dalloc(p, &p->xp.scratch, want))) return rc;
         p->xp.scratch_bytes = want;
     }
-    bool ok = true;
+    bool ok = !refused("tensor_maps");
     for (int i = 0; ok && i < 4; i++)
         ok = xp_map_acts(&p->xp.mA[i], p->xp.AQ, p->xp.AS, rows, g.dim, 8 << i) == 0 && xp_map_acts(&p->xp.mATT[i], p->xp.AQ, p->xp.AS, rows, p->qd, 8 << i) == 0 &&
              xp_map_acts(&p->xp.mH[i], p->xp.HQ, p->xp.HS, rows, g.hidden_dim, 8 << i) == 0;
@@ -1338,7 +1345,7 @@ int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide) {
         auto &m = p->xp.maps[l];
         ok = xp_map_weights(&m.qkv, L.tqkv) == 0 && xp_map_weights(&m.wo, L.two) == 0 && xp_map_weights(&m.gu, L.tgu) == 0 && xp_map_weights(&m.w2, L.tw2) == 0;
     }
-    if (!ok) return B200_OK; // a tensor map that the driver does not make: rows stays 0, and prompts go token by token
+    if (!ok) return fail(p, B200_ERR_UNSUPPORTED, "the driver does not make the tensor maps");
     p->xp.rows = rows;
     return B200_OK;
 }
@@ -1832,6 +1839,7 @@ int b200_forward_batch_prefill(b200_plan *p, const int32_t *tokens, int32_t n, i
         int rc2 = exact_prefill(p, n, start_pos);
         if (rc2) return rc2;
         CK(cudaStreamSynchronize(p->stream));
+        p->xp.chunks++;
         return check_device_error(p);
     }
     CK(cudaMemcpyAsync(p->seq_tokens, p->h_ids, (size_t)n * 4, cudaMemcpyHostToDevice, p->stream));
@@ -1924,6 +1932,15 @@ int b200_prefill_info(b200_plan *p, int32_t *mode, int32_t *launches, float *dev
     if (mode) *mode = p->prefill.ready ? p->prefill.mode : B200_PREFILL_EXACT;
     if (launches) *launches = p->launches_prefill;
     if (device_ms) *device_ms = p->prefill_ms;
+    return B200_OK;
+}
+
+int b200_exact_prefill_info(b200_plan *p, int32_t *rows, int64_t *chunks, const char **why) {
+    if (!p) return B200_ERR_BAD_ARG;
+    if (rows) *rows = !p->xp.rows ? 0 : p->prefill_batch < p->cfg.context_length ? p->prefill_batch : p->cfg.context_length;
+    if (chunks) *chunks = p->xp.chunks;
+    if (why) *why = p->xp.rows ? "" : p->ly ? "layered plans have no exact prefill of their own" : p->cfg.tp_size > 1 ? "the plan is tensor-parallel"
+                  : p->prefill_batch <= 1 ? "the plan was created with prefill_batch_size <= 1" : p->xp.why.c_str();
     return B200_OK;
 }
 

@@ -199,6 +199,10 @@ class B200MasterPlan:
         """(active mode, kernels launched, device ms) of the last tensor-core prefill chunk."""
         return self._native.prefill_info()
 
+    def exact_prefill_info(self):
+        """(longest chunk that the exact prefill multiplies at once, 0: token by token; chunks so multiplied so far; why none are)."""
+        return self._native.exact_prefill_info()
+
     # -Dllama.cudaGraphs-style switch of the decode implementation (both bit-identical): "graph" = one CUDA graph of
     # 5 to 7 kernels per layer, "persistent" = one persistent kernel per token (csrc/decode_persistent.cuh)
     DECODE_GRAPH, DECODE_PERSISTENT = 0, 1

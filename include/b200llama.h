@@ -363,6 +363,10 @@ int b200_set_prefill_mode(b200_plan *plan, int32_t mode);
 /* Active mode, kernels launched and device milliseconds of the last tensor-core chunk (any pointer may be NULL). */
 int b200_prefill_info(b200_plan *plan, int32_t *mode, int32_t *launches, float *device_ms);
 
+/* The exact path: longest chunk that is multiplied at once (0: chunks go token by token, and *why says for what reason; else *why is empty), and how many chunks were
+ * multiplied at once so far (a chunk of one token is a single-token step).  Any pointer may be NULL; *why lives as long as the plan. */
+int b200_exact_prefill_info(b200_plan *plan, int32_t *rows, int64_t *chunks, const char **why);
+
 /* How the single-token forwards (b200_forward_decode / _prefill / b200_decode_sequence) run.  Both replace
  * TornadoVMMasterPlanSingleToken.tornadoVMForwardDecode's N+2 TaskGraph executions
  * (TornadoVMMasterPlanSingleToken.java:68-95) and produce bit-identical results:

@@ -22,7 +22,8 @@ def token_by_token(pkg, model, toks):
     return cache, x, logits
 
 
-def check(pkg, model, toks, chunks, batch):
+def check(pkg, model, toks, chunks, batch, why=""):
+    """Chunks of more than one token are multiplied at once; with `why` (a word of the reason) they go token by token, as in the plan that they are compared with."""
     cache, x, logits = token_by_token(pkg, model, toks)
     plan = pkg.B200MasterPlan(model, prefill_batch_size=batch)
     at = 0
@@ -30,6 +31,8 @@ def check(pkg, model, toks, chunks, batch):
         plan.forward_batch_prefill(toks[at:at + n], at)
         at += n
     assert at == len(toks) - 1
+    rows, multiplied, reason = plan.exact_prefill_info()
+    assert (rows, multiplied) == ((0, 0) if why else (min(batch, model.configuration.context_length), sum(n > 1 for n in chunks))) and (why in reason if why else not reason)
     for got, want in zip(kv(plan, model.configuration, at), cache):
         assert np.array_equal(got, want)
     assert np.array_equal(plan.read_buffer("x", model.configuration.dim).view(np.uint32), x)
