@@ -134,7 +134,6 @@ __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const in
 #define XP_STAGES 3
 #define XP_ROWS 64
 #define XP_THREADS 128
-#define XP_SPINS (1 << 22)
 struct XpMaps { CUtensorMap q, s; }; // quants; scales
 template <int NJ> struct XpTile {
     static constexpr int TOK = 8 * NJ;
@@ -142,9 +141,13 @@ template <int NJ> struct XpTile {
     static constexpr int HV = 33 * TOK * 4; // gate/up: the tile's 32 hidden units (+ 1: no bank conflicts) per token
     static constexpr int BYTES = 1024 + XP_STAGES * STAGE + 16 * XP_STAGES;
 };
-__device__ __forceinline__ bool xp_wait(unsigned bar, unsigned parity) { // bounded: false = given up
-    unsigned ok = 0;
-    for (int i = 0; i < XP_SPINS && !ok; i++)
+// Bounded: false = given up, after a second or once a wait has given up anywhere (the host's error word).  The clock is looked at every 256th time: read every time it
+// cost a prompt of 512 tokens 26 of 2226 us.
+#define XP_WAIT_NS 1000000000ull
+__device__ __forceinline__ bool xp_wait(unsigned bar, unsigned parity, const unsigned *err) {
+    unsigned long long t0 = 0;
+    for (unsigned i = 1;; i++) {
+        unsigned ok;
         asm volatile(
             "{\n"
             ".reg .pred p;\n"
@@ -154,7 +157,12 @@ __device__ __forceinline__ bool xp_wait(unsigned bar, unsigned parity) { // boun
             : "=r"(ok)
             : "r"(bar), "r"(parity)
             : "memory");
-    return ok != 0;
+        if (ok) return true;
+        if (i & 255u) continue;
+        const unsigned long long t = gtime_ns();
+        if (!t0) t0 = t;
+        if (t - t0 > XP_WAIT_NS || *reinterpret_cast<const volatile unsigned *>(err)) return false;
+    }
 }
 __device__ __forceinline__ void xp_load4(unsigned dst, const CUtensorMap *map, int x, int seg, int group, unsigned bar) {
     asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst), "l"(map), "r"(x), "r"(0), "r"(seg),
@@ -171,6 +179,7 @@ template <int MODE, int NJ>
 __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant__ XpMaps map_w, const __grid_constant__ XpMaps map_a, TileMat W, int lds, int n, float *__restrict__ out, int ldo,
                                                         int8_t *__restrict__ HQ, float *__restrict__ HS, XpLast last, float one_f, unsigned *err) {
     using T = XpTile<NJ>;
+    static_assert(T::HV <= XP_STAGES * T::STAGE, "the gate/up epilogue's rows take the ring's place");
     constexpr int TOK = T::TOK, MI = NJ >= 4 ? 2 : 1, NW = NJ / MI; // a warp's tile: 16 MI rows x 8 NW tokens
     extern __shared__ unsigned char smraw[];
     unsigned char *const ring = reinterpret_cast<unsigned char *>(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023); // (the swizzle is by address)
@@ -208,9 +217,9 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant
     const unsigned a_base = T::A_Q + ar * 128, b_base = T::B_Q + bt * 128, as_base = T::B_S + (wtok + 2 * (lane & 3)) * 4, ws_base = T::A_S + (wrow + (lane >> 2)) * 16;
     int stage = 0, c_in_seg = 0, c = 0;
     unsigned ph = 0;
-    bool ok = true;
+    bool ok = true, dead = false; // dead (thread 0): a stage did not come free, nothing is fetched any more
     for (; c < n_chunks; c++) {
-        if (!(ok = __all_sync(0xffffffffu, xp_wait(full0 + 8 * stage, ph)))) break;
+        if (!(ok = __all_sync(0xffffffffu, !dead && xp_wait(full0 + 8 * stage, ph, err)))) break;
         const unsigned s = smb + stage * T::STAGE;
         __half2 ws[MI][2][2]; // scales of blocks {0, 1}, {2, 3}
 #pragma unroll
@@ -267,15 +276,15 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant
         __syncwarp();
         if (lane == 0) mbar_arrive(empty0 + 8 * stage);
         if (tid == 0 && c + XP_STAGES < n_chunks) { // the stage goes to the chunk after the next two, once every warp is done with it
-            ok = xp_wait(empty0 + 8 * stage, ph);
-            if (ok) fetch();
+            dead = !xp_wait(empty0 + 8 * stage, ph, err);
+            if (!dead) fetch();
         }
         if (++stage == XP_STAGES) { stage = 0; ph ^= 1u; }
         if (++c_in_seg == cps) c_in_seg = 0;
     }
     if (!ok && lane == 0) { // (a wait gave up: the host is told, and nothing leaves with its copies in flight)
         *reinterpret_cast<volatile unsigned *>(err) = 200u;
-        for (int q = c; q < n_chunks && q < c + XP_STAGES; q++) xp_wait(full0 + 8 * (q % XP_STAGES), (q / XP_STAGES) & 1);
+        for (int q = c; q < n_chunks && q < c + XP_STAGES; q++) xp_wait(full0 + 8 * (q % XP_STAGES), (q / XP_STAGES) & 1, err);
     }
 
     const int r0 = wrow + (lane >> 2), t0 = wtok + 2 * (lane & 3);

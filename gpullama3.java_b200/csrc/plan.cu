@@ -1664,8 +1664,9 @@ cudaGraphExec_t prefill_graph(b200_plan *p, int pos) {
 int check_device_error(b200_plan *p) {
     if (p->h_err && *reinterpret_cast<volatile unsigned *>(p->h_err)) {
         const unsigned code = *reinterpret_cast<volatile unsigned *>(p->h_err);
-        return fail(p, B200_ERR_STATE, "a device-side wait timed out (code %u: 1+phase of the persistent decode kernel, 100+slot of a tensor-parallel flag, 200 the "
-                                       "batched exact prefill's operand ring): a peer rank is missing or the ranks' call sequences diverged; the plan must be freed", code);
+        if (code == 200u) return fail(p, B200_ERR_STATE, "a copy into the operand ring of the exact prefill's product did not arrive in time; the plan must be freed");
+        return fail(p, B200_ERR_STATE, "a device-side wait timed out (code %u: 1+phase of the persistent decode kernel, 100+slot of a tensor-parallel flag): a peer "
+                                       "rank is missing or the ranks' call sequences diverged; the plan must be freed", code);
     }
     return B200_OK;
 }
@@ -2210,6 +2211,49 @@ int b200_test_seqsum(const float *terms, int32_t n, float *out, int32_t *info) {
 int b200_test_seqsum2(const float *terms, int32_t n, int32_t threads, float *out, int32_t *info) {
     if (threads != 3 && threads != 256 && threads != 512 && threads != 1024) return B200_ERR_BAD_ARG;
     return run_seqsum_hook(terms, n, threads, out, info);
+}
+
+// One tile of the exact prefill's product on zeros (64 rows x 640 columns x 16 tokens), three times: as it is, with activation boxes of half the tile, whose stages never fill, and as
+// it is again.
+int b200_test_exact_prefill_wait(uint32_t *codes, float *ms) {
+    if (!codes || !ms) return B200_ERR_BAD_ARG;
+    constexpr int COLS = 640, TOK = 16;
+    b200_plan *p = nullptr; // (CK)
+    TileMat W{nullptr, XP_ROWS, COLS, COLS, 1, smv_unit_bytes(COLS)};
+    const size_t w_bytes = (size_t)XP_ROWS * W.unit_bytes, q_bytes = (size_t)64 * COLS, s_bytes = (size_t)64 * (COLS / 32) * 4, o_bytes = (size_t)TOK * XP_ROWS * 4;
+    unsigned char *mem = nullptr;
+    unsigned *err = nullptr, *d_err = nullptr;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    auto run = [&]() -> int {
+        CK(cudaMalloc(&mem, w_bytes + q_bytes + s_bytes + o_bytes));
+        CK(cudaMemset(mem, 0, w_bytes + q_bytes + s_bytes + o_bytes));
+        CK(cudaHostAlloc(&err, 64, cudaHostAllocMapped));
+        CK(cudaHostGetDevicePointer((void **)&d_err, err, 0));
+        for (cudaEvent_t &e : ev) CK(cudaEventCreate(&e));
+        W.base = mem;
+        const int8_t *q = reinterpret_cast<const int8_t *>(mem + w_bytes);
+        const float *s = reinterpret_cast<const float *>(mem + w_bytes + q_bytes);
+        XpMaps mw, ma[2];
+        if (xp_map_weights(&mw, W) || xp_map_acts(&ma[0], q, s, 64, COLS, TOK) || xp_map_acts(&ma[1], q, s, 64, COLS, TOK / 2)) return B200_ERR_UNSUPPORTED;
+        CK(cudaFuncSetAttribute(k_xp_gemm<XP_STORE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::BYTES));
+        for (int i = 0; i < 3; i++) {
+            *err = 0u;
+            CK(cudaEventRecord(ev[0]));
+            k_xp_gemm<XP_STORE, 2><<<dim3(1, 1), XP_THREADS, XpTile<2>::BYTES>>>(mw, ma[i == 1], W, 64, TOK, reinterpret_cast<float *>(mem + w_bytes + q_bytes + s_bytes), XP_ROWS, nullptr, nullptr,
+                                                                                XpLast{}, 1.0f, d_err);
+            CK(cudaGetLastError());
+            CK(cudaEventRecord(ev[1]));
+            CK(cudaDeviceSynchronize());
+            codes[i] = *reinterpret_cast<volatile unsigned *>(err);
+            CK(cudaEventElapsedTime(ms + i, ev[0], ev[1]));
+        }
+        return B200_OK;
+    };
+    const int rc = run();
+    for (cudaEvent_t e : ev) if (e) cudaEventDestroy(e);
+    if (err) cudaFreeHost(err);
+    cudaFree(mem);
+    return rc;
 }
 
 int b200_requant_kquant(int32_t ggml_type, const void *src, int64_t n_elems, void *dst_q8_0) {

@@ -457,6 +457,10 @@ int b200_test_seqsum(const float *terms, int32_t n, float *out, int32_t *info /*
  * (csrc/seqsum3.cuh); info = {items walked, fallbacks}. */
 int b200_test_seqsum2(const float *terms, int32_t n, int32_t threads, float *out, int32_t *info /* nullable */);
 
+/* Test hook for the bounded waits of the exact prefill's product (csrc/exact_prefill.cuh): codes[3] and ms[3] are the error word and the time of one tile whose operands
+ * arrive, of one whose operands arrive in part (its waits give up: 200), and of the first again. */
+int b200_test_exact_prefill_wait(uint32_t *codes, float *ms);
+
 /* Test hook for the device-side K-quant -> Q8_0 re-quantiser the upload pipeline applies to Q4_K / Q5_K / Q6_K tensors (csrc/kquant.cuh;
  * replaces ModelLoader.dequantizeToQ8_0TornadoTensor, model/loader/ModelLoader.java:173-224): host K-quant blocks in, host GGUF Q8_0
  * blocks (34 bytes per 32 elements) out, byte-identical to the reference's.  n_elems % 256 == 0. */

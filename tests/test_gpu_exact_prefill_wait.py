@@ -1,0 +1,17 @@
+"""The bounded waits of the exact prefill's product (csrc/exact_prefill.cuh, xp_wait): a tile whose operands arrive in part only (its stages never fill) ends with the error word set,
+every warp of it, and the context goes on as before."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_operands_that_do_not_arrive(pkg, make_model):
+    before, starved, after = pkg.native.test_exact_prefill_wait()
+    assert before[0] == 0 and before[1] < 900
+    assert starved[0] == 200 and 1000 <= starved[1] < 1100  # the first wait in full, the drained stages a tenth of a millisecond each
+    assert after[0] == 0 and after[1] < 10
+    model = make_model("tiny-llama", pkg.gguf.GGMLType.Q8_0, ctx=32)
+    plan = pkg.B200MasterPlan(model, prefill_batch_size=16)
+    plan.forward_batch_prefill(list(range(3, 14)), 0)
+    assert plan.exact_prefill_info()[1] == 1
+    plan.free()
