@@ -141,6 +141,7 @@ struct b200_plan {
         std::vector<Maps> maps;
         XpMaps mA[4], mATT[4], mH[4]; // activations in tiles of 8, 16, 32, 64 tokens: AQ with rows of dim and of the query width, HQ
         int64_t chunks = 0;           // multiplied at once so far
+        int tile = -1;                // token tile of every product, as an index into {64, 32, 16, 8} (B200_XP_TILE=64|32|16|8; -1: by the model)
         std::string why;              // rows == 0: why not
     } xp;
     // persistent decode kernel
@@ -1346,6 +1347,9 @@ int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide) {
         ok = xp_map_weights(&m.qkv, L.tqkv) == 0 && xp_map_weights(&m.wo, L.two) == 0 && xp_map_weights(&m.gu, L.tgu) == 0 && xp_map_weights(&m.w2, L.tw2) == 0;
     }
     if (!ok) return fail(p, B200_ERR_UNSUPPORTED, "the driver does not make the tensor maps");
+    if (const char *e = getenv("B200_XP_TILE"))
+        for (int i = 0; i < 4; i++)
+            if (atoi(e) == 64 >> i) p->xp.tile = i;
     p->xp.rows = rows;
     return B200_OK;
 }
@@ -1374,7 +1378,7 @@ int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps (&ma)
         const float t = std::max(per_sm * tiles[i].share, tiles[i].chain + (per_sm - 1) * tiles[i].share / 3.f);
         if (i == 0 || t < least) { best = i; least = t; }
     }
-    switch (best) {
+    switch (p->xp.tile >= 0 ? p->xp.tile : best) {
     case 0: return go(std::integral_constant<int, 8>());
     case 1: return go(std::integral_constant<int, 4>());
     case 2: return go(std::integral_constant<int, 2>());
