@@ -79,7 +79,7 @@ struct PdArgs {
     unsigned evict_first;      // 1: the weight stream's bulk copies carry an L2 evict_first policy -- 8 GB of single-use weights per token
                                // otherwise churn the 126 MB L2 and push out the KV rows, x, the norm weights and the prefetched tiles
     unsigned max_fly;          // experiment knob (B200_PD_MAXFLY): bulk copies one CTA keeps in flight; 0 = no limit but the ring (default:
-                               // limiting it never helped the dependent phases and always slowed the stream, profiles/r2_run3_knob_sweep.log)
+                               // limiting it never helped the dependent phases and always slowed the stream)
     // tensor parallelism (tp.n == 1: everything below unused)
     TpCtx tp;
     unsigned pd_flags_off;     // offset of the persistent kernel's epoch flags [PD_S_SLOTS][TP_MAX] in every rank's comm buffer
@@ -134,7 +134,7 @@ __host__ __device__ inline PdSmem pd_layout(int dim, int qd, int hidden, int hea
 // ---- bounded waits ----------------------------------------------------------------------------------------------------------
 // Polls are RELAXED loads; ONE acquire load of the same word follows the successful one.  (ld.acquire in the loop compiles to a
 // load plus CCTL.IVALL: every poll of thread 0 threw away the whole L1 of its SM; a trailing fence.acq_rel.sys instead costs a
-// MEMBAR.SYS per wait, which made tensor-parallel steps ~20 % slower -- profiles/r2_tp2_fences.log.)
+// MEMBAR.SYS per wait, which made tensor-parallel steps ~20 % slower.)
 __device__ __forceinline__ unsigned pd_ld_relaxed_gpu(const unsigned *p) {
     unsigned v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const in
 // add: a packed add behind a packed product comes out as ONE fused operation (measured; also where the 1 is a constant of the kernel, so it is an argument).
 // Integers are converted by the conversion instruction: accumulators that start at 0x4B400000 and a subtraction cost four register moves for every mma (gate/up
 // product 411 against 392 us).  Gate/up of 512 tokens, 8B layer: 560 us with scalar adds and cp.async fetches by all threads, 392 us so (FMA pipe 50 %, issue slots
-// 64 %; 19 warp instructions per 16 x 8 tile and block, 15 of them the arithmetic and its operands); Wo + W2 341 -> 281 us, QKV 121 -> 90 us.
+// 64 %; 19 warp instructions per 16 x 8 tile and block, 10 of them the conversions, products and adds); Wo + W2 341 -> 281 us, QKV 121 -> 90 us.
 // tcgen05.mma.kind::i8 does not pay here: a sum is read back after every 32 columns, so each block costs a round trip product - barrier - tcgen05.ld - barrier; with 2 to
 // 4 accumulator buffers, a warp each for loads and products and up to 24 warps on the sums it took 410 us (32-token tiles) to 494 us.
 // A CTA is 4 warps: 64 weight rows (16 groups of the tile-major layout) x 8 * NJ tokens; with 32 tokens and more a warp owns 32 rows and half of the tokens

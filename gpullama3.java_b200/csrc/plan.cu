@@ -612,12 +612,12 @@ void read_knobs(b200_plan *p) {
     size_t b = e ? (size_t)atoi(e) * 1024 : SMV_SMEM_BUDGET_MAX;
     p->smv_budget = b > SMV_SMEM_BUDGET_MAX ? SMV_SMEM_BUDGET_MAX : b;
     p->smv_budget_cols = m ? atoi(m) : 0;
-    const char *w = getenv("B200_L2_WINDOW_KB"); // experimental: measured slower on B200 (profiles/), off by default
+    const char *w = getenv("B200_L2_WINDOW_KB"); // experimental: measured slower on B200, off by default
     p->l2_window = (unsigned)((w ? atoi(w) : 0) * 1024);
     const char *a = getenv("B200_PD_L2_AHEAD"); // persistent kernel: tiles of L2 look-ahead while the ring is full
     p->pd_l2_ahead = a ? (unsigned)atoi(a) : 0u;
     const char *f = getenv("B200_PD_MAXFLY"); // persistent kernel: bulk copies in flight per CTA (0 = unlimited)
-    p->pd_max_fly = f ? (unsigned)atoi(f) : 0u; // measured (profiles/r2_run3_knob_sweep.log): any limit below the ring depth only slows the stream
+    p->pd_max_fly = f ? (unsigned)atoi(f) : 0u; // measured: any limit below the ring depth only slows the stream
     const char *ev = getenv("B200_PD_EVICT_FIRST"); // persistent kernel: L2 evict_first policy on the weight stream (default on)
     p->pd_evict_first = ev ? (unsigned)atoi(ev) : 1u;
     const char *g = getenv("B200_PD_STAGES"); // persistent kernel: cap on the ring depth
@@ -625,7 +625,7 @@ void read_knobs(b200_plan *p) {
     const char *v = getenv("B200_NORM_V2");
     p->norm_v2 = !(v && v[0] == '0');
     const char *d = getenv("B200_DECODE");
-    // default: the CUDA graph -- measured faster than the persistent kernel on the same box (profiles/r2_final_a.log: 313.6 vs 285.1 tok/s,
+    // default: the CUDA graph -- measured faster than the persistent kernel on the same GPU (313.6 vs 285.1 tok/s,
     // 8B Q8_0; under tensor parallelism by 10-21 %).  B200_DECODE=persistent or b200_set_decode_mode select the one-kernel-per-token path.
     p->decode_mode = (d && !strcmp(d, "persistent")) ? B200_DECODE_PERSISTENT : B200_DECODE_GRAPH;
 }
@@ -1497,10 +1497,10 @@ int prefill_init(b200_plan *p) {
     {
         const char *e = getenv("B200_GEMM_2CTA");
         c.pair = !(e && e[0] == '0') && nqkv % 256 == 0 && g.dim % 256 == 0 && g.hidden_dim % 128 == 0;
-        const char *e2 = getenv("B200_GEMM_PERSIST"); // persistent CTA-pair kernel (double-buffered TMEM) for QKV and gate/up: validated on the
+        const char *e2 = getenv("B200_GEMM_PERSIST"); // persistent CTA-pair kernel (double-buffered TMEM) for QKV and gate/up; =0 selects the one-tile kernels
         c.persist = !(e2 && e2[0] == '0');
         const char *e3 = getenv("B200_GEMM_PERSIST_RESID"); // =1: Wo / W2 through the persistent kernel too (split-K folded into its work list); experimental
-        c.persist_resid = c.persist && e3 && e3[0] == '1';            // GPU (tests/test_gpu_prefill.py, profiles/r2_run1_first_green.log); =0 selects the one-tile kernels
+        c.persist_resid = c.persist && e3 && e3[0] == '1';
     }
     if (!ok) { c.why = "cuTensorMapEncodeTiled rejected a tensor map"; return B200_OK; }
     if (g.head_size == 128) {

@@ -100,7 +100,7 @@ __device__ __forceinline__ void bulk_g2s(unsigned dst, const void *src, unsigned
                  : "memory");
 }
 // The same copy with an L2 evict_first policy: single-use weight tiles must not push the KV rows, activations and norm weights out of L2
-// (measured on the persistent kernel: +6 % tokens/s, profiles/r2_run6_evict_first_qwen3.log).
+// (measured on the persistent kernel: +6 % tokens/s).
 __device__ __forceinline__ unsigned long long l2_policy_evict_first() {
     unsigned long long pol;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));

@@ -371,7 +371,7 @@ int b200_exact_prefill_info(b200_plan *plan, int32_t *rows, int64_t *chunks, con
  * TornadoVMMasterPlanSingleToken.tornadoVMForwardDecode's N+2 TaskGraph executions
  * (TornadoVMMasterPlanSingleToken.java:68-95) and produce bit-identical results:
  *   B200_DECODE_GRAPH       one CUDA graph of 5 kernels per layer (7 where the norm is a launch) with programmatic-dependent-launch edges (the default:
- *                           measured 3.19 ms vs 3.51 ms per token on Llama-3-8B Q8_0, profiles/r2_final_a.log);
+ *                           measured 3.19 ms vs 3.51 ms per token on Llama-3-8B Q8_0);
  *   B200_DECODE_PERSISTENT  ONE persistent kernel per token (csrc/decode_persistent.cuh): one CTA per SM streams the
  *                           weights of every matrix through a shared-memory ring while epoch counters order the phases.
  *                           Available when the plan fits (Q8_0 streaming layout, head size 64/128); the environment

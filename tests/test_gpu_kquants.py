@@ -1,4 +1,4 @@
-"""GPU tests of the K-quant load path (csrc/kquant.cuh inside the upload pipeline, SURVEY 8(f) N4) through the C ABI.
+"""GPU tests of the K-quant load path (csrc/kquant.cuh inside the upload pipeline) through the C ABI.
 
 Bar: byte-exact.  The device re-quantiser must produce the very Q8_0 blocks ModelLoader.dequantizeToQ8_0TornadoTensor builds on the host
 (model/loader/ModelLoader.java:173-224, restated in oracle/oracle.c and pinned against gguf-py in tests/test_kquants.py), and a plan

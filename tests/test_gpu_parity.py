@@ -1,7 +1,7 @@
 """GPU parity tests: the CUDA path, called through the C ABI (ctypes -> libb200llama.so), against
 the CPU oracle on the same seeded synthetic GGUF models.  Bar: logits BIT-EXACT (uint32 view
 equal) and greedy token ids identical for both Q8_0 and FP16 weights -- the kernels reproduce
-the CPU path's float evaluation order (DESIGN.md "Exactness"), so no tolerance is needed."""
+the CPU path's float evaluation order, so no tolerance is needed."""
 import numpy as np
 import pytest
 
@@ -77,7 +77,7 @@ def test_decode_f16_bit_exact(pkg, orc, make_model, shape, lanes):
 @pytest.mark.parametrize("shape,lanes", [("mid-llama-1b", 16), ("mid-llama", 16), ("mid-llama", 8), ("mid-qwen3-4b", 16)])
 def test_decode_mid_geometries_f16(pkg, orc, shape, lanes):
     """FP16 plans on the per-warp bulk-copy rings (csrc/stream_matvec_f16.cuh) at the real layer geometries, bit-exact vs the oracle:
-    Llama-3.2-1B (dim 2048, hidden 8192, tied classifier), Llama-3-8B (config 3: hidden 14336 -> a 57 KB activation
+    Llama-3.2-1B (dim 2048, hidden 8192, tied classifier), Llama-3-8B (hidden 14336 -> a 57 KB activation
     next to the rings), Qwen3-4B (dim 2560 -> 256-column segments).  A warp laps its ring many times per matvec; the 8-lane species
     puts four rows (two gate + two up) into one warp."""
     sh = pkg.synth.SHAPES[shape]
@@ -134,7 +134,7 @@ def mid_model(pkg, name, ctx):
 @pytest.mark.parametrize("mode", MODES)
 @pytest.mark.parametrize("shape", ["mid-llama", "mid-qwen3-4b", "mid-llama-1b", "mid-llama-70b"])
 def test_decode_mid_geometries_q8(pkg, orc, shape, mode):
-    """2-layer cuts of the BASELINE geometries, bit-exact vs the oracle: Llama-3-8B (dim 4096, hidden 14336 = 7 column segments,
+    """2-layer cuts of the benchmarked geometries, bit-exact vs the oracle: Llama-3-8B (dim 4096, hidden 14336 = 7 column segments,
     32/8 heads), Qwen3-4B (dim 2560 / hidden 9728 / q width 4096: three different segment widths, q/k norm, NeoX rope),
     Llama-3.2-1B (head 64, tied classifier), Llama-3-70B (dim 8192 / hidden 28672 / 64 heads).  The ring laps many times per matvec."""
     m = mid_model(pkg, shape, 16)
@@ -224,7 +224,7 @@ def test_batch_prefill_generation_loop(pkg, orc, make_model):
 
 
 def test_mistral_named_model_runs_the_llama_path(pkg, orc, tmp_path):
-    """SURVEY 8(f) N4: Mistral = the Llama forward through the same kernels (Mistral.java -> InferenceCore.forwardJava)."""
+    """Mistral = the Llama forward through the same kernels (Mistral.java -> InferenceCore.forwardJava)."""
     path = str(tmp_path / "mistral.gguf")
     pkg.synth.write_model(path, "tiny-llama", pkg.gguf.GGMLType.Q8_0, seed=11, display_name="Mistral-7B-Instruct synthetic")
     m = pkg.load_model(path, 24)
@@ -247,7 +247,7 @@ def test_modes_interleave(pkg, orc, make_model):
 
 
 def test_long_context_score_row_in_global_memory(pkg, orc, make_model):
-    """A context too long for the shared-memory score row (ADVICE r1: real checkpoints default to 131072) builds a plan and stays bit-exact."""
+    """A context too long for the shared-memory score row (real checkpoints default to 131072) builds a plan and stays bit-exact."""
     m = make_model("tiny-llama", pkg.gguf.GGMLType.Q8_0, 20000)
     for mode in MODES:
         run_stream(pkg, orc, m, 16, 6, check_kv=False, mode=mode)

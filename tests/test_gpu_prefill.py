@@ -5,7 +5,7 @@ FP16 before each GEMM, as in the reference's MMA prefill, TransformerBatchPrefil
   * GEMM building block vs an fp32 matmul of the same fp16 operands: |err| <= 2^-14 * K^(1/2) * max|ref|-ish;
     asserted as max|err| <= 1e-4 * max|ref| (measured 8e-6 .. 2e-5; only the fp32 summation order differs);
   * KV cache after prefill and the logits of the following decode step vs the CPU oracle:
-    max|err| <= 2^-8 * max|ref| (SURVEY.md 8d "FP16-scale tolerance"; measured 2e-4 .. 1.2e-3)."""
+    max|err| <= 2^-8 * max|ref| (FP16-scale tolerance; measured 2e-4 .. 1.2e-3)."""
 import os
 
 import numpy as np

@@ -1,4 +1,4 @@
-"""the device-side temperature / top-p sampler (csrc/sampler.cuh behind b200_forward_decode_sample) against the
+"""The device-side temperature / top-p sampler (csrc/sampler.cuh behind b200_forward_decode_sample) against the
 oracle's restatement of Sampler.java / CategoricalSampler.java / ToppSampler.java: same logits (bit-exact forward), same uniform
 number -> same token id, for greedy, categorical and top-p sampling."""
 import numpy as np

@@ -89,8 +89,8 @@ def test_generation_loop_conventions(pkg):
 
 
 def test_mistral_loads_for_the_forward_pass_only(pkg, tmp_path):
-    """a Mistral GGUF uses the Llama forward and weight slots (MistralModelLoader.java:92-113); its context is clamped
-    to the model's (:45-46).  Its tokenizer family is NOT implemented and must be rejected up front (ADVICE r1), not mis-tokenised."""
+    """A Mistral GGUF uses the Llama forward and weight slots (MistralModelLoader.java:92-113); its context is clamped
+    to the model's (:45-46).  Its tokenizer family is NOT implemented and must be rejected up front, not mis-tokenised."""
     path = str(tmp_path / "mistral.gguf")
     pkg.synth.write_model(path, "tiny-llama", pkg.gguf.GGMLType.Q8_0, seed=3, display_name="Mistral-7B-Instruct synthetic")
     m = pkg.load_model(path, 10 ** 6)
@@ -102,7 +102,7 @@ def test_mistral_loads_for_the_forward_pass_only(pkg, tmp_path):
 
 
 def test_phi3_loads_with_fused_tensors(pkg, tmp_path):
-    """a Phi-3 GGUF (Phi3ModelLoader.java:51-113): head size = dim / heads, the requested context length is kept, the
+    """A Phi-3 GGUF (Phi3ModelLoader.java:51-113): head size = dim / heads, the requested context length is kept, the
     fused attn_qkv / ffn_up tensors are present instead of q/k/v/gate; its SentencePiece tokenizer is rejected up front."""
     G = pkg.gguf.GGMLType
     path = str(tmp_path / "phi3.gguf")

@@ -1,11 +1,11 @@
-"""K-quant load path (SURVEY 8(f) N4) and third-party pins of the data formats -- CPU.
+"""K-quant load path and third-party pins of the data formats -- CPU.
 
 The reference's accelerator path re-quantises Q4_K / Q5_K / Q6_K tensors to Q8_0 while loading (ModelLoader.java:163,173-224) and then
 computes as for a Q8_0 file.  The oracle restates the element reads and the re-quantiser (oracle/oracle.c); here:
   * the element reads are PINNED against gguf-py (llama.cpp's own Python implementation of the formats, pinned in this image as
     gguf 0.19) -- bit-equal floats for all three formats, and the same for Q8_0 / F16 through the product's own dequantiser;
   * the re-quantiser is checked against a second, vectorised numpy restatement, and its rounding rule against hand-computed ties;
-  * the product's GGUF reader and writer are pinned against gguf-py's GGUFReader / GGUFWriter (SURVEY 8(f) N1);
+  * the product's GGUF reader and writer are pinned against gguf-py's GGUFReader / GGUFWriter;
   * the loader maps K-quant file types to a Q8_0 configuration (AbstractModelLoader.java:45-47).
 The device side (csrc/kquant.cuh) is compared with the oracle in tests/test_gpu_kquants.py."""
 import os

@@ -204,7 +204,7 @@ def test_golden_fixture(orc, pkg, make_model):
 
 
 def test_sampler_restatements_agree(pkg, orc):
-    """SURVEY 8(f) N3 (parity unpinned: no JDK): the product's Python restatement of L32X64MixRandom equals the oracle's C
+    """Parity unpinned (no JDK): the product's Python restatement of L32X64MixRandom equals the oracle's C
     restatement, and the oracle's C sampler (Sampler.java / CategoricalSampler.java / ToppSampler.java line by line, heap
     included) equals an independent numpy formulation on random logits."""
     for seed in (0, 1, 42, -7, 2 ** 40 + 3):

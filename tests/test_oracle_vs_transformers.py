@@ -1,6 +1,6 @@
 """STRUCTURAL pin of the oracle against an independent implementation (CPU).
 
-No JDK exists in this image, so the oracle cannot be compared with the reference's own output ("parity unpinned").  What can
+No JDK exists in this image, so the oracle cannot be compared with the reference's own output.  What can
 be checked here is everything except the float summation order: the oracle's forward pass (oracle/oracle.c, a restatement of
 InferenceCore.forwardJava / forwardJavaQwen3, inference/InferenceCore.java:39-172,565-697) is run on a seeded synthetic GGUF model and
 compared with Hugging Face transformers' LlamaForCausalLM / Qwen3ForCausalLM / Phi3ForCausalLM evaluating THE SAME weights in float64 -- an implementation

@@ -217,7 +217,7 @@ def test_native_is_faster_than_the_restatement(pkg, tor, vocabs):
 
 
 def test_encode_agrees_with_huggingface_tokenizers(pkg, tor, vocabs):
-    """THIRD-PARTY pin (SURVEY 8(f) N2 was checked only against this repository's own restatement): Hugging Face `tokenizers` (the Rust
+    """THIRD-PARTY pin (the tokenizer was checked only against this repository's own restatement): Hugging Face `tokenizers` (the Rust
     BPE) configured with the reference's pipeline ORDER -- byte-level symbol mapping first, THEN the pre-tokenisation regex on the mapped
     text (LlamaTokenizer.java:164-200 does exactly this, which is why words are not split at spaces there), then BPE over the chunk --
     produces the same ids as the native tokenizer and as the oracle on the synthetic vocabularies (whose token ids are in merge order, so

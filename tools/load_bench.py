@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""time the load of a model FROM A GGUF FILE ON DISK through the upload pipeline (the counterpart of the
+"""Time the load of a model FROM A GGUF FILE ON DISK through the upload pipeline (the counterpart of the
 reference's load-time metric, ModelLoader.java:102-106, and its first-execution copy-in, TornadoVMMasterPlanSingleToken.java:51-54).
 
     python tools/load_bench.py [workload] [dir]   ->  gpurun_out/load_bench_<workload>.json
@@ -34,7 +34,7 @@ def main():
     size = os.path.getsize(path)
     del tensors, plan_order
     out = {"workload": workload, "file_bytes": size, "synthesise_s": gen_s, "write_s": write_s, "runs": []}
-    for label, env in (("pipelined", {}), ("blocking (round 1)", {"B200_UPLOAD_SYNC": "1"}), ("pipelined, 8 host threads", {"B200_UPLOAD_THREADS": "8"})):
+    for label, env in (("pipelined", {}), ("blocking", {"B200_UPLOAD_SYNC": "1"}), ("pipelined, 8 host threads", {"B200_UPLOAD_THREADS": "8"})):
         os.environ.update(env)
         try:
             t0 = time.time()
