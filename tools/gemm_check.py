@@ -37,5 +37,5 @@ for (m, n, k) in shapes:
     rec = {"two_cta": two, "resid": os.environ.get("B200_GEMM_RESID", "0"), "stages": os.environ.get("B200_GEMM_STAGES", "3"), "m": m, "n": n, "k": k, "max_abs_err": err, "ref_max": scale, "ms": ms, "tflops": 2.0 * m * n * k / (ms * 1e-3) / 1e12}
     print(json.dumps(rec), flush=True)
     out.append(rec)
-os.makedirs("gpurun_out", exist_ok=True)
-json.dump(out, open("gpurun_out/gemm_check_s%s_2cta%d_r%s.json" % (os.environ.get("B200_GEMM_STAGES", "3"), two, os.environ.get("B200_GEMM_RESID", "0")), "w"), indent=1)
+os.makedirs("out", exist_ok=True)
+json.dump(out, open("out/gemm_check_s%s_2cta%d_r%s.json" % (os.environ.get("B200_GEMM_STAGES", "3"), two, os.environ.get("B200_GEMM_RESID", "0")), "w"), indent=1)

@@ -2,7 +2,7 @@
 """Time the load of a model FROM A GGUF FILE ON DISK through the upload pipeline (the counterpart of the
 reference's load-time metric, ModelLoader.java:102-106, and its first-execution copy-in, TornadoVMMasterPlanSingleToken.java:51-54).
 
-    python tools/load_bench.py [workload] [dir]   ->  gpurun_out/load_bench_<workload>.json
+    python tools/load_bench.py [workload] [dir]   ->  out/load_bench_<workload>.json
 
 Writes a seeded synthetic GGUF of the real shape (no checkpoints offline), drops it from the process (the page cache may still hold it:
 reported as "warm"), then: parse + mmap (gguf.GGUFFile), b200_plan_create (pinned double buffer -> copy stream -> device staging ->
@@ -52,8 +52,8 @@ def main():
             for k in env:
                 del os.environ[k]
     os.remove(path)
-    os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-    with open(os.path.join(ROOT, "gpurun_out", f"load_bench_{workload}.json"), "w") as f:
+    os.makedirs(os.path.join(ROOT, "out"), exist_ok=True)
+    with open(os.path.join(ROOT, "out", f"load_bench_{workload}.json"), "w") as f:
         json.dump(out, f, indent=1)
     print(json.dumps(out))
 

@@ -2,7 +2,7 @@
 """Summarise an ncu launch list (`ncu --metrics gpu__time_duration.sum[,dram__bytes_read.sum,dram__bytes_write.sum] --csv --log-file X.csv ...`)
 per kernel: launches, total and mean duration, share of the listed time, DRAM bytes per launch.
 
-    python tools/ncu_summary.py gpurun_out/launches.csv [skip_first_n_launches] > profiles/launches.summary.txt
+    python tools/ncu_summary.py out/launches.csv [skip_first_n_launches] > profiles/launches.summary.txt
 
 Per-launch times under ncu are cold-cache and serialised (no PDL overlap): the kernel SHARES are what to compare with the bench, never the absolutes."""
 import csv

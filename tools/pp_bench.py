@@ -37,6 +37,6 @@ att_flops = 4.0 * sh.q_dim * sh.n_layers * (n * (n + 1) / 2)
 rec = {"shape": shape, "n": n, "mode": info[0], "launches": info[1], "device_ms": dev, "wall_ms": wall, "tok_s_device": n / dev * 1e3, "tok_s_e2e": n / wall * 1e3,
        "tflops": (gemm_flops + att_flops) / (dev * 1e-3) / 1e12, "gemm_tflop": gemm_flops / 1e12, "att_tflop": att_flops / 1e12, "build_s": t1 - t0, "plan_s": t2 - t1}
 print(json.dumps(rec), flush=True)
-os.makedirs("gpurun_out", exist_ok=True)
-json.dump(rec, open(f"gpurun_out/pp_bench_{shape}_{n}.json", "w"), indent=1)
+os.makedirs("out", exist_ok=True)
+json.dump(rec, open(f"out/pp_bench_{shape}_{n}.json", "w"), indent=1)
 plan.free()

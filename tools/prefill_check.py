@@ -56,5 +56,5 @@ for shape in shapes:
     print(json.dumps(rec), flush=True)
     out.append(rec)
     plan.free()
-os.makedirs("gpurun_out", exist_ok=True)
-json.dump(out, open("gpurun_out/prefill_check%s.json" % ("_q8" if os.environ.get("PREFILL_QUANT") == "q8" else ""), "w"), indent=1)
+os.makedirs("out", exist_ok=True)
+json.dump(out, open("out/prefill_check%s.json" % ("_q8" if os.environ.get("PREFILL_QUANT") == "q8" else ""), "w"), indent=1)

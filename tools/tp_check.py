@@ -3,7 +3,7 @@
 Every rank builds the same seeded model, uploads its share, decodes a teacher-forced stream and a greedy
 stream with BOTH decode implementations (CUDA graph / persistent kernel); rank 0 compares every argmax with the
 CPU oracle (token-exact expected: row sharding keeps the reference's summation order) and the residual stream bit
-for bit, and writes gpurun_out/tp_check_<shape>_tp<N>.json."""
+for bit, and writes out/tp_check_<shape>_tp<N>.json."""
 import json
 import os
 import sys
@@ -67,8 +67,8 @@ for mode in ("graph", "persistent"):
         print(f"[tp{world}] {mode}: {r}", flush=True)
 if rank == 0:
     report["ok"] = bool(ok)
-    os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-    with open(os.path.join(ROOT, "gpurun_out", f"tp_check_{shape}_tp{world}.json"), "w") as f:
+    os.makedirs(os.path.join(ROOT, "out"), exist_ok=True)
+    with open(os.path.join(ROOT, "out", f"tp_check_{shape}_tp{world}.json"), "w") as f:
         json.dump(report, f, indent=1)
     print("RESULT", "OK" if ok else "MISMATCH", flush=True)
 plan.free()
