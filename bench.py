@@ -642,7 +642,7 @@ def parity_gate(plan, tokens, ref, want_logits: bool):
     if dmax is not None:
         out["max_abs_dlogit"] = dmax
         out["logits_bit_equal"] = bit_equal
-        out["tolerance"] = "0 (decode reproduces the CPU path's float order; FP16-scale 2^-8*max|logit| would be the north-star bound)"
+        out["tolerance"] = "0 (decode reproduces the CPU path's float order; FP16-scale 2^-8*max|logit| would be an FP16 bound)"
     return out
 
 
