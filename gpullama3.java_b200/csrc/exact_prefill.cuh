@@ -48,6 +48,18 @@ __device__ __forceinline__ xp_f2 xp_fma2(xp_f2 a, xp_f2 b, xp_f2 c) {
     return r;
 }
 
+// four quants as bytes, and four bytes as FP16 numbers (1024 + 128 + q has q + 128 in its low byte)
+__device__ __forceinline__ unsigned xp_bytes(const int (&q)[4]) { return (q[0] & 0xff) | (q[1] & 0xff) << 8 | (q[2] & 0xff) << 16 | (unsigned)q[3] << 24; }
+__device__ __forceinline__ void xp_halves(unsigned q, unsigned &lo, unsigned &hi) {
+    const __half2 bias = __floats2half2_rn(1152.0f, 1152.0f);
+    q ^= 0x80808080u;
+    lo = __byte_perm(q, 0x64646464u, 0x4140);
+    hi = __byte_perm(q, 0x64646464u, 0x4342);
+    const __half2 a = __hsub2(*reinterpret_cast<__half2 *>(&lo), bias), b = __hsub2(*reinterpret_cast<__half2 *>(&hi), bias);
+    lo = *reinterpret_cast<const unsigned *>(&a);
+    hi = *reinterpret_cast<const unsigned *>(&b);
+}
+
 // ---- RMSNorm + Q8_0 quantisation of one token's row (InferenceCore.rmsnorm, InferenceCore.java:39-48) ------------------------------
 // One CTA per token, E entries per thread in registers, the sum of squares by seqsum3.cuh (a literal chain by one thread, the rows of a chunk side by
 // side, took 22 us at dim 4096).  EMBED: the row is gathered from the embedding table first.
@@ -60,7 +72,7 @@ struct XpLast {
 struct XpSync { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
 template <bool EMBED, int E>
 __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const int *__restrict__ tok, DevMat emb, const float *__restrict__ w, float eps, int dim,
-                                                 int8_t *__restrict__ AQ, float *__restrict__ AS, int lds, XpLast out1) {
+                                                 int8_t *__restrict__ AQ, __half *__restrict__ AH, float *__restrict__ AS, int lds, XpLast out1) {
     __shared__ __align__(16) float sq[256 * E];
     __shared__ SeqSum3Scratch scratch;
     constexpr int TPB = 32 / E; // threads of a quantisation block
@@ -109,7 +121,11 @@ __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const in
             const float s = __fmul_rn(v[k + u], ainv);
             p |= ((unsigned)__float2int_rz(__fadd_rn(s, copysignf(0.5f, s))) & 0xffu) << (8 * u);
         }
-        *reinterpret_cast<unsigned *>(AQ + (size_t)b * dim + base + k) = p;
+        if (AH) {
+            uint2 h;
+            xp_halves(p, h.x, h.y);
+            *reinterpret_cast<uint2 *>(AH + (size_t)b * dim + base + k) = h;
+        } else *reinterpret_cast<unsigned *>(AQ + (size_t)b * dim + base + k) = p;
         if (last) *reinterpret_cast<unsigned *>(out1.xq + base + k) = p;
     }
     if (tid % TPB == 0) {
@@ -177,7 +193,7 @@ __device__ __forceinline__ xp_f2 xp_lds64(unsigned a) {
 
 template <int MODE, int NJ>
 __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant__ XpMaps map_w, const __grid_constant__ XpMaps map_a, TileMat W, int lds, int n, float *__restrict__ out, int ldo,
-                                                        int8_t *__restrict__ HQ, float *__restrict__ HS, XpLast last, float one_f, unsigned *err) {
+                                                        int8_t *__restrict__ HQ, __half *__restrict__ HH, float *__restrict__ HS, XpLast last, float one_f, unsigned *err) {
     using T = XpTile<NJ>;
     static_assert(T::HV <= XP_STAGES * T::STAGE, "the gate/up epilogue's rows take the ring's place");
     constexpr int TOK = T::TOK, MI = NJ >= 4 ? 2 : 1, NW = NJ / MI; // a warp's tile: 16 MI rows x 8 NW tokens
@@ -310,7 +326,8 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant
             const float v = hv[t * 33 + lane];
             float as;
             const int q = quant_block_lane(v, as);
-            HQ[(size_t)(tok0 + t) * hidden + blockIdx.x * 32 + lane] = (int8_t)q;
+            if (HH) HH[(size_t)(tok0 + t) * hidden + blockIdx.x * 32 + lane] = __int2half_rn((int8_t)q);
+            else HQ[(size_t)(tok0 + t) * hidden + blockIdx.x * 32 + lane] = (int8_t)q;
             if (lane == 0) HS[(size_t)blockIdx.x * lds + tok0 + t] = as;
             if (tok0 + t == n - 1) {
                 last.hb[blockIdx.x * 32 + lane] = v;
@@ -337,14 +354,14 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant
             }
 }
 
-// The tile-major matrix as {column of a segment, slot of a group, segment, group}: a box is 128 bytes of quants, or 16 of scales, of one segment in 16 groups =
-// 64 rows.  Behind the segment's last column a box of quants holds scales: blocks that are not multiplied.
-inline int xp_map_weights(XpMaps *maps, const TileMat &W) {
+// The tile-major matrix as {column of a segment, slot of a group, segment, group}: a box is 128 bytes of quants, or 16 of scales, of one segment in `rows`
+// rows.  Behind the segment's last column a box of quants holds scales: blocks that are not multiplied.
+inline int xp_map_weights(XpMaps *maps, const TileMat &W, int rows) {
     pg::EncodeTiledFn fn = pg::encode_fn();
     if (!fn) return -1;
     cuuint64_t dims[4] = {(cuuint64_t)W.unit_bytes, 4, (cuuint64_t)W.nseg, (cuuint64_t)(W.rows / 4)};
     cuuint64_t strides[3] = {(cuuint64_t)W.unit_bytes, (cuuint64_t)W.unit_bytes * 4, (cuuint64_t)W.unit_bytes * 4 * W.nseg};
-    cuuint32_t box[4] = {128, 4, 1, XP_ROWS / 4}, sbox[4] = {16, 4, 1, XP_ROWS / 4}, estr[4] = {1, 1, 1, 1};
+    cuuint32_t box[4] = {128, 4, 1, (cuuint32_t)rows / 4}, sbox[4] = {16, 4, 1, (cuuint32_t)rows / 4}, estr[4] = {1, 1, 1, 1};
     void *base = const_cast<unsigned char *>(W.base);
     const CUresult q = fn(&maps->q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -352,14 +369,14 @@ inline int xp_map_weights(XpMaps *maps, const TileMat &W) {
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return q == CUDA_SUCCESS && s == CUDA_SUCCESS ? 0 : -2;
 }
-// int8 activations [rows][cols] and their scales [blocks][rows]: boxes of 128 columns x the tile's tokens, and of the tile's tokens x 4 blocks
-inline int xp_map_acts(XpMaps *maps, const int8_t *q, const float *s, int rows, int cols, int nt) {
+// activations [rows][cols] (int8: boxes of 128 columns x the tile's tokens; FP16: of 64 columns) and their scales [blocks][rows] (boxes of the tile's tokens x 4 blocks)
+inline int xp_map_acts(XpMaps *maps, const void *q, bool halves, const float *s, int rows, int cols, int nt) {
     pg::EncodeTiledFn fn = pg::encode_fn();
     if (!fn) return -1;
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols}, sdims[2] = {(cuuint64_t)rows, (cuuint64_t)cols / 32}, sstrides[1] = {(cuuint64_t)rows * 4};
-    cuuint32_t box[2] = {128, (cuuint32_t)nt}, sbox[2] = {(cuuint32_t)nt, 4}, estr[2] = {1, 1};
-    const CUresult rq = fn(&maps->q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t *>(q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * (halves ? 2 : 1)}, sdims[2] = {(cuuint64_t)rows, (cuuint64_t)cols / 32}, sstrides[1] = {(cuuint64_t)rows * 4};
+    cuuint32_t box[2] = {halves ? 64u : 128u, (cuuint32_t)nt}, sbox[2] = {(cuuint32_t)nt, 4}, estr[2] = {1, 1};
+    const CUresult rq = fn(&maps->q, halves ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     const CUresult rs = fn(&maps->s, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(s), sdims, sstrides, sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return rq == CUDA_SUCCESS && rs == CUDA_SUCCESS ? 0 : -2;
@@ -424,7 +441,7 @@ __host__ __device__ inline size_t xp_att_smem_bytes(int hs, int qt, int nt, bool
 }
 template <int HS, int QI, int XP_ATT_THREADS>
 __global__ void __launch_bounds__(XP_ATT_THREADS) k_xp_attention(const float *__restrict__ QKV, const float *__restrict__ kc, const float *__restrict__ vc, int n_heads, int n_kv_heads,
-                                                                 int n, int start_pos, float sqrt_hs, int8_t *__restrict__ AQ, float *__restrict__ AS, int lds, float *scratch, XpLast last) {
+                                                                 int n, int start_pos, float sqrt_hs, int8_t *__restrict__ AQ, __half *__restrict__ AH, float *__restrict__ AS, int lds, float *scratch, XpLast last) {
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = HS + 4, QG = XP_ATT_THREADS / 32, QT = QG * QI;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -598,7 +615,8 @@ __global__ void __launch_bounds__(XP_ATT_THREADS) k_xp_attention(const float *__
             const int r = k / (HS / 32), blk = k % (HS / 32);
             float as;
             const int q = quant_block_lane(sq[r * LD + blk * 32 + lane], as);
-            AQ[(size_t)(q0 + r) * qd + h * HS + blk * 32 + lane] = (int8_t)q;
+            if (AH) AH[(size_t)(q0 + r) * qd + h * HS + blk * 32 + lane] = __int2half_rn((int8_t)q);
+            else AQ[(size_t)(q0 + r) * qd + h * HS + blk * 32 + lane] = (int8_t)q;
             if (lane == 0) AS[(size_t)(h * (HS / 32) + blk) * lds + q0 + r] = as;
             if (q0 + r == n - 1) {
                 last.xq[h * HS + blk * 32 + lane] = (int8_t)q;

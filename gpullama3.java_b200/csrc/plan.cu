@@ -7,7 +7,7 @@
 #include "prefill.cuh"
 #include "stream_matvec.cuh"
 #include "stream_matvec_f16.cuh"
-#include "exact_prefill.cuh"
+#include "exact_prefill_umma.cuh"
 #include "kquant.cuh"
 #include "decode_persistent.cuh"
 #include "sampler.cuh"
@@ -137,11 +137,14 @@ struct b200_plan {
         int8_t *AQ = nullptr, *HQ = nullptr;
         float *scratch = nullptr; // score rows of contexts whose rows do not fit shared memory
         size_t scratch_bytes = 0;
+        __half *AH = nullptr, *HH = nullptr; // the quants as FP16 numbers, for the tcgen05 product (exact_prefill_umma.cuh; nullptr: no room)
+        float *G = nullptr;                  // its gate and up rows
         struct Maps { XpMaps qkv, wo, gu, w2; }; // a layer's weights
-        std::vector<Maps> maps;
+        std::vector<Maps> maps, maps_umma;
         XpMaps mA[4], mATT[4], mH[4]; // activations in tiles of 8, 16, 32, 64 tokens: AQ with rows of dim and of the query width, HQ
+        XpMaps hA, hATT, hH;          // the same as FP16, in tiles of 128
         int64_t chunks = 0;           // multiplied at once so far
-        int tile = -1;                // token tile of every product, as an index into {64, 32, 16, 8} (B200_XP_TILE=64|32|16|8; -1: by the model)
+        int tile = -1;                // kernel of every product, as an index into XP_KERNELS (B200_XP_TILE; -1: by the model)
         std::string why;              // rows == 0: why not
     } xp;
     // persistent decode kernel
@@ -1288,10 +1291,22 @@ template <typename F> int xp_by_head_size(int hs, F &&f) { // f(integral_constan
     if (hs == 96) return f(std::integral_constant<int, 96>());
     return f(std::integral_constant<int, 32>());
 }
+// The kernels of a product, and the least time by this model: an SM works its CTAs off at `share` each, but no faster than the chain of one CTA, which the others
+// lengthen a little (both in ns per column block, measured at 1 - 28 CTAs per SM, 36 - 512 tokens, 4B and 8B layers).  A wide tile has the cheaper token, a
+// narrow one the shorter chain and the evener spread: Wo and W2 of the 4B layer at 200 tokens 62.4 us in tiles of 64, 47.5 of 32, 45.9 of 16, 69.7 of 8.
+// The last two are the tcgen05 kernel's, in tiles of 128 tokens and so many rows: its CTAs have an SM to themselves, walk their tiles one after the other and take `fixed` ns
+// to set up and to fill.  8B layer, 512 tokens, tcgen05 and mma.sync, us: QKV 82 and 90, Wo 53 and 63, gate/up 303 + 30 and 388, W2 149 and 218.
+struct XpKernel { int code, tok, rows; float chain, share, fixed; }; // code: B200_XP_TILE
+const XpKernel XP_KERNELS[] = {{64, 64, XP_ROWS, 240.f, 120.f, 0.f}, {32, 32, XP_ROWS, 185.f, 75.f, 0.f}, {16, 16, XP_ROWS, 150.f, 46.f, 0.f}, {8, 8, XP_ROWS, 140.f, 35.f, 0.f},
+                               {12896, XT_TOK, 96, 0.f, 284.f, 6000.f}, {128128, XT_TOK, 128, 0.f, 340.f, 6000.f}};
+const int XP_N_KERNELS = sizeof(XP_KERNELS) / sizeof(XP_KERNELS[0]), XP_UMMA = 4; // the first of the tcgen05 kernels
+const float XP_SWIGLU = 0.0041f; // ns for a hidden unit of a token: k_xt_swiglu, behind the tcgen05 kernel's gate/up product
+
 const size_t XP_SMEM_MAX = 220 * 1024;
 const size_t XP_SCRATCH_MAX = (size_t)256 << 20;
 
 int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide);
+int exact_prefill_umma_alloc(b200_plan *p, int rows, int wide);
 size_t xp_rope_smem_bytes(const b200_config &g) { return (size_t)(g.n_heads + g.n_kv_heads) * (g.head_size + 1) * 4; } // k_xp_rope_kv: a token's query and key heads
 
 // Buffers of one chunk.  Plans off the streaming path (row-major weights) and tensor-parallel ones keep the token-by-token graph, and so do plans that these buffers
@@ -1312,8 +1327,18 @@ int exact_prefill_init(b200_plan *p) {
         p->xp = {};
         p->xp.why = why;
         p->prefill.tok = tok;
+        return B200_OK;
+    }
+    if (chunk < XT_TOK / 2) return B200_OK; // (a tile of 128 tokens would be mostly empty)
+    if ((rc = alloc_optional(p, &done, [&]() -> int { return exact_prefill_umma_alloc(p, rows, wide); }, &why))) return rc;
+    if (!done) {
+        p->xp.AH = nullptr;
+        p->xp.maps_umma.clear();
     }
     return B200_OK;
+}
+bool xp_map_layer(decltype(b200_plan::xp)::Maps *m, const LayerW &L, int rows) {
+    return xp_map_weights(&m->qkv, L.tqkv, rows) == 0 && xp_map_weights(&m->wo, L.two, rows) == 0 && xp_map_weights(&m->gu, L.tgu, rows) == 0 && xp_map_weights(&m->w2, L.tw2, rows) == 0;
 }
 int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide) {
     const b200_config &g = p->cfg;
@@ -1338,51 +1363,85 @@ int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide) {
     }
     bool ok = !refused("tensor_maps");
     for (int i = 0; ok && i < 4; i++)
-        ok = xp_map_acts(&p->xp.mA[i], p->xp.AQ, p->xp.AS, rows, g.dim, 8 << i) == 0 && xp_map_acts(&p->xp.mATT[i], p->xp.AQ, p->xp.AS, rows, p->qd, 8 << i) == 0 &&
-             xp_map_acts(&p->xp.mH[i], p->xp.HQ, p->xp.HS, rows, g.hidden_dim, 8 << i) == 0;
+        ok = xp_map_acts(&p->xp.mA[i], p->xp.AQ, false, p->xp.AS, rows, g.dim, 8 << i) == 0 && xp_map_acts(&p->xp.mATT[i], p->xp.AQ, false, p->xp.AS, rows, p->qd, 8 << i) == 0 &&
+             xp_map_acts(&p->xp.mH[i], p->xp.HQ, false, p->xp.HS, rows, g.hidden_dim, 8 << i) == 0;
     p->xp.maps.resize(g.n_layers);
     for (int l = 0; ok && l < g.n_layers; l++) {
         const LayerW &L = p->layers[l];
         auto &m = p->xp.maps[l];
-        ok = xp_map_weights(&m.qkv, L.tqkv) == 0 && xp_map_weights(&m.wo, L.two) == 0 && xp_map_weights(&m.gu, L.tgu) == 0 && xp_map_weights(&m.w2, L.tw2) == 0;
+        ok = xp_map_layer(&m, L, XP_ROWS);
     }
     if (!ok) return fail(p, B200_ERR_UNSUPPORTED, "the driver does not make the tensor maps");
     if (const char *e = getenv("B200_XP_TILE"))
-        for (int i = 0; i < 4; i++)
-            if (atoi(e) == 64 >> i) p->xp.tile = i;
+        for (int i = 0; i < XP_N_KERNELS; i++)
+            if (atoi(e) == XP_KERNELS[i].code) p->xp.tile = i;
     p->xp.rows = rows;
     return B200_OK;
 }
 
+// What the tcgen05 product reads and writes besides.  Without it every chunk takes the mma.sync product.
+int exact_prefill_umma_alloc(b200_plan *p, int rows, int wide) {
+    const b200_config &g = p->cfg;
+    auto &c = p->xp;
+    int rc;
+    if ((rc = dalloc(p, &c.AH, (size_t)rows * wide * 2))) return rc;
+    if ((rc = dalloc(p, &c.HH, (size_t)rows * g.hidden_dim * 2))) return rc;
+    if ((rc = dalloc(p, &c.G, (size_t)rows * 2 * g.hidden_dim * 4))) return rc;
+    CK(cudaMemset(c.AH, 0, (size_t)rows * wide * 2)); // (as AQ and HQ)
+    CK(cudaMemset(c.HH, 0, (size_t)rows * g.hidden_dim * 2));
+    bool ok = xp_map_acts(&c.hA, c.AH, true, c.AS, rows, g.dim, XT_TOK) == 0 && xp_map_acts(&c.hATT, c.AH, true, c.AS, rows, p->qd, XT_TOK) == 0 &&
+              xp_map_acts(&c.hH, c.HH, true, c.HS, rows, g.hidden_dim, XT_TOK) == 0;
+    c.maps_umma.resize(g.n_layers);
+    for (int l = 0; ok && l < g.n_layers; l++) ok = xp_map_layer(&c.maps_umma[l], p->layers[l], XT_BOX);
+    return ok ? B200_OK : fail(p, B200_ERR_UNSUPPORTED, "the driver does not make the tensor maps of the tcgen05 product");
+}
+
 XpLast xp_last(const b200_plan *p) { return XpLast{p->xq, p->hq, p->xs, p->hs, p->hb}; }
 
+int xp_kernel(const b200_plan *p, const TileMat &W, int n, bool gateup = false) { // the product's kernel, an index into XP_KERNELS
+    if (p->xp.tile >= 0 && (p->xp.tile < XP_UMMA || p->xp.AH)) return p->xp.tile;
+    int best = 0;
+    float least = 0.f;
+    for (int i = 0; i < (p->xp.AH ? XP_N_KERNELS : XP_UMMA); i++) {
+        const XpKernel &k = XP_KERNELS[i];
+        const int ctas = (W.rows + k.rows - 1) / k.rows * ((n + k.tok - 1) / k.tok), per_sm = (ctas + p->n_sms - 1) / p->n_sms;
+        const float t = std::max(per_sm * k.share, k.chain + (per_sm - 1) * k.share / 3.f) * (W.cols / 32) + k.fixed + (gateup && i >= XP_UMMA ? XP_SWIGLU * n * (W.rows / 2) : 0.f);
+        if (i == 0 || t < least) { best = i; least = t; }
+    }
+    return best;
+}
+// MODE XP_GATEUP: hidden units, as bytes to hq or (hh) as FP16 numbers
 template <int MODE>
-int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps (&ma)[4], int n, float *out, int ldo, int8_t *hq, float *hs) {
-    const int mt = (W.rows + XP_ROWS - 1) / XP_ROWS;
+int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps &mw_umma, const XpMaps (&ma)[4], const XpMaps &ma_umma, int n, float *out, int ldo, int8_t *hq, __half *hh, float *hs) {
     auto go = [&](auto nj) -> int {
         constexpr int NJ = decltype(nj)::value;
         auto kern = k_xp_gemm<MODE, NJ>;
         CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<NJ>::BYTES));
-        kern<<<dim3(mt, (n + 8 * NJ - 1) / (8 * NJ)), XP_THREADS, XpTile<NJ>::BYTES, p->stream>>>(mw, ma[NJ == 8 ? 3 : NJ == 4 ? 2 : NJ - 1], W, p->xp.rows, n, out, ldo, hq, hs, xp_last(p), 1.0f, p->d_err);
+        kern<<<dim3((W.rows + XP_ROWS - 1) / XP_ROWS, (n + 8 * NJ - 1) / (8 * NJ)), XP_THREADS, XpTile<NJ>::BYTES, p->stream>>>(mw, ma[NJ == 8 ? 3 : NJ == 4 ? 2 : NJ - 1], W, p->xp.rows, n, out, ldo, hq, hh, hs, xp_last(p), 1.0f, p->d_err);
         CK(cudaGetLastError());
         return B200_OK;
     };
-    // The token tile with the least time by this model: an SM works its CTAs off at `share` each, but no faster than the chain of one CTA, which the others
-    // lengthen a little (both in ns per column block, measured at 1 - 28 CTAs per SM, 36 - 512 tokens, 4B and 8B layers).  A wide tile has the cheaper token, a
-    // narrow one the shorter chain and the evener spread: Wo and W2 of the 4B layer at 200 tokens 62.4 us in tiles of 64, 47.5 of 32, 45.9 of 16, 69.7 of 8.
-    static const struct { int tok; float chain, share; } tiles[4] = {{64, 240.f, 120.f}, {32, 185.f, 75.f}, {16, 150.f, 46.f}, {8, 140.f, 35.f}};
-    int best = 0;
-    float least = 0.f;
-    for (int i = 0; i < 4; i++) {
-        const int ctas = mt * ((n + tiles[i].tok - 1) / tiles[i].tok), per_sm = (ctas + p->n_sms - 1) / p->n_sms;
-        const float t = std::max(per_sm * tiles[i].share, tiles[i].chain + (per_sm - 1) * tiles[i].share / 3.f);
-        if (i == 0 || t < least) { best = i; least = t; }
-    }
-    switch (p->xp.tile >= 0 ? p->xp.tile : best) {
+    auto go_umma = [&](auto rows) -> int { // a CTA per SM
+        constexpr int N = decltype(rows)::value;
+        auto kern = k_xt_gemm<MODE == XP_RESID ? XP_RESID : XP_STORE, N>;
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XtSmem<N>::BYTES));
+        const int tiles = (n + XT_TOK - 1) / XT_TOK * ((W.rows + N - 1) / N);
+        kern<<<std::min(tiles, p->n_sms), XT_THREADS, XtSmem<N>::BYTES, p->stream>>>(mw_umma, ma_umma, W, n, MODE == XP_GATEUP ? p->xp.G : out, MODE == XP_GATEUP ? W.rows : ldo, 1.0f, p->d_err);
+        CK(cudaGetLastError());
+        if (MODE == XP_GATEUP) {
+            const int hidden = W.rows / 2;
+            k_xt_swiglu<<<dim3((hidden / 32 + 15) / 16, n), 256, 0, p->stream>>>(p->xp.G, hidden, n, hq, hh, hs, p->xp.rows, xp_last(p));
+            CK(cudaGetLastError());
+        }
+        return B200_OK;
+    };
+    switch (xp_kernel(p, W, n, MODE == XP_GATEUP)) {
     case 0: return go(std::integral_constant<int, 8>());
     case 1: return go(std::integral_constant<int, 4>());
     case 2: return go(std::integral_constant<int, 2>());
-    default: return go(std::integral_constant<int, 1>());
+    case 3: return go(std::integral_constant<int, 1>());
+    case 4: return go_umma(std::integral_constant<int, 96>());
+    default: return go_umma(std::integral_constant<int, 128>());
     }
 }
 
@@ -1394,16 +1453,17 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     const size_t ctx_kv = (size_t)g.context_length * p->kvd;
     const size_t rope_smem = xp_rope_smem_bytes(g);
     CK(cudaFuncSetAttribute(k_xp_rope_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
-    auto norm = [&](bool embed, const float *w) {
+    auto halves = [&](const TileMat &W, __half *h, bool gateup = false) { return xp_kernel(p, W, n, gateup) >= XP_UMMA ? h : nullptr; }; // what the product of W reads: FP16 quants, or bytes
+    auto norm = [&](bool embed, const float *w, __half *ah) {
         return by_norm_terms(g.dim, [&](auto e_c) -> int {
             constexpr int E = decltype(e_c)::value;
-            if (embed) k_xp_norm<true, E><<<n, 256, 0, p->stream>>>(c.X, p->prefill.tok, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, xp_last(p));
-            else k_xp_norm<false, E><<<n, 256, 0, p->stream>>>(c.X, nullptr, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, c.AS, c.rows, xp_last(p));
+            if (embed) k_xp_norm<true, E><<<n, 256, 0, p->stream>>>(c.X, p->prefill.tok, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, ah, c.AS, c.rows, xp_last(p));
+            else k_xp_norm<false, E><<<n, 256, 0, p->stream>>>(c.X, nullptr, p->emb, w, g.rms_norm_eps, g.dim, c.AQ, ah, c.AS, c.rows, xp_last(p));
             CK(cudaGetLastError());
             return B200_OK;
         });
     };
-    auto attention = [&](float *kc, float *vc) {
+    auto attention = [&](float *kc, float *vc, __half *ah) {
         return xp_by_head_size(g.head_size, [&](auto hs_c) -> int {
             constexpr int HS = decltype(hs_c)::value;
             const int nt = start_pos + n;
@@ -1417,7 +1477,7 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
                     if ((size_t)ctas > slots) ctas = (int)slots;
                 }
                 CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
-                kern<<<ctas, threads, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, c.AS, c.rows, scratch ? c.scratch : nullptr, xp_last(p));
+                kern<<<ctas, threads, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, ah, c.AS, c.rows, scratch ? c.scratch : nullptr, xp_last(p));
                 CK(cudaGetLastError());
                 return B200_OK;
             };
@@ -1429,18 +1489,18 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     };
     for (int l = 0; l < g.n_layers; l++) {
         const LayerW &L = p->layers[l];
-        const auto &m = c.maps[l];
+        const auto &m = c.maps[l], &mu = c.maps_umma.empty() ? m : c.maps_umma[l];
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
         int rc;
-        if ((rc = norm(l == 0, L.attn_norm))) return rc;
-        if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, m.qkv, c.mA, n, c.QKV, nqkv, nullptr, nullptr))) return rc;
+        if ((rc = norm(l == 0, L.attn_norm, halves(L.tqkv, c.AH)))) return rc;
+        if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, m.qkv, mu.qkv, c.mA, c.hA, n, c.QKV, nqkv, nullptr, nullptr, nullptr))) return rc;
         k_xp_rope_kv<<<n, 256, rope_smem, p->stream>>>(c.QKV, kc, vc, g.head_size, g.n_heads, g.n_kv_heads, p->kflags, L.q_norm, L.k_norm, g.rms_norm_eps, p->rope_cr, p->rope_ci, start_pos);
         CK(cudaGetLastError());
-        if ((rc = attention(kc, vc))) return rc;
-        if ((rc = xp_gemm<XP_RESID>(p, L.two, m.wo, c.mATT, n, c.X, g.dim, nullptr, nullptr))) return rc;
-        if ((rc = norm(false, L.ffn_norm))) return rc;
-        if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, m.gu, c.mA, n, nullptr, 0, c.HQ, c.HS))) return rc;
-        if ((rc = xp_gemm<XP_RESID>(p, L.tw2, m.w2, c.mH, n, c.X, g.dim, nullptr, nullptr))) return rc;
+        if ((rc = attention(kc, vc, halves(L.two, c.AH)))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, L.two, m.wo, mu.wo, c.mATT, c.hATT, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
+        if ((rc = norm(false, L.ffn_norm, halves(L.tgu, c.AH, true)))) return rc;
+        if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, m.gu, mu.gu, c.mA, c.hA, n, nullptr, 0, c.HQ, halves(L.tw2, c.HH), c.HS))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, L.tw2, m.w2, mu.w2, c.mH, c.hH, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
     }
     // the single-token buffers hold what the last token's own step would have left there (the others: XpLast)
     CK(cudaMemcpyAsync(p->x, c.X + (size_t)(n - 1) * g.dim, (size_t)g.dim * 4, cudaMemcpyDeviceToDevice, p->stream));
@@ -2238,12 +2298,12 @@ int b200_test_exact_prefill_wait(uint32_t *codes, float *ms) {
         const int8_t *q = reinterpret_cast<const int8_t *>(mem + w_bytes);
         const float *s = reinterpret_cast<const float *>(mem + w_bytes + q_bytes);
         XpMaps mw, ma[2];
-        if (xp_map_weights(&mw, W) || xp_map_acts(&ma[0], q, s, 64, COLS, TOK) || xp_map_acts(&ma[1], q, s, 64, COLS, TOK / 2)) return B200_ERR_UNSUPPORTED;
+        if (xp_map_weights(&mw, W, XP_ROWS) || xp_map_acts(&ma[0], q, false, s, 64, COLS, TOK) || xp_map_acts(&ma[1], q, false, s, 64, COLS, TOK / 2)) return B200_ERR_UNSUPPORTED;
         CK(cudaFuncSetAttribute(k_xp_gemm<XP_STORE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::BYTES));
         for (int i = 0; i < 3; i++) {
             *err = 0u;
             CK(cudaEventRecord(ev[0]));
-            k_xp_gemm<XP_STORE, 2><<<dim3(1, 1), XP_THREADS, XpTile<2>::BYTES>>>(mw, ma[i == 1], W, 64, TOK, reinterpret_cast<float *>(mem + w_bytes + q_bytes + s_bytes), XP_ROWS, nullptr, nullptr,
+            k_xp_gemm<XP_STORE, 2><<<dim3(1, 1), XP_THREADS, XpTile<2>::BYTES>>>(mw, ma[i == 1], W, 64, TOK, reinterpret_cast<float *>(mem + w_bytes + q_bytes + s_bytes), XP_ROWS, nullptr, nullptr, nullptr,
                                                                                 XpLast{}, 1.0f, d_err);
             CK(cudaGetLastError());
             CK(cudaEventRecord(ev[1]));

@@ -1,0 +1,42 @@
+"""The tcgen05 product of the exact Q8_0 prefill (csrc/exact_prefill_umma.cuh): the cache and the logits behind the chunk are the token-by-token path's bit for bit.  Every product of
+the layer in tiles of 128 tokens x 96 or 128 weight rows (B200_XP_TILE): ragged and whole token tiles, row tiles that the rows do not fill, segments that are no multiple of a stage's
+128 columns, more tiles than SMs, and block scales over the whole FP16 range (subnormal, negative, large)."""
+import numpy as np
+import pytest
+
+from test_gpu_exact_prefill import check
+
+pytestmark = pytest.mark.gpu
+CODES = {96: "12896", 128: "128128"}
+
+
+def run(pkg, shape, chunks, scales=None):
+    S, Q8, n = pkg.synth, pkg.gguf.GGMLType.Q8_0, sum(chunks)
+    tensors = S.build_tensors_fast(shape, Q8, seed=n)
+    if scales is not None:
+        for name, (kind, dims, raw) in tensors.items():
+            if len(dims) == 2 and name.startswith("blk."):
+                raw.reshape(-1, 34)[:, :2] = scales(np.random.default_rng(len(name)), raw.size // 34).astype(np.float16).view(np.uint8).reshape(-1, 2)
+    model = pkg.loader.model_from_tensors(shape, Q8, tensors, n + 4)
+    check(pkg, model, np.random.default_rng(n).integers(0, shape.vocab, n + 1), chunks, n)
+
+
+# (dim, hidden, heads, key/value heads, head size): rows of three and of seven segments of 27 and 23 blocks; 96 + 2 * 32 rows and rows of 64 and 96 columns
+@pytest.mark.parametrize("geometry", [(2592, 5152, 8, 2, 128), (64, 96, 3, 1, 32)])
+@pytest.mark.parametrize("rows", [96, 128])
+def test_tiles(pkg, monkeypatch, geometry, rows):
+    dim, hidden, heads, kv, hs = geometry
+    monkeypatch.setenv("B200_XP_TILE", CODES[rows])
+    run(pkg, pkg.synth.Shape("qwen3", dim, hidden, 2, heads, kv, hs, 128, False, 500000.0, 1e-5), [3, 128, 257])
+
+
+@pytest.mark.parametrize("rows", [96, 128])
+def test_several_tiles_per_sm(pkg, monkeypatch, rows):
+    monkeypatch.setenv("B200_XP_TILE", CODES[rows])
+    run(pkg, pkg.synth.SHAPES["mid-llama"], [129, 300])
+
+
+@pytest.mark.parametrize("rows", [96, 128])
+def test_scales(pkg, monkeypatch, rows):
+    monkeypatch.setenv("B200_XP_TILE", CODES[rows])
+    run(pkg, pkg.synth.SHAPES["tiny-llama"], [130], lambda rng, n: np.ldexp(rng.choice([-1.0, 1.0], n) * rng.uniform(1.0, 2.0, n), rng.integers(-26, -2, n)))
