@@ -5,7 +5,7 @@
 // there token i only reads the cache rows that the earlier tokens of the same layer have written.  Per layer:
 //
 //   AQ <- Q8_0(rmsnorm(X) * w)                 k_xp_norm       a CTA per token
-//   QKV <- AQ [Wq;Wk;Wv]^T                     k_xp_gemm<XP_STORE>
+//   QKV <- AQ [Wq;Wk;Wv]^T                     k_xp_gemm<XP_STORE>, or k_xt_gemm (exact_prefill_umma.cuh)
 //   q, k <- (Qwen3 head norm,) rotation; k, v -> cache     k_xp_rope_kv
 //   AQ <- Q8_0(softmax(q k^T / sqrt(hs)) v)    k_xp_attention  a CTA per (64, 32 or 8 tokens, head)
 //   X += AQ Wo^T                               k_xp_gemm<XP_RESID>
@@ -13,8 +13,8 @@
 //   HQ <- Q8_0(silu(AQ W1^T) * (AQ W3^T))      k_xp_gemm<XP_GATEUP>
 //   X += HQ W2^T                               k_xp_gemm<XP_RESID>
 //
-// Measured on two layers of the 8B geometry, 512 tokens and the decode step behind them: 109.8 ms token by token, 2.25 ms here; two layers of the 4B
-// Qwen3 geometry, 36 tokens: 5.36 ms and 0.52 ms.
+// Measured on two layers of the 8B geometry, 512 tokens and the decode step behind them: 109.8 ms token by token, 1.98 ms here; two layers of the 4B
+// Qwen3 geometry, 36 tokens: 5.36 ms and 0.47 ms.
 #pragma once
 #include "prefill_gemm.cuh"
 #include "stream_matvec.cuh"
@@ -71,7 +71,7 @@ struct XpLast {
 };
 struct XpSync { __device__ __forceinline__ void operator()() const { __syncthreads(); } };
 template <bool EMBED, int E>
-__global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const int *__restrict__ tok, DevMat emb, const float *__restrict__ w, float eps, int dim,
+__global__ void __launch_bounds__(256, E <= 16 ? 4 : 1) k_xp_norm(float *__restrict__ X, const int *__restrict__ tok, DevMat emb, const float *__restrict__ w, float eps, int dim,
                                                  int8_t *__restrict__ AQ, __half *__restrict__ AH, float *__restrict__ AS, int lds, XpLast out1) {
     __shared__ __align__(16) float sq[256 * E];
     __shared__ SeqSum3Scratch scratch;
@@ -113,20 +113,36 @@ __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const in
     if (!live) return;
     const float qs = __fdiv_rn(amax, 127.0f), as = __half2float(__float2half_rn(qs)), ainv = qs != 0.0f ? __fdiv_rn(1.0f, qs) : 0.0f; // quant_block_lane's arithmetic
     const bool last = b == (int)gridDim.x - 1;
+    unsigned q[E / 4];
 #pragma unroll
     for (int k = 0; k < E; k += 4) {
-        unsigned p = 0;
+        int u[4];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const float s = __fmul_rn(v[k + u], ainv);
-            p |= ((unsigned)__float2int_rz(__fadd_rn(s, copysignf(0.5f, s))) & 0xffu) << (8 * u);
+        for (int j = 0; j < 4; j++) {
+            const float s = __fmul_rn(v[k + j], ainv);
+            u[j] = __float2int_rz(__fadd_rn(s, copysignf(0.5f, s)));
         }
-        if (AH) {
-            uint2 h;
-            xp_halves(p, h.x, h.y);
-            *reinterpret_cast<uint2 *>(AH + (size_t)b * dim + base + k) = h;
-        } else *reinterpret_cast<unsigned *>(AQ + (size_t)b * dim + base + k) = p;
-        if (last) *reinterpret_cast<unsigned *>(out1.xq + base + k) = p;
+        q[k / 4] = xp_bytes(u);
+        if (last) *reinterpret_cast<unsigned *>(out1.xq + base + k) = q[k / 4];
+    }
+    if (AH) {
+#pragma unroll
+        for (int k = 0; k < E; k += E >= 8 ? 8 : 4) {
+            uint4 h;
+            xp_halves(q[k / 4], h.x, h.y);
+            if (E >= 8) {
+                xp_halves(q[E >= 8 ? k / 4 + 1 : 0], h.z, h.w);
+                *reinterpret_cast<uint4 *>(AH + (size_t)b * dim + base + k) = h;
+            } else *reinterpret_cast<uint2 *>(AH + (size_t)b * dim + base + k) = make_uint2(h.x, h.y);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < E; k += E >= 16 ? 16 : E) {
+            int8_t *dst = AQ + (size_t)b * dim + base + k;
+            if (E >= 16) *reinterpret_cast<uint4 *>(dst) = make_uint4(q[k / 4], q[E >= 16 ? k / 4 + 1 : 0], q[E >= 16 ? k / 4 + 2 : 0], q[E >= 16 ? k / 4 + 3 : 0]);
+            else if (E >= 8) *reinterpret_cast<uint2 *>(dst) = make_uint2(q[0], q[E >= 8 ? 1 : 0]);
+            else *reinterpret_cast<unsigned *>(dst) = q[0];
+        }
     }
     if (tid % TPB == 0) {
         AS[(size_t)(base / 32) * lds + b] = as;
@@ -140,22 +156,24 @@ __global__ void __launch_bounds__(256) k_xp_norm(float *__restrict__ X, const in
 // products and an ordered add, and those run on the CUDA cores, two values at a time (f32x2).  The ordered add is fma(acc, 1, term), which rounds like the
 // add: a packed add behind a packed product comes out as ONE fused operation (measured; also where the 1 is a constant of the kernel, so it is an argument).
 // Integers are converted by the conversion instruction: accumulators that start at 0x4B400000 and a subtraction cost four register moves for every mma (gate/up
-// product 411 against 392 us).  Gate/up of 512 tokens, 8B layer: 560 us with scalar adds and cp.async fetches by all threads, 392 us so (FMA pipe 50 %, issue slots
-// 64 %; 19 warp instructions per 16 x 8 tile and block, 10 of them the conversions, products and adds); Wo + W2 341 -> 281 us, QKV 121 -> 90 us.
-// tcgen05.mma.kind::i8 does not pay here: a sum is read back after every 32 columns, so each block costs a round trip product - barrier - tcgen05.ld - barrier; with 2 to
-// 4 accumulator buffers, a warp each for loads and products and up to 24 warps on the sums it took 410 us (32-token tiles) to 494 us.
-// A CTA is 4 warps: 64 weight rows (16 groups of the tile-major layout) x 8 * NJ tokens; with 32 tokens and more a warp owns 32 rows and half of the tokens
-// (every B fragment and activation scale serves two row tiles), else 16 rows and all of them.  Three stages of 128 columns come in by TMA (thread 0 issues: weights and
-// their scales straight out of the tile-major layout by a 4-D map), rows of 128 bytes swizzled so that ldmatrix is conflict-free.
-#define XP_STAGES 3
+// product 411 against 392 us).
+// A CTA is 4 warps that multiply: 64 weight rows (16 groups of the tile-major layout) x 8 * NJ tokens; with 32 tokens and more a warp owns 32 rows and half of the tokens
+// (every B fragment and activation scale serves two row tiles), else 16 rows and all of them; and one that fetches: a ring of stages of 128 columns comes in by TMA (weights and
+// their scales straight out of the tile-major layout by a 4-D map), rows of 128 bytes swizzled so that ldmatrix is conflict-free.  A multiplying warp that waited for the others and
+// issued the fetches between its chunks held the whole CTA up by half of its time: gate/up of 512 tokens, 8B layer, 388 us against 328 us so; W2 of 36 tokens, 4B layer, 43 against 28 us (a
+// deeper ring alone 43, all operands of a chunk in registers ahead 46).  Issue slots: 19 warp instructions per 16 x 8 tile and block, 10 of them the conversions, products and adds.
+// Long chunks' QKV, Wo and W2 are exact_prefill_umma.cuh's.
+#define XP_STAGES 3      // of a ring, at least;
+#define XP_STAGES_MAX 8  // and at most: as many as the CTAs of an SM have room for
 #define XP_ROWS 64
-#define XP_THREADS 128
+#define XP_THREADS 128 // that multiply; a fifth warp fetches
 struct XpMaps { CUtensorMap q, s; }; // quants; scales
 template <int NJ> struct XpTile {
     static constexpr int TOK = 8 * NJ;
     static constexpr int A_Q = 0, B_Q = XP_ROWS * 128, A_S = B_Q + TOK * 128, B_S = A_S + XP_ROWS * 16, BYTES_IN = B_S + 4 * TOK * 4, STAGE = (BYTES_IN + 1023) & ~1023;
     static constexpr int HV = 33 * TOK * 4; // gate/up: the tile's 32 hidden units (+ 1: no bank conflicts) per token
-    static constexpr int BYTES = 1024 + XP_STAGES * STAGE + 16 * XP_STAGES;
+    static constexpr int RESIDENT = NJ == 8 ? 3 : 4; // CTAs of an SM (registers)
+    static constexpr int bytes(int stages) { return 1024 + stages * STAGE + 16 * stages; }
 };
 // Bounded: false = given up, after a second or once a wait has given up anywhere (the host's error word).  The clock is looked at every 256th time: read every time it
 // cost a prompt of 512 tokens 26 of 2226 us.
@@ -192,34 +210,44 @@ __device__ __forceinline__ xp_f2 xp_lds64(unsigned a) {
 }
 
 template <int MODE, int NJ>
-__global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant__ XpMaps map_w, const __grid_constant__ XpMaps map_a, TileMat W, int lds, int n, float *__restrict__ out, int ldo,
-                                                        int8_t *__restrict__ HQ, __half *__restrict__ HH, float *__restrict__ HS, XpLast last, float one_f, unsigned *err) {
+__global__ void __launch_bounds__(XP_THREADS + 32, XpTile<NJ>::RESIDENT) k_xp_gemm(const __grid_constant__ XpMaps map_w, const __grid_constant__ XpMaps map_a, TileMat W, int lds, int n, float *__restrict__ out, int ldo,
+                                                        int8_t *__restrict__ HQ, __half *__restrict__ HH, float *__restrict__ HS, XpLast last, float one_f, int stages, unsigned *err) {
     using T = XpTile<NJ>;
     static_assert(T::HV <= XP_STAGES * T::STAGE, "the gate/up epilogue's rows take the ring's place");
     constexpr int TOK = T::TOK, MI = NJ >= 4 ? 2 : 1, NW = NJ / MI; // a warp's tile: 16 MI rows x 8 NW tokens
     extern __shared__ unsigned char smraw[];
     unsigned char *const ring = reinterpret_cast<unsigned char *>(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023); // (the swizzle is by address)
-    const unsigned smb = smem_u32(ring), full0 = smb + XP_STAGES * T::STAGE, empty0 = full0 + 8 * XP_STAGES;
+    const unsigned smb = smem_u32(ring), full0 = smb + stages * T::STAGE, empty0 = full0 + 8 * stages;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int row0 = blockIdx.x * XP_ROWS, tok0 = blockIdx.y * TOK;
     const int nbs = W.seg >> 5, cps = (nbs + 3) >> 2, n_chunks = W.nseg * cps; // blocks per segment, chunks of <= 4 blocks per segment
-    int f_seg = 0, f_c = 0, f_stage = 0; // (thread 0) the next chunk to fetch
-    auto fetch = [&]() {
-        const unsigned s = smb + f_stage * T::STAGE, bar = full0 + 8 * f_stage;
-        mbar_expect_tx(bar, T::BYTES_IN);
-        xp_load4(s + T::A_Q, &map_w.q, 128 * f_c, f_seg, row0 >> 2, bar);
-        pg::tma_load_2d(s + T::B_Q, &map_a.q, f_seg * W.seg + 128 * f_c, tok0, bar);
-        xp_load4(s + T::A_S, &map_w.s, W.seg + ((8 * f_c) & ~15), f_seg, row0 >> 2, bar); // 8 scales of a row, 16 bytes
-        pg::tma_load_2d(s + T::B_S, &map_a.s, tok0, f_seg * nbs + 4 * f_c, bar);
-        if (++f_c == cps) { f_c = 0; f_seg++; }
-        if (++f_stage == XP_STAGES) f_stage = 0;
-    };
     if (tid == 0) {
-        for (int s = 0; s < XP_STAGES; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, XP_THREADS / 32); }
+        for (int s = 0; s < stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, XP_THREADS / 32); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int s = 0; s < XP_STAGES && s < n_chunks; s++) fetch();
     }
     __syncthreads();
+    if (warp == XP_THREADS / 32) { // ---- fetches, by a warp of their own: one of the others that waited for the rest and issued them held the whole CTA up
+        if (lane == 0) {
+            int c = 0, stage = 0;
+            unsigned ph = 1; // (a fresh stage is empty: the wait for the phase before the first one returns at once)
+            bool ok = true;
+            for (int seg = 0; ok && seg < W.nseg; seg++)
+                for (int cs = 0; cs < cps; cs++, c++) {
+                    if (!(ok = xp_wait(empty0 + 8 * stage, ph, err))) break;
+                    const unsigned s = smb + stage * T::STAGE, bar = full0 + 8 * stage;
+                    mbar_expect_tx(bar, T::BYTES_IN);
+                    xp_load4(s + T::A_Q, &map_w.q, 128 * cs, seg, row0 >> 2, bar);
+                    pg::tma_load_2d(s + T::B_Q, &map_a.q, seg * W.seg + 128 * cs, tok0, bar);
+                    xp_load4(s + T::A_S, &map_w.s, W.seg + ((8 * cs) & ~15), seg, row0 >> 2, bar); // 8 scales of a row, 16 bytes
+                    pg::tma_load_2d(s + T::B_S, &map_a.s, tok0, seg * nbs + 4 * cs, bar);
+                    if (++stage == stages) { stage = 0; ph ^= 1u; }
+                }
+            if (!ok) // (a wait gave up: nothing leaves with its copies in flight)
+                for (int q = max(0, c - stages); q < c; q++) xp_wait(full0 + 8 * (q % stages), (q / stages) & 1, err);
+        }
+        if (MODE == XP_GATEUP) { __syncthreads(); __syncthreads(); } // (the epilogue's)
+        return;
+    }
 
     xp_f2 acc[MI][NW][2]; // [row tile][token tile][row lane/4 | row lane/4 + 8], tokens 2 (lane % 4), + 1
 #pragma unroll
@@ -231,11 +259,11 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant
     const int ar = wrow + (lane & 15), ap = lane >> 4;                              // ldmatrix: A row, 16-byte half
     const int bt = wtok + (NW > 1 ? ((lane >> 4) << 3) + (lane & 7) : (lane & 7)), bp = (lane >> 3) & 1; // B token (of 16), half
     const unsigned a_base = T::A_Q + ar * 128, b_base = T::B_Q + bt * 128, as_base = T::B_S + (wtok + 2 * (lane & 3)) * 4, ws_base = T::A_S + (wrow + (lane >> 2)) * 16;
-    int stage = 0, c_in_seg = 0, c = 0;
+    int stage = 0, c_in_seg = 0;
     unsigned ph = 0;
-    bool ok = true, dead = false; // dead (thread 0): a stage did not come free, nothing is fetched any more
-    for (; c < n_chunks; c++) {
-        if (!(ok = __all_sync(0xffffffffu, !dead && xp_wait(full0 + 8 * stage, ph, err)))) break;
+    bool ok = true;
+    for (int c = 0; c < n_chunks; c++) {
+        if (!(ok = __all_sync(0xffffffffu, xp_wait(full0 + 8 * stage, ph, err)))) break;
         const unsigned s = smb + stage * T::STAGE;
         __half2 ws[MI][2][2]; // scales of blocks {0, 1}, {2, 3}
 #pragma unroll
@@ -291,17 +319,10 @@ __global__ void __launch_bounds__(XP_THREADS, 4) k_xp_gemm(const __grid_constant
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(empty0 + 8 * stage);
-        if (tid == 0 && c + XP_STAGES < n_chunks) { // the stage goes to the chunk after the next two, once every warp is done with it
-            dead = !xp_wait(empty0 + 8 * stage, ph, err);
-            if (!dead) fetch();
-        }
-        if (++stage == XP_STAGES) { stage = 0; ph ^= 1u; }
+        if (++stage == stages) { stage = 0; ph ^= 1u; }
         if (++c_in_seg == cps) c_in_seg = 0;
     }
-    if (!ok && lane == 0) { // (a wait gave up: the host is told, and nothing leaves with its copies in flight)
-        *reinterpret_cast<volatile unsigned *>(err) = 200u;
-        for (int q = c; q < n_chunks && q < c + XP_STAGES; q++) xp_wait(full0 + 8 * (q % XP_STAGES), (q / XP_STAGES) & 1, err);
-    }
+    if (!ok && lane == 0) *reinterpret_cast<volatile unsigned *>(err) = 200u; // (a wait gave up: the host is told)
 
     const int r0 = wrow + (lane >> 2), t0 = wtok + 2 * (lane & 3);
     if (MODE == XP_GATEUP) { // rows of a group: gate 2G, gate 2G + 1, up 2G, up 2G + 1; the CTA's 64 rows are one 32-unit block of the hidden row

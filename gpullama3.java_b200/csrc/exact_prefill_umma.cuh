@@ -8,8 +8,8 @@
 // the tensor cores are on the next.
 //
 // Bound by: the sums.  Two warps a scheduler; a step of 16 columns (two tcgen05.ld, a wait, 8 packed products and 8 packed adds) takes 95 cycles and a block about 220 besides, in
-// which its barrier is waited for and handed back: 600 cycles for N = 128 (FMA pipe 50 %, tensor pipe 32 %).  Measured for the gate/up product of 512 tokens, 8B layer: 303 us (388 us with
-// mma.sync, k_xp_gemm, which converts, multiplies twice and adds).  Without effect (all 296 - 360 us): 12 and 16 warps of 32 columns, 8 or 32 columns a step, the next step's columns loaded ahead, all
+// which its barrier is waited for and handed back: 600 cycles for N = 128 (FMA pipe 50 %, tensor pipe 32 %).  Measured, 512 tokens, 8B layer: W2 149 us, Wo 53, QKV 82 gate/up 303 (185, 60, 86 and 328 us with mma.sync,
+// k_xp_gemm, which converts, multiplies twice and adds).  Without effect (gate/up 296 - 360 us): 12 and 16 warps of 32 columns, 8 or 32 columns a step, the next step's columns loaded ahead, all
 // columns loaded at once (setmaxnreg), neither conversion nor scale products; kind::i8 and a conversion in the sums 335 us; one warp that did not walk together for the products 434 us.
 //
 // Warps: 0-7 sums (warp w: lanes 32 (w % 4) .., columns (w / 4) N / 2 ..), 8-11 turn a stage's bytes into FP16 operands (thread = weight row) and its scales into S's operands
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_xt_gemm(const __grid_constant
 
 // ---- hidden units behind the gate/up product: Q8_0(silu(gate) * up), FP16 quants (or bytes) and scales -------------------------------
 // A warp takes two blocks of 32 units of a token, a lane two units: G's columns come in groups gate 2g, gate 2g + 1, up 2g, up 2g + 1.  A launch of its own because the double
-// precision of the activation would stand between the tiles of the product: 360 us in its epilogue against 296 + 31 us, 512 tokens, 8B layer.
+// precision of the activation would stand between the tiles of the product: 360 us in its epilogue against 303 + 30 us, 512 tokens, 8B layer.
 __global__ void __launch_bounds__(256) k_xt_swiglu(const float *__restrict__ G, int hidden, int n, int8_t *__restrict__ HQ, __half *__restrict__ HH, float *__restrict__ HS, int lds, XpLast last) {
     const int lane = threadIdx.x & 31, pair = blockIdx.x * 8 + (threadIdx.x >> 5), t = blockIdx.y, unit = pair * 64 + 2 * lane;
     if (pair * 64 >= hidden) return;

@@ -138,7 +138,7 @@ struct b200_plan {
         float *scratch = nullptr; // score rows of contexts whose rows do not fit shared memory
         size_t scratch_bytes = 0;
         __half *AH = nullptr, *HH = nullptr; // the quants as FP16 numbers, for the tcgen05 product (exact_prefill_umma.cuh; nullptr: no room)
-        float *G = nullptr;                  // its gate and up rows
+        float *G = nullptr;                  // the gate and up rows of chunks whose SwiGLU is a launch of its own
         struct Maps { XpMaps qkv, wo, gu, w2; }; // a layer's weights
         std::vector<Maps> maps, maps_umma;
         XpMaps mA[4], mATT[4], mH[4]; // activations in tiles of 8, 16, 32, 64 tokens: AQ with rows of dim and of the query width, HQ
@@ -1292,15 +1292,18 @@ template <typename F> int xp_by_head_size(int hs, F &&f) { // f(integral_constan
     return f(std::integral_constant<int, 32>());
 }
 // The kernels of a product, and the least time by this model: an SM works its CTAs off at `share` each, but no faster than the chain of one CTA, which the others
-// lengthen a little (both in ns per column block, measured at 1 - 28 CTAs per SM, 36 - 512 tokens, 4B and 8B layers).  A wide tile has the cheaper token, a
-// narrow one the shorter chain and the evener spread: Wo and W2 of the 4B layer at 200 tokens 62.4 us in tiles of 64, 47.5 of 32, 45.9 of 16, 69.7 of 8.
+// lengthen a little (both in ns per column block, measured at 1 - 49 CTAs per SM, 36 - 512 tokens, 4B and 8B layers).  A wide tile has the cheaper token, a
+// narrow one the shorter chain and the evener spread: W2 of the 4B layer at 36 tokens 48 us in tiles of 64, 35 of 32, 28 of 16 and of 8; gate/up of the 8B layer at 512 tokens 328, 358, 504
+// and 884 us.
 // The last two are the tcgen05 kernel's, in tiles of 128 tokens and so many rows: its CTAs have an SM to themselves, walk their tiles one after the other and take `fixed` ns
-// to set up and to fill.  8B layer, 512 tokens, tcgen05 and mma.sync, us: QKV 82 and 90, Wo 53 and 63, gate/up 303 + 30 and 388, W2 149 and 218.
+// to set up and to fill.  8B layer, 512 tokens, tcgen05 and the best of the others, us: QKV 82 and 86, Wo 53 and 60, gate/up 303 and 328, W2 149 and 185.
 struct XpKernel { int code, tok, rows; float chain, share, fixed; }; // code: B200_XP_TILE
-const XpKernel XP_KERNELS[] = {{64, 64, XP_ROWS, 240.f, 120.f, 0.f}, {32, 32, XP_ROWS, 185.f, 75.f, 0.f}, {16, 16, XP_ROWS, 150.f, 46.f, 0.f}, {8, 8, XP_ROWS, 140.f, 35.f, 0.f},
+const XpKernel XP_KERNELS[] = {{64, 64, XP_ROWS, 158.f, 103.f, 0.f}, {32, 32, XP_ROWS, 115.f, 58.f, 0.f}, {16, 16, XP_ROWS, 91.f, 40.f, 0.f}, {8, 8, XP_ROWS, 91.f, 34.f, 0.f},
                                {12896, XT_TOK, 96, 0.f, 284.f, 6000.f}, {128128, XT_TOK, 128, 0.f, 340.f, 6000.f}};
+// From so many tokens on SwiGLU is a launch behind the gate/up product: in double precision in the product's epilogue it holds up the CTAs that multiply (8B layer, 512 tokens 384 -> 333 us,
+// then on tcgen05; whole prompts of 129 - 513 tokens 0 - 3 % shorter, of 37 - 97 the same).
+const int XP_SPLIT_TOKENS = 128;
 const int XP_N_KERNELS = sizeof(XP_KERNELS) / sizeof(XP_KERNELS[0]), XP_UMMA = 4; // the first of the tcgen05 kernels
-const float XP_SWIGLU = 0.0041f; // ns for a hidden unit of a token: k_xt_swiglu, behind the tcgen05 kernel's gate/up product
 
 const size_t XP_SMEM_MAX = 220 * 1024;
 const size_t XP_SCRATCH_MAX = (size_t)256 << 20;
@@ -1398,44 +1401,59 @@ int exact_prefill_umma_alloc(b200_plan *p, int rows, int wide) {
 
 XpLast xp_last(const b200_plan *p) { return XpLast{p->xq, p->hq, p->xs, p->hs, p->hb}; }
 
-int xp_kernel(const b200_plan *p, const TileMat &W, int n, bool gateup = false) { // the product's kernel, an index into XP_KERNELS
-    if (p->xp.tile >= 0 && (p->xp.tile < XP_UMMA || p->xp.AH)) return p->xp.tile;
+int xp_kernel(const b200_plan *p, const TileMat &W, int n) { // the product's kernel, an index into XP_KERNELS
+    const int kernels = p->xp.AH ? XP_N_KERNELS : XP_UMMA;
+    if (p->xp.tile >= 0 && p->xp.tile < kernels) return p->xp.tile;
     int best = 0;
     float least = 0.f;
-    for (int i = 0; i < (p->xp.AH ? XP_N_KERNELS : XP_UMMA); i++) {
+    for (int i = 0; i < kernels; i++) {
         const XpKernel &k = XP_KERNELS[i];
         const int ctas = (W.rows + k.rows - 1) / k.rows * ((n + k.tok - 1) / k.tok), per_sm = (ctas + p->n_sms - 1) / p->n_sms;
-        const float t = std::max(per_sm * k.share, k.chain + (per_sm - 1) * k.share / 3.f) * (W.cols / 32) + k.fixed + (gateup && i >= XP_UMMA ? XP_SWIGLU * n * (W.rows / 2) : 0.f);
+        const float t = std::max(per_sm * k.share, k.chain + (per_sm - 1) * k.share / 3.f) * (W.cols / 32) + k.fixed;
         if (i == 0 || t < least) { best = i; least = t; }
     }
     return best;
 }
-// MODE XP_GATEUP: hidden units, as bytes to hq or (hh) as FP16 numbers
+// out (MODE XP_STORE) or out += the product (XP_RESID); XP_GATEUP: hidden units, as bytes to hq or (hh) as FP16 numbers
 template <int MODE>
 int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps &mw_umma, const XpMaps (&ma)[4], const XpMaps &ma_umma, int n, float *out, int ldo, int8_t *hq, __half *hh, float *hs) {
+    const int kernel = xp_kernel(p, W, n);
+    if constexpr (MODE == XP_GATEUP)
+        if (kernel >= XP_UMMA || (p->xp.G && n >= XP_SPLIT_TOKENS)) { // SwiGLU in a launch of its own
+            const int hidden = W.rows / 2;
+            int rc = xp_gemm<XP_STORE>(p, W, mw, mw_umma, ma, ma_umma, n, p->xp.G, W.rows, nullptr, nullptr, nullptr);
+            if (rc) return rc;
+            k_xt_swiglu<<<dim3((hidden / 32 + 15) / 16, n), 256, 0, p->stream>>>(p->xp.G, hidden, n, hq, hh, hs, p->xp.rows, xp_last(p));
+            CK(cudaGetLastError());
+            return B200_OK;
+        }
     auto go = [&](auto nj) -> int {
         constexpr int NJ = decltype(nj)::value;
+        using T = XpTile<NJ>;
         auto kern = k_xp_gemm<MODE, NJ>;
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<NJ>::BYTES));
-        kern<<<dim3((W.rows + XP_ROWS - 1) / XP_ROWS, (n + 8 * NJ - 1) / (8 * NJ)), XP_THREADS, XpTile<NJ>::BYTES, p->stream>>>(mw, ma[NJ == 8 ? 3 : NJ == 4 ? 2 : NJ - 1], W, p->xp.rows, n, out, ldo, hq, hh, hs, xp_last(p), 1.0f, p->d_err);
+        const dim3 grid((W.rows + XP_ROWS - 1) / XP_ROWS, (n + 8 * NJ - 1) / (8 * NJ));
+        // the CTAs that an SM has at a time share its memory: few of them have deep rings (a chunk's fetch takes about as long as three chunks of a narrow tile; W2 of the 4B
+        // layer, 36 tokens: 33.7 us with three stages, 27.6 with five)
+        const int per_sm = std::min(((int)(grid.x * grid.y) + p->n_sms - 1) / p->n_sms, T::RESIDENT);
+        const int stages = std::max(XP_STAGES, std::min(XP_STAGES_MAX, ((int)XP_SMEM_MAX / per_sm - 2048) / (T::STAGE + 16)));
+        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::bytes(stages)));
+        kern<<<grid, XP_THREADS + 32, T::bytes(stages), p->stream>>>(mw, ma[NJ == 8 ? 3 : NJ == 4 ? 2 : NJ - 1], W, p->xp.rows, n, out, ldo, hq, hh, hs, xp_last(p), 1.0f, stages, p->d_err);
         CK(cudaGetLastError());
         return B200_OK;
     };
     auto go_umma = [&](auto rows) -> int { // a CTA per SM
-        constexpr int N = decltype(rows)::value;
-        auto kern = k_xt_gemm<MODE == XP_RESID ? XP_RESID : XP_STORE, N>;
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XtSmem<N>::BYTES));
-        const int tiles = (n + XT_TOK - 1) / XT_TOK * ((W.rows + N - 1) / N);
-        kern<<<std::min(tiles, p->n_sms), XT_THREADS, XtSmem<N>::BYTES, p->stream>>>(mw_umma, ma_umma, W, n, MODE == XP_GATEUP ? p->xp.G : out, MODE == XP_GATEUP ? W.rows : ldo, 1.0f, p->d_err);
-        CK(cudaGetLastError());
-        if (MODE == XP_GATEUP) {
-            const int hidden = W.rows / 2;
-            k_xt_swiglu<<<dim3((hidden / 32 + 15) / 16, n), 256, 0, p->stream>>>(p->xp.G, hidden, n, hq, hh, hs, p->xp.rows, xp_last(p));
+        if constexpr (MODE == XP_GATEUP) return fail(p, B200_ERR_UNSUPPORTED, "the tcgen05 product has no gate/up form");
+        else {
+            constexpr int N = decltype(rows)::value;
+            auto kern = k_xt_gemm<MODE, N>;
+            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XtSmem<N>::BYTES));
+            const int tiles = (n + XT_TOK - 1) / XT_TOK * ((W.rows + N - 1) / N);
+            kern<<<std::min(tiles, p->n_sms), XT_THREADS, XtSmem<N>::BYTES, p->stream>>>(mw_umma, ma_umma, W, n, out, ldo, 1.0f, p->d_err);
             CK(cudaGetLastError());
+            return B200_OK;
         }
-        return B200_OK;
     };
-    switch (xp_kernel(p, W, n, MODE == XP_GATEUP)) {
+    switch (kernel) {
     case 0: return go(std::integral_constant<int, 8>());
     case 1: return go(std::integral_constant<int, 4>());
     case 2: return go(std::integral_constant<int, 2>());
@@ -1453,7 +1471,7 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     const size_t ctx_kv = (size_t)g.context_length * p->kvd;
     const size_t rope_smem = xp_rope_smem_bytes(g);
     CK(cudaFuncSetAttribute(k_xp_rope_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
-    auto halves = [&](const TileMat &W, __half *h, bool gateup = false) { return xp_kernel(p, W, n, gateup) >= XP_UMMA ? h : nullptr; }; // what the product of W reads: FP16 quants, or bytes
+    auto halves = [&](const TileMat &W, __half *h) { return xp_kernel(p, W, n) >= XP_UMMA ? h : nullptr; }; // what the product of W reads: FP16 quants, or bytes
     auto norm = [&](bool embed, const float *w, __half *ah) {
         return by_norm_terms(g.dim, [&](auto e_c) -> int {
             constexpr int E = decltype(e_c)::value;
@@ -1498,7 +1516,7 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
         CK(cudaGetLastError());
         if ((rc = attention(kc, vc, halves(L.two, c.AH)))) return rc;
         if ((rc = xp_gemm<XP_RESID>(p, L.two, m.wo, mu.wo, c.mATT, c.hATT, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
-        if ((rc = norm(false, L.ffn_norm, halves(L.tgu, c.AH, true)))) return rc;
+        if ((rc = norm(false, L.ffn_norm, halves(L.tgu, c.AH)))) return rc;
         if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, m.gu, mu.gu, c.mA, c.hA, n, nullptr, 0, c.HQ, halves(L.tw2, c.HH), c.HS))) return rc;
         if ((rc = xp_gemm<XP_RESID>(p, L.tw2, m.w2, mu.w2, c.mH, c.hH, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
     }
@@ -2299,12 +2317,12 @@ int b200_test_exact_prefill_wait(uint32_t *codes, float *ms) {
         const float *s = reinterpret_cast<const float *>(mem + w_bytes + q_bytes);
         XpMaps mw, ma[2];
         if (xp_map_weights(&mw, W, XP_ROWS) || xp_map_acts(&ma[0], q, false, s, 64, COLS, TOK) || xp_map_acts(&ma[1], q, false, s, 64, COLS, TOK / 2)) return B200_ERR_UNSUPPORTED;
-        CK(cudaFuncSetAttribute(k_xp_gemm<XP_STORE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::BYTES));
+        CK(cudaFuncSetAttribute(k_xp_gemm<XP_STORE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::bytes(XP_STAGES)));
         for (int i = 0; i < 3; i++) {
             *err = 0u;
             CK(cudaEventRecord(ev[0]));
-            k_xp_gemm<XP_STORE, 2><<<dim3(1, 1), XP_THREADS, XpTile<2>::BYTES>>>(mw, ma[i == 1], W, 64, TOK, reinterpret_cast<float *>(mem + w_bytes + q_bytes + s_bytes), XP_ROWS, nullptr, nullptr, nullptr,
-                                                                                XpLast{}, 1.0f, d_err);
+            k_xp_gemm<XP_STORE, 2><<<dim3(1, 1), XP_THREADS + 32, XpTile<2>::bytes(XP_STAGES)>>>(mw, ma[i == 1], W, 64, TOK, reinterpret_cast<float *>(mem + w_bytes + q_bytes + s_bytes), XP_ROWS, nullptr, nullptr, nullptr,
+                                                                                XpLast{}, 1.0f, XP_STAGES, d_err);
             CK(cudaGetLastError());
             CK(cudaEventRecord(ev[1]));
             CK(cudaDeviceSynchronize());
