@@ -401,6 +401,8 @@ __global__ void k_swiglu(float *__restrict__ hb, const float *__restrict__ hb2, 
 //   output   : xb = sum_t a_t * v_t, sequentially over t per element (saxpyInPlace, FloatTensor.java:221-227)
 // The current position's k/v come from shared memory / the packed qkv vector, older ones from the
 // FP32 cache.  Output as floats (xb) and/or quantised to Q8_0 (activation of the Wo matvec).
+// Bound by its chain.  The rows of earlier positions are asked for in front of the dependency wait, products are made by all four threads of a quad at once and only the adds go through it in
+// turn, and quarters without positions are left out: 13400 -> 7800 cycles at position 20 (64 entries a head), 18900 -> 13300 at position 100 (128 entries).
 // ------------------------------------------------------------------------------------------
 #define ATT_THREADS 512 // four threads per key (scores) and per output element (weighted sum): head size <= ATT_THREADS / 4
 
@@ -413,7 +415,8 @@ __global__ void k_swiglu(float *__restrict__ hb, const float *__restrict__ hb2, 
 //   output    a CTA owns 32 elements of the head: one warp walks the positions (one dependent add each: 4 cycles per position, the bound of this part),
 //             the others stage V rows and the quotients ahead of it.
 // Decode step of two layers of the 8B geometry at position 3000: 562 us with a CTA per head, 316 us so (277 us since the norms run inside the
-// matvecs); the dependent adds alone are 6.3 us a layer.
+// matvecs, 246 us now); the dependent adds alone are 6.9 us a layer.  Of a layer's 35 us (65000 cycles) the scores take 14000, the maximum and its barrier 4000, the exponentials 3500, their sum 7500,
+// the values 31000.
 #define ATT_SPLIT 128
 #define ATT_KW 8           // scoring warps of a CTA
 #define ATT_KSTAGES 4      // stages of a scoring warp's ring
@@ -560,40 +563,76 @@ __device__ __forceinline__ void attention_split(float *sm, float *qkv, const flo
     }
     __syncthreads();
     const float sum = S.sum.result;
-    // ---- output (saxpyInPlace, FloatTensor.java:221-227): warp 0 walks, the others stay a stage ahead
+    // ---- output (saxpyInPlace, FloatTensor.java:221-227): warp 0 adds, the others stay ahead of it: stages on their way, and the next one's rows multiplied by their weights where they lie.
+    // Up to 4096 positions the exponentials are all in shared memory still and become the weights there at once; a longer row's come from L2 stage by stage.  3000 positions, 128 entries a
+    // head: 42000 cycles with warp 0 multiplying too and every weight from L2 (a round trip per stage that the adds did not cover), 34000 with the weights in place, 31000 so; the adds
+    // alone are 13000 (4.3 cycles each).
+    const bool whole = nt <= 4096;
     auto weights = [&](int c) {
         const int i = tid - 32, t = c * ATT_VT + i;
         if (i >= 0 && i < ATT_VT && t < nt) S.a[c & 1][i] = __fdiv_rn(ldcg_f32c(row + t), sum);
     };
-    weights(0);
+    auto multiply = [&](int c, int t0, int n_thr) { // stage c by threads t0 of n_thr
+        float4 *v = reinterpret_cast<float4 *>(S.ring) + (c % ATT_VSTAGES) * ATT_VT * 8;
+        const float *a = whole ? S.e + c * ATT_VT : S.a[c & 1];
+        const int n = min(ATT_VT, pos - c * ATT_VT) * 8;
+        for (int i = t0; i < n; i += n_thr) {
+            const float w = a[i >> 3];
+            const float4 x = v[i];
+            v[i] = make_float4(__fmul_rn(w, x.x), __fmul_rn(w, x.y), __fmul_rn(w, x.z), __fmul_rn(w, x.w));
+        }
+    };
+    if (whole)
+        for (int t = tid; t < nt; t += ATT_THREADS) S.e[t] = __fdiv_rn(S.e[t], sum);
+    else { weights(0); weights(1); }
+    asm volatile("cp.async.wait_group %0;" ::"n"(ATT_VSTAGES - 2) : "memory");
+    __syncthreads();
+    multiply(0, tid, ATT_THREADS);
     float acc = 0.0f;
     for (int c = 0; c < n_vc; c++) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(ATT_VSTAGES - 2) : "memory");
-        __syncthreads(); // stage c and its weights are there for every thread, and stage c - 1 is consumed
+        asm volatile("cp.async.wait_group %0;" ::"n"(ATT_VSTAGES - 3) : "memory");
+        __syncthreads(); // stage c is multiplied, stage c + 1 and its weights are there for every thread, and stage c - 1 is consumed
         if (warp == 0) {
-            const float *v = reinterpret_cast<const float *>(S.ring) + (c % ATT_VSTAGES) * ATT_VT * 32 + lane, *a = S.a[c & 1];
+            const float *v = reinterpret_cast<const float *>(S.ring) + (c % ATT_VSTAGES) * ATT_VT * 32 + lane;
             const int n = min(ATT_VT, pos - c * ATT_VT);
             int t = 0;
-            for (; t + 16 <= n; t += 16) {
-                float p[16];
+            if (n >= 16) { // sixteen products are read while the sixteen before them are added
+                float p0[16], p1[16];
+                auto read = [&](int t, float (&p)[16]) {
 #pragma unroll
-                for (int u = 0; u < 16; u += 4) {
-                    const float4 w = *reinterpret_cast<const float4 *>(a + t + u);
-                    p[u] = __fmul_rn(w.x, v[(t + u) * 32]); p[u + 1] = __fmul_rn(w.y, v[(t + u + 1) * 32]);
-                    p[u + 2] = __fmul_rn(w.z, v[(t + u + 2) * 32]); p[u + 3] = __fmul_rn(w.w, v[(t + u + 3) * 32]);
+                    for (int u = 0; u < 16; u++) p[u] = v[(t + u) * 32];
+                };
+                auto add = [&](const float (&p)[16]) {
+#pragma unroll
+                    for (int u = 0; u < 16; u++) acc = __fadd_rn(p[u], acc);
+                };
+                read(0, p0);
+                for (; t + 48 <= n; t += 32) {
+                    read(t + 16, p1);
+                    add(p0);
+                    read(t + 32, p0);
+                    add(p1);
                 }
-#pragma unroll
-                for (int u = 0; u < 16; u++) acc = __fadd_rn(p[u], acc);
+                if (t + 32 <= n) {
+                    read(t + 16, p1);
+                    add(p0);
+                    add(p1);
+                    t += 32;
+                } else {
+                    add(p0);
+                    t += 16;
+                }
             }
-            for (; t < n; t++) acc = __fadd_rn(__fmul_rn(a[t], v[t * 32]), acc);
+            for (; t < n; t++) acc = __fadd_rn(v[t * 32], acc);
         } else {
             if (c + ATT_VSTAGES - 1 < n_vc) fetch_v(c + ATT_VSTAGES - 1, tid - 32, ATT_THREADS - 32);
-            weights(c + 1);
+            if (c + 1 < n_vc) multiply(c + 1, tid - 32, ATT_THREADS - 32);
+            if (!whole) weights(c + 2);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     if (warp == 0) {
-        const float wl = __fdiv_rn(ldcg_f32c(row + pos), sum);
+        const float wl = whole ? S.e[pos] : __fdiv_rn(ldcg_f32c(row + pos), sum);
         const int d = rank * 32 + lane;
         acc = __fadd_rn(__fmul_rn(wl, vcur[d]), acc);
         if (xb) xb[h * HS + d] = acc;
@@ -634,19 +673,39 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     pdl_launch_dependents();
     const int kv_mul = n_heads / n_kv_heads, kvh = h / kv_mul;
     const int qd = n_heads * HS, kvd = n_kv_heads * HS;
-    pdl_wait();
-    trace_mark(tr, 2);
-    const int pos = st->pos, nt = pos + 1;
+    const int pos = st->pos, nt = pos + 1; // set before the step's first kernel started and left alone until its last one
     const bool split = cluster > 1; // (the host launches clusters from ATT_SPLIT positions on)
-    if (!split) { // K/V rows of the earlier positions -> L2, one 128-byte line per request, so the score loads below hit L2 (the weight stream carries an
-      // evict_first policy; without the prefetch these rows come from HBM every layer)
-        constexpr int LINES = HS / 32;
-        for (int i = tid; i < pos * LINES; i += ATT_THREADS) {
+    // K and V rows of the earlier positions were written by earlier steps, so they are asked for in front of the wait: the first pass' rows into registers, the others
+    // into L2, one 128-byte line per request (the weight stream carries an evict_first policy; without the prefetch these rows come from HBM every layer).
+    constexpr int LINES = HS / 32;
+    if (!split) {
+        for (int i = tid + ATT_THREADS / 4 * LINES; i < pos * LINES; i += ATT_THREADS) {
             const size_t off = (size_t)(i / LINES) * kvd + kvh * HS + (i % LINES) * 32;
             asm volatile("prefetch.global.L2 [%0];" ::"l"(kc + off));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(vc + off));
         }
     }
+    constexpr int QE = HS / 4, QV = HS / 16, VB = 32;
+    const int quad = tid & 3, qbase = lane & ~3, vd = tid >> 2;
+    const bool vlive = vd < HS;
+    float vv[VB];
+    float4 kk[QV];
+    auto load_k = [&](int t) { // this thread's quarter of row t
+        const float4 *k = reinterpret_cast<const float4 *>(kc + (size_t)t * kvd + kvh * HS + quad * QE);
+#pragma unroll
+        for (int u = 0; u < QV; u++) kk[u] = t < pos ? __ldg(k + u) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto load_v = [&](int d, bool live, int t0) { // rows [t0, t0 + VB) of element d
+        const float *vcol = vc + kvh * HS + d;
+#pragma unroll
+        for (int u = 0; u < VB; u++) vv[u] = (live && t0 + u < pos) ? __ldg(vcol + (size_t)(t0 + u) * kvd) : 0.0f;
+    };
+    if (!split) {
+        load_k(tid >> 2);
+        load_v(vd, vlive, quad * VB);
+    }
+    pdl_wait();
+    trace_mark(tr, 2);
     const float *qsrc = qkv + h * HS, *ksrc = qkv + qd + kvh * HS, *vsrc = qkv + qd + kvd + kvh * HS;
     // ---- prologue: threads [0,HALF) rotate q pairs, threads [HALF,HS) rotate k pairs
     if (tid < HS) {
@@ -710,42 +769,32 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
             return;
         }
     }
-    // ---- scores (scalarDot, FloatTensor.java:86-92: one sequential unfused mul/add chain per key).  Four threads share a key: each loads
-    // ITS quarter of the K row at once (one round trip per pass of ATT_THREADS/4 keys), then the chain runs through the quad in element
-    // order, handed on by shuffle.  The V rows of the first round of the weighted sum are requested here too (they do not depend on the scores).
-    constexpr int QE = HS / 4, QV = HS / 16, VB = 32;
-    const int quad = tid & 3, qbase = lane & ~3, vd = tid >> 2;
-    const bool vlive = vd < HS;
-    float vv[VB];
-    {
-        const float *vcol = vc + kvh * HS + vd;
-#pragma unroll
-        for (int u = 0; u < VB; u++) vv[u] = (vlive && quad * VB + u < pos) ? __ldg(vcol + (size_t)(quad * VB + u) * kvd) : 0.0f;
-    }
+    // ---- scores (scalarDot, FloatTensor.java:86-92: one sequential unfused mul/add chain per key).  Four threads share a key: each has
+    // ITS quarter of the K row and makes its products, then the adds run through the quad in element order, handed on by shuffle.
     float lmax = -INFINITY;
 #pragma unroll 1
     for (int t0 = 0; t0 < nt; t0 += ATT_THREADS / 4) {
         const int t = t0 + (tid >> 2);
-        float4 kk[QV];
-        if (t < pos) {
-            const float4 *k = reinterpret_cast<const float4 *>(kc + (size_t)t * kvd + kvh * HS + quad * QE);
+        if (t0 > 0) load_k(t);
+        if (t == pos) {
 #pragma unroll
-            for (int u = 0; u < QV; u++) kk[u] = __ldg(k + u);
-        } else {
+            for (int u = 0; u < QV; u++) kk[u] = *reinterpret_cast<const float4 *>(sk + quad * QE + 4 * u);
+        }
 #pragma unroll
-            for (int u = 0; u < QV; u++) kk[u] = t == pos ? *reinterpret_cast<const float4 *>(sk + quad * QE + 4 * u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int u = 0; u < QV; u++) {
+            const float4 q = *reinterpret_cast<const float4 *>(sq + quad * QE + 4 * u);
+            kk[u] = make_float4(__fmul_rn(q.x, kk[u].x), __fmul_rn(q.y, kk[u].y), __fmul_rn(q.z, kk[u].z), __fmul_rn(q.w, kk[u].w));
         }
         float acc = 0.0f;
 #pragma unroll 1
         for (int qd4 = 0; qd4 < 4; qd4++) {
             if (quad == qd4) {
-                const float *qq = sq + qd4 * QE;
 #pragma unroll
                 for (int u = 0; u < QV; u++) {
-                    acc = __fadd_rn(acc, __fmul_rn(qq[4 * u + 0], kk[u].x));
-                    acc = __fadd_rn(acc, __fmul_rn(qq[4 * u + 1], kk[u].y));
-                    acc = __fadd_rn(acc, __fmul_rn(qq[4 * u + 2], kk[u].z));
-                    acc = __fadd_rn(acc, __fmul_rn(qq[4 * u + 3], kk[u].w));
+                    acc = __fadd_rn(acc, kk[u].x);
+                    acc = __fadd_rn(acc, kk[u].y);
+                    acc = __fadd_rn(acc, kk[u].z);
+                    acc = __fadd_rn(acc, kk[u].w);
                 }
             }
             acc = __shfl_sync(0xffffffffu, acc, qbase + qd4);
@@ -765,11 +814,20 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     for (int t = tid; t < nt; t += ATT_THREADS) att[t] = (float)exp((double)__fsub_rn(att[t], mx));
     __syncthreads();
     if (tid == 0) {
-        float sum = 0.0f;
+        float sum = 0.0f, c[8], n[8];
         int t = 0;
-        for (; t + 4 <= nt; t += 4) {
-            const float a0 = att[t], a1 = att[t + 1], a2 = att[t + 2], a3 = att[t + 3];
-            sum = __fadd_rn(sum, a0); sum = __fadd_rn(sum, a1); sum = __fadd_rn(sum, a2); sum = __fadd_rn(sum, a3);
+        if (nt >= 8) { // eight terms are read while the eight before them are added
+#pragma unroll
+            for (int u = 0; u < 8; u++) c[u] = att[u];
+            for (; t + 8 <= nt; t += 8) {
+                if (t + 16 <= nt)
+#pragma unroll
+                    for (int u = 0; u < 8; u++) n[u] = att[t + 8 + u];
+#pragma unroll
+                for (int u = 0; u < 8; u++) sum = __fadd_rn(sum, c[u]);
+#pragma unroll
+                for (int u = 0; u < 8; u++) c[u] = n[u];
+            }
         }
         for (; t < nt; t++) sum = __fadd_rn(sum, att[t]);
         s_val[0] = sum;
@@ -784,23 +842,28 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     for (int vd0 = 0; vd0 < HS; vd0 += ATT_THREADS / 4) { // one pass for head sizes up to 128
         const int d = vd0 + vd;
         const bool live = d < HS;
-        const float *vcol = vc + kvh * HS + d;
         const float vcur = live ? vsrc[d] : 0.0f; // current position: straight from the packed qkv vector
         float acc = 0.0f;
 #pragma unroll 1
         for (int r0 = 0; r0 < pos; r0 += 4 * VB) {
-            if (r0 > 0 || vd0 > 0) { // (round 0 of the first pass was requested before the scores)
-                const int vt0 = r0 + quad * VB;
+            const int vt0 = r0 + quad * VB;
+            if (r0 > 0 || vd0 > 0) load_v(d, live, vt0); // (round 0 of the first pass was requested in front of the wait)
 #pragma unroll
-                for (int u = 0; u < VB; u++) vv[u] = (live && vt0 + u < pos) ? __ldg(vcol + (size_t)(vt0 + u) * kvd) : 0.0f;
-            }
+            for (int u = 0; u < VB; u++)
+                if (vt0 + u < pos) vv[u] = __fmul_rn(att[vt0 + u], vv[u]);
 #pragma unroll 1
-            for (int qd4 = 0; qd4 < 4; qd4++) {
+            for (int qd4 = 0; qd4 < 4 && r0 + qd4 * VB < pos; qd4++) { // (quarters behind the last position add nothing)
                 if (quad == qd4) {
-                    const int vt0 = r0 + qd4 * VB;
+                    if (vt0 + VB <= pos) {
 #pragma unroll
-                    for (int u = 0; u < VB; u++)
-                        if (vt0 + u < pos) acc = __fadd_rn(__fmul_rn(att[vt0 + u], vv[u]), acc);
+                        for (int u = 0; u < VB; u++) acc = __fadd_rn(vv[u], acc);
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < VB; u++) {
+                            const float more = __fadd_rn(vv[u], acc);
+                            acc = vt0 + u < pos ? more : acc;
+                        }
+                    }
                 }
                 acc = __shfl_sync(0xffffffffu, acc, qbase + qd4);
             }
