@@ -1165,6 +1165,8 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool vali
 // ways), looks the distances up meanwhile, asks for the first tiles of its values before the softmax, and the parts are merged over distributed shared
 // memory, every CTA finishing its share of the head's entries.  Lanes that share a row take four of them at a time (U; one where a stage holds no more than a row per
 // group).  32 heads of 64, 900 keys, cap and distance table: 27 us there, 17 us with one row at a time, 13 us with four; 32 heads of 128, 2000 keys: 56 and 38 us.
+// Latent rows (LATENT): seven rows of 576 fill a stage, so a CTA's 64 keys took ten stages and their values, which lie in the same rows, eight more; all at once and once only, the step of the
+// 16-head layer takes 145 us instead of 154 at 511 keys, 131 instead of 142 at 60.  Separate keys and values that way lose (16 heads of 64, 100 keys: 130 instead of 121 us).
 // grid (splits, heads), cluster (splits), LY_ATT_THREADS threads; dynamic shared memory step_att_smem_floats(...) floats.
 // ---------------------------------------------------------------------------------------------------------------------
 #define LY_STEP_STAGES 4
@@ -1176,6 +1178,13 @@ __host__ __device__ inline int step_att_chunk(int window, int splits) { // most 
 __host__ __device__ inline size_t step_att_smem_floats(int dk, int dv, int window, int splits) {
     return (size_t)dk + step_att_chunk(window, splits) + 4 * LY_ATT_THREADS + dv + 4 + LY_STEP_STAGES * LY_STEP_STAGE_FLOATS;
 }
+// LATENT: values lie inside the key rows (latent attention), all of a CTA's rows have room beside the rest, and they are read once.
+__host__ __device__ inline bool step_att_latent(const float *kc, const float *vc, const WindowAttn &a) {
+    return a.kv_heads == 1 && a.k_heads <= 1 && a.maps <= 1 && a.ldk == a.ldv && vc >= kc && vc + a.dv <= kc + a.dk && (vc - kc) % 4 == 0;
+}
+__host__ __device__ inline size_t step_att_latent_floats(int dk, int dv, int window, int splits) {
+    return step_att_smem_floats(dk, dv, window, splits) - LY_STEP_STAGES * LY_STEP_STAGE_FLOATS + (size_t)step_att_chunk(window, splits) * dk;
+}
 __device__ __forceinline__ float ld_cluster_f32(const float *p, int rank) { // the same shared variable of another CTA of the cluster
     unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
     float v;
@@ -1185,7 +1194,7 @@ __device__ __forceinline__ float ld_cluster_f32(const float *p, int rank) { // t
 }
 __device__ __forceinline__ void cluster_barrier() { asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory"); }
 
-template <int U> // rows of a lane group at a time
+template <int U, bool LATENT = false> // rows of a lane group at a time
 __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *__restrict__ P, WindowAttn a, const float *__restrict__ kc, const float *__restrict__ vc,
                                                                    const StepState *__restrict__ st, float *__restrict__ out) {
     extern __shared__ __align__(16) float sm[];
@@ -1221,13 +1230,27 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *
             for (int c = sub * 4; c < w; c += lpr * 4) cp_async16(dst + r * w + c, src + c, true);
         }
     };
-    const int kper = LY_STEP_STAGE_FLOATS / a.dk < 64 ? LY_STEP_STAGE_FLOATS / a.dk : 64, vper = LY_STEP_STAGE_FLOATS / a.dv < 64 ? LY_STEP_STAGE_FLOATS / a.dv : 64;
-    const int ktiles = (nk + kper - 1) / kper, vtiles = (nk + vper - 1) / vper;
+    // LATENT: all rows are asked for at once, in four groups, and nothing is refilled
+    const int kmost = LY_STEP_STAGE_FLOATS / a.dk < 64 ? LY_STEP_STAGE_FLOATS / a.dk : 64, vper = LY_STEP_STAGE_FLOATS / a.dv < 64 ? LY_STEP_STAGE_FLOATS / a.dv : 64;
+    const int kper = LATENT ? (nk + LY_STEP_STAGES - 1) / LY_STEP_STAGES : kmost;
+    const int ktiles = nk > 0 ? (nk + kper - 1) / kper : 0, vtiles = LATENT ? 0 : (nk + vper - 1) / vper;
     const float *kb = kc + (size_t)gk * a.dk, *vb = vc + (size_t)g * a.dv;
     const int klpr = lanes_row(a.dk), vlpr = lanes_row(a.dv);
+    auto fetch_rows = [&](int r0, int n) { // (LATENT) the CTA's rows [r0, r0 + n)
+        const int sub = lane & (klpr - 1), rows = 32 / klpr;
+        for (int r = r0 + warp * rows + lane / klpr; r < r0 + n; r += (LY_ATT_THREADS / 32) * rows) {
+            int slot = slot0 + r;
+            if (slot >= a.ring) slot %= a.ring;
+            const float *src = kb + (size_t)slot * a.ldk;
+            for (int c = sub * 4; c < a.dk; c += klpr * 4) cp_async16(ring + r * a.dk + c, src + c, true);
+        }
+    };
 #pragma unroll
     for (int i = 0; i < LY_STEP_STAGES; i++) {
-        if (i < ktiles) fetch(kb, a.ldk, a.dk, kper, klpr, i);
+        if (i < ktiles) {
+            if (LATENT) fetch_rows(i * kper, nk - i * kper < kper ? nk - i * kper : kper);
+            else fetch(kb, a.ldk, a.dk, kper, klpr, i);
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     for (int i = tid; i < a.dk; i += LY_ATT_THREADS) qs[i] = P[(size_t)h * a.dk + i];
@@ -1237,7 +1260,7 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *
     for (int i = 0; i < ktiles; i++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(LY_STEP_STAGES - 1) : "memory");
         __syncthreads();
-        const float *kt = ring + (i % LY_STEP_STAGES) * LY_STEP_STAGE_FLOATS;
+        const float *kt = LATENT ? ring + (size_t)i * kper * a.dk : ring + (i % LY_STEP_STAGES) * LY_STEP_STAGE_FLOATS;
         const int n = nk - i * kper < kper ? nk - i * kper : kper, sub = lane & (klpr - 1), rows = 32 / klpr;
         const int hop = (LY_ATT_THREADS / 32) * rows;
         for (int w0 = warp * rows; w0 < n; w0 += U * hop) { // (their chains of products, shuffles and cap run side by side)
@@ -1270,7 +1293,7 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *
                     mx = fmaxf(mx, e);
                 }
         }
-        if (i + LY_STEP_STAGES < ktiles) { // (uniform) refill the stage when every warp is done with it
+        if (!LATENT && i + LY_STEP_STAGES < ktiles) { // (uniform) refill the stage when every warp is done with it
             __syncthreads();
             fetch(kb, a.ldk, a.dk, kper, klpr, i + LY_STEP_STAGES);
         }
@@ -1278,11 +1301,12 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     mx = block_max(mx, red); // also: the ring is free, the scores are written
+    if (!LATENT)
 #pragma unroll
-    for (int i = 0; i < LY_STEP_STAGES; i++) { // values on their way through the softmax
-        if (i < vtiles) fetch(vb, a.ldv, a.dv, vper, vlpr, i);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
+        for (int i = 0; i < LY_STEP_STAGES; i++) { // values on their way through the softmax
+            if (i < vtiles) fetch(vb, a.ldv, a.dv, vper, vlpr, i);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
     float sum = 0.0f;
     for (int j = tid; j < nk; j += LY_ATT_THREADS) {
         const float w = expf(sc[j] - mx);
@@ -1292,6 +1316,15 @@ __global__ void __launch_bounds__(LY_ATT_THREADS) k_step_attention(const float *
     sum = block_sum(sum, red);
     const int tpk = a.dv / 4, groups = LY_ATT_THREADS / tpk, grp = tid / tpk, d0 = (tid % tpk) * 4;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (LATENT && grp < groups) {
+        const float *v0 = ring + (vc - kc) + d0;
+#pragma unroll 4
+        for (int r = grp; r < nk; r += groups) {
+            const float w = sc[r];
+            const float4 v = *reinterpret_cast<const float4 *>(v0 + (size_t)r * a.dk);
+            acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
+        }
+    }
     for (int i = 0; i < vtiles; i++) {
         asm volatile("cp.async.wait_group %0;" ::"n"(LY_STEP_STAGES - 1) : "memory");
         __syncthreads();

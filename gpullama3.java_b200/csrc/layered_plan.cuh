@@ -395,10 +395,15 @@ static int ly_step_attention(b200_plan *p, int heads, int window, const float *q
     Layered &Y = *p->ly;
     int sp = 1;
     if (Y.split.o && window >= 64) { sp = p->n_sms / heads; if (sp > Y.max_splits) sp = Y.max_splits; if (sp < 1) sp = 1; }
-    const size_t sm = ly::step_att_smem_floats(wa.dk, wa.dv, wa.window, sp) * 4;
-    if ((wa.dk | wa.dv | wa.ldk | wa.ldv) % 4 == 0 && wa.dk <= 1024 && wa.dv <= 4 * LY_ATT_THREADS && sm <= (size_t)Y.smem_max)
-        return launch_cluster(p, p->use_pdl, sp, LY_STEP_STAGE_FLOATS / wa.dk >= 2 * (LY_ATT_THREADS / 32) ? ly::k_step_attention<4> : ly::k_step_attention<1>, dim3(sp, heads),
-                              dim3(LY_ATT_THREADS), sm, q, wa, kc, vc, st, out);
+    if ((wa.dk | wa.dv | wa.ldk | wa.ldv) % 4 == 0 && wa.dk <= 1024 && wa.dv <= 4 * LY_ATT_THREADS) {
+        const size_t sm = ly::step_att_smem_floats(wa.dk, wa.dv, wa.window, sp) * 4;
+        // latent rows once and at once where they fit beside the rest (a CTA an SM: splits x heads are no more than that), else through the ring
+        const size_t latent = ly::step_att_latent_floats(wa.dk, wa.dv, wa.window, sp) * 4;
+        if (ly::step_att_latent(kc, vc, wa) && latent <= (size_t)Y.smem_max && sp * heads <= p->n_sms)
+            return launch_cluster(p, p->use_pdl, sp, ly::k_step_attention<2, true>, dim3(sp, heads), dim3(LY_ATT_THREADS), latent, q, wa, kc, vc, st, out);
+        if (sm <= (size_t)Y.smem_max)
+            return launch_cluster(p, p->use_pdl, sp, LY_STEP_STAGE_FLOATS / wa.dk >= 2 * (LY_ATT_THREADS / 32) ? ly::k_step_attention<4> : ly::k_step_attention<1>, dim3(sp, heads), dim3(LY_ATT_THREADS), sm, q, wa, kc, vc, st, out);
+    }
     return launch_k(p, p->use_pdl, ly::k_window_attention<float>, dim3(1, heads, sp), dim3(LY_ATT_THREADS), general_smem, q, ldq, wa, kc, vc, st, out, ldo,
                     sp > 1 ? Y.split : ly::KeySplit{nullptr, nullptr, nullptr});
 }
@@ -839,6 +844,7 @@ static int ly_build(b200_plan *p, const b200_layered_config *cfg, const b200_lay
             CK(set_max_dyn(ly::k_window_attention<float>, Y.smem_max));
             CK(set_max_dyn(ly::k_step_attention<1>, Y.smem_max));
             CK(set_max_dyn(ly::k_step_attention<4>, Y.smem_max));
+            CK(set_max_dyn(ly::k_step_attention<2, true>, Y.smem_max));
             CK(set_max_dyn(ly::k_window_attention<ly::bf16>, Y.smem_max));
             CK(set_max_dyn(ly::k_window_attention_mma<64, 64>, Y.smem_max));
             CK(set_max_dyn(ly::k_window_attention_mma<64, 64, 64>, Y.smem_max));
