@@ -1335,7 +1335,8 @@ int exact_prefill_init(b200_plan *p) {
     if (chunk < XT_TOK / 2) return B200_OK; // (a tile of 128 tokens would be mostly empty)
     if ((rc = alloc_optional(p, &done, [&]() -> int { return exact_prefill_umma_alloc(p, rows, wide); }, &why))) return rc;
     if (!done) {
-        p->xp.AH = nullptr;
+        p->xp.AH = p->xp.HH = nullptr;
+        p->xp.G = nullptr;
         p->xp.maps_umma.clear();
     }
     return B200_OK;
@@ -1392,7 +1393,7 @@ int exact_prefill_umma_alloc(b200_plan *p, int rows, int wide) {
     if ((rc = dalloc(p, &c.G, (size_t)rows * 2 * g.hidden_dim * 4))) return rc;
     CK(cudaMemset(c.AH, 0, (size_t)rows * wide * 2)); // (as AQ and HQ)
     CK(cudaMemset(c.HH, 0, (size_t)rows * g.hidden_dim * 2));
-    bool ok = xp_map_acts(&c.hA, c.AH, true, c.AS, rows, g.dim, XT_TOK) == 0 && xp_map_acts(&c.hATT, c.AH, true, c.AS, rows, p->qd, XT_TOK) == 0 &&
+    bool ok = !refused("umma") && xp_map_acts(&c.hA, c.AH, true, c.AS, rows, g.dim, XT_TOK) == 0 && xp_map_acts(&c.hATT, c.AH, true, c.AS, rows, p->qd, XT_TOK) == 0 &&
               xp_map_acts(&c.hH, c.HH, true, c.HS, rows, g.hidden_dim, XT_TOK) == 0;
     c.maps_umma.resize(g.n_layers);
     for (int l = 0; ok && l < g.n_layers; l++) ok = xp_map_layer(&c.maps_umma[l], p->layers[l], XT_BOX);

@@ -40,3 +40,16 @@ def test_several_tiles_per_sm(pkg, monkeypatch, rows):
 def test_scales(pkg, monkeypatch, rows):
     monkeypatch.setenv("B200_XP_TILE", CODES[rows])
     run(pkg, pkg.synth.SHAPES["tiny-llama"], [130], lambda rng, n: np.ldexp(rng.choice([-1.0, 1.0], n) * rng.uniform(1.0, 2.0, n), rng.integers(-26, -2, n)))
+
+
+def test_without_its_buffers(pkg, monkeypatch):
+    """A driver that does not make its tensor maps: the chunk takes the other product, with none of its buffers."""
+    used = []
+    for refuse in ("umma", ""):
+        monkeypatch.setenv("B200_TEST_REFUSE", refuse)
+        run(pkg, pkg.synth.SHAPES["small-llama"], [300])
+        S, Q8 = pkg.synth, pkg.gguf.GGMLType.Q8_0
+        plan = pkg.B200MasterPlan(pkg.loader.model_from_tensors(S.SHAPES["small-llama"], Q8, S.build_tensors_fast(S.SHAPES["small-llama"], Q8, seed=1), 304), prefill_batch_size=300)
+        used.append(plan.device_bytes)
+        plan.free()
+    assert used[0] < used[1]
