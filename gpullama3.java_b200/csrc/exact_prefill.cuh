@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(256, E <= 16 ? 4 : 1) k_xp_norm(float *__restr
 // (every B fragment and activation scale serves two row tiles), else 16 rows and all of them; and one that fetches: a ring of stages of 128 columns comes in by TMA (weights and
 // their scales straight out of the tile-major layout by a 4-D map), rows of 128 bytes swizzled so that ldmatrix is conflict-free.  A multiplying warp that waited for the others and
 // issued the fetches between its chunks held the whole CTA up by half of its time: gate/up of 512 tokens, 8B layer, 388 us against 328 us so; W2 of 36 tokens, 4B layer, 43 against 28 us (a
-// deeper ring alone 43, all operands of a chunk in registers ahead 46).  Issue slots: 19 warp instructions per 16 x 8 tile and block, 10 of them the conversions, products and adds.
+// deeper ring alone 43, all operands of a chunk in registers ahead 46).  Issue slots: 15.7 warp instructions per 16 x 8 tile and block, 10 of them the conversions, products and
+// adds (65 % of the slots, FMA pipe 57 %).
 // Long chunks' QKV, Wo and W2 are exact_prefill_umma.cuh's.
 #define XP_STAGES 3      // of a ring, at least;
 #define XP_STAGES_MAX 8  // and at most: as many as the CTAs of an SM have room for
