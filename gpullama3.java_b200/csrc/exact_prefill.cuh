@@ -243,9 +243,10 @@ __global__ void __launch_bounds__(XP_THREADS + 32, XpTile<NJ>::RESIDENT) k_xp_ge
                     pg::tma_load_2d(s + T::B_S, &map_a.s, tok0, seg * nbs + 4 * cs, bar);
                     if (++stage == stages) { stage = 0; ph ^= 1u; }
                 }
-            if (!ok) // (a wait gave up: nothing leaves with its copies in flight)
-                for (int q = max(0, c - stages); q < c; q++) xp_wait(full0 + 8 * (q % stages), (q / stages) & 1, err);
+            // Nothing leaves with its copies in flight, whoever gave up: a multiplying warp whose wait did goes on without looking at its stages, and all chunks may be under way by then.
+            for (int q = max(0, c - stages); q < c; q++) xp_wait(full0 + 8 * (q % stages), (q / stages) & 1, err);
         }
+        __syncwarp();
         if (MODE == XP_GATEUP) { __syncthreads(); __syncthreads(); } // (the epilogue's)
         return;
     }
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(XP_THREADS + 32, XpTile<NJ>::RESIDENT) k_xp_ge
 
     const int r0 = wrow + (lane >> 2), t0 = wtok + 2 * (lane & 3);
     if (MODE == XP_GATEUP) { // rows of a group: gate 2G, gate 2G + 1, up 2G, up 2G + 1; the CTA's 64 rows are one 32-unit block of the hidden row
-        __syncthreads(); // (every fetch has landed: a warp is here behind its last chunk)
+        __syncthreads(); // (every fetch has landed: the fetching warp is here behind its last one)
         float *hv = reinterpret_cast<float *>(ring);
 #pragma unroll
         for (int i = 0; i < MI; i++)

@@ -2300,9 +2300,8 @@ int b200_test_seqsum2(const float *terms, int32_t n, int32_t threads, float *out
 }
 
 // One tile of the exact prefill's product on zeros (64 rows x 640 columns x 16 tokens), three times: as it is, with activation boxes of half the tile, whose stages never fill, and as
-// it is again.
-int b200_test_exact_prefill_wait(uint32_t *codes, float *ms) {
-    if (!codes || !ms) return B200_ERR_BAD_ARG;
+// it is again.  form 0: a ring of three stages, so that the fetching warp waits too; 1: of eight, so that all chunks are under way at once; 2: that and the gate/up epilogue.
+static int run_exact_prefill_wait(int form, uint32_t *codes, float *ms) {
     constexpr int COLS = 640, TOK = 16;
     b200_plan *p = nullptr; // (CK)
     TileMat W{nullptr, XP_ROWS, COLS, COLS, 1, smv_unit_bytes(COLS)};
@@ -2319,15 +2318,24 @@ int b200_test_exact_prefill_wait(uint32_t *codes, float *ms) {
         W.base = mem;
         const int8_t *q = reinterpret_cast<const int8_t *>(mem + w_bytes);
         const float *s = reinterpret_cast<const float *>(mem + w_bytes + q_bytes);
+        unsigned char *o = mem + w_bytes + q_bytes + s_bytes;
         XpMaps mw, ma[2];
         if (xp_map_weights(&mw, W, XP_ROWS) || xp_map_acts(&ma[0], q, false, s, 64, COLS, TOK) || xp_map_acts(&ma[1], q, false, s, 64, COLS, TOK / 2)) return B200_ERR_UNSUPPORTED;
-        CK(cudaFuncSetAttribute(k_xp_gemm<XP_STORE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::bytes(XP_STAGES)));
+        auto launch = [&](const XpMaps &acts) -> int {
+            const int stages = form == 0 ? XP_STAGES : XP_STAGES_MAX;
+            // (hidden units: 32 of 16 tokens as bytes, their scales, and the last token's units, bytes and scale)
+            const XpLast last{nullptr, reinterpret_cast<int8_t *>(o + 2304), nullptr, reinterpret_cast<float *>(o + 2560), reinterpret_cast<float *>(o + 2048)};
+            auto kern = form == 2 ? k_xp_gemm<XP_GATEUP, 2> : k_xp_gemm<XP_STORE, 2>;
+            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::bytes(stages)));
+            kern<<<dim3(1, 1), XP_THREADS + 32, XpTile<2>::bytes(stages)>>>(mw, acts, W, 64, TOK, reinterpret_cast<float *>(o), XP_ROWS, reinterpret_cast<int8_t *>(o), nullptr,
+                                                                            reinterpret_cast<float *>(o + 1024), last, 1.0f, stages, d_err);
+            CK(cudaGetLastError());
+            return B200_OK;
+        };
         for (int i = 0; i < 3; i++) {
             *err = 0u;
             CK(cudaEventRecord(ev[0]));
-            k_xp_gemm<XP_STORE, 2><<<dim3(1, 1), XP_THREADS + 32, XpTile<2>::bytes(XP_STAGES)>>>(mw, ma[i == 1], W, 64, TOK, reinterpret_cast<float *>(mem + w_bytes + q_bytes + s_bytes), XP_ROWS, nullptr, nullptr, nullptr,
-                                                                                XpLast{}, 1.0f, XP_STAGES, d_err);
-            CK(cudaGetLastError());
+            if (int rc = launch(ma[i == 1])) return rc;
             CK(cudaEventRecord(ev[1]));
             CK(cudaDeviceSynchronize());
             codes[i] = *reinterpret_cast<volatile unsigned *>(err);
@@ -2340,6 +2348,11 @@ int b200_test_exact_prefill_wait(uint32_t *codes, float *ms) {
     if (err) cudaFreeHost(err);
     cudaFree(mem);
     return rc;
+}
+int b200_test_exact_prefill_wait(uint32_t *codes, float *ms) { return b200_test_exact_prefill_wait_form(0, codes, ms); }
+int b200_test_exact_prefill_wait_form(int32_t form, uint32_t *codes, float *ms) {
+    if (!codes || !ms || form < 0 || form > 2) return B200_ERR_BAD_ARG;
+    return run_exact_prefill_wait(form, codes, ms);
 }
 
 int b200_requant_kquant(int32_t ggml_type, const void *src, int64_t n_elems, void *dst_q8_0) {

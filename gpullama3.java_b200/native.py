@@ -72,7 +72,7 @@ class Tensor(C.Structure):
 
 
 EXPORTS = ["b200_plan_create_layered", "b200_forward_batch_logits", "b200_layered_info", "b200_plan_create", "b200_forward_decode", "b200_forward_prefill", "b200_forward_batch_prefill", "b200_set_prefill_mode", "b200_prefill_info", "b200_exact_prefill_info",
-           "b200_set_decode_mode", "b200_decode_info", "b200_trace_persistent", "b200_test_seqsum2", "b200_test_exact_prefill_wait", "b200_forward_decode_sample", "b200_upload_info", "b200_requant_kquant",
+           "b200_set_decode_mode", "b200_decode_info", "b200_trace_persistent", "b200_test_seqsum2", "b200_test_exact_prefill_wait", "b200_test_exact_prefill_wait_form", "b200_forward_decode_sample", "b200_upload_info", "b200_requant_kquant",
            "b200_decode_sequence", "b200_time_kernel", "b200_tp_handle", "b200_tp_attach", "b200_trace_decode", "b200_profile_norm", "b200_test_seqsum", "b200_gemm_f16", "b200_kv_reset", "b200_read_buffer", "b200_launches_per_decode",
            "b200_device_bytes", "b200_plan_free", "b200_last_error", "b200_version"]
 
@@ -110,6 +110,7 @@ def lib() -> C.CDLL:
     L.b200_test_seqsum2.argtypes = [vp, i32, i32, C.POINTER(C.c_float), C.POINTER(i32)]
     L.b200_prefill_info.argtypes = [vp, C.POINTER(i32), C.POINTER(i32), C.POINTER(C.c_float)]
     L.b200_test_exact_prefill_wait.argtypes = [C.POINTER(C.c_uint32), C.POINTER(C.c_float)]
+    L.b200_test_exact_prefill_wait_form.argtypes = [C.c_int32, C.POINTER(C.c_uint32), C.POINTER(C.c_float)]
     L.b200_exact_prefill_info.argtypes = [vp, C.POINTER(i32), C.POINTER(C.c_int64), C.POINTER(C.c_char_p)]
     L.b200_gemm_f16.argtypes = [vp, vp, vp, i32, i32, i32, i32, C.POINTER(C.c_float)]
     L.b200_time_kernel.argtypes = [vp, i32, i32, C.POINTER(C.c_float), C.POINTER(C.c_int64)]
@@ -147,10 +148,10 @@ def test_seqsum(terms, want_info: bool = False, threads: int = 0):
     return (out.value, info[0], info[1]) if want_info else out.value
 
 
-def test_exact_prefill_wait():
-    """[(error word, milliseconds)] of a tile whose operands arrive, of one whose operands arrive in part, and of the first again."""
+def test_exact_prefill_wait(form: int = 0):
+    """[(error word, milliseconds)] of a tile whose operands arrive, of one whose operands arrive in part, and of the first again (``form``: b200llama.h)."""
     codes, ms = (C.c_uint32 * 3)(), (C.c_float * 3)()
-    rc = lib().b200_test_exact_prefill_wait(codes, ms)
+    rc = lib().b200_test_exact_prefill_wait_form(form, codes, ms)
     if rc != B200_OK:
         _raise(rc, "b200_test_exact_prefill_wait failed")
     return list(zip(codes, ms))

@@ -15,3 +15,12 @@ def test_operands_that_do_not_arrive(pkg, make_model):
     plan.forward_batch_prefill(list(range(3, 14)), 0)
     assert plan.exact_prefill_info()[1] == 1
     plan.free()
+
+
+@pytest.mark.parametrize("form", [1, 2])
+def test_all_operands_under_way(pkg, form):
+    """The fetching warp has issued every chunk when the multiplying warps give up: it waits for their copies, as long as a copy takes and no longer than a wait's limit."""
+    before, starved, after = pkg.native.test_exact_prefill_wait(form)
+    assert before[0] == 0 and before[1] < 900
+    assert starved[0] == 200 and 1000 <= starved[1] < 1100
+    assert after[0] == 0 and after[1] < 10
