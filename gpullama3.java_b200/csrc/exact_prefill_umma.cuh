@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_xt_gemm(const __grid_constant
     } else {
         if (warp == XT_SUM_WARPS + 4) { // ---- fetches
             if (lane == 0) {
-                int it = 0;
+                int it = 0, n_w = 0, n_a = 0; // the chunk; chunks whose weights, whose activations are under way or there
                 bool ok = true;
                 for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
                     const int tok0 = tile % m_tiles * XT_TOK, row0 = tile / m_tiles * N;
@@ -164,18 +164,20 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_xt_gemm(const __grid_constant
                             xp_load4(w + T::W_Q + r * 128, &map_w.q, 128 * cs, seg, (row0 + r) >> 2, wbar);
                             xp_load4(w + T::W_S + r * 16, &map_w.s, W.seg + ((8 * cs) & ~15), seg, (row0 + r) >> 2, wbar); // 8 scales of a row, 16 bytes
                         }
-                        if (it >= 2 && !(ok = xp_wait(aempty0 + 8 * as, ((it >> 1) - 1) & 1, err))) { it++; break; } // (the weights of this chunk are on their way)
+                        n_w = it + 1;
+                        if (it >= 2 && !(ok = xp_wait(aempty0 + 8 * as, ((it >> 1) - 1) & 1, err))) break;
                         mbar_expect_tx(abar, T::A_STAGE);
                         pg::tma_load_2d(a, &map_a.q, seg * W.seg + 128 * cs, tok0, abar);
                         pg::tma_load_2d(a + T::A_TILE, &map_a.q, seg * W.seg + 128 * cs + 64, tok0, abar);
+                        n_a = it + 1;
                         if (++cs == cps) { cs = 0; seg++; }
                     }
                 }
-                if (!ok) { // (nothing leaves with its copies in flight)
-                    for (int q = max(0, it - XT_W_STAGES); q < it; q++) xp_wait(wfull0 + 8 * (q % XT_W_STAGES), (q / XT_W_STAGES) & 1, err);
-                    for (int q = max(0, it - 3); q < it; q++) xp_wait(afull0 + 8 * (q & 1), (q >> 1) & 1, err);
-                }
+                // Nothing leaves with its copies in flight, whoever gave up: the others go to the block's last barrier without looking at their stages.
+                for (int q = max(0, n_w - XT_W_STAGES); q < n_w; q++) xp_wait(wfull0 + 8 * (q % XT_W_STAGES), (q / XT_W_STAGES) & 1, err);
+                for (int q = max(0, n_a - 2); q < n_a; q++) xp_wait(afull0 + 8 * (q & 1), (q >> 1) & 1, err);
             }
+            __syncwarp();
         } else if (warp == XT_SUM_WARPS + 5) { // ---- products: the warp walks together (addresses and phases stay in uniform registers), one lane issues
             constexpr uint32_t idesc = pg::umma_idesc_f16(XT_TOK, N);
             uint32_t lead;
@@ -218,14 +220,12 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_xt_gemm(const __grid_constant
                     if (++as == 2) { as = 0; ph_a ^= 1u; }
                     if (++cs == cps) cs = 0;
                 }
-            if (!ok) { // (nothing leaves with its products in flight)
-                if (lead) {
-                    *reinterpret_cast<volatile unsigned *>(err) = 200u;
-                    pg::umma_commit(fin);
-                    xp_wait(fin, 0, err);
-                }
-                __syncwarp();
+            if (lead) { // no columns go back with products in flight, whoever gave up
+                if (!ok) *reinterpret_cast<volatile unsigned *>(err) = 200u;
+                pg::umma_commit(fin);
+                xp_wait(fin, 0, err);
             }
+            __syncwarp();
         } else if (warp < XT_SUM_WARPS + 4) { // ---- operands
             const int r = tid - XT_SUM_WARPS * 32; // weight row, and token
             int ws = 0, h = 0, sb = 0;

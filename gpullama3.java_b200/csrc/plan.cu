@@ -2299,13 +2299,15 @@ int b200_test_seqsum2(const float *terms, int32_t n, int32_t threads, float *out
     return run_seqsum_hook(terms, n, threads, out, info);
 }
 
-// One tile of the exact prefill's product on zeros (64 rows x 640 columns x 16 tokens), three times: as it is, with activation boxes of half the tile, whose stages never fill, and as
-// it is again.  form 0: a ring of three stages, so that the fetching warp waits too; 1: of eight, so that all chunks are under way at once; 2: that and the gate/up epilogue.
+// One tile of the exact prefill's product on zeros, three times: as it is, with activation boxes of half the tile, whose stages never fill, and as it is again.
+//   form 0: k_xp_gemm, 64 rows x 640 columns x 16 tokens, a ring of three stages, so that the fetching warp waits too; 1: of eight, so that all chunks are under way at once; 2: that and
+//   the gate/up epilogue; 3: k_xt_gemm, 128 rows x 640 columns x 128 tokens, activations in part: every role waits; 4: 256 columns, scales in part, with all chunks under way at once.
 static int run_exact_prefill_wait(int form, uint32_t *codes, float *ms) {
-    constexpr int COLS = 640, TOK = 16;
+    const bool umma = form >= 3;
+    const int cols = form == 4 ? 256 : 640, rows = umma ? 128 : XP_ROWS, tok = umma ? XT_TOK : 16, tok_pad = umma ? XT_TOK : 64;
     b200_plan *p = nullptr; // (CK)
-    TileMat W{nullptr, XP_ROWS, COLS, COLS, 1, smv_unit_bytes(COLS)};
-    const size_t w_bytes = (size_t)XP_ROWS * W.unit_bytes, q_bytes = (size_t)64 * COLS, s_bytes = (size_t)64 * (COLS / 32) * 4, o_bytes = (size_t)TOK * XP_ROWS * 4;
+    TileMat W{nullptr, rows, cols, cols, 1, smv_unit_bytes(cols)};
+    const size_t w_bytes = (size_t)rows * W.unit_bytes, q_bytes = (size_t)tok_pad * cols * (umma ? 2 : 1), s_bytes = (size_t)tok_pad * (cols / 32) * 4, o_bytes = (size_t)tok * rows * 4;
     unsigned char *mem = nullptr;
     unsigned *err = nullptr, *d_err = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -2316,26 +2318,32 @@ static int run_exact_prefill_wait(int form, uint32_t *codes, float *ms) {
         CK(cudaHostGetDevicePointer((void **)&d_err, err, 0));
         for (cudaEvent_t &e : ev) CK(cudaEventCreate(&e));
         W.base = mem;
-        const int8_t *q = reinterpret_cast<const int8_t *>(mem + w_bytes);
+        const unsigned char *q = mem + w_bytes;
         const float *s = reinterpret_cast<const float *>(mem + w_bytes + q_bytes);
         unsigned char *o = mem + w_bytes + q_bytes + s_bytes;
-        XpMaps mw, ma[2];
-        if (xp_map_weights(&mw, W, XP_ROWS) || xp_map_acts(&ma[0], q, false, s, 64, COLS, TOK) || xp_map_acts(&ma[1], q, false, s, 64, COLS, TOK / 2)) return B200_ERR_UNSUPPORTED;
+        XpMaps mw, whole, half;
+        if (xp_map_weights(&mw, W, umma ? XT_BOX : XP_ROWS) || xp_map_acts(&whole, q, umma, s, tok_pad, cols, tok) || xp_map_acts(&half, q, umma, s, tok_pad, cols, tok / 2)) return B200_ERR_UNSUPPORTED;
+        const XpMaps starved = form == 3 ? XpMaps{half.q, whole.s} : form == 4 ? XpMaps{whole.q, half.s} : half;
         auto launch = [&](const XpMaps &acts) -> int {
-            const int stages = form == 0 ? XP_STAGES : XP_STAGES_MAX;
-            // (hidden units: 32 of 16 tokens as bytes, their scales, and the last token's units, bytes and scale)
-            const XpLast last{nullptr, reinterpret_cast<int8_t *>(o + 2304), nullptr, reinterpret_cast<float *>(o + 2560), reinterpret_cast<float *>(o + 2048)};
-            auto kern = form == 2 ? k_xp_gemm<XP_GATEUP, 2> : k_xp_gemm<XP_STORE, 2>;
-            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::bytes(stages)));
-            kern<<<dim3(1, 1), XP_THREADS + 32, XpTile<2>::bytes(stages)>>>(mw, acts, W, 64, TOK, reinterpret_cast<float *>(o), XP_ROWS, reinterpret_cast<int8_t *>(o), nullptr,
-                                                                            reinterpret_cast<float *>(o + 1024), last, 1.0f, stages, d_err);
+            if (umma) {
+                CK(cudaFuncSetAttribute(k_xt_gemm<XP_STORE, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, XtSmem<128>::BYTES));
+                k_xt_gemm<XP_STORE, 128><<<1, XT_THREADS, XtSmem<128>::BYTES>>>(mw, acts, W, tok, reinterpret_cast<float *>(o), rows, 1.0f, d_err);
+            } else {
+                const int stages = form == 0 ? XP_STAGES : XP_STAGES_MAX;
+                // (hidden units: 32 of 16 tokens as bytes, their scales, and the last token's units, bytes and scale)
+                const XpLast last{nullptr, reinterpret_cast<int8_t *>(o + 2304), nullptr, reinterpret_cast<float *>(o + 2560), reinterpret_cast<float *>(o + 2048)};
+                auto kern = form == 2 ? k_xp_gemm<XP_GATEUP, 2> : k_xp_gemm<XP_STORE, 2>;
+                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::bytes(stages)));
+                kern<<<dim3(1, 1), XP_THREADS + 32, XpTile<2>::bytes(stages)>>>(mw, acts, W, tok_pad, tok, reinterpret_cast<float *>(o), rows, reinterpret_cast<int8_t *>(o), nullptr,
+                                                                                reinterpret_cast<float *>(o + 1024), last, 1.0f, stages, d_err);
+            }
             CK(cudaGetLastError());
             return B200_OK;
         };
         for (int i = 0; i < 3; i++) {
             *err = 0u;
             CK(cudaEventRecord(ev[0]));
-            if (int rc = launch(ma[i == 1])) return rc;
+            if (int rc = launch(i == 1 ? starved : whole)) return rc;
             CK(cudaEventRecord(ev[1]));
             CK(cudaDeviceSynchronize());
             codes[i] = *reinterpret_cast<volatile unsigned *>(err);
@@ -2351,7 +2359,7 @@ static int run_exact_prefill_wait(int form, uint32_t *codes, float *ms) {
 }
 int b200_test_exact_prefill_wait(uint32_t *codes, float *ms) { return b200_test_exact_prefill_wait_form(0, codes, ms); }
 int b200_test_exact_prefill_wait_form(int32_t form, uint32_t *codes, float *ms) {
-    if (!codes || !ms || form < 0 || form > 2) return B200_ERR_BAD_ARG;
+    if (!codes || !ms || form < 0 || form > 4) return B200_ERR_BAD_ARG;
     return run_exact_prefill_wait(form, codes, ms);
 }
 

@@ -460,7 +460,8 @@ int b200_test_seqsum2(const float *terms, int32_t n, int32_t threads, float *out
 /* Test hook for the bounded waits of the exact prefill's product (csrc/exact_prefill.cuh): codes[3] and ms[3] are the error word and the time of one tile whose operands
  * arrive, of one whose operands arrive in part (its waits give up: 200), and of the first again. */
 int b200_test_exact_prefill_wait(uint32_t *codes, float *ms);
-/* ... of form 0: that tile; 1: with all its operands under way at once; 2: so, with the gate/up epilogue. */
+/* ... of form 0: that tile; 1: with all its operands under way at once; 2: so, with the gate/up epilogue; of the product on tcgen05 (csrc/exact_prefill_umma.cuh) 3: a tile whose
+ * activations arrive in part; 4: one whose scales do, with all its operands under way at once. */
 int b200_test_exact_prefill_wait_form(int32_t form, uint32_t *codes, float *ms);
 
 /* Test hook for the device-side K-quant -> Q8_0 re-quantiser the upload pipeline applies to Q4_K / Q5_K / Q6_K tensors (csrc/kquant.cuh;
