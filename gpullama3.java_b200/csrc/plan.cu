@@ -1308,6 +1308,36 @@ const int XP_N_KERNELS = sizeof(XP_KERNELS) / sizeof(XP_KERNELS[0]), XP_UMMA = 4
 const size_t XP_SMEM_MAX = 220 * 1024;
 const size_t XP_SCRATCH_MAX = (size_t)256 << 20;
 
+// The kernels' shared memory limits, the device's, ONCE per plan and never in front of a launch: a limit belongs to the function on a device, not to the launch or the plan, and rings are as deep as
+// the call leaves room for.  Set to a launch's own need, one thread's could be lowered by another's between its setting and its launch, which the driver then refused.
+template <typename... K> int set_max_dyn_all(b200_plan *p, int maxdyn, K... kerns) {
+    cudaError_t e = cudaSuccess;
+    ((e = e == cudaSuccess ? set_max_dyn(kerns, maxdyn) : e), ...);
+    CK(e);
+    return B200_OK;
+}
+int xp_smem_attrs(b200_plan *p, int device) { // the products'
+    int maxdyn = 0;
+    CK(cudaDeviceGetAttribute(&maxdyn, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    return set_max_dyn_all(p, maxdyn, k_xp_gemm<XP_STORE, 8>, k_xp_gemm<XP_STORE, 4>, k_xp_gemm<XP_STORE, 2>, k_xp_gemm<XP_STORE, 1>, k_xp_gemm<XP_RESID, 8>, k_xp_gemm<XP_RESID, 4>, k_xp_gemm<XP_RESID, 2>,
+                           k_xp_gemm<XP_RESID, 1>, k_xp_gemm<XP_GATEUP, 8>, k_xp_gemm<XP_GATEUP, 4>, k_xp_gemm<XP_GATEUP, 2>, k_xp_gemm<XP_GATEUP, 1>, k_xt_gemm<XP_STORE, 96>, k_xt_gemm<XP_STORE, 128>,
+                           k_xt_gemm<XP_RESID, 96>, k_xt_gemm<XP_RESID, 128>);
+}
+int xp_smem_attrs(b200_plan *p) {
+    int maxdyn = 0;
+    CK(cudaDeviceGetAttribute(&maxdyn, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device));
+    int rc = xp_smem_attrs(p, p->device);
+    if (!rc) rc = set_max_dyn_all(p, maxdyn, k_xp_rope_kv);
+    if (!rc)
+        rc = xp_by_head_size(p->cfg.head_size, [&](auto hs_c) -> int {
+            constexpr int HS = decltype(hs_c)::value;
+            int rc = set_max_dyn_all(p, maxdyn, k_xp_attention<HS, 4, 512>, k_xp_attention<HS, 1, 256>);
+            if constexpr (HS >= 128) return rc ? rc : set_max_dyn_all(p, maxdyn, k_xp_attention<HS, 2, 512>);
+            else return rc ? rc : set_max_dyn_all(p, maxdyn, k_xp_attention<HS, 4, 256>);
+        });
+    return rc;
+}
+
 int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide);
 int exact_prefill_umma_alloc(b200_plan *p, int rows, int wide);
 size_t xp_rope_smem_bytes(const b200_config &g) { return (size_t)(g.n_heads + g.n_kv_heads) * (g.head_size + 1) * 4; } // k_xp_rope_kv: a token's query and key heads
@@ -1318,6 +1348,7 @@ size_t xp_rope_smem_bytes(const b200_config &g) { return (size_t)(g.n_heads + g.
 int exact_prefill_init(b200_plan *p) {
     const b200_config &g = p->cfg;
     if (p->wtype != B200_GGML_Q8_0 || !p->use_stream || g.tp_size > 1) { p->xp.why = "the plan's weights are not Q8_0 on the streaming path"; return B200_OK; }
+    if (int rc = xp_smem_attrs(p)) return rc;
     if (xp_rope_smem_bytes(g) > XP_SMEM_MAX) { p->xp.why = "a token's query and key heads are wider than shared memory"; return B200_OK; }
     const int chunk = p->prefill_batch < g.context_length ? p->prefill_batch : g.context_length;
     const int rows = (chunk + 63) / 64 * 64, nqkv = p->qd + 2 * p->kvd, wide = p->qd > g.dim ? p->qd : g.dim;
@@ -1437,7 +1468,6 @@ int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps &mw_u
         // layer, 36 tokens: 33.7 us with three stages, 27.6 with five)
         const int per_sm = std::min(((int)(grid.x * grid.y) + p->n_sms - 1) / p->n_sms, T::RESIDENT);
         const int stages = std::max(XP_STAGES, std::min(XP_STAGES_MAX, ((int)XP_SMEM_MAX / per_sm - 2048) / (T::STAGE + 16)));
-        CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::bytes(stages)));
         kern<<<grid, XP_THREADS + 32, T::bytes(stages), p->stream>>>(mw, ma[NJ == 8 ? 3 : NJ == 4 ? 2 : NJ - 1], W, p->xp.rows, n, out, ldo, hq, hh, hs, xp_last(p), 1.0f, stages, p->d_err);
         CK(cudaGetLastError());
         return B200_OK;
@@ -1447,7 +1477,6 @@ int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps &mw_u
         else {
             constexpr int N = decltype(rows)::value;
             auto kern = k_xt_gemm<MODE, N>;
-            CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XtSmem<N>::BYTES));
             const int tiles = (n + XT_TOK - 1) / XT_TOK * ((W.rows + N - 1) / N);
             kern<<<std::min(tiles, p->n_sms), XT_THREADS, XtSmem<N>::BYTES, p->stream>>>(mw_umma, ma_umma, W, n, out, ldo, 1.0f, p->d_err);
             CK(cudaGetLastError());
@@ -1471,7 +1500,6 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     const int nqkv = p->qd + 2 * p->kvd;
     const size_t ctx_kv = (size_t)g.context_length * p->kvd;
     const size_t rope_smem = xp_rope_smem_bytes(g);
-    CK(cudaFuncSetAttribute(k_xp_rope_kv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
     auto halves = [&](const TileMat &W, __half *h) { return xp_kernel(p, W, n) >= XP_UMMA ? h : nullptr; }; // what the product of W reads: FP16 quants, or bytes
     auto norm = [&](bool embed, const float *w, __half *ah) {
         return by_norm_terms(g.dim, [&](auto e_c) -> int {
@@ -1495,7 +1523,6 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
                     const size_t slots = c.scratch_bytes / ((size_t)qt * xp_score_stride(nt) * 4);
                     if ((size_t)ctas > slots) ctas = (int)slots;
                 }
-                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
                 kern<<<ctas, threads, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, ah, c.AS, c.rows, scratch ? c.scratch : nullptr, xp_last(p));
                 CK(cudaGetLastError());
                 return B200_OK;
@@ -2321,19 +2348,20 @@ static int run_exact_prefill_wait(int form, uint32_t *codes, float *ms) {
         const unsigned char *q = mem + w_bytes;
         const float *s = reinterpret_cast<const float *>(mem + w_bytes + q_bytes);
         unsigned char *o = mem + w_bytes + q_bytes + s_bytes;
+        int dev = 0;
+        CK(cudaGetDevice(&dev));
+        if (int rc = xp_smem_attrs(p, dev)) return rc;
         XpMaps mw, whole, half;
         if (xp_map_weights(&mw, W, umma ? XT_BOX : XP_ROWS) || xp_map_acts(&whole, q, umma, s, tok_pad, cols, tok) || xp_map_acts(&half, q, umma, s, tok_pad, cols, tok / 2)) return B200_ERR_UNSUPPORTED;
         const XpMaps starved = form == 3 ? XpMaps{half.q, whole.s} : form == 4 ? XpMaps{whole.q, half.s} : half;
         auto launch = [&](const XpMaps &acts) -> int {
             if (umma) {
-                CK(cudaFuncSetAttribute(k_xt_gemm<XP_STORE, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, XtSmem<128>::BYTES));
                 k_xt_gemm<XP_STORE, 128><<<1, XT_THREADS, XtSmem<128>::BYTES>>>(mw, acts, W, tok, reinterpret_cast<float *>(o), rows, 1.0f, d_err);
             } else {
                 const int stages = form == 0 ? XP_STAGES : XP_STAGES_MAX;
                 // (hidden units: 32 of 16 tokens as bytes, their scales, and the last token's units, bytes and scale)
                 const XpLast last{nullptr, reinterpret_cast<int8_t *>(o + 2304), nullptr, reinterpret_cast<float *>(o + 2560), reinterpret_cast<float *>(o + 2048)};
                 auto kern = form == 2 ? k_xp_gemm<XP_GATEUP, 2> : k_xp_gemm<XP_STORE, 2>;
-                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XpTile<2>::bytes(stages)));
                 kern<<<dim3(1, 1), XP_THREADS + 32, XpTile<2>::bytes(stages)>>>(mw, acts, W, tok_pad, tok, reinterpret_cast<float *>(o), rows, reinterpret_cast<int8_t *>(o), nullptr,
                                                                                 reinterpret_cast<float *>(o + 1024), last, 1.0f, stages, d_err);
             }
