@@ -289,9 +289,9 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_xt_gemm(const __grid_constant
 
 // ---- hidden units behind the gate/up product: Q8_0(silu(gate) * up), FP16 quants (or bytes) and scales -------------------------------
 // A warp takes two blocks of 32 units of a token, a lane two units: G's columns come in groups gate 2g, gate 2g + 1, up 2g, up 2g + 1.  A launch of its own because the double
-// precision of the activation would stand between the tiles of the product: 360 us in its epilogue against 303 + 30 us, 512 tokens, 8B layer.
+// precision of the activation would stand between the tiles of the product: 360 us in its epilogue against 303 + 30 us, 512 tokens, 8B layer.  Tokens are the grid's x: y ends at 65535.
 __global__ void __launch_bounds__(256) k_xt_swiglu(const float *__restrict__ G, int hidden, int n, int8_t *__restrict__ HQ, __half *__restrict__ HH, float *__restrict__ HS, int lds, XpLast last) {
-    const int lane = threadIdx.x & 31, pair = blockIdx.x * 8 + (threadIdx.x >> 5), t = blockIdx.y, unit = pair * 64 + 2 * lane;
+    const int lane = threadIdx.x & 31, pair = blockIdx.y * 8 + (threadIdx.x >> 5), t = blockIdx.x, unit = pair * 64 + 2 * lane;
     if (pair * 64 >= hidden) return;
     const bool live = unit < hidden; // (an odd number of blocks)
     float4 g = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -1455,7 +1455,7 @@ int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps &mw_u
             const int hidden = W.rows / 2;
             int rc = xp_gemm<XP_STORE>(p, W, mw, mw_umma, ma, ma_umma, n, p->xp.G, W.rows, nullptr, nullptr, nullptr);
             if (rc) return rc;
-            k_xt_swiglu<<<dim3((hidden / 32 + 15) / 16, n), 256, 0, p->stream>>>(p->xp.G, hidden, n, hq, hh, hs, p->xp.rows, xp_last(p));
+            k_xt_swiglu<<<dim3(n, (hidden / 32 + 15) / 16), 256, 0, p->stream>>>(p->xp.G, hidden, n, hq, hh, hs, p->xp.rows, xp_last(p));
             CK(cudaGetLastError());
             return B200_OK;
         }
