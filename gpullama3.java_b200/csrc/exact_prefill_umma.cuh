@@ -177,7 +177,6 @@ __global__ void __launch_bounds__(XT_THREADS, 1) k_xt_gemm(const __grid_constant
                 for (int q = max(0, n_w - XT_W_STAGES); q < n_w; q++) xp_wait(wfull0 + 8 * (q % XT_W_STAGES), (q / XT_W_STAGES) & 1, err);
                 for (int q = max(0, n_a - 2); q < n_a; q++) xp_wait(afull0 + 8 * (q & 1), (q >> 1) & 1, err);
             }
-            __syncwarp();
         } else if (warp == XT_SUM_WARPS + 5) { // ---- products: the warp walks together (addresses and phases stay in uniform registers), one lane issues
             constexpr uint32_t idesc = pg::umma_idesc_f16(XT_TOK, N);
             uint32_t lead;
