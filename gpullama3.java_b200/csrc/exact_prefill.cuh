@@ -391,11 +391,14 @@ inline int xp_map_weights(XpMaps *maps, const TileMat &W, int rows) {
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return q == CUDA_SUCCESS && s == CUDA_SUCCESS ? 0 : -2;
 }
-// activations [rows][cols] (int8: boxes of 128 columns x the tile's tokens; FP16: of 64 columns) and their scales [blocks][rows] (boxes of the tile's tokens x 4 blocks)
-inline int xp_map_acts(XpMaps *maps, const void *q, bool halves, const float *s, int rows, int cols, int nt) {
+// activations [rows][cols] (int8: boxes of 128 columns x the tile's tokens; FP16: of 64 columns) and their scales [blocks][lds] (boxes of the tile's tokens x 4 blocks), from token `first` on
+inline int xp_map_acts(XpMaps *maps, const void *q, bool halves, const float *s, int lds, int cols, int nt, int first = 0) {
+    const int rows = lds - first;
+    q = static_cast<const int8_t *>(q) + (size_t)first * cols * (halves ? 2 : 1);
+    s += first;
     pg::EncodeTiledFn fn = pg::encode_fn();
     if (!fn) return -1;
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * (halves ? 2 : 1)}, sdims[2] = {(cuuint64_t)rows, (cuuint64_t)cols / 32}, sstrides[1] = {(cuuint64_t)rows * 4};
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * (halves ? 2 : 1)}, sdims[2] = {(cuuint64_t)rows, (cuuint64_t)cols / 32}, sstrides[1] = {(cuuint64_t)lds * 4};
     cuuint32_t box[2] = {halves ? 64u : 128u, (cuuint32_t)nt}, sbox[2] = {(cuuint32_t)nt, 4}, estr[2] = {1, 1};
     const CUresult rq = fn(&maps->q, halves ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

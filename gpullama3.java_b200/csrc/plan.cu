@@ -138,11 +138,13 @@ struct b200_plan {
         float *scratch = nullptr; // score rows of contexts whose rows do not fit shared memory
         size_t scratch_bytes = 0;
         __half *AH = nullptr, *HH = nullptr; // the quants as FP16 numbers, for the tcgen05 product (exact_prefill_umma.cuh; nullptr: no room)
-        float *G = nullptr;                  // the gate and up rows of chunks whose SwiGLU is a launch of its own
+        float *G = nullptr;                  // the gate and up rows of a slice of tokens (XP_SLICE) whose SwiGLU is a launch of its own
         struct Maps { XpMaps qkv, wo, gu, w2; }; // a layer's weights
         std::vector<Maps> maps, maps_umma;
         XpMaps mA[4], mATT[4], mH[4]; // activations in tiles of 8, 16, 32, 64 tokens: AQ with rows of dim and of the query width, HQ
         XpMaps hA, hATT, hH;          // the same as FP16, in tiles of 128
+        struct Slice { XpMaps m[4], h; };
+        std::vector<Slice> slices;    // AQ and AH with rows of dim, from the second slice on
         int64_t chunks = 0;           // multiplied at once so far
         int tile = -1;                // kernel of every product, as an index into XP_KERNELS (B200_XP_TILE; -1: by the model)
         std::string why;              // rows == 0: why not
@@ -1303,6 +1305,8 @@ const XpKernel XP_KERNELS[] = {{64, 64, XP_ROWS, 158.f, 103.f, 0.f}, {32, 32, XP
 // From so many tokens on SwiGLU is a launch behind the gate/up product: in double precision in the product's epilogue it holds up the CTAs that multiply (8B layer, 512 tokens 384 -> 333 us,
 // then on tcgen05; whole prompts of 129 - 513 tokens 0 - 3 % shorter, of 37 - 97 the same).
 const int XP_SPLIT_TOKENS = 128;
+// ... of so many tokens at a time: its gate and up rows are 32-bit floats in a buffer that the plan keeps (8B layer: 0.9 GB; 15 GB for a chunk of 131072 tokens at once).
+const int XP_SLICE = 8192;
 const int XP_N_KERNELS = sizeof(XP_KERNELS) / sizeof(XP_KERNELS[0]), XP_UMMA = 4; // the first of the tcgen05 kernels
 
 const size_t XP_SMEM_MAX = 220 * 1024;
@@ -1369,6 +1373,7 @@ int exact_prefill_init(b200_plan *p) {
         p->xp.AH = p->xp.HH = nullptr;
         p->xp.G = nullptr;
         p->xp.maps_umma.clear();
+        p->xp.slices.clear();
     }
     return B200_OK;
 }
@@ -1421,11 +1426,17 @@ int exact_prefill_umma_alloc(b200_plan *p, int rows, int wide) {
     int rc;
     if ((rc = dalloc(p, &c.AH, (size_t)rows * wide * 2))) return rc;
     if ((rc = dalloc(p, &c.HH, (size_t)rows * g.hidden_dim * 2))) return rc;
-    if ((rc = dalloc(p, &c.G, (size_t)rows * 2 * g.hidden_dim * 4))) return rc;
+    if ((rc = dalloc(p, &c.G, (size_t)std::min(rows, XP_SLICE) * 2 * g.hidden_dim * 4))) return rc;
     CK(cudaMemset(c.AH, 0, (size_t)rows * wide * 2)); // (as AQ and HQ)
     CK(cudaMemset(c.HH, 0, (size_t)rows * g.hidden_dim * 2));
     bool ok = !refused("umma") && xp_map_acts(&c.hA, c.AH, true, c.AS, rows, g.dim, XT_TOK) == 0 && xp_map_acts(&c.hATT, c.AH, true, c.AS, rows, p->qd, XT_TOK) == 0 &&
               xp_map_acts(&c.hH, c.HH, true, c.HS, rows, g.hidden_dim, XT_TOK) == 0;
+    c.slices.resize((rows - 1) / XP_SLICE);
+    for (int i = 0; ok && i < (int)c.slices.size(); i++) {
+        const int first = (i + 1) * XP_SLICE;
+        ok = xp_map_acts(&c.slices[i].h, c.AH, true, c.AS, rows, g.dim, XT_TOK, first) == 0;
+        for (int k = 0; ok && k < 4; k++) ok = xp_map_acts(&c.slices[i].m[k], c.AQ, false, c.AS, rows, g.dim, 8 << k, first) == 0;
+    }
     c.maps_umma.resize(g.n_layers);
     for (int l = 0; ok && l < g.n_layers; l++) ok = xp_map_layer(&c.maps_umma[l], p->layers[l], XT_BOX);
     return ok ? B200_OK : fail(p, B200_ERR_UNSUPPORTED, "the driver does not make the tensor maps of the tcgen05 product");
@@ -1448,15 +1459,20 @@ int xp_kernel(const b200_plan *p, const TileMat &W, int n) { // the product's ke
 }
 // out (MODE XP_STORE) or out += the product (XP_RESID); XP_GATEUP: hidden units, as bytes to hq or (hh) as FP16 numbers
 template <int MODE>
-int xp_gemm(b200_plan *p, const TileMat &W, const XpMaps &mw, const XpMaps &mw_umma, const XpMaps (&ma)[4], const XpMaps &ma_umma, int n, float *out, int ldo, int8_t *hq, __half *hh, float *hs) {
-    const int kernel = xp_kernel(p, W, n);
+int xp_gemm(b200_plan *p, int kernel, const TileMat &W, const XpMaps &mw, const XpMaps &mw_umma, const XpMaps (&ma)[4], const XpMaps &ma_umma, int n, float *out, int ldo, int8_t *hq, __half *hh,
+            float *hs) {
     if constexpr (MODE == XP_GATEUP)
         if (kernel >= XP_UMMA || (p->xp.G && n >= XP_SPLIT_TOKENS)) { // SwiGLU in a launch of its own
             const int hidden = W.rows / 2;
-            int rc = xp_gemm<XP_STORE>(p, W, mw, mw_umma, ma, ma_umma, n, p->xp.G, W.rows, nullptr, nullptr, nullptr);
-            if (rc) return rc;
-            k_xt_swiglu<<<dim3(n, (hidden / 32 + 15) / 16), 256, 0, p->stream>>>(p->xp.G, hidden, n, hq, hh, hs, p->xp.rows, xp_last(p));
-            CK(cudaGetLastError());
+            for (int i = 0, first = 0; first < n; i++, first += XP_SLICE) {
+                const int m = std::min(n - first, XP_SLICE);
+                const auto *slice = i ? &p->xp.slices[i - 1] : nullptr;
+                int rc = xp_gemm<XP_STORE>(p, kernel, W, mw, mw_umma, slice ? slice->m : ma, slice ? slice->h : ma_umma, m, p->xp.G, W.rows, nullptr, nullptr, nullptr);
+                if (rc) return rc;
+                const size_t at = (size_t)first * hidden;
+                k_xt_swiglu<<<dim3(m, (hidden / 32 + 15) / 16), 256, 0, p->stream>>>(p->xp.G, hidden, n - first, hq + at, hh ? hh + at : nullptr, hs + first, p->xp.rows, xp_last(p));
+                CK(cudaGetLastError());
+            }
             return B200_OK;
         }
     auto go = [&](auto nj) -> int {
@@ -1500,7 +1516,10 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     const int nqkv = p->qd + 2 * p->kvd;
     const size_t ctx_kv = (size_t)g.context_length * p->kvd;
     const size_t rope_smem = xp_rope_smem_bytes(g);
-    auto halves = [&](const TileMat &W, __half *h) { return xp_kernel(p, W, n) >= XP_UMMA ? h : nullptr; }; // what the product of W reads: FP16 quants, or bytes
+    // the layers are alike; a product's kernel says what it reads: FP16 quants, or bytes
+    const LayerW &first = p->layers[0];
+    const int k_qkv = xp_kernel(p, first.tqkv, n), k_wo = xp_kernel(p, first.two, n), k_gu = xp_kernel(p, first.tgu, n), k_w2 = xp_kernel(p, first.tw2, n);
+    auto halves = [&](int kernel, __half *h) { return kernel >= XP_UMMA ? h : nullptr; };
     auto norm = [&](bool embed, const float *w, __half *ah) {
         return by_norm_terms(g.dim, [&](auto e_c) -> int {
             constexpr int E = decltype(e_c)::value;
@@ -1541,15 +1560,15 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
         const auto &m = c.maps[l], &mu = c.maps_umma.empty() ? m : c.maps_umma[l];
         float *kc = p->key_cache + (size_t)l * ctx_kv, *vc = p->value_cache + (size_t)l * ctx_kv;
         int rc;
-        if ((rc = norm(l == 0, L.attn_norm, halves(L.tqkv, c.AH)))) return rc;
-        if ((rc = xp_gemm<XP_STORE>(p, L.tqkv, m.qkv, mu.qkv, c.mA, c.hA, n, c.QKV, nqkv, nullptr, nullptr, nullptr))) return rc;
+        if ((rc = norm(l == 0, L.attn_norm, halves(k_qkv, c.AH)))) return rc;
+        if ((rc = xp_gemm<XP_STORE>(p, k_qkv, L.tqkv, m.qkv, mu.qkv, c.mA, c.hA, n, c.QKV, nqkv, nullptr, nullptr, nullptr))) return rc;
         k_xp_rope_kv<<<n, 256, rope_smem, p->stream>>>(c.QKV, kc, vc, g.head_size, g.n_heads, g.n_kv_heads, p->kflags, L.q_norm, L.k_norm, g.rms_norm_eps, p->rope_cr, p->rope_ci, start_pos);
         CK(cudaGetLastError());
-        if ((rc = attention(kc, vc, halves(L.two, c.AH)))) return rc;
-        if ((rc = xp_gemm<XP_RESID>(p, L.two, m.wo, mu.wo, c.mATT, c.hATT, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
-        if ((rc = norm(false, L.ffn_norm, halves(L.tgu, c.AH)))) return rc;
-        if ((rc = xp_gemm<XP_GATEUP>(p, L.tgu, m.gu, mu.gu, c.mA, c.hA, n, nullptr, 0, c.HQ, halves(L.tw2, c.HH), c.HS))) return rc;
-        if ((rc = xp_gemm<XP_RESID>(p, L.tw2, m.w2, mu.w2, c.mH, c.hH, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
+        if ((rc = attention(kc, vc, halves(k_wo, c.AH)))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, k_wo, L.two, m.wo, mu.wo, c.mATT, c.hATT, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
+        if ((rc = norm(false, L.ffn_norm, halves(k_gu, c.AH)))) return rc;
+        if ((rc = xp_gemm<XP_GATEUP>(p, k_gu, L.tgu, m.gu, mu.gu, c.mA, c.hA, n, nullptr, 0, c.HQ, halves(k_w2, c.HH), c.HS))) return rc;
+        if ((rc = xp_gemm<XP_RESID>(p, k_w2, L.tw2, m.w2, mu.w2, c.mH, c.hH, n, c.X, g.dim, nullptr, nullptr, nullptr))) return rc;
     }
     // the single-token buffers hold what the last token's own step would have left there (the others: XpLast)
     CK(cudaMemcpyAsync(p->x, c.X + (size_t)(n - 1) * g.dim, (size_t)g.dim * 4, cudaMemcpyDeviceToDevice, p->stream));
