@@ -1302,9 +1302,11 @@ template <typename F> int xp_by_head_size(int hs, F &&f) { // f(integral_constan
 struct XpKernel { int code, tok, rows; float chain, share, fixed; }; // code: B200_XP_TILE
 const XpKernel XP_KERNELS[] = {{64, 64, XP_ROWS, 158.f, 103.f, 0.f}, {32, 32, XP_ROWS, 115.f, 58.f, 0.f}, {16, 16, XP_ROWS, 91.f, 40.f, 0.f}, {8, 8, XP_ROWS, 91.f, 34.f, 0.f},
                                {12896, XT_TOK, 96, 0.f, 284.f, 6000.f}, {128128, XT_TOK, 128, 0.f, 340.f, 6000.f}};
-// From so many tokens on SwiGLU is a launch behind the gate/up product: in double precision in the product's epilogue it holds up the CTAs that multiply (8B layer, 512 tokens 384 -> 333 us,
-// then on tcgen05; whole prompts of 129 - 513 tokens 0 - 3 % shorter, of 37 - 97 the same).
-const int XP_SPLIT_TOKENS = 128;
+// From so many hidden units per SM on, over all tokens, SwiGLU is a launch behind the gate/up product: in double precision in the product's epilogue it holds up the CTAs that multiply
+// (8B layer, 512 tokens 384 -> 333 us, then on tcgen05), but a launch and a pass over the rows cost a small product more.  Two or three layers and a step, behind the product against in the
+// epilogue: at 900 - 2700 units per SM (256 wide models, 64 - 512 tokens) 0.4 - 8 us more (2 %), 2700 - 7200 (1536 to 4096 wide, 64 - 250 tokens) between 0.5 % less and 1.6 % more, 7700 and
+// above 0.3 % more to 2.9 % less (8B, 99 tokens 832 and 851 us; 1B, 128 tokens, 7100 units: 427 and 420; 512 tokens, 28300: 909 and 930).
+const int XP_SPLIT_UNITS = 7500;
 // ... of so many tokens at a time: its gate and up rows are 32-bit floats in a buffer that the plan keeps (8B layer: 0.9 GB; 15 GB for a chunk of 131072 tokens at once).
 const int XP_SLICE = 8192;
 const int XP_N_KERNELS = sizeof(XP_KERNELS) / sizeof(XP_KERNELS[0]), XP_UMMA = 4; // the first of the tcgen05 kernels
@@ -1462,7 +1464,7 @@ template <int MODE>
 int xp_gemm(b200_plan *p, int kernel, const TileMat &W, const XpMaps &mw, const XpMaps &mw_umma, const XpMaps (&ma)[4], const XpMaps &ma_umma, int n, float *out, int ldo, int8_t *hq, __half *hh,
             float *hs) {
     if constexpr (MODE == XP_GATEUP)
-        if (kernel >= XP_UMMA || (p->xp.G && n >= XP_SPLIT_TOKENS)) { // SwiGLU in a launch of its own
+        if (kernel >= XP_UMMA || (p->xp.G && (int64_t)n * (W.rows / 2) >= (int64_t)XP_SPLIT_UNITS * p->n_sms)) { // SwiGLU in a launch of its own
             const int hidden = W.rows / 2;
             for (int i = 0, first = 0; first < n; i++, first += XP_SLICE) {
                 const int m = std::min(n - first, XP_SLICE);

@@ -53,3 +53,9 @@ def test_without_its_buffers(pkg, monkeypatch):
         used.append(plan.device_bytes)
         plan.free()
     assert used[0] < used[1]
+
+
+@pytest.mark.parametrize("side", [0, 1])
+def test_swiglu_line(pkg, side):
+    """On both sides of the line from which SwiGLU is a launch behind the gate/up product (csrc/plan.cu, XP_SPLIT_UNITS hidden units per SM): 12288 units are 90.3 tokens on 148 SMs."""
+    run(pkg, pkg.synth.Shape("qwen3", 256, 12288, 1, 2, 1, 128, 128, False, 500000.0, 1e-5), [90 + side])
