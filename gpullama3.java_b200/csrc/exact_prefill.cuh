@@ -244,7 +244,10 @@ __global__ void __launch_bounds__(XP_THREADS + 32, XpTile<NJ>::RESIDENT) k_xp_ge
                     if (++stage == stages) { stage = 0; ph ^= 1u; }
                 }
             // Nothing leaves with its copies in flight, whoever gave up: a multiplying warp whose wait did goes on without looking at its stages, and all chunks may be under way by then.
-            for (int q = max(0, c - stages); q < c; q++) xp_wait(full0 + 8 * (q % stages), (q / stages) & 1, err);
+            for (c = min(c, stages); c > 0; c--) { // (the newest first: behind it the others have landed too, as a rule)
+                if (stage == 0) { stage = stages; ph ^= 1u; }
+                xp_wait(full0 + 8 * --stage, ph ^ 1u, err);
+            }
         } // (the other lanes are gone, or at the barrier below: held at one of the warp's instead they made the product 1 - 2 % slower)
         if (MODE == XP_GATEUP) { __syncthreads(); __syncthreads(); } // (the epilogue's)
         return;

@@ -51,8 +51,13 @@ def product(n_chunks, stages, rng, give_up, wait=True, drain="always", gateup=Fa
                 stage, ph = 0, ph ^ 1
             yield
         if drain == "always" or (drain == "own" and not ok):
-            for q in range(max(0, issued - stages), issued):
-                while filled[q % stages] % 2 == (q // stages) & 1:  # (its limit is far above the time of a copy)
+            for _ in range(min(issued, stages)):
+                if stage == 0:
+                    stage, ph = stages, ph ^ 1
+                stage -= 1
+                while filled[stage] % 2 == ph ^ 1:  # (its limit is far above the time of a copy)
+                    if not any(s == stage for s, _ in in_flight):
+                        raise Hazard("waits for what was never issued")
                     yield
         yield from epilogue()
 
