@@ -401,8 +401,9 @@ __global__ void k_swiglu(float *__restrict__ hb, const float *__restrict__ hb2, 
 //   output   : xb = sum_t a_t * v_t, sequentially over t per element (saxpyInPlace, FloatTensor.java:221-227)
 // The current position's k/v come from shared memory / the packed qkv vector, older ones from the
 // FP32 cache.  Output as floats (xb) and/or quantised to Q8_0 (activation of the Wo matvec).
-// Bound by its chain.  The rows of earlier positions are asked for in front of the dependency wait, products are made by all four threads of a quad at once and only the adds go through it in
-// turn, and quarters without positions are left out: 13400 -> 7800 cycles at position 20 (64 entries a head), 18900 -> 13300 at position 100 (128 entries).
+// Bound by its chain.  The rows of earlier positions are asked for in front of the dependency wait, products are made by all four threads of a quad at once and only the
+// adds go through it in turn, and quarters without positions are left out: 13400 -> 7800 cycles at position 20 (64 entries a head), 18900 -> 13300 at position 100 (128
+// entries).
 // ------------------------------------------------------------------------------------------
 #define ATT_THREADS 512 // four threads per key (scores) and per output element (weighted sum): head size <= ATT_THREADS / 4
 
@@ -563,10 +564,10 @@ __device__ __forceinline__ void attention_split(float *sm, float *qkv, const flo
     }
     __syncthreads();
     const float sum = S.sum.result;
-    // ---- output (saxpyInPlace, FloatTensor.java:221-227): warp 0 adds, the others stay ahead of it: stages on their way, and the next one's rows multiplied by their weights where they lie.
-    // Up to 4096 positions the exponentials are all in shared memory still and become the weights there at once; a longer row's come from L2 stage by stage.  3000 positions, 128 entries a
-    // head: 42000 cycles with warp 0 multiplying too and every weight from L2 (a round trip per stage that the adds did not cover), 34000 with the weights in place, 31000 so; the adds
-    // alone are 13000 (4.3 cycles each).
+    // ---- output (saxpyInPlace, FloatTensor.java:221-227): warp 0 adds, the others stay ahead of it: stages on their way, and the next one's rows multiplied by their
+    // weights where they lie.  Up to 4096 positions the exponentials are all in shared memory still and become the weights there at once; a longer row's come from L2 stage
+    // by stage.  3000 positions, 128 entries a head: 42000 cycles with warp 0 multiplying too and every weight from L2 (a round trip per stage that the adds did not cover),
+    // 34000 with the weights in place, 31000 so; the adds alone are 13000 (4.3 cycles each).
     const bool whole = nt <= 4096;
     auto weights = [&](int c) {
         const int i = tid - 32, t = c * ATT_VT + i;
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     const int pos = st->pos, nt = pos + 1; // set before the step's first kernel started and left alone until its last one
     const bool split = cluster > 1; // (the host launches clusters from ATT_SPLIT positions on)
     // K and V rows of the earlier positions were written by earlier steps, so they are asked for in front of the wait: the first pass' rows into registers, the others
-    // into L2, one 128-byte line per request (the weight stream carries an evict_first policy; without the prefetch these rows come from HBM every layer).
+    // into L2, one 128-byte line per request (the weight stream carries an evict_first policy; without the prefetch they could come from HBM every layer).
     constexpr int LINES = HS / 32;
     if (!split) {
         for (int i = tid + ATT_THREADS / 4 * LINES; i < pos * LINES; i += ATT_THREADS) {

@@ -5,13 +5,15 @@
 // there token i only reads the cache rows that the earlier tokens of the same layer have written.  Per layer:
 //
 //   AQ <- Q8_0(rmsnorm(X) * w)                 k_xp_norm       a CTA per token
-//   QKV <- AQ [Wq;Wk;Wv]^T                     k_xp_gemm<XP_STORE>, or k_xt_gemm (exact_prefill_umma.cuh)
+//   QKV <- AQ [Wq;Wk;Wv]^T                     k_xp_gemm<XP_STORE>
 //   q, k <- (Qwen3 head norm,) rotation; k, v -> cache     k_xp_rope_kv
 //   AQ <- Q8_0(softmax(q k^T / sqrt(hs)) v)    k_xp_attention  a CTA per (64, 32 or 8 tokens, head)
 //   X += AQ Wo^T                               k_xp_gemm<XP_RESID>
 //   AQ <- Q8_0(rmsnorm(X) * w)                 k_xp_norm
-//   HQ <- Q8_0(silu(AQ W1^T) * (AQ W3^T))      k_xp_gemm<XP_GATEUP>
+//   HQ <- Q8_0(silu(AQ W1^T) * (AQ W3^T))      k_xp_gemm<XP_GATEUP>, or k_xp_gemm<XP_STORE> and k_xt_swiglu (exact_prefill_umma.cuh) where there is much of it
 //   X += HQ W2^T                               k_xp_gemm<XP_RESID>
+//
+// Each of the four products is k_xt_gemm's (exact_prefill_umma.cuh, tcgen05) where the host's time model says so: long chunks.  Its operands are FP16 numbers, AH and HH in AQ's and HQ's place.
 //
 // Measured on two layers of the 8B geometry, 512 tokens and the decode step behind them: 109.8 ms token by token, 1.94 ms here; two layers of the 4B
 // Qwen3 geometry, 36 tokens: 5.36 ms and 0.44 ms.
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(256, E <= 16 ? 4 : 1) k_xp_norm(float *__restr
 // issued the fetches between its chunks held the whole CTA up by half of its time: gate/up of 512 tokens, 8B layer, 388 us against 328 us so; W2 of 36 tokens, 4B layer, 43 against 28 us (a
 // deeper ring alone 43, all operands of a chunk in registers ahead 46).  Issue slots: 15.7 warp instructions per 16 x 8 tile and block, 10 of them the conversions, products and
 // adds (65 % of the slots, FMA pipe 57 %).
-// Long chunks' QKV, Wo and W2 are exact_prefill_umma.cuh's.
+// Long chunks' products are exact_prefill_umma.cuh's.
 #define XP_STAGES 3      // of a ring, at least;
 #define XP_STAGES_MAX 8  // and at most: as many as the CTAs of an SM have room for
 #define XP_ROWS 64

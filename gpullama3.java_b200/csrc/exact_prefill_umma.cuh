@@ -8,9 +8,10 @@
 // the tensor cores are on the next.
 //
 // Bound by: the sums.  Two warps a scheduler; a step of 16 columns (two tcgen05.ld, a wait, 8 packed products and 8 packed adds) takes 95 cycles and a block about 220 besides, in
-// which its barrier is waited for and handed back: 600 cycles for N = 128 (FMA pipe 50 %, tensor pipe 32 %).  Measured, 512 tokens, 8B layer: W2 149 us, Wo 53, QKV 82 gate/up 303 (185, 60, 86 and 328 us with mma.sync,
-// k_xp_gemm, which converts, multiplies twice and adds).  Without effect (gate/up 296 - 360 us): 12 and 16 warps of 32 columns, 8 or 32 columns a step, the next step's columns loaded ahead, all
-// columns loaded at once (setmaxnreg), neither conversion nor scale products; kind::i8 and a conversion in the sums 335 us; one warp that did not walk together for the products 434 us.
+// which its barrier is waited for and handed back: 600 cycles for N = 128 (FMA pipe 50 %, tensor pipe 32 %).  Measured, 512 tokens, 8B layer: W2 149 us, Wo 53, QKV 82,
+// gate/up 303 (185, 60, 86 and 328 us with mma.sync, k_xp_gemm, which converts, multiplies twice and adds).  Without effect (gate/up 296 - 360 us): 12 and 16 warps of
+// 32 columns, 8 or 32 columns a step, the next step's columns loaded ahead, all columns loaded at once (setmaxnreg), neither conversion nor scale products; kind::i8 and a
+// conversion in the sums 335 us; one warp that did not walk together for the products 434 us.
 //
 // Warps: 0-7 sums (warp w: lanes 32 (w % 4) .., columns (w / 4) N / 2 ..), 8-11 turn a stage's bytes into FP16 operands (thread = weight row) and its scales into S's operands
 // (one column of a zeroed tile), 12 TMA, 13 MMA.

@@ -397,7 +397,8 @@ static int ly_step_attention(b200_plan *p, int heads, int window, const float *q
     if (Y.split.o && window >= 64) { sp = p->n_sms / heads; if (sp > Y.max_splits) sp = Y.max_splits; if (sp < 1) sp = 1; }
     if ((wa.dk | wa.dv | wa.ldk | wa.ldv) % 4 == 0 && wa.dk <= 1024 && wa.dv <= 4 * LY_ATT_THREADS) {
         const size_t sm = ly::step_att_smem_floats(wa.dk, wa.dv, wa.window, sp) * 4;
-        // latent rows once and at once where they fit beside the rest (a CTA an SM: splits x heads are no more than that), else through the ring
+        // latent rows once and at once where those of the whole window (a causal layer's: the plan's context) fit beside the rest (a CTA an SM: splits x heads are no more than that), else
+        // through the ring
         const size_t latent = ly::step_att_latent_floats(wa.dk, wa.dv, wa.window, sp) * 4;
         if (ly::step_att_latent(kc, vc, wa) && latent <= (size_t)Y.smem_max && sp * heads <= p->n_sms)
             return launch_cluster(p, p->use_pdl, sp, ly::k_step_attention<2, true>, dim3(sp, heads), dim3(LY_ATT_THREADS), latent, q, wa, kc, vc, st, out);

@@ -1548,9 +1548,9 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
                 CK(cudaGetLastError());
                 return B200_OK;
             };
-            // 64 tokens per CTA (16 warps) share the staged keys and values while their score rows fit shared memory, else 32 (heads of 128 and more by 16 warps of two tokens: with eight of four, one CTA an SM, a
-            // third of the issue slots; 8B layer, 512 tokens 190 -> 174 us; smaller heads have no work for 16 in the value pass); a chunk too small to
-            // fill the SMs that way takes 8
+            // 64 tokens per CTA (16 warps) share the staged keys and values while their score rows fit shared memory, else 32: heads of 128 and more by 16 warps of two
+            // tokens (with eight of four, one CTA an SM, a third of the issue slots were used: 8B layer, 512 tokens 190 -> 174 us; smaller heads have no work for 16 warps in
+            // the value pass).  A chunk too small to fill the SMs that way takes 8.
             if ((n + 63) / 64 * g.n_heads >= p->n_sms && fits(64)) return go(k_xp_attention<HS, 4, 512>, 512, 64);
             if ((n + 31) / 32 * g.n_heads < p->n_sms) return go(k_xp_attention<HS, 1, 256>, 256, 8);
             if constexpr (HS >= 128) return go(k_xp_attention<HS, 2, 512>, 512, 32);

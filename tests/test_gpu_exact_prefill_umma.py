@@ -1,6 +1,6 @@
 """The tcgen05 product of the exact Q8_0 prefill (csrc/exact_prefill_umma.cuh): the cache and the logits behind the chunk are the token-by-token path's bit for bit.  Every product of
 the layer in tiles of 128 tokens x 96 or 128 weight rows (B200_XP_TILE): ragged and whole token tiles, row tiles that the rows do not fill, segments that are no multiple of a stage's
-128 columns, more tiles than SMs, and block scales over the whole FP16 range (subnormal, negative, large)."""
+128 columns, more tiles than SMs, and block scales over the whole FP16 range (subnormal, negative, large), on both sides of it at once where results stay finite."""
 import numpy as np
 import pytest
 
@@ -16,9 +16,11 @@ def run(pkg, shape, chunks, scales=None):
     if scales is not None:
         for name, (kind, dims, raw) in tensors.items():
             if len(dims) == 2 and name.startswith("blk."):
-                raw.reshape(-1, 34)[:, :2] = scales(np.random.default_rng(len(name)), raw.size // 34).astype(np.float16).view(np.uint8).reshape(-1, 2)
+                raw.reshape(-1, 34)[:, :2] = scales(np.random.default_rng(len(name)), raw.size // 34, name).astype(np.float16).view(np.uint8).reshape(-1, 2)
     model = pkg.loader.model_from_tensors(shape, Q8, tensors, n + 4)
-    check(pkg, model, np.random.default_rng(n).integers(0, shape.vocab, n + 1), chunks, n)
+    toks = np.random.default_rng(n).integers(0, shape.vocab, n + 1)
+    check(pkg, model, toks, chunks, n)
+    return model, toks
 
 
 # (dim, hidden, heads, key/value heads, head size): rows of three and of seven segments of 27 and 23 blocks; 96 + 2 * 32 rows and rows of 64 and 96 columns
@@ -39,7 +41,25 @@ def test_several_tiles_per_sm(pkg, monkeypatch, rows):
 @pytest.mark.parametrize("rows", [96, 128])
 def test_scales(pkg, monkeypatch, rows):
     monkeypatch.setenv("B200_XP_TILE", CODES[rows])
-    run(pkg, pkg.synth.SHAPES["tiny-llama"], [130], lambda rng, n: np.ldexp(rng.choice([-1.0, 1.0], n) * rng.uniform(1.0, 2.0, n), rng.integers(-26, -2, n)))
+    run(pkg, pkg.synth.SHAPES["tiny-llama"], [130], lambda rng, n, name: np.ldexp(rng.choice([-1.0, 1.0], n) * rng.uniform(1.0, 2.0, n), rng.integers(-26, -2, n)))
+
+
+@pytest.mark.parametrize("rows", [96, 128])
+def test_large_scales(pkg, monkeypatch, rows):
+    """Scales up to the largest FP16 numbers in queries, keys, gates and the attention's output, against values and up rows of the smallest, so that the hidden rows' scales and the logits stay finite."""
+    exponents = {"attn_q": (6, 16), "attn_k": (6, 16), "attn_v": (-24, -14), "attn_output": (6, 16), "ffn_gate": (6, 16), "ffn_up": (-24, -14), "ffn_down": (-12, -4)}
+    monkeypatch.setenv("B200_XP_TILE", CODES[rows])
+
+    def scales(rng, n, name):
+        lo, hi = exponents[name.split(".")[2]]
+        return np.ldexp(rng.choice([-1.0, 1.0], n) * rng.uniform(1.0, 1.99, n), rng.integers(lo, hi, n))
+
+    model, toks = run(pkg, pkg.synth.SHAPES["tiny-llama"], [130], scales)
+    plan = pkg.B200MasterPlan(model, prefill_batch_size=130)
+    plan.forward_batch_prefill(toks[:130], 0)
+    assert np.isfinite(plan.forward_decode(int(toks[130]), 130)[0]).all()
+    assert np.abs(plan.read_buffer("qkv", 64)).max() > 1e6
+    plan.free()
 
 
 def test_without_its_buffers(pkg, monkeypatch):
