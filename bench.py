@@ -810,7 +810,7 @@ def main():
             per_kernel[name] = {"ms": m, "GB/s": b / (m / 1e3) / 1e9, "bytes": b, "frac": b / (m / 1e3) / 1e9 / peak}
     persistent = dmode == 1
     traffic = None
-    tpath = os.path.join(ROOT, "profiles", "r2_decode_traffic.json")  # dram bytes per launch from the committed ncu --set full capture
+    tpath = os.path.join(ROOT, "profiles", "decode_traffic.json")  # dram bytes per launch from the committed ncu --set full capture
     if world == 1 and WORKLOAD == "llama-3-8b" and QUANT == "q8_0" and os.path.exists(tpath):
         with open(tpath) as f:
             traffic = json.load(f).get("persistent" if persistent else "graph")

@@ -64,7 +64,7 @@ __device__ __noinline__ void tp_wait(const TpCtx &t, int slot, unsigned seq) {
     unsigned long long t0 = 0;
     for (int k = 0; k < t.n; k++) {
         for (;;) {
-            unsigned v; // relaxed polls, ONE acquire fence after the last flag: ld.acquire in the loop is a load + CCTL.IVALL (an L1 flush per poll)
+            unsigned v; // relaxed polls, ONE acquire fence after the last flag: an ld.acquire in the loop empties the L1 at every poll
             asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(f + k) : "memory");
             if ((int)(v - seq) >= 0) break;
             if ((++it & 255u) == 0u && t.err) {
@@ -79,7 +79,7 @@ __device__ __noinline__ void tp_wait(const TpCtx &t, int slot, unsigned seq) {
             }
         }
     }
-    { // one acquire load after the relaxed polls (flags are monotone); a fence.acq_rel.sys here is a MEMBAR.SYS per wait
+    { // one acquire load after the relaxed polls (flags are monotone); a fence.acq_rel.sys per wait made tensor-parallel steps ~20 % slower
         unsigned v;
         asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
     }
@@ -151,7 +151,7 @@ __device__ __forceinline__ int quant_block_lane(float v, float &ascale) {
     return __float2int_rz(__fadd_rn(s, copysignf(0.5f, s)));
 }
 
-// 256-bit read-only streaming load (LDG.E.256 on sm_100a): one whole Q8_0 quant block per lane.
+// 256-bit read-only streaming load: one whole Q8_0 quant block per lane.
 __device__ __forceinline__ void ldg256_stream(const void *p, int (&r)[8]) {
     asm("ld.global.nc.L1::no_allocate.v8.s32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -175,7 +175,7 @@ __device__ __forceinline__ float f16_bits_to_f32_daz(unsigned h) {
 // Weight matrix as stored on the device.
 //   Q8_0: qs = int8 [rows][cols] row-major, sc = f16 scale [rows][cols/32]
 //         (GGUF's 34-byte blocks split at upload so the quants are 32-byte aligned: same
-//          1.0625 B/element, one LDG.256 per block).
+//          1.0625 B/element, one 256-bit load per block).
 //   F16 : qs = f16 [rows][cols], sc unused.  F32: qs = float.
 struct DevMat {
     const void *qs;

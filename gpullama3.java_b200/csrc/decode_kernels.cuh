@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(T, 1) k_test_seqsum2(const float *__restrict__
 //   per 32-block b:  isum_b = sum aq*wq (int32, exact);  term_b = (float)isum_b * (wScale_b * aScale_b)
 //   result = ((term_0 + term_1) + term_2) + ...      strictly in block order.
 // The activation quantisation is row-independent, so it arrives pre-quantised (xq, xs).
-// Mapping: a warp owns R rows; lane l owns blocks l, l+32, ... of each row (one LDG.256 per block,
+// Mapping: a warp owns R rows; lane l owns blocks l, l+32, ... of each row (one 256-bit load per block,
 // the warp reads 1 KB contiguous per instruction); block terms go to shared memory and lanes
 // 0..R-1 then walk their row's terms in order.
 // ------------------------------------------------------------------------------------------
@@ -214,7 +214,7 @@ __device__ __forceinline__ void q8_row_terms(const int8_t *__restrict__ qs, cons
 
 // Stage the quantised activation in shared memory as two planes of 16-byte half-blocks
 // (plane p holds bytes [16p,16p+16) of every block) so that lanes reading consecutive
-// blocks hit consecutive 16-byte slots: conflict-free LDS.128.
+// blocks hit consecutive 16-byte slots: no bank conflicts in their 16-byte loads.
 __device__ __forceinline__ void stage_activation(const int8_t *__restrict__ xq, const float *__restrict__ xs, int cols,
                                                  int4 *sxq, float *sxs) {
     const int nb = cols >> 5;

@@ -30,7 +30,7 @@
 #include "stream_matvec.cuh"
 
 #define PD_WARPS 16                     // consumer warps: 4 per SM sub-partition -- every phase of this kernel is a chain of dependent instructions,
-                                        // and the ncu samples (profiles/r2_pd_full_v2.summary.txt) show warps waiting on their own previous result
+                                        // and the ncu samples (profiles/persistent_decode_full.summary.txt) show warps waiting on their own previous result
 #define PD_CT (PD_WARPS * 32)           // consumer threads
 #define PD_THREADS (PD_CT + 32)         // + the producer warp
 #define PD_MAX_STAGES 32
@@ -132,9 +132,9 @@ __host__ __device__ inline PdSmem pd_layout(int dim, int qd, int hidden, int hea
 }
 
 // ---- bounded waits ----------------------------------------------------------------------------------------------------------
-// Polls are RELAXED loads; ONE acquire load of the same word follows the successful one.  (ld.acquire in the loop compiles to a
-// load plus CCTL.IVALL: every poll of thread 0 threw away the whole L1 of its SM; a trailing fence.acq_rel.sys instead costs a
-// MEMBAR.SYS per wait, which made tensor-parallel steps ~20 % slower.)
+// Polls are RELAXED loads; ONE acquire load of the same word follows the successful one.  (An ld.acquire in the loop makes every
+// poll of thread 0 an acquire, behind which its SM's L1 starts empty; a trailing fence.acq_rel.sys per wait instead made
+// tensor-parallel steps ~20 % slower.)
 __device__ __forceinline__ unsigned pd_ld_relaxed_gpu(const unsigned *p) {
     unsigned v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -185,7 +185,7 @@ __device__ __noinline__ void pd_arrive(const PdArgs &a, int slot, unsigned targe
         const bool x = cross && a.tp.n > 1;
         // gpu-scope fence per CTA, ONE system-scope fence by the last arriver below: the CTAs' peer stores reach system scope through the
         // cumulativity of the fence chain (CTA store -> fence.gpu -> atomic -> last arriver's atomic -> fence.sys -> flag).  A per-CTA
-        // __threadfence_system() here cost ~7 us per exchange at tp2 (148 MEMBAR.SYS waiting on NVLink round trips).
+        // __threadfence_system() here cost ~7 us per exchange at tp2 (148 system fences waiting on NVLink round trips).
         __threadfence();
         const unsigned old = atomicAdd(a.sync + slot, 1u);
         if (x && old + 1u == target) {

@@ -1,5 +1,5 @@
-// seqsum2.cuh -- the exact sequential-sum accumulator of the decode path's RMSNorms (the algorithm is validated on
-// the CPU by tools/seqsum2/proto.c, on the GPU by tools/seqsum2/harness.cu and tests/test_gpu_parity.py).
+// seqsum2.cuh -- the exact sequential-sum accumulator of the decode path's RMSNorms (tests/test_gpu_parity.py has the
+// adversarial cases).
 //
 // Same contract as block_seqsum_exact (seqsum.cuh): the bit-exact value of  s = 0; for (i) s = s + t[i]  for non-negative
 // float terms (InferenceCore.rmsnorm's accumulator, InferenceCore.java:39-48), evaluated by one CTA.  Where the first

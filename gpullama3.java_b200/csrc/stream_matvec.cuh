@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(SMV_THREADS, 1) k_stream_matvec_q8(SmvArgs a, 
     float *terms = reinterpret_cast<float *>(smem + L.off_terms) + (size_t)warp * 4 * L.nbs_pad;
     const unsigned char *sact = smem + L.off_xq;
     const float *sxs = reinterpret_cast<const float *>(smem + L.off_xs);
-    const int hsel = (lane >> 2) & 1; // half-swap: conflict-free LDS.128 over 32-byte strides
+    const int hsel = (lane >> 2) & 1; // half-swap: 16-byte loads over 32-byte strides without bank conflicts
 
     float *hvals = reinterpret_cast<float *>(smem + L.off_hvals);
     float best = -INFINITY;

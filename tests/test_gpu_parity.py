@@ -90,7 +90,7 @@ def test_decode_mid_geometries_f16(pkg, orc, shape, lanes):
                                               ("tiny-phi3-gqa", "Q8_0", "persistent"), ("tiny-phi3-gqa", "F16", "graph")])
 def test_decode_phi3_bit_exact(pkg, orc, make_model, shape, quant, mode):
     """Phi-3 (InferenceCore.forwardJavaPhi3, InferenceCore.java:699-800): fused attn_qkv / gate-up tensors split by rows at upload,
-    NeoX-pair RoPE without q/k norm.  Mini-like (multi-head, head size 96: graph only, FP16 through the round-1 kernels since dim 384
+    NeoX-pair RoPE without q/k norm.  Mini-like (multi-head, head size 96: graph only, FP16 through the non-streaming kernels since dim 384
     is not a multiple of 256) and medium-like (GQA, head size 128: also the persistent kernel and the FP16 rings)."""
     m = make_model(shape, getattr(pkg.gguf.GGMLType, quant), 24)
     assert m.model_type == "PHI_3" and m.configuration.arch == 2
@@ -106,8 +106,8 @@ def test_decode_phi3_mini_geometry(pkg, orc, quant):
     run_stream(pkg, orc, m, 16, 4, check_kv=True)
 
 
-def test_decode_f16_round1_kernels_still_exact(pkg, orc, make_model, monkeypatch):
-    """B200_F16_STREAM=0 keeps the round-1 launches (k_matvec_f16 + separate SwiGLU), the fallback for shapes the rings do not fit."""
+def test_decode_f16_non_streaming_kernels_still_exact(pkg, orc, make_model, monkeypatch):
+    """B200_F16_STREAM=0 keeps the non-streaming launches (k_matvec_f16 + separate SwiGLU), the fallback for shapes the rings do not fit."""
     monkeypatch.setenv("B200_F16_STREAM", "0")
     m = make_model("tiny-llama", pkg.gguf.GGMLType.F16, 24)
     run_stream(pkg, orc, m, 16, 8)

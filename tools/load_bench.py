@@ -6,7 +6,7 @@ reference's load-time metric, ModelLoader.java:102-106, and its first-execution 
 
 Writes a seeded synthetic GGUF of the real shape (no checkpoints offline), drops it from the process (the page cache may still hold it:
 reported as "warm"), then: parse + mmap (gguf.GGUFFile), b200_plan_create (pinned double buffer -> copy stream -> device staging ->
-repack kernels), and the same with the blocking round-1 path (B200_UPLOAD_SYNC=1)."""
+repack kernels), and the same with the blocking path (B200_UPLOAD_SYNC=1)."""
 import json
 import os
 import sys
