@@ -13,7 +13,8 @@
 //   HQ <- Q8_0(silu(AQ W1^T) * (AQ W3^T))      k_xp_gemm<XP_GATEUP>, or k_xp_gemm<XP_STORE> and k_xt_swiglu (exact_prefill_umma.cuh) where there is much of it
 //   X += HQ W2^T                               k_xp_gemm<XP_RESID>
 //
-// Each of the four products is k_xt_gemm's (exact_prefill_umma.cuh, tcgen05) where the host's time model says so: long chunks.  Its operands are FP16 numbers, AH and HH in AQ's and HQ's place.
+// Each of the four products is k_xt_gemm's (exact_prefill_umma.cuh, tcgen05) where the host's time model says so: long chunks.  Its operands are FP16 numbers, AH
+// and HH in AQ's and HQ's place.
 //
 // Measured on two layers of the 8B geometry, 512 tokens and the decode step behind them: 109.8 ms token by token, 1.94 ms here; two layers of the 4B
 // Qwen3 geometry, 36 tokens: 5.36 ms and 0.44 ms.
@@ -396,7 +397,8 @@ inline int xp_map_weights(XpMaps *maps, const TileMat &W, int rows) {
                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return q == CUDA_SUCCESS && s == CUDA_SUCCESS ? 0 : -2;
 }
-// activations [rows][cols] (int8: boxes of 128 columns x the tile's tokens; FP16: of 64 columns) and their scales [blocks][lds] (boxes of the tile's tokens x 4 blocks), from token `first` on
+// activations [rows][cols] (int8: boxes of 128 columns x the tile's tokens; FP16: of 64 columns) and their scales [blocks][lds] (boxes of the tile's tokens x 4
+// blocks), from token `first` on
 inline int xp_map_acts(XpMaps *maps, const void *q, bool halves, const float *s, int lds, int cols, int nt, int first = 0) {
     const int rows = lds - first;
     q = static_cast<const int8_t *>(q) + (size_t)first * cols * (halves ? 2 : 1);

@@ -1165,10 +1165,10 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, bool vali
 // ways), looks the distances up meanwhile, asks for the first tiles of its values before the softmax, and the parts are merged over distributed shared
 // memory, every CTA finishing its share of the head's entries.  Lanes that share a row take four of them at a time (U; one where a stage holds no more than a row per
 // group).  32 heads of 64, 900 keys, cap and distance table: 27 us there, 17 us with one row at a time, 13 us with four; 32 heads of 128, 2000 keys: 56 and 38 us.
-// Latent rows (LATENT): seven rows of 576 fill a stage, so a CTA's 64 keys took ten stages and their values, which lie in the same rows, eight more; all at once and once only,
-// the step of the 16-head layer takes 145 us instead of 154 at 511 keys, 131 instead of 142 at 60.  Shared memory is asked for by the plan's context, so that is where its reach ends: with eight
-// splits, contexts of 768 for rows of 576 and 512 value entries, of 1632 for rows of 272 and 256; beyond, every position takes the ring (511 keys: 154 us).  Separate keys and values that way lose
-// (16 heads of 64, 100 keys: 130 instead of 121 us).
+// Latent rows (LATENT): seven rows of 576 fill a stage, so a CTA's 64 keys took ten stages and their values, which lie in the same rows, eight more; all at once
+// and once only, the step of the 16-head layer takes 145 us instead of 154 at 511 keys, 131 instead of 142 at 60.  Shared memory is asked for by the plan's
+// context, so that is where its reach ends: with eight splits, contexts of 768 for rows of 576 and 512 value entries, of 1632 for rows of 272 and 256; beyond,
+// every position takes the ring (511 keys: 154 us).  Separate keys and values that way lose (16 heads of 64, 100 keys: 130 instead of 121 us).
 // grid (splits, heads), cluster (splits), LY_ATT_THREADS threads; dynamic shared memory step_att_smem_floats(...) floats.
 // ---------------------------------------------------------------------------------------------------------------------
 #define LY_STEP_STAGES 4

@@ -1302,10 +1302,11 @@ template <typename F> int xp_by_head_size(int hs, F &&f) { // f(integral_constan
 struct XpKernel { int code, tok, rows; float chain, share, fixed; }; // code: B200_XP_TILE
 const XpKernel XP_KERNELS[] = {{64, 64, XP_ROWS, 158.f, 103.f, 0.f}, {32, 32, XP_ROWS, 115.f, 58.f, 0.f}, {16, 16, XP_ROWS, 91.f, 40.f, 0.f}, {8, 8, XP_ROWS, 91.f, 34.f, 0.f},
                                {12896, XT_TOK, 96, 0.f, 284.f, 6000.f}, {128128, XT_TOK, 128, 0.f, 340.f, 6000.f}};
-// From so many hidden units per SM on, over all tokens, SwiGLU is a launch behind the gate/up product: in double precision in the product's epilogue it holds up the CTAs that multiply
-// (8B layer, 512 tokens 384 -> 333 us, then on tcgen05), but a launch and a pass over the rows cost a small product more.  Two or three layers and a step, behind the product against in the
-// epilogue: at 900 - 2700 units per SM (256 wide models, 64 - 512 tokens) 0.4 - 8 us more (2 %), 2700 - 7200 (1536 to 4096 wide, 64 - 250 tokens) between 0.5 % less and 1.6 % more, 7700 and
-// above 0.3 % more to 2.9 % less (8B, 99 tokens 832 and 851 us; 1B, 128 tokens, 7100 units: 427 and 420; 512 tokens, 28300: 909 and 930).
+// From so many hidden units per SM on, over all tokens, SwiGLU is a launch behind the gate/up product: in double precision in the product's epilogue it holds up the
+// CTAs that multiply (8B layer, 512 tokens 384 -> 333 us, then on tcgen05), but a launch and a pass over the rows cost a small product more.  Two or three layers
+// and a step, behind the product against in the epilogue: at 900 - 2700 units per SM (256 wide models, 64 - 512 tokens) 0.4 - 8 us more (2 %), 2700 - 7200 (1536 to
+// 4096 wide, 64 - 250 tokens) between 0.5 % less and 1.6 % more, 7700 and above 0.3 % more to 2.9 % less (8B, 99 tokens 832 and 851 us; 1B, 128 tokens, 7100 units:
+// 427 and 420; 512 tokens, 28300: 909 and 930).
 const int XP_SPLIT_UNITS = 7500;
 // ... of so many tokens at a time: its gate and up rows are 32-bit floats in a buffer that the plan keeps (8B layer: 0.9 GB; 15 GB for a chunk of 131072 tokens at once).
 const int XP_SLICE = 8192;
@@ -1314,8 +1315,9 @@ const int XP_N_KERNELS = sizeof(XP_KERNELS) / sizeof(XP_KERNELS[0]), XP_UMMA = 4
 const size_t XP_SMEM_MAX = 220 * 1024;
 const size_t XP_SCRATCH_MAX = (size_t)256 << 20;
 
-// The kernels' shared memory limits, the device's, ONCE per plan and never in front of a launch: a limit belongs to the function on a device, not to the launch or the plan, and rings are as deep as
-// the call leaves room for.  Set to a launch's own need, one thread's could be lowered by another's between its setting and its launch, which the driver then refused.
+// The kernels' shared memory limits, the device's, ONCE per plan and never in front of a launch: a limit belongs to the function on a device, not to the launch or
+// the plan, and rings are as deep as the call leaves room for.  Set to a launch's own need, one thread's could be lowered by another's between its setting and its
+// launch, which the driver then refused.
 template <typename... K> int set_max_dyn_all(b200_plan *p, int maxdyn, K... kerns) {
     cudaError_t e = cudaSuccess;
     ((e = e == cudaSuccess ? set_max_dyn(kerns, maxdyn) : e), ...);
@@ -1325,9 +1327,10 @@ template <typename... K> int set_max_dyn_all(b200_plan *p, int maxdyn, K... kern
 int xp_smem_attrs(b200_plan *p, int device) { // the products'
     int maxdyn = 0;
     CK(cudaDeviceGetAttribute(&maxdyn, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    return set_max_dyn_all(p, maxdyn, k_xp_gemm<XP_STORE, 8>, k_xp_gemm<XP_STORE, 4>, k_xp_gemm<XP_STORE, 2>, k_xp_gemm<XP_STORE, 1>, k_xp_gemm<XP_RESID, 8>, k_xp_gemm<XP_RESID, 4>, k_xp_gemm<XP_RESID, 2>,
-                           k_xp_gemm<XP_RESID, 1>, k_xp_gemm<XP_GATEUP, 8>, k_xp_gemm<XP_GATEUP, 4>, k_xp_gemm<XP_GATEUP, 2>, k_xp_gemm<XP_GATEUP, 1>, k_xt_gemm<XP_STORE, 96>, k_xt_gemm<XP_STORE, 128>,
-                           k_xt_gemm<XP_RESID, 96>, k_xt_gemm<XP_RESID, 128>);
+    return set_max_dyn_all(p, maxdyn, k_xp_gemm<XP_STORE, 8>, k_xp_gemm<XP_STORE, 4>, k_xp_gemm<XP_STORE, 2>, k_xp_gemm<XP_STORE, 1>,
+                           k_xp_gemm<XP_RESID, 8>, k_xp_gemm<XP_RESID, 4>, k_xp_gemm<XP_RESID, 2>, k_xp_gemm<XP_RESID, 1>,
+                           k_xp_gemm<XP_GATEUP, 8>, k_xp_gemm<XP_GATEUP, 4>, k_xp_gemm<XP_GATEUP, 2>, k_xp_gemm<XP_GATEUP, 1>,
+                           k_xt_gemm<XP_STORE, 96>, k_xt_gemm<XP_STORE, 128>, k_xt_gemm<XP_RESID, 96>, k_xt_gemm<XP_RESID, 128>);
 }
 int xp_smem_attrs(b200_plan *p) {
     int maxdyn = 0;
@@ -2373,7 +2376,8 @@ static int run_exact_prefill_wait(int form, uint32_t *codes, float *ms) {
         CK(cudaGetDevice(&dev));
         if (int rc = xp_smem_attrs(p, dev)) return rc;
         XpMaps mw, whole, half;
-        if (xp_map_weights(&mw, W, umma ? XT_BOX : XP_ROWS) || xp_map_acts(&whole, q, umma, s, tok_pad, cols, tok) || xp_map_acts(&half, q, umma, s, tok_pad, cols, tok / 2)) return B200_ERR_UNSUPPORTED;
+        if (xp_map_weights(&mw, W, umma ? XT_BOX : XP_ROWS) || xp_map_acts(&whole, q, umma, s, tok_pad, cols, tok) || xp_map_acts(&half, q, umma, s, tok_pad, cols, tok / 2))
+            return B200_ERR_UNSUPPORTED;
         const XpMaps starved = form == 3 ? XpMaps{half.q, whole.s} : form == 4 ? XpMaps{whole.q, half.s} : half;
         auto launch = [&](const XpMaps &acts) -> int {
             if (umma) {

@@ -1,7 +1,8 @@
-"""CPU model of the operand ring of the exact Q8_0 prefill's product (csrc/exact_prefill.cuh, k_xp_gemm) as a warp of its own fills it, with the kernel's stage and phase
-expressions, for rings of 3 to 8 stages under random interleavings, where waits may give up at any time: no copy lands in a stage that a warp has still to read, every warp ends, a product
-without a wait that gave up has read every chunk, and no copy is on its way where the gate/up form takes the ring for its hidden units or the block ends.  Found out where planted: a fetching
-warp that does not wait for a stage to come free, and one that waits for its last copies only if a wait of its own gave up, or not at all."""
+"""CPU model of the operand ring of the exact Q8_0 prefill's product (csrc/exact_prefill.cuh, k_xp_gemm) as a warp of its own fills it, with the kernel's stage and
+phase expressions, for rings of 3 to 8 stages under random interleavings, where waits may give up at any time: no copy lands in a stage that a warp has still to
+read, every warp ends, a product without a wait that gave up has read every chunk, and no copy is on its way where the gate/up form takes the ring for its hidden
+units or the block ends.  Found out where planted: a fetching warp that does not wait for a stage to come free, and one that waits for its last copies only if a wait
+of its own gave up, or not at all."""
 import random
 
 import pytest

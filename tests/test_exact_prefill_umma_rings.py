@@ -1,8 +1,9 @@
-"""CPU model of the rings of the exact Q8_0 prefill's tcgen05 product (csrc/exact_prefill_umma.cuh, k_xt_gemm) with the kernel's stage and phase expressions: weights as bytes with both scales,
-activations, weights as FP16, the scales' operands and the sums' columns, under random interleavings of the fetching lane, the operand warps, the product warp, the summing warps, the copies and the
-products, where waits may give up at any time.  Nothing is overwritten that has still to be read, everything that is read is the chunk's, half's or block's own, every role ends, a run without a wait that
-gave up has summed every block, and no copy or product is in flight when the block ends, nor is one waited for that was never issued.  Found out where planted: a fetching lane or a product warp
-that looks back only if a wait of its own gave up, a look back over more activation stages than there are, and waits that are left out."""
+"""CPU model of the rings of the exact Q8_0 prefill's tcgen05 product (csrc/exact_prefill_umma.cuh, k_xt_gemm) with the kernel's stage and phase expressions: weights
+as bytes with both scales, activations, weights as FP16, the scales' operands and the sums' columns, under random interleavings of the fetching lane, the operand
+warps, the product warp, the summing warps, the copies and the products, where waits may give up at any time.  Nothing is overwritten that has still to be read,
+everything that is read is the chunk's, half's or block's own, every role ends, a run without a wait that gave up has summed every block, and no copy or product is
+in flight when the block ends, nor is one waited for that was never issued.  Found out where planted: a fetching lane or a product warp that looks back only if a
+wait of its own gave up, a look back over more activation stages than there are, and waits that are left out."""
 import random
 
 import pytest

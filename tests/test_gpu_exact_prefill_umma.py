@@ -46,7 +46,8 @@ def test_scales(pkg, monkeypatch, rows):
 
 @pytest.mark.parametrize("rows", [96, 128])
 def test_large_scales(pkg, monkeypatch, rows):
-    """Scales up to the largest FP16 numbers in queries, keys, gates and the attention's output, against values and up rows of the smallest, so that the hidden rows' scales and the logits stay finite."""
+    """Scales up to the largest FP16 numbers in queries, keys, gates and the attention's output, against values and up rows of the smallest, so that the hidden rows'
+    scales and the logits stay finite."""
     exponents = {"attn_q": (6, 16), "attn_k": (6, 16), "attn_v": (-24, -14), "attn_output": (6, 16), "ffn_gate": (6, 16), "ffn_up": (-24, -14), "ffn_down": (-12, -4)}
     monkeypatch.setenv("B200_XP_TILE", CODES[rows])
 

@@ -1,5 +1,5 @@
-"""The bounded waits of the exact prefill's products (csrc/exact_prefill.cuh, xp_wait; csrc/exact_prefill_umma.cuh): a tile whose operands arrive in part only (its stages never fill) ends with the error word set,
-every warp of it, and the context goes on as before."""
+"""The bounded waits of the exact prefill's products (csrc/exact_prefill.cuh, xp_wait; csrc/exact_prefill_umma.cuh): a tile whose operands arrive in part only (its
+stages never fill) ends with the error word set, every warp of it, and the context goes on as before."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -19,8 +19,8 @@ def test_operands_that_do_not_arrive(pkg, make_model):
 
 @pytest.mark.parametrize("form", [1, 2, 3, 4])
 def test_other_tiles(pkg, form):
-    """1, 2 and 4: the fetching warp has issued every chunk when the others give up, and waits for their copies, as long as a copy takes and no longer than a wait's limit; 3: on tcgen05, every
-    role waits."""
+    """1, 2 and 4: the fetching warp has issued every chunk when the others give up, and waits for their copies, as long as a copy takes and no longer than a wait's
+    limit; 3: on tcgen05, every role waits."""
     before, starved, after = pkg.native.test_exact_prefill_wait(form)
     assert before[0] == 0 and before[1] < 900
     assert starved[0] == 200 and 1000 <= starved[1] < 1100
