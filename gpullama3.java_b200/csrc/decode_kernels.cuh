@@ -685,10 +685,6 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
             asm volatile("prefetch.global.L2 [%0];" ::"l"(kc + off));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(vc + off));
         }
-        constexpr int VLINES = LINES - ATT_THREADS / 4 / 32; // (heads of 256: the registers hold the first 128 entries of those rows' values, so the others are asked for here)
-        if constexpr (VLINES > 0)
-            for (int i = tid; i < min(pos, ATT_THREADS / 4) * VLINES; i += ATT_THREADS)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(vc + (size_t)(i / VLINES) * kvd + kvh * HS + ATT_THREADS / 4 + (i % VLINES) * 32));
     }
     constexpr int QE = HS / 4, QV = HS / 16, VB = 32;
     const int quad = tid & 3, qbase = lane & ~3, vd = tid >> 2;
@@ -707,6 +703,8 @@ __global__ void __launch_bounds__(ATT_THREADS) k_attention(float *__restrict__ q
     };
     if (!split) {
         load_k(tid >> 2);
+        if constexpr (HS > ATT_THREADS / 4) // (the registers hold the first 128 value entries: the others of these rows, four lines each, are asked for here)
+            if ((tid >> 2) < pos) asm volatile("prefetch.global.L2 [%0];" ::"l"(vc + (size_t)(tid >> 2) * kvd + kvh * HS + ATT_THREADS / 4 + quad * 32));
         load_v(vd, vlive, quad * VB);
     }
     pdl_wait();
