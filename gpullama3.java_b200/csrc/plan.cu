@@ -146,6 +146,7 @@ struct b200_plan {
         struct Slice { XpMaps m[4], h; };
         std::vector<Slice> slices;    // AQ and AH with rows of dim, from the second slice on
         int64_t chunks = 0;           // multiplied at once so far
+        unsigned smem_set = 0;        // kernels whose shared memory limit this plan has set (xp_smem_limit)
         int tile = -1;                // kernel of every product, as an index into XP_KERNELS (B200_XP_TILE; -1: by the model)
         std::string why;              // rows == 0: why not
     } xp;
@@ -1315,36 +1316,15 @@ const int XP_N_KERNELS = sizeof(XP_KERNELS) / sizeof(XP_KERNELS[0]), XP_UMMA = 4
 const size_t XP_SMEM_MAX = 220 * 1024;
 const size_t XP_SCRATCH_MAX = (size_t)256 << 20;
 
-// The kernels' shared memory limits, the device's, ONCE per plan and never in front of a launch: a limit belongs to the function on a device, not to the launch or
-// the plan, and rings are as deep as the call leaves room for.  Set to a launch's own need, one thread's could be lowered by another's between its setting and its
-// launch, which the driver then refused.
-template <typename... K> int set_max_dyn_all(b200_plan *p, int maxdyn, K... kerns) {
-    cudaError_t e = cudaSuccess;
-    ((e = e == cudaSuccess ? set_max_dyn(kerns, maxdyn) : e), ...);
-    CK(e);
+// A kernel's shared memory limit: the same for every launch of an instance, set in front of a plan's first (one that is not launched is not loaded).  It belongs to the
+// function on a device, not to the launch or the plan, and rings are as deep as the call leaves room for: set to a launch's own need, one thread's could be lowered by
+// another's between its setting and its launch, which the driver then refused.
+enum { XP_ID_ATTENTION = 3 * XP_N_KERNELS, XP_ID_ROPE = XP_ID_ATTENTION + 3 }; // bits of xp.smem_set; a product's: MODE * XP_N_KERNELS + kernel
+template <typename K> int xp_smem_limit(b200_plan *p, int id, K kern, size_t limit) {
+    if (p->xp.smem_set >> id & 1u) return B200_OK;
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+    p->xp.smem_set |= 1u << id;
     return B200_OK;
-}
-int xp_smem_attrs(b200_plan *p, int device) { // the products'
-    int maxdyn = 0;
-    CK(cudaDeviceGetAttribute(&maxdyn, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    return set_max_dyn_all(p, maxdyn, k_xp_gemm<XP_STORE, 8>, k_xp_gemm<XP_STORE, 4>, k_xp_gemm<XP_STORE, 2>, k_xp_gemm<XP_STORE, 1>,
-                           k_xp_gemm<XP_RESID, 8>, k_xp_gemm<XP_RESID, 4>, k_xp_gemm<XP_RESID, 2>, k_xp_gemm<XP_RESID, 1>,
-                           k_xp_gemm<XP_GATEUP, 8>, k_xp_gemm<XP_GATEUP, 4>, k_xp_gemm<XP_GATEUP, 2>, k_xp_gemm<XP_GATEUP, 1>,
-                           k_xt_gemm<XP_STORE, 96>, k_xt_gemm<XP_STORE, 128>, k_xt_gemm<XP_RESID, 96>, k_xt_gemm<XP_RESID, 128>);
-}
-int xp_smem_attrs(b200_plan *p) {
-    int maxdyn = 0;
-    CK(cudaDeviceGetAttribute(&maxdyn, cudaDevAttrMaxSharedMemoryPerBlockOptin, p->device));
-    int rc = xp_smem_attrs(p, p->device);
-    if (!rc) rc = set_max_dyn_all(p, maxdyn, k_xp_rope_kv);
-    if (!rc)
-        rc = xp_by_head_size(p->cfg.head_size, [&](auto hs_c) -> int {
-            constexpr int HS = decltype(hs_c)::value;
-            int rc = set_max_dyn_all(p, maxdyn, k_xp_attention<HS, 4, 512>, k_xp_attention<HS, 1, 256>);
-            if constexpr (HS >= 128) return rc ? rc : set_max_dyn_all(p, maxdyn, k_xp_attention<HS, 2, 512>);
-            else return rc ? rc : set_max_dyn_all(p, maxdyn, k_xp_attention<HS, 4, 256>);
-        });
-    return rc;
 }
 
 int exact_prefill_alloc(b200_plan *p, int rows, int nqkv, int wide);
@@ -1357,7 +1337,6 @@ size_t xp_rope_smem_bytes(const b200_config &g) { return (size_t)(g.n_heads + g.
 int exact_prefill_init(b200_plan *p) {
     const b200_config &g = p->cfg;
     if (p->wtype != B200_GGML_Q8_0 || !p->use_stream || g.tp_size > 1) { p->xp.why = "the plan's weights are not Q8_0 on the streaming path"; return B200_OK; }
-    if (int rc = xp_smem_attrs(p)) return rc;
     if (xp_rope_smem_bytes(g) > XP_SMEM_MAX) { p->xp.why = "a token's query and key heads are wider than shared memory"; return B200_OK; }
     const int chunk = p->prefill_batch < g.context_length ? p->prefill_batch : g.context_length;
     const int rows = (chunk + 63) / 64 * 64, nqkv = p->qd + 2 * p->kvd, wide = p->qd > g.dim ? p->qd : g.dim;
@@ -1489,6 +1468,7 @@ int xp_gemm(b200_plan *p, int kernel, const TileMat &W, const XpMaps &mw, const 
         // layer, 36 tokens: 33.7 us with three stages, 27.6 with five)
         const int per_sm = std::min(((int)(grid.x * grid.y) + p->n_sms - 1) / p->n_sms, T::RESIDENT);
         const int stages = std::max(XP_STAGES, std::min(XP_STAGES_MAX, ((int)XP_SMEM_MAX / per_sm - 2048) / (T::STAGE + 16)));
+        if (int rc = xp_smem_limit(p, MODE * XP_N_KERNELS + kernel, kern, XP_SMEM_MAX)) return rc;
         kern<<<grid, XP_THREADS + 32, T::bytes(stages), p->stream>>>(mw, ma[NJ == 8 ? 3 : NJ == 4 ? 2 : NJ - 1], W, p->xp.rows, n, out, ldo, hq, hh, hs, xp_last(p), 1.0f, stages, p->d_err);
         CK(cudaGetLastError());
         return B200_OK;
@@ -1498,6 +1478,7 @@ int xp_gemm(b200_plan *p, int kernel, const TileMat &W, const XpMaps &mw, const 
         else {
             constexpr int N = decltype(rows)::value;
             auto kern = k_xt_gemm<MODE, N>;
+            if (int rc = xp_smem_limit(p, MODE * XP_N_KERNELS + kernel, kern, XtSmem<N>::BYTES)) return rc;
             const int tiles = (n + XT_TOK - 1) / XT_TOK * ((W.rows + N - 1) / N);
             kern<<<std::min(tiles, p->n_sms), XT_THREADS, XtSmem<N>::BYTES, p->stream>>>(mw_umma, ma_umma, W, n, out, ldo, 1.0f, p->d_err);
             CK(cudaGetLastError());
@@ -1521,6 +1502,7 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
     const int nqkv = p->qd + 2 * p->kvd;
     const size_t ctx_kv = (size_t)g.context_length * p->kvd;
     const size_t rope_smem = xp_rope_smem_bytes(g);
+    if (int rc = xp_smem_limit(p, XP_ID_ROPE, k_xp_rope_kv, XP_SMEM_MAX)) return rc;
     // the layers are alike; a product's kernel says what it reads: FP16 quants, or bytes
     const LayerW &first = p->layers[0];
     const int k_qkv = xp_kernel(p, first.tqkv, n), k_wo = xp_kernel(p, first.two, n), k_gu = xp_kernel(p, first.tgu, n), k_w2 = xp_kernel(p, first.tw2, n);
@@ -1547,6 +1529,7 @@ int exact_prefill(b200_plan *p, int n, int start_pos) {
                     const size_t slots = c.scratch_bytes / ((size_t)qt * xp_score_stride(nt) * 4);
                     if ((size_t)ctas > slots) ctas = (int)slots;
                 }
+                if (int rc = xp_smem_limit(p, XP_ID_ATTENTION + (qt == 64 ? 0 : qt == 8 ? 1 : 2), kern, XP_SMEM_MAX)) return rc;
                 kern<<<ctas, threads, smem, p->stream>>>(c.QKV, kc, vc, g.n_heads, g.n_kv_heads, n, start_pos, (float)sqrt((double)HS), c.AQ, ah, c.AS, c.rows, scratch ? c.scratch : nullptr, xp_last(p));
                 CK(cudaGetLastError());
                 return B200_OK;
@@ -2372,21 +2355,20 @@ static int run_exact_prefill_wait(int form, uint32_t *codes, float *ms) {
         const unsigned char *q = mem + w_bytes;
         const float *s = reinterpret_cast<const float *>(mem + w_bytes + q_bytes);
         unsigned char *o = mem + w_bytes + q_bytes + s_bytes;
-        int dev = 0;
-        CK(cudaGetDevice(&dev));
-        if (int rc = xp_smem_attrs(p, dev)) return rc;
         XpMaps mw, whole, half;
         if (xp_map_weights(&mw, W, umma ? XT_BOX : XP_ROWS) || xp_map_acts(&whole, q, umma, s, tok_pad, cols, tok) || xp_map_acts(&half, q, umma, s, tok_pad, cols, tok / 2))
             return B200_ERR_UNSUPPORTED;
         const XpMaps starved = form == 3 ? XpMaps{half.q, whole.s} : form == 4 ? XpMaps{whole.q, half.s} : half;
         auto launch = [&](const XpMaps &acts) -> int {
             if (umma) {
+                CK(cudaFuncSetAttribute(k_xt_gemm<XP_STORE, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, XtSmem<128>::BYTES)); // (as xp_smem_limit)
                 k_xt_gemm<XP_STORE, 128><<<1, XT_THREADS, XtSmem<128>::BYTES>>>(mw, acts, W, tok, reinterpret_cast<float *>(o), rows, 1.0f, d_err);
             } else {
                 const int stages = form == 0 ? XP_STAGES : XP_STAGES_MAX;
                 // (hidden units: 32 of 16 tokens as bytes, their scales, and the last token's units, bytes and scale)
                 const XpLast last{nullptr, reinterpret_cast<int8_t *>(o + 2304), nullptr, reinterpret_cast<float *>(o + 2560), reinterpret_cast<float *>(o + 2048)};
                 auto kern = form == 2 ? k_xp_gemm<XP_GATEUP, 2> : k_xp_gemm<XP_STORE, 2>;
+                CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XP_SMEM_MAX));
                 kern<<<dim3(1, 1), XP_THREADS + 32, XpTile<2>::bytes(stages)>>>(mw, acts, W, tok_pad, tok, reinterpret_cast<float *>(o), rows, reinterpret_cast<int8_t *>(o), nullptr,
                                                                                 reinterpret_cast<float *>(o + 1024), last, 1.0f, stages, d_err);
             }
